@@ -99,21 +99,22 @@ int reinit_iterations(const Grid* g, const Options* o) {
   return n;
 }
 
-void dev_reinit(DevVolume& v, double*& data, const Grid* g, const Options* o) {
+// one field, or two at once (the second with the WENO5 derivative arrays, free
+// between inner loops, as its scratch)
+void dev_reinit(DevVolume& v, double** data, int nf, const Grid* g, const Options* o) {
   PhaseTimer pt(v, PH_REINIT);
-  const Box& b = v.box;
-  const double dx = g->dx[0], dy = g->dx[1], dz = g->dx[2];
-  const double dt_r = 0.5 * g->dx[0];
-  const int iters = reinit_iterations(g, o);
-  QSS_CK(cudaMemcpyAsync(v.r_phi0, data, v.n * sizeof(double), cudaMemcpyDeviceToDevice, v.stream));
-  launch_distance0(v.stream, b, v.r_phi0, v.r_dist, dx, dy, dz);
-  ImposeArgs none{};
-  for (int it = 0; it < iters; it++) {
-    launch_reinit_step(v.stream, b, data, v.r_phi0, v.r_dist, v.r_next, dt_r, dx, dy, dz);
-    launch_ghost(v.stream, b, v.r_next, nullptr, none, nullptr);
-    std::swap(data, v.r_next);
-  }
+  ReinitArrays f[2] = {{data[0], v.r_phi0, v.r_dist, v.r_next},
+                       {nf > 1 ? data[1] : nullptr, v.dplus[0], v.dplus[1], v.dplus[2]}};
+  launch_reinit(v.stream, v.box, f, nf, reinit_iterations(g, o), 0.5 * g->dx[0], g->dx[0], g->dx[1], g->dx[2]);
   QSS_CK(cudaGetLastError());
+  data[0] = f[0].data;
+  v.r_phi0 = f[0].phi0;
+  v.r_next = f[0].next;
+  if (nf > 1) {
+    data[1] = f[1].data;
+    v.dplus[0] = f[1].phi0;
+    v.dplus[2] = f[1].next;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -305,8 +306,10 @@ double dev_const_curv(DevVolume& v, bool var, Options* o, QSS_DataArrays* p, Gri
     }
     if (o->check_connectivity) {
       dev_trap(v, g, o);
-      dev_reinit(v, v.mask_w, g, o);
-      dev_reinit(v, v.mask_nw, g, o);
+      double* trapped[2] = {v.mask_w, v.mask_nw};
+      dev_reinit(v, trapped, 2, g, o);
+      v.mask_w = trapped[0];
+      v.mask_nw = trapped[1];
       if (var && o->conserve_imbibe) {
         launch_trapvel(v.stream, v.box, v.mask_nw, v.vel_n, v.bcoef, v.vx, v.vy, v.vz, g->dx[0]);
         v.nsrc_slabs = 0;
@@ -315,7 +318,7 @@ double dev_const_curv(DevVolume& v, bool var, Options* o, QSS_DataArrays* p, Gri
       launch_merge(v.stream, v.n, v.phi, v.mask_nw);
     }
     if (fp_out) fprintf(fp_out, "Reinitializing....");
-    dev_reinit(v, v.phi, g, o);
+    dev_reinit(v, &v.phi, 1, g, o);
     if (fp_out) fprintf(fp_out, "Reinitialized\n");
     v.dirty[H_PHI] = true;
     max_abs_err = dev_maxnorm(v, o);
@@ -365,7 +368,7 @@ void upload_for_const_curv(DevVolume& v, QSS_DataArrays* p, const Options* o, bo
 }  // namespace
 
 // shared with qss_fortran_abi.cu / qss_paths.cu
-void path_reinit(DevVolume& v, double*& data, const Grid* g, const Options* o) { dev_reinit(v, data, g, o); }
+void path_reinit(DevVolume& v, double*& data, const Grid* g, const Options* o) { dev_reinit(v, &data, 1, g, o); }
 void path_trap(DevVolume& v, const Grid* g, const Options* o) { dev_trap(v, g, o); }
 double path_const_curv(DevVolume& v, bool var, Options* o, QSS_DataArrays* p, Grid* g, FILE* fp, double a) {
   return dev_const_curv(v, var, o, p, g, fp, a);

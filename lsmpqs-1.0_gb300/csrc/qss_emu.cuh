@@ -1,22 +1,22 @@
 // qss_emu.cuh -- IEEE-754 binary64 arithmetic (round to nearest even) on the
 // integer pipes.
 //
-// On GB300 the FP64 pipe issues one warp instruction per ~64 cycles per
-// scheduler, while the integer pipes accept one every one or two cycles, and
-// the WENO5 kernels of this library keep the FP64 pipe 80-85 % busy with the
-// integer pipes nearly idle.  The functions below compute the correctly
+// On GB300 the FP64 pipe takes one warp instruction per 77 cycles and
+// scheduler (measured for DADD, DMUL and DFMA alike), a 32-bit ALU
+// instruction 2 cycles of the ALU pipe and an integer product 2 cycles of
+// the FMA pipe, all three side by side; and the WENO5 kernels of this library
+// are bound by the FP64 pipe.  The functions below compute the correctly
 // rounded IEEE results of x/y, sqrt(x), x*y, x+y, exact power-of-two
 // scalings and comparisons from the operands' bit patterns with 32/64-bit integer
 // instructions, so that part of the FP64 work moves to otherwise idle
-// pipes.  Each function has a fast path for normal operands whose result is
-// normal (plus signed zeros where cheap) and falls back to the native FP64
+// pipes.  Each function has a fast path for operands in a middle range of
+// exponents (plus signed zeros where cheap) and falls back to the native FP64
 // instruction for everything else (subnormals, infinities, NaNs, overflow,
 // underflow), so every result is bit-identical to the native operation on
-// all inputs.  The division reciprocal is seeded by the single-precision
-// reciprocal approximation and refined by two Newton steps in fixed point;
-// the quotient is then verified and corrected with its exact 128-bit integer
-// remainder, so the reciprocal's accuracy affects only speed, never the
-// result (a quotient still off after one correction falls back to native).
+// all inputs.  Divisions and square roots start from the single-precision
+// approximations (rcp / rsqrt.approx, whose error bounds the PTX manual
+// states) and proceed by two digits with exact remainders, as in long
+// division; the bounds that make the last digit right are stated with each.
 //
 // The header compiles for the host too (g++), where the same code is tested
 // against the host's IEEE double arithmetic.
@@ -43,6 +43,24 @@
 
 namespace qss_emu {
 
+// The native instruction of a fallback.  Volatile, so that the compiler does
+// not issue it ahead of the test that rarely selects it: one FP64
+// instruction costs as much as a whole integer-pipe product.
+#ifdef __CUDA_ARCH__
+#define QSS_EMU_NATIVE(name, ptx)                                                       \
+  __device__ __forceinline__ double name(double x, double y) {                          \
+    double r;                                                                           \
+    asm volatile(ptx " %0, %1, %2;" : "=d"(r) : "d"(x), "d"(y));                        \
+    return r;                                                                           \
+  }
+QSS_EMU_NATIVE(native_mul, "mul.rn.f64")
+QSS_EMU_NATIVE(native_add, "add.rn.f64")
+#undef QSS_EMU_NATIVE
+#else
+QSS_EMU_HD double native_mul(double x, double y) { return x * y; }
+QSS_EMU_HD double native_add(double x, double y) { return x + y; }
+#endif
+
 constexpr uint64_t kMant = (1ull << 52) - 1;
 constexpr uint64_t kHidden = 1ull << 52;
 constexpr uint64_t kSign = 1ull << 63;
@@ -68,14 +86,6 @@ QSS_EMU_HD double from_bits(uint64_t u) {
 #endif
 }
 
-QSS_EMU_HD uint64_t umulhi(uint64_t a, uint64_t b) {
-#ifdef __CUDA_ARCH__
-  return __umul64hi(a, b);
-#else
-  return (uint64_t)(((unsigned __int128)a * b) >> 64);
-#endif
-}
-
 QSS_EMU_HD int clz64(uint64_t x) {
 #ifdef __CUDA_ARCH__
   return __clzll((long long)x);
@@ -84,34 +94,102 @@ QSS_EMU_HD int clz64(uint64_t x) {
 #endif
 }
 
-// 53 x 53-bit product of two mantissas as (hi, lo) of a 128-bit value, from
-// four 32 x 32 -> 64-bit products (the high words are below 2^21)
-QSS_EMU_HD void mul53(uint64_t a, uint64_t b, uint64_t& hi, uint64_t& lo) {
-  const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32);
-  const uint32_t b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
-  const uint64_t p00 = (uint64_t)a0 * b0;
-  const uint64_t mid = (uint64_t)a0 * b1 + (uint64_t)a1 * b0;  // < 2^54
-  const uint64_t p11 = (uint64_t)a1 * b1;
-  lo = p00 + (mid << 32);
-  hi = p11 + (mid >> 32) + (lo < p00 ? 1u : 0u);
+// ---------------------------------------------------------------------------
+// 32-bit words.  A 32-bit logic, shift or compare instruction occupies the
+// ALU pipe for 2 cycles of a scheduler, an integer product (32 x 32 -> 64
+// included) the FMA pipe for 2, both at the same time, and one FP64
+// instruction the FP64 pipe for 77 (GB300, measured); so the routines below
+// work on 32-bit words, keep the count of ALU instructions low, and leave
+// the exponent arithmetic packed in the high word.
+
+QSS_EMU_HD uint32_t hi32(double x) { return (uint32_t)(bits(x) >> 32); }
+QSS_EMU_HD uint32_t lo32(double x) { return (uint32_t)bits(x); }
+QSS_EMU_HD uint64_t pack64(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
+
+// low word of (hi:lo) >> s and high word of (hi:lo) << s, 0 <= s <= 31
+QSS_EMU_HD uint32_t fsr(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_r(lo, hi, s);
+#else
+  return (uint32_t)((((uint64_t)hi << 32) | lo) >> s);
+#endif
+}
+QSS_EMU_HD uint32_t fsl(uint32_t lo, uint32_t hi, uint32_t s) {
+#ifdef __CUDA_ARCH__
+  return __funnelshift_l(lo, hi, s);
+#else
+  return (uint32_t)(((((uint64_t)hi << 32) | lo) << s) >> 32);
+#endif
 }
 
-// ---------------------------------------------------------------------------
-// reciprocal of a mantissa m in (2^52, 2^53): V ~ 2^116 / m in (2^63, 2^64)
-//
-// With D = m 2^11 in [2^63, 2^64) and Dh = D >> 32, the top 32 bits of V are
-// S ~ 2^63 / Dh.  The seed S0 comes from the single-precision reciprocal
-// approximation (about 2^-22 relative); one Newton step in 32-bit fixed
-// point gives S1 to about 2^-31; one more step against the full D gives V to
-// about 2^-62.  Only speed depends on these accuracies (see div()).
+// high word of the 53-bit significand
+QSS_EMU_HD uint32_t mant_hi(uint32_t h) { return (h & 0xfffffu) | 0x100000u; }
 
-QSS_EMU_HD uint32_t recip_seed32(uint64_t D) {
-  // single-precision value of the top 24 bits of D / 2^63, in [1, 2)
-  const uint32_t fb = 0x3f800000u | (uint32_t)((D >> 40) & 0x7fffffu);
+// 32 x 32 -> 64-bit product plus a word
+QSS_EMU_HD uint64_t madw(uint32_t a, uint32_t b, uint64_t c) {
+#ifdef __CUDA_ARCH__
+  uint64_t r;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+  return r;
+#else
+  return (uint64_t)a * b + c;
+#endif
+}
+QSS_EMU_HD uint32_t mulhi32(uint32_t a, uint32_t b) { return (uint32_t)(((uint64_t)a * b) >> 32); }
+
+// Round to nearest even: (hi:lo) plus one where the discarded bits are at
+// least half a unit (half holds them left-aligned: its top bit), then the
+// lowest bit cleared where they were exactly half (rest is nonzero where
+// anything lies below half).
+QSS_EMU_HD double round_pack(uint32_t hi, uint32_t lo, uint32_t half, uint32_t rest) {
+#ifdef __CUDA_ARCH__
+  asm("{\n\t.reg .u32 t;\n\t"
+      "add.cc.u32 t, %2, %2;\n\t"
+      "addc.cc.u32 %1, %1, 0;\n\t"
+      "addc.u32 %0, %0, 0;\n\t}"
+      : "+r"(hi), "+r"(lo)
+      : "r"(half));
+  if (((half ^ 0x80000000u) | rest) == 0u) lo &= ~1u;
+  return __hiloint2double((int)hi, (int)lo);
+#else
+  uint64_t r = (((uint64_t)hi << 32) | lo) + (half >> 31);
+  if (((half ^ 0x80000000u) | rest) == 0u) r &= ~1ull;
+  return from_bits(r);
+#endif
+}
+
+// The fast paths take operands with exponents in [-255, 256]: products and
+// quotients of two such are normal.  2 h - 0x60000000 (sign shifted out) is
+// below 2^30 exactly there.
+QSS_EMU_HD uint32_t win(uint32_t h) { return h * 2u - 0x60000000u; }
+QSS_EMU_HD bool in_window(uint32_t xh) { return win(xh) < 0x40000000u; }
+QSS_EMU_HD bool in_window(uint32_t xh, uint32_t yh) { return (win(xh) | win(yh)) < 0x40000000u; }
+
+// ---------------------------------------------------------------------------
+// x / y
+//
+// Significands N and D in [2^52, 2^53), N doubled where N < D (N'), so that
+// N' / D is in [1, 2); d = D / 2^52.  The quotient N' 2^52 / D is built from
+// two digits q1 2^26 + q2 with exact remainders, which need only their low
+// 64 bits because their size is known:
+//   S0   rcp.approx of the top 24 bits of d, 2^24 / d to 2^-22 relative
+//        (truncation of d and 1 ulp of the approximation)
+//   S1   one Newton step in fixed point: 2^30 / d, off by (-0.01, 1.5) units
+//   q1   floor(x - 1/2) for x = (N' >> 22) S1 / 2^34, so that
+//        R1 = N' 2^26 - q1 D has R1 / D in [0.125, 1.625)
+//   q2   floor((R1 + 2^23 >> 24) S1 / 2^32), so that
+//        R2 = R1 2^26 - q2 D has R2 / D in [-0.43, 1.13)
+// and the correctly rounded quotient is q1 2^26 + q2 + (2 R2 > D) (no
+// quotient lies half-way between two 53-bit numbers).  T = D - 2 R2.
+// On the host, where the seed may be perturbed, a seed outside its bound
+// falls back to the native division.
+
+QSS_EMU_HD uint32_t recip_seed(uint32_t mh, uint32_t ml) {
+  const uint32_t fb = fsl(ml, mh, 3) + 0x3f000000u;  // the float in [1, 2) of the top 24 bits
 #ifdef __CUDA_ARCH__
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
-  uint32_t rb = __float_as_uint(r);
+  const uint32_t rb = __float_as_uint(r);
 #else
   float f, r;
   memcpy(&f, &fb, 4);
@@ -120,76 +198,44 @@ QSS_EMU_HD uint32_t recip_seed32(uint64_t D) {
   memcpy(&rb, &r, 4);
   rb = QSS_EMU_SEED_ADJUST(rb);
 #endif
-  // 1/f lies in (0.5, 1]; an approximation outside [0.5, 1) is clamped to the
-  // nearest end, which keeps the seed within 2^-22 of the true value
-  if (rb >= 0x3f800000u) return 0xffffffffu;
-  if (rb < 0x3f000000u) return 0x80000000u;
-  return ((rb & 0x7fffffu) | 0x800000u) << 8;  // r 2^32
+  return rb - 0x3e800000u;  // r 2^24, 2^24 itself for r = 1
 }
 
-QSS_EMU_HD uint64_t recip116(uint64_t m) {
-  const uint64_t D = m << 11;
-  const uint32_t Dh = (uint32_t)(D >> 32);
-  uint32_t S = recip_seed32(D);
-  {
-    // E = 2^63 - Dh S (|E| < 2^43 for a seed within 2^-20), S <- S + S E / 2^63
-    const int64_t E = (int64_t)((1ull << 63) - (uint64_t)Dh * S);
-    const int64_t c = ((int64_t)S * (E >> 12)) >> 51;
-    S = (uint32_t)((int64_t)S + c);
-  }
-  // T = D S (96 bits) as T >> 32; e = (2^95 - T) >> 32 (|e| < 2^34 for S
-  // within 2^-29), V = S 2^32 + S e / 2^31
-  const uint64_t lo = (D & 0xffffffffull) * S, hi = (D >> 32) * S;
-  const uint64_t T32 = hi + (lo >> 32);
-  const int64_t e = (int64_t)((1ull << 63) - T32);
-  const int64_t c = ((int64_t)S * (e >> 3)) >> 28;
-  return ((uint64_t)S << 32) + (uint64_t)c;
+// S1 of the significand (mh:ml)
+QSS_EMU_HD uint32_t recip30(uint32_t mh, uint32_t ml, bool& ok) {
+  const uint32_t S0 = recip_seed(mh, ml);
+  const uint64_t P = (uint64_t)fsl(ml, mh, 11) * S0;  // 2^55 - e
+#ifndef __CUDA_ARCH__
+  ok = P - ((1ull << 55) - (1ull << 34)) < (1ull << 35);
+#endif
+  const int32_t E = (int32_t)fsr((uint32_t)P, (uint32_t)(P >> 32), 8);  // floor(-e / 2^8)
+  const int32_t c = (int32_t)((uint64_t)((int64_t)E * (int32_t)S0) >> 32) >> 9;
+  return S0 * 64u - (uint32_t)c;
 }
 
-// ---------------------------------------------------------------------------
-// x / y
+// quotient of the normal numbers (xh:xl) / (yh:yl) where it is normal
+QSS_EMU_HD double div_win(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl, bool& ok) {
+  const uint32_t mxh = mant_hi(xh), myh = mant_hi(yh);
+  const uint64_t mx = pack64(mxh, xl), my = pack64(myh, yl);
+  const uint32_t s = mx < my ? 1u : 0u;
+  const uint32_t S1 = recip30(myh, yl, ok);
+  const uint32_t nh = fsr(xl, mxh, 22u - s);
+  const uint32_t q1 = (mulhi32(nh, S1) - 2u) >> 2;
+  const uint64_t R1c = pack64(fsl(xl, mxh, 26u + s), xl << (26u + s)) + (1ull << 23) - (uint64_t)q1 * my;  // R1 + 2^23
+  const uint32_t q2 = mulhi32(fsr((uint32_t)R1c, (uint32_t)(R1c >> 32), 24), S1);
+  const uint64_t T = (uint64_t)(2u * q2 + 1u) * my + (1ull << 50) - (R1c << 27);
+  const uint64_t Q = madw(q1, 1u << 26, q2 + (uint32_t)(T >> 63));
+  // (exponent - 1) << 52 plus the 53-bit significand; the signs add up mod 2
+  const uint32_t e = (xh - mxh) - (yh - myh) + ((1022u - s) << 20);
+  return from_bits(pack64((uint32_t)(Q >> 32) + e, (uint32_t)Q));
+}
 
 QSS_EMU_HD double div(double x, double y) {
-  const uint64_t bx = bits(x), by = bits(y);
-  const uint32_t ex = (uint32_t)(bx >> 52) & 0x7ffu, ey = (uint32_t)(by >> 52) & 0x7ffu;
-  if (ex - 1u < 2046u && ey - 1u < 2046u) {
-    const uint64_t sign = (bx ^ by) & kSign;
-    const uint64_t mx = (bx & kMant) | kHidden, my = (by & kMant) | kHidden;
-    const int s = mx < my ? 1 : 0;
-    const uint64_t N = mx << s;                  // N / my in [1, 2)
-    const int e = (int)ex - (int)ey + 1023 - s;  // biased exponent of the quotient
-    if (e >= 1 && e <= 2046) {
-      uint64_t Q = N, R = 0;  // power-of-two divisor: exact
-      bool ok = true;
-      if (my != kHidden) {
-        Q = umulhi(N, recip116(my));  // ~ floor(N 2^52 / my)
-        // exact 128-bit N 2^52 - Q my = (rhi, rlo)
-        uint64_t phi, plo;
-        mul53(Q, my, phi, plo);
-        const uint64_t nlo = N << 52;
-        R = nlo - plo;
-        const uint64_t rhi = (N >> 12) - phi - (nlo < plo ? 1u : 0u);
-        if (rhi == 0) {
-          if (R >= my) {  // Q one too small
-            Q += 1;
-            R -= my;
-            ok = R < my;
-          }
-        } else if (rhi == ~0ull && R + my < my) {  // -my <= R < 0: Q one too large
-          Q -= 1;
-          R += my;
-        } else {
-          ok = false;
-        }
-      }
-      if (ok && Q >= kHidden && Q < (kHidden << 1)) {
-        const uint64_t r2 = R << 1;
-        const uint64_t up = (r2 > my || (r2 == my && (Q & 1))) ? 1u : 0u;
-        // (e - 1) << 52 plus the 53-bit significand: a carry out of the
-        // significand increments the exponent (to infinity at the top)
-        return from_bits(sign | ((((uint64_t)(e - 1)) << 52) + Q + up));
-      }
-    }
+  const uint32_t xh = hi32(x), yh = hi32(y);
+  if (in_window(xh, yh)) {
+    bool ok = true;
+    const double q = div_win(xh, lo32(x), yh, lo32(y), ok);
+    if (ok) return q;
   }
   return QSS_EMU_FALLBACK(0, x / y);
 }
@@ -197,126 +243,137 @@ QSS_EMU_HD double div(double x, double y) {
 // ---------------------------------------------------------------------------
 // sqrt(x)
 //
-// x = M 2^(2k-52) with M = mx or 2 mx (53-54 bits) so that v = M / 2^52 lies
-// in [1, 4); the significand is Q = floor(sqrt(M 2^52)) in [2^52, 2^53),
-// rounded up when the remainder M 2^52 - Q^2 exceeds Q (no ties exist).  Q
-// comes from the single-precision reciprocal square root, one Newton step in
-// 32-bit fixed point and one correction against the full M; the exact
-// 128-bit remainder then verifies and corrects it.
+// x = M 2^(2k-52) with M = mx or 2 mx, so that v = M / 2^52 is in [1, 4); the
+// root's significand sqrt(M 2^52) = S 2^26 comes from two digits:
+//   Y0   rsqrt.approx of the top 24 bits of v, 2^24 / sqrt(v) to 2^-22
+//   Y1   one Newton step: 2^30 / sqrt(v), off by less than a unit
+//   q1   (M >> 22) Y1 / 2^34 rounded, so that d1 = S - q1 is within +-0.88;
+//        R1 = M - q1^2 = d1 (2 S - d1) fits 32 bits
+//   q2   floor((2 R1 + 1) Y1 / 2^32): d1 2^26 less d1^2 / (2 sqrt(v)) <= 0.39
+// so that S 2^26 - (q1 2^26 + q2) is in (-0.5, 1.5) and the rounded root is
+// Q = q1 2^26 + q2, plus one where M 2^52 - Q^2 > Q (no root lies half-way).
+
+// root of the positive normal number (xh:xl)
+QSS_EMU_HD double sqrt_win(uint32_t xh, uint32_t xl, bool& ok) {
+  const uint32_t ex = xh >> 20, odd = ~ex & 1u;
+  const uint32_t mh = mant_hi(xh);
+  const uint64_t M = pack64(mh, xl) << odd;
+  const uint32_t fb = 0x3f800000u + (odd << 23) + fsl(xl, mh & 0xfffffu, 3);
+#ifdef __CUDA_ARCH__
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
+  const uint32_t rb = __float_as_uint(r);
+#else
+  float f, r;
+  memcpy(&f, &fb, 4);
+  r = 1.0f / ::sqrtf(f);
+  uint32_t rb;
+  memcpy(&rb, &r, 4);
+  rb = QSS_EMU_SEED_ADJUST(rb);
+#endif
+  // r = 1 would make Y0^2 >> 16 overflow 32 bits
+  const uint32_t Y0 = rb < 0x3f800000u ? rb - 0x3e800000u : 0xffffffu;
+  const uint32_t Mt = fsr(xl, mh, 22u - odd);  // v 2^30
+  const uint64_t P = (uint64_t)Mt * (uint32_t)(((uint64_t)Y0 * Y0) >> 16);  // 2^62 - e
+#ifndef __CUDA_ARCH__
+  ok = P - ((1ull << 62) - (1ull << 42)) < (1ull << 43);
+#endif
+  const int32_t E = (int32_t)fsr((uint32_t)P, (uint32_t)(P >> 32), 16);  // floor(-e / 2^16)
+  const int32_t c = (int32_t)((uint64_t)((int64_t)E * (int32_t)Y0) >> 32) >> 9;
+  const uint32_t Y1 = Y0 * 64u - (uint32_t)c;
+  const uint32_t q1 = ((uint32_t)(((uint64_t)Mt * Y1) >> 32) + 2u) >> 2;
+  const int32_t R1 = (int32_t)((uint32_t)M - q1 * q1);
+  const int32_t q2 = (int32_t)((uint64_t)((int64_t)(2 * R1 + 1) * (int32_t)Y1) >> 32);
+  const uint64_t Q = ((uint64_t)q1 << 26) + (uint64_t)(int64_t)q2;
+  const uint64_t T = Q + Q * Q - (M << 52);  // Q - (M 2^52 - Q^2)
+  const uint32_t e = (((ex + 1023u - odd) >> 1) - 1u) << 20;
+  return from_bits(Q + (T >> 63) + ((uint64_t)e << 32));
+}
+QSS_EMU_HD double sqrt_win(uint32_t xh, uint32_t xl) {
+  bool ok = true;
+  return sqrt_win(xh, xl, ok);
+}
 
 QSS_EMU_HD double sqrt(double x) {
-  const uint64_t bx = bits(x);
-  const uint32_t ex = (uint32_t)(bx >> 52);  // sign bit included: negative x fails the test
-  if (ex - 1u < 2046u) {
-    const int E = (int)ex - 1023;
-    const int odd = E & 1;
-    const uint64_t M = ((bx & kMant) | kHidden) << odd;  // v = M / 2^52 in [1, 4)
-    const uint32_t fb = ((uint32_t)(127 + odd) << 23) | (uint32_t)((bx >> 29) & 0x7fffffu);
-#ifdef __CUDA_ARCH__
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(fb)));
-    uint32_t rb = __float_as_uint(r);
-#else
-    float f, r;
-    memcpy(&f, &fb, 4);
-    r = 1.0f / ::sqrtf(f);
-    uint32_t rb;
-    memcpy(&rb, &r, 4);
-    rb = QSS_EMU_SEED_ADJUST(rb);
-#endif
-    // 1/sqrt(v) in (0.5, 1] as Y = r 2^32 (clamped to the interval)
-    uint32_t Y;
-    if (rb >= 0x3f800000u) Y = 0xffffffffu;
-    else if (rb < 0x3f000000u) Y = 0x80000000u;
-    else Y = ((rb & 0x7fffffu) | 0x800000u) << 8;
-    const uint32_t Mt = (uint32_t)(M >> 22);  // v 2^30
-    {
-      // Newton step for the reciprocal square root: Y <- Y (3 - v Y^2) / 2
-      const uint64_t G = (uint64_t)Mt * Y;                   // v r 2^62
-      const uint64_t H = umulhi(G, (uint64_t)Y << 32);       // v r^2 2^62
-      const int64_t d = (int64_t)((3ull << 62) - H);          // ~ 2^63 (3 - v r^2)/2 ... scaled below
-      // Y (3 - v r^2) / 2 = Y d / 2^63
-      const uint64_t t = umulhi((uint64_t)Y << 32, (uint64_t)d);  // Y d / 2^32
-      Y = (uint32_t)(t >> 31);
-    }
-    // q0 = v r 2^52 (about 2^-30 relative), then q1 = q0 + (T - q0^2) r / 2
-    uint64_t Q = ((uint64_t)Mt * Y) >> 10;
-    {
-      uint64_t shi, slo;
-      mul53(Q, Q, shi, slo);
-      const uint64_t tlo = M << 52, thi = M >> 12;
-      const uint64_t elo = tlo - slo;
-      const uint64_t ehi = thi - shi - (tlo < slo ? 1u : 0u);
-      // e = (ehi:elo) signed, |e| < 2^80; e >> 16 fits 64 bits
-      const int64_t e16 = (int64_t)((ehi << 48) | (elo >> 16));
-      const bool neg = e16 < 0;
-      const uint64_t ae = neg ? (uint64_t)(-e16) : (uint64_t)e16;
-      // e r / 2 in units of Q: e16 2^16 Y / 2^32 / 2 / 2^52 = e16 Y / 2^69
-      const uint64_t c = umulhi(ae, (uint64_t)Y << 32) >> 37;
-      Q = neg ? Q - c : Q + c;
-    }
-    // exact remainder T - Q^2 and a correction of at most one unit
-    uint64_t shi, slo;
-    mul53(Q, Q, shi, slo);
-    const uint64_t tlo = M << 52, thi = M >> 12;
-    uint64_t R = tlo - slo;
-    const uint64_t rhi = thi - shi - (tlo < slo ? 1u : 0u);
+  const uint32_t xh = hi32(x);
+  if (xh - 0x30000000u < 0x20000000u) {  // positive, exponent in [-255, 256]
     bool ok = true;
-    if (rhi == 0) {
-      if (R > 2 * Q) {  // Q one too small
-        Q += 1;
-        R -= 2 * Q - 1;
-        ok = R <= 2 * Q;
-      }
-    } else if (rhi == ~0ull && R + 2 * Q - 1 < 2 * Q - 1) {  // -(2Q - 1) <= R < 0: Q one too large
-      R += 2 * Q - 1;
-      Q -= 1;
-    } else {
-      ok = false;
-    }
-    if (ok && Q >= kHidden && Q < (kHidden << 1)) {
-      const uint64_t up = R > Q ? 1u : 0u;
-      const uint64_t eb = (uint64_t)((E >> 1) + 1023);
-      return from_bits(((eb - 1) << 52) + Q + up);
-    }
-  } else if ((bx & kAbs) == 0) {
+    const double r = sqrt_win(xh, lo32(x), ok);
+    if (ok) return r;
+  } else if ((bits(x) & kAbs) == 0) {
     return x;  // sqrt(+-0) = +-0
   }
   return QSS_EMU_FALLBACK(3, ::sqrt(x));
 }
 
 // ---------------------------------------------------------------------------
-// x * y
+// x * y: the 106-bit product in four words, the significand taken from it by
+// one funnel shift per word (by 20 or 21 bits), then rounded.
+
+// product of the normal numbers (xh:xl), (yh:yl), times 2^k, where it is normal
+QSS_EMU_HD double mul_win(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl, int k = 0) {
+  const uint32_t mxh = mant_hi(xh), myh = mant_hi(yh);
+  const uint64_t p00 = (uint64_t)xl * yl;
+  const uint64_t t = madw(mxh, yl, madw(xl, myh, p00 >> 32));  // < 2^55
+  const uint64_t p11 = madw(mxh, myh, t >> 32);
+  const uint32_t w0 = (uint32_t)p00, w1 = (uint32_t)t, w2 = (uint32_t)p11, w3 = (uint32_t)(p11 >> 32);
+  const uint32_t top = w3 >> 9;  // product >= 2^105
+  const uint32_t sh = 20u + top;
+  const uint32_t e = (xh - mxh) + (yh - myh) + ((uint32_t)(k - 1022) << 20) + top * 0x100000u;
+  return round_pack(fsr(w2, w3, sh) + e, fsr(w1, w2, sh), fsr(0u, w1, sh), w0);
+}
+
+// square of the normal number (xh:xl), sign ignored, times 2^k, where normal
+QSS_EMU_HD double sq_win(uint32_t xh, uint32_t xl, int k = 0) {
+  const uint32_t mh = mant_hi(xh);
+  const uint64_t p00 = (uint64_t)xl * xl;
+  const uint64_t t = madw(2u * mh, xl, p00 >> 32);
+  const uint64_t p11 = madw(mh, mh, t >> 32);
+  const uint32_t w0 = (uint32_t)p00, w1 = (uint32_t)t, w2 = (uint32_t)p11, w3 = (uint32_t)(p11 >> 32);
+  const uint32_t top = w3 >> 9;
+  const uint32_t sh = 20u + top;
+  const uint32_t e = 2u * (xh - mh) + ((uint32_t)(k - 1022) << 20) + top * 0x100000u;
+  return round_pack(fsr(w2, w3, sh) + e, fsr(w1, w2, sh), fsr(0u, w1, sh), w0);
+}
 
 QSS_EMU_HD double mul(double x, double y) {
+  const uint32_t xh = hi32(x), yh = hi32(y);
+  if (in_window(xh, yh)) return mul_win(xh, lo32(x), yh, lo32(y));
   const uint64_t bx = bits(x), by = bits(y);
-  const uint32_t ex = (uint32_t)(bx >> 52) & 0x7ffu, ey = (uint32_t)(by >> 52) & 0x7ffu;
-  const uint64_t sign = (bx ^ by) & kSign;
-  if (ex - 1u < 2046u && ey - 1u < 2046u) {
-    const uint64_t mx = (bx & kMant) | kHidden, my = (by & kMant) | kHidden;
-    uint64_t hi, lo;
-    mul53(mx, my, hi, lo);  // product in [2^104, 2^106)
-    const int top = (int)(hi >> 41);  // 1 if the product is >= 2^105
-    const int e = (int)ex + (int)ey - 1023 + top;
-    if (e >= 1 && e <= 2046) {
-      uint64_t sig, rem, half;
-      if (top) {
-        sig = (hi << 11) | (lo >> 53);
-        rem = lo & ((1ull << 53) - 1);
-        half = 1ull << 52;
-      } else {
-        sig = (hi << 12) | (lo >> 52);
-        rem = lo & ((1ull << 52) - 1);
-        half = 1ull << 51;
-      }
-      const uint64_t up = (rem > half || (rem == half && (sig & 1))) ? 1u : 0u;
-      return from_bits(sign | ((((uint64_t)(e - 1)) << 52) + sig + up));
-    }
-  } else if ((((bx & kAbs) == 0) && ey - 1u < 2046u) || (((by & kAbs) == 0) && ex - 1u < 2046u) ||
-             (((bx | by) & kAbs) == 0)) {
-    return from_bits(sign);  // zero times a finite nonzero normal, or zero times zero
+  const uint32_t ex = (xh >> 20) & 0x7ffu, ey = (yh >> 20) & 0x7ffu;
+  if ((((bx & kAbs) == 0) && ey != 0x7ffu) || (((by & kAbs) == 0) && ex != 0x7ffu))
+    return from_bits((bx ^ by) & kSign);  // zero times a finite number
+  return QSS_EMU_FALLBACK(1, native_mul(x, y));
+}
+
+// ---------------------------------------------------------------------------
+// x + y of non-negative operands (+0 included; no NaN): no cancellation, so
+// the larger significand grows by at most one bit
+
+// a >= b by their high words, a in the window (or any normal number whose
+// double is finite); b may be +0 or subnormal
+QSS_EMU_HD double add_ordered(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl) {
+  const uint32_t mah = mant_hi(ah), mbh = mant_hi(bh);
+  const uint32_t d = ((ah - mah) - (bh - mbh)) >> 20;
+  if (d < 32u) {  // b is normal here
+    const uint64_t s = pack64(mah, al) + pack64(mbh >> d, fsr(bl, mbh, d));
+    const uint32_t f = fsr(0u, bl, d);  // bits of b below a's unit, left-aligned; bit 0 clear
+    const uint32_t sl = (uint32_t)s, sh = (uint32_t)(s >> 32), top = sh >> 21;
+    return round_pack((sh >> top) + (ah - mah) + top * 0x100000u, fsr(sl, sh, top), fsr(f, sl, top), 0u);
   }
-  return QSS_EMU_FALLBACK(1, x * y);
+  if (d >= 54u) return from_bits(pack64(ah, al));  // b is below half a unit of a
+  return QSS_EMU_FALLBACK(2, native_add(from_bits(pack64(ah, al)), from_bits(pack64(bh, bl))));
+}
+
+// the larger operand known to be in the window
+QSS_EMU_HD double add_pos(double x, double y) {
+  const bool sw = hi32(x) < hi32(y);
+  return add_ordered(sw ? hi32(y) : hi32(x), sw ? lo32(y) : lo32(x), sw ? hi32(x) : hi32(y), sw ? lo32(x) : lo32(y));
+}
+
+QSS_EMU_HD double add_nonneg(double x, double y) {
+  if (in_window(hi32(x) < hi32(y) ? hi32(y) : hi32(x))) return add_pos(x, y);
+  return QSS_EMU_FALLBACK(2, native_add(x, y));
 }
 
 // ---------------------------------------------------------------------------
@@ -369,7 +426,7 @@ QSS_EMU_HD double add(double x, double y) {
   } else if ((ba & kAbs) == 0) {  // both zero
     return from_bits(ba & bb & kSign);
   }
-  return QSS_EMU_FALLBACK(2, x + y);
+  return QSS_EMU_FALLBACK(2, native_add(x, y));
 }
 
 QSS_EMU_HD double neg(double x);
@@ -378,6 +435,7 @@ QSS_EMU_HD double sub(double x, double y) { return add(x, neg(y)); }
 // x * 2^k for a small integer k (exact unless the result leaves the normal range)
 QSS_EMU_HD double scale2(double x, int k) {
   const uint64_t b = bits(x);
+  if (in_window((uint32_t)(b >> 32))) return from_bits(b + ((uint64_t)(int64_t)k << 52));
   const int e = (int)((b >> 52) & 0x7ffu);
   if (e >= 1 && e <= 2046 && e + k >= 1 && e + k <= 2046)
     return from_bits(b + ((uint64_t)(int64_t)k << 52));

@@ -86,6 +86,9 @@ __global__ void k_emu_selftest(long long n, uint64_t seed, unsigned long long* c
     if (!same(qss_emu::div(x, y), __ddiv_rn(x, y))) note(counts, 0, x, y, first_flag, first);
     if (!same(qss_emu::mul(x, y), __dmul_rn(x, y))) note(counts, 1, x, y, first_flag, first);
     if (!same(qss_emu::add(x, y), __dadd_rn(x, y))) note(counts, 2, x, y, first_flag, first);
+    const double ux = fabs(x), uy = fabs(y);
+    if (ux == ux && uy == uy && !same(qss_emu::add_nonneg(ux, uy), __dadd_rn(ux, uy)))
+      note(counts, 2, ux, uy, first_flag, first);
     if (!same(qss_emu::sub(x, y), __dsub_rn(x, y))) note(counts, 3, x, y, first_flag, first);
     const int k = (int)((r >> 16) % 9) - 4;
     const double p2 = qss_emu::from_bits((uint64_t)(1023 + k) << 52);  // 2^k

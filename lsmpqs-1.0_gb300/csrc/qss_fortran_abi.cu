@@ -387,7 +387,7 @@ void qss3dcomputereinitializationeqnrhssubcellfixorder1_(double* reinit_rhs, con
   h2d(dp, phi, bytes);
   h2d(d0, phi0, bytes);
   h2d(dd, distance0, bytes);
-  launch_reinit_rhs(abi_stream(), bx, dp.d(), d0.d(), dd.d(), dr.d(), *dx, *dy, *dz);
+  launch_reinit_rhs(abi_stream(), bx, dp.d(), d0.d(), dd.d(), dr.d(), false, *dx, *dy, *dz);
   d2h(reinit_rhs, dr, bytes);
   finish();
   ABI_END

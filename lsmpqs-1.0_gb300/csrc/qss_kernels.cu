@@ -345,13 +345,19 @@ __global__ void k_distance0(Box b, const double* __restrict__ phi0, double* dist
   const int k = b.klo + blockIdx.z * blockDim.z + threadIdx.z;
   if (i > b.ihi || j > b.jhi || k > b.khi) return;
   const int64_t c = b.idx(i, j, k), sy = b.sy(), sz = b.sz();
-  const double zero_tol = 1.e-5, zero = 0.0;
+  const double zero_tol = 1.e-5;
   const double max_dx = dmax(dmax(dx, dy), dz);
   const double cc = phi0[c];
   const double n[6] = {phi0[c + 1], phi0[c - 1], phi0[c + sy], phi0[c - sy], phi0[c + sz], phi0[c - sz]};
+  // opposite signs, zero counted as negative; the tests on the integer pipes
+  // (a native comparison occupies the FP64 pipe like an addition)
   bool near = false;
+  const bool pos = qss_emu::gt0(cc), nonpos = qss_emu::lt0(cc) || (qss_emu::bits(cc) & qss_emu::kAbs) == 0;
 #pragma unroll
-  for (int q = 0; q < 6; q++) near = near || (n[q] > zero && cc <= zero) || (n[q] <= zero && cc > zero);
+  for (int q = 0; q < 6; q++) {
+    const bool np = qss_emu::gt0(n[q]);
+    near = near || (np && nonpos) || (!np && pos && !qss_emu::isnan_bits(qss_emu::bits(n[q])));
+  }
   if (!near) {
     distance0[c] = -1000.0 * max_dx;
     return;
@@ -510,52 +516,148 @@ __device__ __forceinline__ double reinit_rhs_diffs(double cc, double p0, double 
 }
 
 // Reinitialisation step at level 2 with each face difference computed once:
-// the difference (phi(c + e) - phi(c)) inv is the plus difference of c and
-// the minus difference of c + e, the same operation on the same operands.
-// A block of 4 warps covers 32 (i) x 4 (j) voxels, each warp an 8 x 4 patch
-// (x neighbours one lane apart, y neighbours eight), and walks `walk` planes
-// along k carrying the z difference; lanes on the patch's low edges and the
-// first plane compute their minus difference themselves.  Per voxel about
-// 3.4 differences instead of 6 for a walk of 16 planes.  Short walks keep
-// small boxes' grids large enough to fill the GPU (see reinit_launch).
+// the difference phi(c + e) - phi(c) is the plus difference of c and the
+// minus difference of c + e, the same operation on the same operands.  A block
+// of 4 warps covers 32 (i) x 4 (j) voxels, each warp an 8 x 4 patch (x
+// neighbours one lane apart, y neighbours eight), and walks `walk` planes
+// along k carrying the z difference.  The 12 minus differences across the
+// patch's low edges are one more instruction: the 4 lanes of the low x edge
+// but the corner compute theirs in x, the 8 of the low y edge theirs in y, and
+// lane 9 the corner's in x.  Short walks keep small boxes' grids large enough
+// to fill the GPU (see reinit_walk_launch).
+//
+// Away from the interface the arithmetic is straight-line: the larger
+// one-sided difference is picked before it is scaled (rounding is monotone),
+// picked, cut off at zero and raised to 2^-255 by one integer maximum on its
+// high word, and scaled, squared and rooted on the integer pipes without a
+// test per operation.  The floor of 2^-255 in place of a zero changes no bit:
+// the root it could reach is below 2^-100, and sgn - root, and phi + dt r,
+// round to the same number.  Differences of 2^100 or more (infinities and
+// NaNs among them) take the general path, reinit_rhs_diffs.  FP64
+// instructions per voxel: 3.4 differences, 2 sums, sgn - root, phi + dt r;
+// that is the kernel's bound.
+//
+// GHOST: the layer next to the fill box is not read but extrapolated from the
+// two voxels inside it (extrap with distance 1, as k_ghost would leave it), so
+// the ghost layers need filling only after the last sweep.
 constexpr int kRWalkMax = 16;
+constexpr int kReinitFields = 2;
 
-__global__ void __launch_bounds__(128) k_reinit_walk(Box b, const double* __restrict__ data,
-                                                     const double* __restrict__ phi0,
-                                                     const double* __restrict__ distance0, double* __restrict__ next,
-                                                     double dt_r, Inv inv, double max_dx, int rhs_only,
-                                                     uint64_t far_bits, int walk) {
+struct ReinitSweep {
+  const double* data[kReinitFields];
+  const double* phi0[kReinitFields];
+  const double* dist[kReinitFields];
+  double* next[kReinitFields];
+  double dt_r, max_dx;
+  Inv inv;
+  uint64_t far_bits;
+  int walk, chunks, rhs_only;
+};
+
+// f + sign(f) |f - g|: extrap(f, g, 1).  Out of line: inlined, its additions
+// would be issued under a predicate by every warp, and an FP64 instruction
+// with no active lane still takes its turn on the pipe.
+__device__ __noinline__ double extrap1(double f, double g) {
+  const uint32_t d = qss_emu::hi32(f - g), low = qss_emu::lo32(f - g);
+  return f + __hiloint2double((int)((d & 0x7fffffffu) | (qss_emu::hi32(f) & 0x80000000u)), (int)low);
+}
+
+__device__ __noinline__ double reinit_general(double cc, double p0, double d0, double px, double py, double pz,
+                                              double mx, double my, double mz, Inv inv, double max_dx,
+                                              uint64_t far_bits) {
+  const double gp[3] = {px * inv.x, py * inv.y, pz * inv.z}, gm[3] = {mx * inv.x, my * inv.y, mz * inv.z};
+  return reinit_rhs_diffs(cc, p0, d0, gp, gm, max_dx, far_bits);
+}
+
+template <bool GHOST>
+__global__ void __launch_bounds__(128, 10) k_reinit_walk(Box b, ReinitSweep a) {
+  using namespace qss_emu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int li = lane & 7, lj = lane >> 3;
-  const int i_raw = b.ilo + blockIdx.x * 32 + 8 * warp + li;
-  const int j_raw = b.jlo + blockIdx.y * 4 + lj;
-  const bool ok = i_raw <= b.ihi && j_raw <= b.jhi;
+  const int field = blockIdx.z / a.chunks, chunk = blockIdx.z - field * a.chunks;
+  const double* __restrict__ data = a.data[field];
+  const int i0 = b.ilo + blockIdx.x * 32 + 8 * warp, j0 = b.jlo + blockIdx.y * 4;
+  const bool ok = i0 + li <= b.ihi && j0 + lj <= b.jhi;
   // lanes past the fill box work on its last row/column (in the box), store nothing
-  const int i = i_raw <= b.ihi ? i_raw : b.ihi;
-  const int j = j_raw <= b.jhi ? j_raw : b.jhi;
-  const int k0 = b.klo + blockIdx.z * walk;
-  const int k1 = k0 + walk - 1 < b.khi ? k0 + walk - 1 : b.khi;
+  const int i = i0 + li <= b.ihi ? i0 + li : b.ihi;
+  const int j = j0 + lj <= b.jhi ? j0 + lj : b.jhi;
+  const int k0 = b.klo + chunk * a.walk;
+  const int k1 = k0 + a.walk - 1 < b.khi ? k0 + a.walk - 1 : b.khi;
   const int64_t sy = b.sy(), sz = b.sz();
-  auto scale = [](double d, double f) -> double { return qss_emu::mul(d, f); };
+  const Inv inv = a.inv;
   int64_t c = b.idx(i, j, k0);
+  // the lane's share of the low edges: a neighbour's offset from c, and whether
+  // that neighbour lies in the ghost layer
+  const bool edge_y = lj == 0, edge_x = li == 0 && lj != 0, corner_x = lane == 9;
+  const bool edge = edge_y || edge_x || corner_x;
+  const int64_t ec = corner_x ? b.idx(i0 <= b.ihi ? i0 : b.ihi, j0, k0) - 1 - c : (edge_y ? -sy : -1);
+  const bool edge_ghost = GHOST && ((edge_y && j0 == b.jlo) || ((edge_x || corner_x) && i0 == b.ilo));
+  const bool xlast = GHOST && i == b.ihi, ylast = GHOST && j == b.jhi;
   double cc = __ldg(data + c);
-  double dzm = scale(cc - __ldg(data + c - sz), inv.z);
+  double zm;
+  if (GHOST && k0 == b.klo) zm = extrap1(cc, __ldg(data + c + sz));
+  else zm = __ldg(data + c - sz);
+  double dzm = cc - zm;
   for (int k = k0; k <= k1; k++) {
-    const double zp = __ldg(data + c + sz);
-    double gp[3], gm[3];
-    gp[0] = scale(__ldg(data + c + 1) - cc, inv.x);
-    gp[1] = scale(__ldg(data + c + sy) - cc, inv.y);
-    gp[2] = scale(zp - cc, inv.z);
-    const double xm = __shfl_up_sync(0xffffffffu, gp[0], 1);
-    const double ym = __shfl_up_sync(0xffffffffu, gp[1], 8);
-    gm[0] = li == 0 ? scale(cc - __ldg(data + c - 1), inv.x) : xm;
-    gm[1] = lj == 0 ? scale(cc - __ldg(data + c - sy), inv.y) : ym;
-    gm[2] = dzm;
-    if (ok) {
-      const double r = reinit_rhs_diffs(cc, phi0[c], distance0[c], gp, gm, max_dx, far_bits);
-      next[c] = rhs_only ? r : data[c] + qss_emu::mul(dt_r, r);
+    double xp = __ldg(data + c + (xlast ? -1 : 1)), yp = __ldg(data + c + (ylast ? -sy : sy));
+    double zp = __ldg(data + c + (GHOST && k == b.khi ? -sz : sz));
+    const double cc0 = __shfl_sync(0xffffffffu, cc, 0);
+    const double eb = corner_x ? cc0 : cc;
+    double em = edge ? __ldg(data + c + ec) : eb;
+    if (GHOST) {
+      if (xlast) xp = extrap1(cc, xp);
+      if (ylast) yp = extrap1(cc, yp);
+      if (k == b.khi) zp = extrap1(cc, zp);
+      if (i0 == b.ilo || j0 == b.jlo) {  // warp-uniform
+        const double xp0 = __shfl_sync(0xffffffffu, xp, 0);
+        if (edge_ghost) em = extrap1(eb, corner_x ? xp0 : (edge_y ? yp : xp));
+      }
     }
-    dzm = gp[2];
+    const double dxp = xp - cc, dyp = yp - cc, dzp = zp - cc, de = eb - em;
+    const double xm = __shfl_up_sync(0xffffffffu, dxp, 1);
+    const double ym = __shfl_up_sync(0xffffffffu, dyp, 8);
+    const double dc = __shfl_sync(0xffffffffu, de, 9);
+    const double dxm = li != 0 ? xm : (lj != 0 ? de : dc);
+    const double dym = lj != 0 ? ym : de;
+    if (ok) {
+      const double p0 = __ldg(a.phi0[field] + c), d0 = __ldg(a.dist[field] + c);
+      // max(-d+, d-, 0) where phi > 0, max(d+, -d-, 0) elsewhere, as signed
+      // 64-bit integers (a negative double is a negative integer)
+      const uint64_t sp = gt0(cc) ? kSign : 0, sm = sp ^ kSign;
+      const int64_t ux = (int64_t)(bits(dxp) ^ sp), vx = (int64_t)(bits(dxm) ^ sm);
+      const int64_t uy = (int64_t)(bits(dyp) ^ sp), vy = (int64_t)(bits(dym) ^ sm);
+      const int64_t uz = (int64_t)(bits(dzp) ^ sp), vz = (int64_t)(bits(dzm) ^ sm);
+      const int64_t wx = ux > vx ? ux : vx, wy = uy > vy ? uy : vy, wz = uz > vz ? uz : vz;
+      const int hx = max((int)(wx >> 32), 0x30000000), hy = max((int)(wy >> 32), 0x30000000),
+                hz = max((int)(wz >> 32), 0x30000000);
+      const uint64_t acc = bits(cc) & kAbs, ap0 = bits(p0) & kAbs;
+      constexpr uint64_t inf = 0x7ff0000000000000ull;
+      const uint64_t tol = 0x3ee4f8b588e368f1ull;  // 1e-5
+      double r;
+      if (bits(d0) == a.far_bits && max(max(hx, hy), hz) < 0x46300000 && acc > tol && acc <= inf && ap0 > tol &&
+          ap0 <= inf) {
+        const double gx = mul_win((uint32_t)hx, (uint32_t)wx, hi32(inv.x), lo32(inv.x));
+        const double gy = mul_win((uint32_t)hy, (uint32_t)wy, hi32(inv.y), lo32(inv.y));
+        const double gz = mul_win((uint32_t)hz, (uint32_t)wz, hi32(inv.z), lo32(inv.z));
+        const double n2 = sq_win(hi32(gx), lo32(gx)) + sq_win(hi32(gy), lo32(gy)) + sq_win(hi32(gz), lo32(gz));
+        const double root = sqrt_win(hi32(n2), lo32(n2));
+        const uint32_t neg0 = hi32(p0) & 0x80000000u;  // sgn = +-1
+        const double sgn = __hiloint2double((int)(0x3ff00000u | neg0), 0);
+        r = sgn + __hiloint2double((int)(hi32(root) ^ neg0 ^ 0x80000000u), (int)lo32(root));
+        if (!a.rhs_only) {
+          // dt r with |r| raised to 2^-255 (r = 0: phi + tiny rounds to phi)
+          const uint32_t ar = hi32(r) & 0x7fffffffu;
+          const double dr = mul_win((ar > 0x30000000u ? ar : 0x30000000u) | (hi32(r) & 0x80000000u), lo32(r),
+                                    hi32(a.dt_r), lo32(a.dt_r));
+          r = cc + dr;
+        }
+      } else {
+        r = reinit_general(cc, p0, d0, dxp, dyp, dzp, dxm, dym, dzm, inv, a.max_dx, a.far_bits);
+        if (!a.rhs_only) r = cc + qss_emu::mul(a.dt_r, r);
+      }
+      a.next[field][c] = r;
+    }
+    dzm = dzp;
     cc = zp;
     c += sz;
   }
@@ -1024,38 +1126,93 @@ static bool reinit_walk() {
   return on != 0;
 }
 
-static void reinit_launch(cudaStream_t s, const Box& b, const double* data, const double* phi0,
-                          const double* distance0, double* out, double dt_r, double dx, double dy, double dz,
-                          int rhs_only) {
+// constants whose products with the kernel's operands stay normal
+static bool middling(double x) { return x > 1e-30 && x < 1e30; }
+
+// one sweep of nf <= 2 fields; from_fill: the ghost layers of data are taken to
+// be the extrapolation of its fill box and may be stale.  Returns false, having
+// done nothing, where this form does not apply.
+static bool reinit_walk_launch(cudaStream_t s, const Box& b, const ReinitArrays* f, int nf, bool from_fill, double dt_r,
+                               double dx, double dy, double dz, int rhs_only) {
   const double max_dx = (dx > dy ? dx : dy) > dz ? (dx > dy ? dx : dy) : dz;
-  const Inv inv{1.0 / dx, 1.0 / dy, 1.0 / dz};
-  const uint64_t far_bits = qss_emu::bits(-1000.0 * max_dx);  // distance0 of voxels away from the interface
-  const int lvl = emu_level();
-  const dim3 grid = fb_grid(b, kBlk3);
-  if (lvl >= 2 && reinit_walk()) {
-    // planes per thread: up to kRWalkMax while the grid keeps ~16 blocks per SM
-    const int64_t xy = (int64_t)((b.fbx() + 31) / 32) * ((b.fby() + 3) / 4);
-    int64_t walk = xy * b.fbz() / (152 * 16);
-    walk = walk < 1 ? 1 : (walk > kRWalkMax ? kRWalkMax : walk);
-    const dim3 gw((b.fbx() + 31) / 32, (b.fby() + 3) / 4, (unsigned)((b.fbz() + walk - 1) / walk));
-    k_reinit_walk<<<gw, 128, 0, s>>>(b, data, phi0, distance0, out, dt_r, inv, max_dx, rhs_only, far_bits,
-                                     (int)walk);
-  } else if (lvl >= 2)
-    k_reinit_step<2><<<grid, kBlk3, 0, s>>>(b, data, phi0, distance0, out, dt_r, inv, max_dx, rhs_only, far_bits);
-  else if (lvl == 1)
-    k_reinit_step<1><<<grid, kBlk3, 0, s>>>(b, data, phi0, distance0, out, dt_r, inv, max_dx, rhs_only, far_bits);
-  else
-    k_reinit_step<0><<<grid, kBlk3, 0, s>>>(b, data, phi0, distance0, out, dt_r, inv, max_dx, rhs_only, far_bits);
+  if (emu_level() < 2 || !reinit_walk() || !middling(dx) || !middling(dy) || !middling(dz) ||
+      !(rhs_only || middling(dt_r)))
+    return false;
+  ReinitSweep a{};
+  for (int q = 0; q < nf; q++) {
+    a.data[q] = f[q].data;
+    a.phi0[q] = f[q].phi0;
+    a.dist[q] = f[q].dist;
+    a.next[q] = f[q].next;
+  }
+  a.dt_r = dt_r;
+  a.max_dx = max_dx;
+  a.inv = Inv{1.0 / dx, 1.0 / dy, 1.0 / dz};
+  a.far_bits = qss_emu::bits(-1000.0 * max_dx);  // distance0 of voxels away from the interface
+  a.rhs_only = rhs_only;
+  // planes per thread: up to kRWalkMax while the grid keeps ~16 blocks per SM
+  const int64_t xy = (int64_t)((b.fbx() + 31) / 32) * ((b.fby() + 3) / 4);
+  int64_t walk = xy * nf * b.fbz() / (152 * 16);
+  a.walk = (int)(walk < 1 ? 1 : (walk > kRWalkMax ? kRWalkMax : walk));
+  a.chunks = (b.fbz() + a.walk - 1) / a.walk;
+  const dim3 g((b.fbx() + 31) / 32, (b.fby() + 3) / 4, (unsigned)(a.chunks * nf));
+  if (from_fill) k_reinit_walk<true><<<g, 128, 0, s>>>(b, a);
+  else k_reinit_walk<false><<<g, 128, 0, s>>>(b, a);
+  return true;
 }
 
-void launch_reinit_step(cudaStream_t s, const Box& b, const double* data, const double* phi0,
-                        const double* distance0, double* next, double dt_r, double dx, double dy, double dz) {
-  reinit_launch(s, b, data, phi0, distance0, next, dt_r, dx, dy, dz, 0);
+static void reinit_launch(cudaStream_t s, const Box& b, const ReinitArrays& f, double dt_r, double dx, double dy,
+                          double dz, int rhs_only) {
+  const double max_dx = (dx > dy ? dx : dy) > dz ? (dx > dy ? dx : dy) : dz;
+  const Inv inv{1.0 / dx, 1.0 / dy, 1.0 / dz};
+  const uint64_t far_bits = qss_emu::bits(-1000.0 * max_dx);
+  const int lvl = emu_level();
+  const dim3 grid = fb_grid(b, kBlk3);
+  if (lvl >= 2)
+    k_reinit_step<2><<<grid, kBlk3, 0, s>>>(b, f.data, f.phi0, f.dist, f.next, dt_r, inv, max_dx, rhs_only, far_bits);
+  else if (lvl == 1)
+    k_reinit_step<1><<<grid, kBlk3, 0, s>>>(b, f.data, f.phi0, f.dist, f.next, dt_r, inv, max_dx, rhs_only, far_bits);
+  else
+    k_reinit_step<0><<<grid, kBlk3, 0, s>>>(b, f.data, f.phi0, f.dist, f.next, dt_r, inv, max_dx, rhs_only, far_bits);
+}
+
+void launch_reinit_sweep(cudaStream_t s, const Box& b, const ReinitArrays* f, int nf, bool from_fill, double dt_r,
+                         double dx, double dy, double dz) {
+  if (reinit_walk_launch(s, b, f, nf, from_fill, dt_r, dx, dy, dz, 0)) return;
+  for (int q = 0; q < nf; q++) {
+    // this form reads the ghost layers
+    if (from_fill) launch_ghost(s, b, const_cast<double*>(f[q].data), nullptr, ImposeArgs{}, nullptr);
+    reinit_launch(s, b, f[q], dt_r, dx, dy, dz, 0);
+  }
 }
 
 void launch_reinit_rhs(cudaStream_t s, const Box& b, const double* data, const double* phi0,
-                       const double* distance0, double* rhs, double dx, double dy, double dz) {
-  reinit_launch(s, b, data, phi0, distance0, rhs, 0.0, dx, dy, dz, 1);
+                       const double* distance0, double* rhs, bool from_fill, double dx, double dy, double dz) {
+  const ReinitArrays f{const_cast<double*>(data), const_cast<double*>(phi0), const_cast<double*>(distance0), rhs};
+  if (reinit_walk_launch(s, b, &f, 1, from_fill, 0.0, dx, dy, dz, 1)) return;
+  if (from_fill) launch_ghost(s, b, const_cast<double*>(data), nullptr, ImposeArgs{}, nullptr);
+  reinit_launch(s, b, f, 0.0, dx, dy, dz, 1);
+}
+
+void launch_reinit(cudaStream_t s, const Box& b, ReinitArrays* f, int nf, int iters, double dt_r, double dx, double dy,
+                   double dz) {
+  if (iters <= 0) return;
+  for (int q = 0; q < nf; q++) {
+    // the input stays where it is, as phi0; the sweeps alternate between the
+    // other two arrays
+    std::swap(f[q].data, f[q].phi0);
+    launch_distance0(s, b, f[q].phi0, f[q].dist, dx, dy, dz);
+  }
+  for (int it = 0; it < iters; it++) {
+    ReinitArrays g[kReinitFields];
+    for (int q = 0; q < nf; q++) {
+      g[q] = f[q];
+      if (it == 0) g[q].data = f[q].phi0;
+    }
+    launch_reinit_sweep(s, b, g, nf, it > 0, dt_r, dx, dy, dz);
+    for (int q = 0; q < nf; q++) std::swap(f[q].data, f[q].next);
+  }
+  for (int q = 0; q < nf; q++) launch_ghost(s, b, f[q].data, nullptr, ImposeArgs{}, nullptr);
 }
 
 void launch_central_grad(cudaStream_t s, const Box& b, const double* f, double* fx, double* fy, double* fz,

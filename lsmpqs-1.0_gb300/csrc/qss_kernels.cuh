@@ -132,11 +132,22 @@ void launch_nsrc(cudaStream_t s, const Box& b, const double* vel_n, int* nsrc, i
 // ---- reinitialisation ---------------------------------------------------
 void launch_distance0(cudaStream_t s, const Box& b, const double* phi0, double* distance0, double dx,
                       double dy, double dz);
-void launch_reinit_step(cudaStream_t s, const Box& b, const double* data, const double* phi0,
-                        const double* distance0, double* next, double dt_r, double dx, double dy,
-                        double dz);
+// One field of a reinitialisation: the current iterate, the initial field, its
+// subcell distances, and where the next iterate goes (ghost-box arrays).
+struct ReinitArrays {
+  double *data, *phi0, *dist, *next;
+};
+// `iters` sweeps of nf (1 or 2) fields at once.  In: data holds the field, the
+// other three are scratch.  Out: data the result, ghost layers included, phi0
+// the initial field; the four pointers of a field may be exchanged.
+void launch_reinit(cudaStream_t s, const Box& b, ReinitArrays* f, int nf, int iters, double dt_r, double dx, double dy,
+                   double dz);
+// one sweep, data -> next on the fill box; from_fill: data's ghost layers are the
+// extrapolation of its fill box and need not have been filled
+void launch_reinit_sweep(cudaStream_t s, const Box& b, const ReinitArrays* f, int nf, bool from_fill, double dt_r,
+                         double dx, double dy, double dz);
 void launch_reinit_rhs(cudaStream_t s, const Box& b, const double* data, const double* phi0,
-                       const double* distance0, double* rhs, double dx, double dy, double dz);
+                       const double* distance0, double* rhs, bool from_fill, double dx, double dy, double dz);
 
 // ---- coefficients -------------------------------------------------------
 void launch_central_grad(cudaStream_t s, const Box& b, const double* f, double* fx, double* fy,

@@ -438,11 +438,9 @@ void reinitializeSubcellFix3d(double* data, Grid* g, Options* o) {
   thread_local QSS_DataArrays key;
   DevVolume& v = volume_for(&key, g);
   QSS_CK(cudaMemcpyAsync(v.scratch, data, v.n * sizeof(double), cudaMemcpyHostToDevice, v.stream));
-  double* d = v.scratch;
-  path_reinit(v, d, g, o);
-  QSS_CK(cudaMemcpyAsync(data, d, v.n * sizeof(double), cudaMemcpyDeviceToHost, v.stream));
+  path_reinit(v, v.scratch, g, o);
+  QSS_CK(cudaMemcpyAsync(data, v.scratch, v.n * sizeof(double), cudaMemcpyDeviceToHost, v.stream));
   QSS_CK(cudaStreamSynchronize(v.stream));
-  if (d != v.scratch) std::swap(v.scratch, v.r_next);
   QSS_API_END(return)
 }
 

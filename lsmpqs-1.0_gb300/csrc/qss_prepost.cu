@@ -13,6 +13,7 @@
 // Every function writes exactly the arrays (and ranges) the reference writes,
 // with the reference's operations in the same order.
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "qss_state.h"
@@ -144,15 +145,20 @@ void reinit_mask_dev(cudaStream_t s, const Box& b, const Grid* g, const Options*
   const double dt_r = 0.5 * g->dx[0];  // cfl_number 0.5
   QSS_CK(cudaMemcpyAsync(scratch2, mask, n * sizeof(double), cudaMemcpyDeviceToDevice, s));  // COPY_DATA
   launch_distance0(s, b, scratch2, scratch1, dx, dy, dz);
-  ImposeArgs none{};
-  double t_r = 0;
-  while (t_r < o->tmax_r) {
-    launch_reinit_rhs(s, b, mask, scratch2, scratch1, rhs, dx, dy, dz);
-    launch_rk(s, b, 1, next, mask, nullptr, rhs, dt_r);
-    launch_ghost(s, b, next, nullptr, none, nullptr);  // signedLinearExtrapolationBCqss(., 9)
-    QSS_CK(cudaMemcpyAsync(mask, next, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    t_r = t_r + dt_r;
+  int iters = 0;
+  for (double t_r = 0; t_r < o->tmax_r; t_r = t_r + dt_r) iters++;
+  if (iters == 0) return;
+  // the reference keeps the RHS of the last iteration only: all sweeps but the
+  // last run fused, alternating between mask and next
+  ReinitArrays f{mask, scratch2, scratch1, next};
+  for (int it = 0; it + 1 < iters; it++) {
+    launch_reinit_sweep(s, b, &f, 1, it > 0, dt_r, dx, dy, dz);
+    std::swap(f.data, f.next);
   }
+  launch_reinit_rhs(s, b, f.data, scratch2, scratch1, rhs, iters > 1, dx, dy, dz);
+  launch_rk(s, b, 1, f.next, f.data, nullptr, rhs, dt_r);
+  launch_ghost(s, b, f.next, nullptr, ImposeArgs{}, nullptr);  // signedLinearExtrapolationBCqss(., 9)
+  QSS_CK(cudaMemcpyAsync(f.data, f.next, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
 }
 
 }  // namespace
