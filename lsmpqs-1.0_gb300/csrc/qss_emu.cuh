@@ -350,25 +350,23 @@ QSS_EMU_HD double mul(double x, double y) {
 // x + y of non-negative operands (+0 included; no NaN): no cancellation, so
 // the larger significand grows by at most one bit
 
-// a >= b by their high words, a in the window (or any normal number whose
-// double is finite); b may be +0 or subnormal
-QSS_EMU_HD double add_ordered(uint32_t ah, uint32_t al, uint32_t bh, uint32_t bl) {
-  const uint32_t mah = mant_hi(ah), mbh = mant_hi(bh);
-  const uint32_t d = ((ah - mah) - (bh - mbh)) >> 20;
-  if (d < 32u) {  // b is normal here
-    const uint64_t s = pack64(mah, al) + pack64(mbh >> d, fsr(bl, mbh, d));
-    const uint32_t f = fsr(0u, bl, d);  // bits of b below a's unit, left-aligned; bit 0 clear
-    const uint32_t sl = (uint32_t)s, sh = (uint32_t)(s >> 32), top = sh >> 21;
-    return round_pack((sh >> top) + (ah - mah) + top * 0x100000u, fsr(sl, sh, top), fsr(f, sl, top), 0u);
-  }
-  if (d >= 54u) return from_bits(pack64(ah, al));  // b is below half a unit of a
-  return QSS_EMU_FALLBACK(2, native_add(from_bits(pack64(ah, al)), from_bits(pack64(bh, bl))));
-}
-
-// the larger operand known to be in the window
+// The larger operand is normal and the sum finite; the smaller may be +0 or
+// subnormal.  No branch: the smaller significand is shifted as three words
+// (a shift of 54 or more leaves less than half a unit of the larger, whatever
+// stands in its place).
 QSS_EMU_HD double add_pos(double x, double y) {
   const bool sw = hi32(x) < hi32(y);
-  return add_ordered(sw ? hi32(y) : hi32(x), sw ? lo32(y) : lo32(x), sw ? hi32(x) : hi32(y), sw ? lo32(x) : lo32(y));
+  const uint32_t ah = sw ? hi32(y) : hi32(x), al = sw ? lo32(y) : lo32(x);
+  const uint32_t bh = sw ? hi32(x) : hi32(y), bl = sw ? lo32(x) : lo32(y);
+  const uint32_t mah = mant_hi(ah), mbh = mant_hi(bh);
+  uint32_t d = ((ah - mah) - (bh - mbh)) >> 20;
+  d = d < 63u ? d : 63u;
+  const bool far = d >= 32u;
+  const uint32_t b2 = far ? 0u : mbh, b1 = far ? mbh : bl, b0 = far ? bl : 0u, t = d & 31u;
+  const uint64_t s = pack64(mah, al) + pack64(b2 >> t, fsr(b1, b2, t));
+  const uint32_t f = fsr(b0, b1, t), rest = fsr(0u, b0, t);  // the bits of b below a's unit
+  const uint32_t sl = (uint32_t)s, sh = (uint32_t)(s >> 32), top = sh >> 21;
+  return round_pack((sh >> top) + (ah - mah) + top * 0x100000u, fsr(sl, sh, top), fsr(f, sl, top), rest | (f & top));
 }
 
 QSS_EMU_HD double add_nonneg(double x, double y) {

@@ -78,11 +78,6 @@ struct Ar {
   }
 };
 
-// out-of-line copies of integer-pipe routines: one copy of the code instead of
-// one per call site keeps the kernels' instruction footprint small
-__device__ __noinline__ double div_outline(double a, double b) { return qss_emu::div(a, b); }
-__device__ __noinline__ double mul_outline(double a, double b) { return qss_emu::mul(a, b); }
-
 struct Face {
   double v, w, t3, c13, c76, c116, c16, c56;
 };
@@ -111,22 +106,6 @@ __device__ __forceinline__ Face make_face_e(double hi, double lo, double inv) {
   f.v = d * inv;
   f.w = f.v * f.v;
   f.t3 = 3.0 * f.v;
-  f.c13 = mul(kC13, f.v);
-  f.c76 = mul(kC76, f.v);
-  f.c116 = mul(kC116, f.v);
-  f.c16 = mul(kC16, f.v);
-  f.c56 = mul(kC56, f.v);
-  return f;
-}
-
-// the face with its square and 3v on the integer pipes as well (tile form)
-__device__ __forceinline__ Face make_face_i(double hi, double lo, double inv) {
-  using qss_emu::mul;
-  Face f;
-  const double d = hi - lo;
-  f.v = d * inv;
-  f.w = mul(f.v, f.v);
-  f.t3 = mul(3.0, f.v);
   f.c13 = mul(kC13, f.v);
   f.c76 = mul(kC76, f.v);
   f.c116 = mul(kC116, f.v);
@@ -183,27 +162,22 @@ __device__ __forceinline__ double eps_of(double w1, double w2, double w3, double
 
 // weights and combination of one side (3d.f:1996-2005) given the candidate
 // stencils and smoothness indicators
-
-template <int EMU, bool SQ, bool MULC = false, bool OUTLINE = false, bool OUTMUL = false>
+template <int EMU, bool SQ>
 __device__ __forceinline__ double weno_weights(double p1, double p2, double p3, double S1, double S2, double S3,
                                                double eps) {
   using Q = Ar<EMU>;
-  auto m2 = [](double x, double y) { return (OUTMUL && EMU >= 2) ? mul_outline(x, y) : Q::mul2(x, y); };
-  auto sq = [&](double t) { return SQ ? m2(t, t) : t * t; };
-  auto dv = [](double x, double y) { return (OUTLINE && EMU >= 1) ? div_outline(x, y) : Q::div(x, y); };
+  auto sq = [](double t) { return SQ ? Q::mul2(t, t) : t * t; };
   double t, a1, a2, a3;
   t = S1 + eps;
-  a1 = dv(0.1, sq(t));
+  a1 = Q::div(0.1, sq(t));
   t = S2 + eps;
-  a2 = dv(0.6, sq(t));
+  a2 = Q::div(0.6, sq(t));
   t = S3 + eps;
-  a3 = dv(0.3, sq(t));
-  const double inv_sum_a = dv(1.0, a1 + a2 + a3);
-  a1 = m2(a1, inv_sum_a);
-  a2 = m2(a2, inv_sum_a);
-  a3 = m2(a3, inv_sum_a);
-  // the combination's products on the integer pipes too when MULC
-  if (MULC) return m2(a1, p1) + m2(a2, p2) + m2(a3, p3);
+  a3 = Q::div(0.3, sq(t));
+  const double inv_sum_a = Q::div(1.0, a1 + a2 + a3);
+  a1 = Q::mul2(a1, inv_sum_a);
+  a2 = Q::mul2(a2, inv_sum_a);
+  a3 = Q::mul2(a3, inv_sum_a);
   return a1 * p1 + a2 * p2 + a3 * p3;
 }
 
@@ -214,7 +188,7 @@ struct AxisArgs {
   double* dminus;
   double inv;
   const Ctl* ctl;
-  int seg_len;  // voxels per thread at EMU >= 1 (SEG at EMU 0)
+  int seg_len;  // voxels per thread (window forms, EMU >= 1) or positions per tile (tile form, EMU 2)
 };
 
 // One thread: SEG consecutive voxels along axis AX starting at s0, inside
@@ -381,46 +355,28 @@ __global__ void __launch_bounds__(128, RING ? 5 : 4) k_weno_axis(AxisArgs a) {
   }
 }
 
-// Tile form of the axis pass: one block holds a tile of TL lines x TP voxels
-// along the pass axis, and every face, centre and eps value of the tile is
-// computed once, by one thread, into shared memory; after a barrier each
-// thread finishes one voxel (the two weight sets and the combinations).
-// Unlike the sliding-window forms no thread carries a window of faces and
-// centres in registers, so the kernel fits 48 registers per thread and five
-// blocks (ten warps per scheduler) stay resident to hide the latency of the
-// integer-pipe arithmetic and of the tile's barriers.  The cost is the tile's
-// halo: 21 faces and 19 centres for 16 voxels of a line (about 7 % more FP64
-// work per voxel than a long window).  Lanes run over the tile's lines (16)
-// and its positions (2 per warp row), so every warp instruction of every
-// phase is full.  Measured on GB300 (whole WENO5 stage, M voxel-steps/s,
-// by-size default of the window forms -> tiles): 64^3 188 -> 338, 128^3
-// 418 -> 476, 192^3 411 -> 501, 256^3 474 -> 509, 384^3 485 -> 514, 512^3
-// 497 -> 516; the FP64 pipe runs 76 % busy at 192^3 (ncu, 4 blocks per SM)
-// against 57 % for the window form.
+// Tile form of the axis pass at EMU 1 (at EMU 2: k_weno_tile below): one block
+// holds a tile of lines x positions along the pass axis, and every face, centre
+// and eps value of the tile is computed once, by one thread, into shared
+// memory; after a barrier each thread finishes one voxel (the two weight sets
+// and the combinations).  Unlike the sliding-window forms no thread carries a
+// window of faces and centres in registers.  Lanes run over the tile's lines
+// and its positions, so every warp instruction of every phase is full.
 // A tile shape: L lines (a power of two) x P voxels along the axis, handled
 // by L * NS threads; thread t works on line t % L and position slot t / L,
 // taking positions slot, slot + NS, ... in each phase.
-template <int L_, int P_, int NS_, int MB_, int MUL_>
+template <int L_, int P_, int NS_, int MB_>
 struct TileGeom {
   static constexpr int L = L_, P = P_, NS = NS_;
   static constexpr int MB = MB_;    // resident blocks per SM the kernel is compiled for
-  static constexpr int MUL = MUL_;  // default integer-pipe / out-of-line arithmetic (tile_mul)
   static constexpr int F = P + 5;  // faces s0-2 .. s0+P+2
   static constexpr int C = P + 3;  // centres s0-1 .. s0+P+1
   static constexpr int E = P + 1;  // eps+ of voxels s0-1 .. s0+P-1
   static constexpr int NT = L * NS;
   static constexpr size_t BYTES = sizeof(double) * (8 * F + 6 * C + E) * L;
 };
-// 16 lines x 16 voxels, 256 threads (faces and centres of the halo take a
-// second round for 5 and 3 slots)
-using Tile16 = TileGeom<16, 16, 16, 5, 6>;
-// 8 lines x 27 voxels, 32 slots, 256 threads: the 32 faces take one round,
-// the 30 centres one (2 slots idle), the 27 voxels one (5 slots idle); lines
-// of a multiple of 27 voxels lose nothing to the last tile; compiled for 6
-// blocks per SM (40 registers): 565 against 553 M voxel-steps/s for the whole
-// stage at 512^3 on GB300 (16 x 16 tiles lose with 6 blocks: 518 against 522
-// M at 192^3)
-using Tile27 = TileGeom<8, 27, 32, 6, 14>;
+using Tile16 = TileGeom<16, 16, 16, 5>;
+using Tile27 = TileGeom<8, 27, 32, 6>;
 
 // the tile kernels ask for all of the unified L1 / shared memory as shared
 // memory, so that five or six blocks of a tile fit on an SM (once per
@@ -432,10 +388,8 @@ void tile_smem_attr(K kernel, bool& done) {
   done = true;
 }
 
-// MUL bit 0: the faces' squares and 3v on the integer pipes; bit 1: the
-// weights' products with the candidate stencils as well (EMU 2 only)
-template <int AX, int EMU, typename G, int MUL = 0>
-__global__ void __launch_bounds__(G::NT, G::MB) k_weno_tile(AxisArgs a) {
+template <int AX, typename G>
+__global__ void __launch_bounds__(G::NT, G::MB) k_weno_tile1(AxisArgs a) {
   if (a.ctl && !a.ctl->active) return;
   constexpr int TL = G::L, TP = G::P, NS = G::NS, TF = G::F, TC = G::C, TE = G::E;
   const Box& b = a.b;
@@ -486,8 +440,7 @@ __global__ void __launch_bounds__(G::NT, G::MB) k_weno_tile(AxisArgs a) {
   // faces m = s0-2+f (between voxels m-1 and m)
   for (int f = slot; f < TF; f += NS) {
     const int m = s0 - 2 + f;
-    const Face fc = (EMU >= 2 && (MUL & 1)) ? make_face_i(ld(m), ld(m - 1), a.inv)
-                                            : make_face_e<EMU>(ld(m), ld(m - 1), a.inv);
+    const Face fc = make_face(ld(m), ld(m - 1), a.inv);
     sf[0][f][line] = fc.v;
     sf[1][f][line] = fc.w;
     sf[2][f][line] = fc.t3;
@@ -506,7 +459,7 @@ __global__ void __launch_bounds__(G::NT, G::MB) k_weno_tile(AxisArgs a) {
     fb.v = sf[0][c + 1][line];
     fd.v = sf[0][c + 2][line];
     fd.t3 = sf[2][c + 2][line];
-    const Centre ct = make_centre<EMU, true>(fa, fb, fd);
+    const Centre ct = make_centre<1, true>(fa, fb, fd);
     sc[0][c][line] = ct.s1p;
     sc[1][c][line] = ct.s2p;
     sc[2][c][line] = ct.s3p;
@@ -527,18 +480,284 @@ __global__ void __launch_bounds__(G::NT, G::MB) k_weno_tile(AxisArgs a) {
   const double pp2_ = (-F(6, t + 4) + F(7, t + 3)) + F(3, t + 2);
   const double pp3_ = (F(3, t + 3) + F(7, t + 2)) - F(6, t + 1);
   const double plus =
-      weno_weights<EMU, true, EMU >= 2 && (MUL & 2), (MUL & 4) != 0, (MUL & 8) != 0>(pp1_, pp2_, pp3_, sc[0][t + 3][line], sc[1][t + 2][line], sc[2][t + 1][line],
-                              se[t + 1][line]);
+      weno_weights<1, true>(pp1_, pp2_, pp3_, sc[0][t + 3][line], sc[1][t + 2][line], sc[2][t + 1][line], se[t + 1][line]);
   // minus: v1..v5 = faces i-2, i-1, i, i+1, i+2 (tile faces t .. t+4)
   const double pm1_ = (F(3, t) - F(4, t + 1)) + F(5, t + 2);
   const double pm2_ = (-F(6, t + 1) + F(7, t + 2)) + F(3, t + 3);
   const double pm3_ = (F(3, t + 2) + F(7, t + 3)) - F(6, t + 4);
   const double minus =
-      weno_weights<EMU, true, EMU >= 2 && (MUL & 2), (MUL & 4) != 0, (MUL & 8) != 0>(pm1_, pm2_, pm3_, sc[3][t][line], sc[4][t + 1][line], sc[5][t + 2][line],
-                              se[t][line]);
+      weno_weights<1, true>(pm1_, pm2_, pm3_, sc[3][t][line], sc[4][t + 1][line], sc[5][t + 2][line], se[t][line]);
   const int64_t o = base + (int64_t)i * stride;
   a.dplus[o] = plus;
   a.dminus[o] = minus;
+}
+
+// ---------------------------------------------------------------------------
+// Tile form at EMU 2: the same three phases with all products, divisions and
+// part of the sums as straight-line integer code.  One test per face (|v| in
+// [2^-200, 2^60] or exactly 0) and one vote per tile replace the test of every
+// operand in every operation; a tile that fails it runs the native
+// instructions.  Inside those bounds
+//   * a square, its multiples and the sums S stay normal, and a difference t
+//     below 2^-255 may be replaced by 2^-255 in a square: S + eps >= 1e-35
+//     rounds to the same number, and nothing else reads it;
+//   * max |v| squared is the largest square (rounding is monotone), so the
+//     faces' squares are not stored;
+//   * S + eps <= 2^131, so its square, 0.1 / it, the weights' sum and its
+//     reciprocal are normal, and a weight is above 2^-700;
+//   * RN(1/3) = 2 RN(1/6), so v / 3 is twice v / 6 after rounding too: it enters
+//     the candidates as the exact product of an FMA, as do 2 v and 4 v.
+// A thread of the last phase computes one side of one voxel: both sides read
+// their stencil through one pointer and a step of either sign, so there is one
+// copy of the code.
+//
+// Bound: the FP64 pipe (one instruction per 77 cycles and scheduler) and the
+// ALU pipe together.  Per voxel ~35 FP64 instructions (additions: the centres'
+// differences 14.4, the candidates and sums 16; the faces 2.4) and ~2200 in
+// all.  The centres' six sums and the weights' sum run on the integer pipes
+// (35 instructions each); with S + eps there as well the ALU becomes the bound
+// (10.95 against 11.3 ms a pass at 512^3, 8 x 27 tiles), with none 13.5 ms.
+// One pass at 512^3 on GB300: 19.64 ms with the earlier tiles and arithmetic,
+// 14.83 with the present arithmetic in them, 10.9 in this form; ncu at 216^3
+// (8 x 27 tiles): FP64 pipe 80 % of its nominal rate (83 is what a stream of
+// independent additions reaches), ALU 71 %.
+//
+// Tile: 4 lines x up to 64 positions, 128 threads, 28 KB, 7 blocks per SM.  The
+// halo costs 5 faces and 3 centres per line of a tile, and 64 positions fill the
+// warps of each phase (9 rounds of faces, 9 of centres, 16 of sides): 10.9 ms
+// against 11.0 for 8 x 27; 256 threads 11.7.  Small grids take shorter tiles
+// (tile_len_for).
+using qss_emu::hi32;
+using qss_emu::lo32;
+
+// t * t * 2^k, |t| raised to at least 2^-255
+__device__ __forceinline__ double sq_floor(double t, int k) {
+  uint32_t h = hi32(t) & 0x7fffffffu;
+  h = h > 0x30000000u ? h : 0x30000000u;
+  return qss_emu::sq_win(h, lo32(t), k);
+}
+// 3 v of a normal v
+__device__ __forceinline__ double times3(double v) {
+  const uint32_t h = hi32(v), mh = qss_emu::mant_hi(h);
+  const uint64_t lo3 = qss_emu::madw(lo32(v), 3u, 0ull);
+  const uint32_t l = (uint32_t)lo3, m = mh * 3u + (uint32_t)(lo3 >> 32);  // 54 or 55 bits
+  const uint32_t top = m >> 22, sh = 1u + top;
+  return qss_emu::round_pack((m >> sh) + (h - mh) + sh * 0x100000u, qss_emu::fsr(l, m, sh), qss_emu::fsr(0u, l, sh), 0u);
+}
+__device__ __forceinline__ double mul_w(double x, double y) {
+  return qss_emu::mul_win(hi32(x), lo32(x), hi32(y), lo32(y));
+}
+__device__ __forceinline__ double div_w(double x, double y) {
+  bool ok = true;
+  return qss_emu::div_win(hi32(x), lo32(x), hi32(y), lo32(y), ok);
+}
+// |x| as an integer that orders like it: the bit pattern without its sign,
+// shifted out (a masked one the compiler takes for fabs, an FP64 instruction)
+__device__ __forceinline__ uint64_t abs_key(double x) { return qss_emu::bits(x) << 1; }
+__device__ __forceinline__ uint64_t max64(uint64_t x, uint64_t y) { return x > y ? x : y; }
+
+constexpr int kTileL = 4, kTileP = 64, kTileThreads = 128, kTileBlocks = 7;
+constexpr int kTileF = kTileP + 5, kTileC = kTileP + 3;
+constexpr size_t kTileBytes = sizeof(double) * (6 * kTileF + 6 * kTileC + kTileP + 1) * kTileL;
+static_assert(kTileBytes <= 48 * 1024, "dynamic shared memory without the opt-in attribute");
+
+// up to three axes in one launch: blockIdx.z runs over the tiles of x, y, z
+// lines in turn (z_end: the first index past each axis's tiles)
+struct TileArgs {
+  Box b;
+  const double* phi;
+  double *dplus[3], *dminus[3];
+  double inv[3];
+  int len[3];  // positions per tile
+  int z_end[3];
+  const Ctl* ctl;
+};
+
+__global__ void __launch_bounds__(kTileThreads, kTileBlocks) k_weno_tile(TileArgs a) {
+  if (a.ctl && !a.ctl->active) return;
+  constexpr int TL = kTileL, TF = kTileF, TC = kTileC, NT = kTileThreads;
+  const Box& b = a.b;
+  // faces: v, 3v and four scaled copies; centres: six smoothness indicators;
+  // eps+ per voxel; all [field][position][line]
+  extern __shared__ double tile_smem[];
+  double* const sf = tile_smem;
+  double* const sc = tile_smem + 6 * TF * TL;
+  double* const se = tile_smem + (6 * TF + 6 * TC) * TL;
+  const int line = threadIdx.x % TL;
+  const int ax = (int)blockIdx.z < a.z_end[0] ? 0 : ((int)blockIdx.z < a.z_end[1] ? 1 : 2);
+  const int tile = blockIdx.z - (ax == 0 ? 0 : (ax == 1 ? a.z_end[0] : a.z_end[1]));
+  const int len = ax == 0 ? a.len[0] : (ax == 1 ? a.len[1] : a.len[2]);
+  const double inv = ax == 0 ? a.inv[0] : (ax == 1 ? a.inv[1] : a.inv[2]);
+  // lanes along j for x lines, along i for y and z lines
+  int p = (ax == 0 ? b.jlo : b.ilo) + blockIdx.x * TL + line;
+  const int plast_line = ax == 0 ? b.jhi : b.ihi;
+  const int q = (ax == 2 ? b.jlo : b.klo) + blockIdx.y, qlast = ax == 2 ? b.jhi : b.khi;
+  const int lo = ax == 0 ? b.ilo : (ax == 1 ? b.jlo : b.klo), hi = ax == 0 ? b.ihi : (ax == 1 ? b.jhi : b.khi);
+  // the grid spans the longest side of each axis (block-uniform)
+  if (q > qlast || p - line > plast_line) return;
+  const bool line_ok = p <= plast_line;
+  if (!line_ok) p = plast_line;  // loads stay in the box; nothing is stored
+  const int s0 = lo + tile * len;
+  int tp = hi - s0 + 1;  // positions of this tile
+  if (tp > len) tp = len;
+  const int64_t base = ax == 0 ? b.idx(0, p, q) : (ax == 1 ? b.idx(p, 0, q) : b.idx(p, q, 0));
+  const int64_t stride = ax == 0 ? 1 : (ax == 1 ? b.sy() : b.sz());
+  const double* __restrict__ phi = a.phi + base + (int64_t)(s0 - 3) * stride;
+
+  double* const dplus = ax == 0 ? a.dplus[0] : (ax == 1 ? a.dplus[1] : a.dplus[2]);
+  double* const dminus = ax == 0 ? a.dminus[0] : (ax == 1 ? a.dminus[1] : a.dminus[2]);
+
+  // faces m = s0-2+f (between voxels m-1 and m)
+  bool ok = true;
+  for (int it = threadIdx.x; it < (tp + 5) * TL; it += NT) {
+    const int f = it / TL;
+    const double v = (__ldg(phi + (int64_t)(f + 1) * stride) - __ldg(phi + (int64_t)f * stride)) * inv;
+    const uint32_t vh = hi32(v), vl = lo32(v), av = vh & 0x7fffffffu;
+    double t3 = v, c76 = v, c116 = v, c16 = v, c56 = v;
+    if ((av | vl) != 0u) {
+      ok = ok && av - 0x33700000u < 0x10400000u;
+      t3 = times3(v);
+      c76 = mul_w(kC76, v);
+      c116 = mul_w(kC116, v);
+      c16 = mul_w(kC16, v);
+      c56 = mul_w(kC56, v);
+    }
+    double* const o = sf + it;
+    o[0] = v;
+    o[1 * TF * TL] = t3;
+    o[2 * TF * TL] = c16;
+    o[3 * TF * TL] = c76;
+    o[4 * TF * TL] = c116;
+    o[5 * TF * TL] = c56;
+  }
+  if (__syncthreads_and(ok)) {
+    // centres s0-1+c from faces c, c+1, c+2; eps+ of voxel s0-1+e from faces e .. e+4
+    for (int it = threadIdx.x; it < (tp + 3) * TL; it += NT) {
+      const double* const o = sf + it;
+      const double va = o[0], vb = o[TL], vd = o[2 * TL], a3 = o[TF * TL], d3 = o[TF * TL + 2 * TL];
+      auto less2b = [&](double x) { return __fma_rn(-2.0, vb, x); };  // x - 2 vb: the product is exact
+      auto less4b = [&](double x) { return __fma_rn(-4.0, vb, x); };
+      const double A = mul_w(k1312, sq_floor(less2b(vd) + va, 0));
+      const double B = mul_w(k1312, sq_floor(less2b(va) + vd, 0));
+      const double Cp = sq_floor(less4b(vd) + a3, -2);
+      const double Dp = sq_floor(less4b(d3) + va, -2);
+      const double Cm = sq_floor(less4b(va) + d3, -2);
+      const double Dm = sq_floor(less4b(a3) + vd, -2);
+      const double E = sq_floor(vd - va, -2);
+      double* const w = sc + it;
+      w[0] = qss_emu::add_pos(A, Cp);
+      w[1 * TC * TL] = qss_emu::add_pos(A, E);
+      w[2 * TC * TL] = qss_emu::add_pos(A, Dp);
+      w[3 * TC * TL] = qss_emu::add_pos(B, Cm);
+      w[4 * TC * TL] = qss_emu::add_pos(B, E);
+      w[5 * TC * TL] = qss_emu::add_pos(B, Dm);
+      if (it < (tp + 1) * TL) {
+        const uint64_t m = max64(max64(max64(abs_key(va), abs_key(vb)), abs_key(vd)),
+                                 max64(abs_key(o[3 * TL]), abs_key(o[4 * TL])));
+        const uint32_t mh = (uint32_t)(m >> 33);
+        double e = mul_w(1e-6, qss_emu::sq_win(mh > 0x30000000u ? mh : 0x30000000u, (uint32_t)(m >> 1)));
+        // 1e-35 is below half a unit of a product of 2^-61 or more
+        if (hi32(e) < 0x3c200000u) e = qss_emu::native_add(e, 1.0e-35);
+        se[it] = e;
+      }
+    }
+    __syncthreads();
+    if (!line_ok) return;
+    const int voxels = tp * TL;
+    for (int it = threadIdx.x; it < 2 * voxels; it += NT) {
+      const bool is_plus = it >= voxels;
+      const int r = is_plus ? it - voxels : it;  // position * TL + line
+      // minus: v1..v5 = faces i-2 .. i+2 (tile faces t .. t+4), plus: faces i+3 .. i-1 (t+5 .. t+1)
+      const int st = is_plus ? -TL : TL;
+      const double* const f = sf + (is_plus ? r + 5 * TL : r);
+      const double* const c = sc + (is_plus ? r + 3 * TL : r + 3 * TC * TL);
+      const double eps = se[is_plus ? r + TL : r];
+      const double s1 = c[0], s2 = (c + st)[TC * TL], s3 = (c + 2 * st)[2 * TC * TL];
+      double t = s1 + eps;
+      double a1 = div_w(0.1, qss_emu::sq_win(hi32(t), lo32(t)));
+      t = s2 + eps;
+      double a2 = div_w(0.6, qss_emu::sq_win(hi32(t), lo32(t)));
+      t = s3 + eps;
+      double a3 = div_w(0.3, qss_emu::sq_win(hi32(t), lo32(t)));
+      const double inv_sum_a = div_w(1.0, qss_emu::add_pos(qss_emu::add_pos(a1, a2), a3));
+      a1 = mul_w(a1, inv_sum_a);
+      a2 = mul_w(a2, inv_sum_a);
+      a3 = mul_w(a3, inv_sum_a);
+      const double* const f2 = f + st;
+      const double* const f3 = f2 + st;
+      const double* const f4 = f3 + st;
+      const double* const f5 = f4 + st;
+      constexpr int K = TF * TL;
+      // v / 3 = 2 (v / 6), rounded alike: the third enters as an exact doubling
+      const double c56_3 = f3[5 * K];
+      const double p1 = __fma_rn(2.0, f[2 * K], -f2[3 * K]) + f3[4 * K];
+      const double p2 = __fma_rn(2.0, f4[2 * K], -f2[2 * K] + c56_3);
+      const double p3 = __fma_rn(2.0, f3[2 * K], f4[5 * K]) - f5[2 * K];
+      double m1, m2, m3;
+      if ((qss_emu::win(hi32(p1)) | qss_emu::win(hi32(p2)) | qss_emu::win(hi32(p3))) < 0x40000000u) {
+        m1 = mul_w(a1, p1);
+        m2 = mul_w(a2, p2);
+        m3 = mul_w(a3, p3);
+      } else {
+        m1 = a1 * p1;
+        m2 = a2 * p2;
+        m3 = a3 * p3;
+      }
+      double* const out = is_plus ? dplus : dminus;
+      out[base + (int64_t)(s0 + r / TL) * stride] = m1 + m2 + m3;
+    }
+    return;
+  }
+  // a tile with values outside the bounds: native instructions
+  for (int it = threadIdx.x; it < (tp + 5) * TL; it += NT) {
+    double* const o = sf + it;
+    const Face fc = make_face(o[0], 0.0, 1.0);
+    o[1 * TF * TL] = fc.t3;
+    o[2 * TF * TL] = fc.c16;
+    o[3 * TF * TL] = fc.c76;
+    o[4 * TF * TL] = fc.c116;
+    o[5 * TF * TL] = fc.c56;
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < (tp + 3) * TL; it += NT) {
+    const double* const o = sf + it;
+    Face fa{}, fb{}, fd{};
+    fa.v = o[0];
+    fa.t3 = o[TF * TL];
+    fb.v = o[TL];
+    fd.v = o[2 * TL];
+    fd.t3 = o[TF * TL + 2 * TL];
+    const Centre ct = make_centre<0, false>(fa, fb, fd);
+    double* const w = sc + it;
+    w[0] = ct.s1p;
+    w[1 * TC * TL] = ct.s2p;
+    w[2 * TC * TL] = ct.s3p;
+    w[3 * TC * TL] = ct.s1m;
+    w[4 * TC * TL] = ct.s2m;
+    w[5 * TC * TL] = ct.s3m;
+    if (it < (tp + 1) * TL) {
+      const double v3 = o[3 * TL], v4 = o[4 * TL];
+      se[it] = 1e-6 * dmax(dmax(dmax(dmax(v4 * v4, v3 * v3), fd.v * fd.v), fb.v * fb.v), fa.v * fa.v) + 1.0e-35;
+    }
+  }
+  __syncthreads();
+  if (!line_ok) return;
+  const int voxels = tp * TL;
+  for (int it = threadIdx.x; it < 2 * voxels; it += NT) {
+    const bool is_plus = it >= voxels;
+    const int r = is_plus ? it - voxels : it;
+    const int st = is_plus ? -TL : TL;
+    const double* const f = sf + (is_plus ? r + 5 * TL : r);
+    const double* const c = sc + (is_plus ? r + 3 * TL : r + 3 * TC * TL);
+    constexpr int K = TF * TL;
+    auto third = [&](int k) { return kC13 * (f + k * st)[0]; };
+    const double p1 = (third(0) - (f + st)[3 * K]) + (f + 2 * st)[4 * K];
+    const double p2 = (-(f + st)[2 * K] + (f + 2 * st)[5 * K]) + third(3);
+    const double p3 = (third(2) + (f + 3 * st)[5 * K]) - (f + 4 * st)[2 * K];
+    double* const out = is_plus ? dplus : dminus;
+    out[base + (int64_t)(s0 + r / TL) * stride] =
+        weno_weights<0, false>(p1, p2, p3, c[0], (c + st)[TC * TL], (c + 2 * st)[2 * TC * TL], se[is_plus ? r + TL : r]);
+  }
 }
 
 struct CombineArgs {
@@ -741,57 +960,91 @@ int default_seg_len(int var, int64_t lines, int along) {
   return var ? seg_len_for(lines, along, 16, along / 64) : seg_len_for(lines, along, 8, (along + SEG - 1) / SEG);
 }
 
-template <int EMU, typename G, int MUL>
-void launch_tile_m(cudaStream_t s, int ax, const AxisArgs& a, int lanes, int other, int along) {
+template <typename G>
+void launch_tile1(cudaStream_t s, int ax, const AxisArgs& a, int lanes, int other, int along) {
   const dim3 gt((lanes + G::L - 1) / G::L, other, (along + G::P - 1) / G::P);
   static bool done[3] = {false, false, false};
   if (ax == 0) {
-    tile_smem_attr(k_weno_tile<0, EMU, G, MUL>, done[0]);
-    k_weno_tile<0, EMU, G, MUL><<<gt, G::NT, G::BYTES, s>>>(a);
+    tile_smem_attr(k_weno_tile1<0, G>, done[0]);
+    k_weno_tile1<0, G><<<gt, G::NT, G::BYTES, s>>>(a);
   } else if (ax == 1) {
-    tile_smem_attr(k_weno_tile<1, EMU, G, MUL>, done[1]);
-    k_weno_tile<1, EMU, G, MUL><<<gt, G::NT, G::BYTES, s>>>(a);
+    tile_smem_attr(k_weno_tile1<1, G>, done[1]);
+    k_weno_tile1<1, G><<<gt, G::NT, G::BYTES, s>>>(a);
   } else {
-    tile_smem_attr(k_weno_tile<2, EMU, G, MUL>, done[2]);
-    k_weno_tile<2, EMU, G, MUL><<<gt, G::NT, G::BYTES, s>>>(a);
+    tile_smem_attr(k_weno_tile1<2, G>, done[2]);
+    k_weno_tile1<2, G><<<gt, G::NT, G::BYTES, s>>>(a);
   }
 }
 
-// $QSSGPU_TILE_MUL (0, 2, 6 or 14; default per geometry, TileGeom::MUL):
-// bit 1 the weights' products with the candidate stencils on the integer
-// pipes, bit 2 one out-of-line copy of the integer-pipe division, bit 3 one
-// out-of-line copy of the integer-pipe product (in the weights); identical
-// results.  GB300, whole WENO5 stage, M voxel-steps/s at 512^3 (8 x 27
-// tiles) / 192^3 (16 x 16): 0: 553.7 / 522.1, 2: 558.5 / 524.5,
-// 6: 580.8 / 546.1, 14: 592.4 / 539.4 (bit 0, the faces' squares and 3v on
-// the integer pipes: no gain; an out-of-line square root and division in the
-// combine kernel: none either; an out-of-line product in the centres' squares:
-// 578.7 / 539.1, a loss).
-int tile_mul() {
-  static const int m = [] {
-    const char* e = getenv("QSSGPU_TILE_MUL");
-    const int v = e ? atoi(e) : -1;
-    return v == 0 || v == 2 || v == 6 || v == 14 ? v : -1;
-  }();
-  return m;
+int line_len(const Box& b, int ax) { return ax == 0 ? b.fbx() : (ax == 1 ? b.fby() : b.fbz()); }
+int line_lanes(const Box& b, int ax) { return ax == 0 ? b.fby() : b.fbx(); }
+int line_rows(const Box& b, int ax) { return ax == 2 ? b.fby() : b.fbz(); }
+
+// lines split evenly into tiles of at most cap positions
+int even_len(int along, int cap) {
+  const int tiles = (along + cap - 1) / cap;
+  return (along + tiles - 1) / tiles;
 }
 
-template <int EMU, typename G>
-void launch_tile(cudaStream_t s, int ax, const AxisArgs& a, int lanes, int other, int along) {
-  switch (EMU >= 2 ? (tile_mul() >= 0 ? tile_mul() : G::MUL) : 0) {
-    case 0: launch_tile_m<EMU, G, 0>(s, ax, a, lanes, other, along); break;
-    case 2: launch_tile_m<EMU, G, 2>(s, ax, a, lanes, other, along); break;
-    case 6: launch_tile_m<EMU, G, 6>(s, ax, a, lanes, other, along); break;
-    default: launch_tile_m<EMU, G, 14>(s, ax, a, lanes, other, along); break;
+// The longest tiles (the smallest halo) that leave about four rounds of blocks
+// for the GPU, down to 8 positions.  Whole stage, M voxel-steps/s, 8-line tiles
+// of up to 8 / 16 / 24 / 27 positions: 24^3 70 / 66 / 63 / 63, 48^3 337 / 340 /
+// 347 / 347, 96^3 703 / 743 / 761 / 760, 128^3 773 / 827 / 837 / 851.
+int tile_cap_for(const Box& b) {
+  int cap = kTileP;
+  while (cap > 8) {
+    int64_t blocks = 0;
+    for (int ax = 0; ax < 3; ax++)
+      blocks += (int64_t)((line_lanes(b, ax) + kTileL - 1) / kTileL) * line_rows(b, ax) *
+                ((line_len(b, ax) + cap - 1) / cap);
+    if (blocks >= (int64_t)152 * kTileBlocks * 4) break;
+    cap /= 2;
   }
+  return cap;
+}
+
+// axes [ax0, ax1) in one launch
+void launch_tiles(cudaStream_t s, const Box& b, const double* phi, const double invs[3], double* const dp[3],
+                  double* const dm[3], const Ctl* ctl, int ax0, int ax1, int cap) {
+  static bool done = false;
+  tile_smem_attr(k_weno_tile, done);
+  TileArgs a;
+  a.b = b;
+  a.phi = phi;
+  a.ctl = ctl;
+  dim3 g(0, 0, 0);
+  for (int ax = 0; ax < 3; ax++) {
+    a.dplus[ax] = dp[ax];
+    a.dminus[ax] = dm[ax];
+    a.inv[ax] = invs[ax];
+    const int along = line_len(b, ax);
+    a.len[ax] = even_len(along, cap < kTileP ? cap : kTileP);
+    if (ax >= ax0 && ax < ax1) {
+      const unsigned x = (line_lanes(b, ax) + kTileL - 1) / kTileL, y = line_rows(b, ax);
+      if (x > g.x) g.x = x;
+      if (y > g.y) g.y = y;
+      g.z += (along + a.len[ax] - 1) / a.len[ax];
+    }
+    a.z_end[ax] = (int)g.z;
+  }
+  k_weno_tile<<<g, kTileThreads, kTileBytes, s>>>(a);
 }
 
 template <int EMU>
 void launch_axis(cudaStream_t s, int ax, int var, AxisArgs a, int lanes, int other, int along, int len) {
   a.seg_len = len;
-  if (var >= 3 && EMU != 0) {
-    if (var == 4) launch_tile<EMU, Tile27>(s, ax, a, lanes, other, along);
-    else launch_tile<EMU, Tile16>(s, ax, a, lanes, other, along);
+  if (var >= 3 && EMU == 2) {
+    double *dp[3] = {}, *dm[3] = {};
+    double invs[3] = {};
+    dp[ax] = a.dplus;
+    dm[ax] = a.dminus;
+    invs[ax] = a.inv;
+    launch_tiles(s, a.b, a.phi, invs, dp, dm, a.ctl, ax, ax + 1, var == 4 ? 27 : 16);
+    return;
+  }
+  if (var >= 3 && EMU == 1) {
+    if (var == 4) launch_tile1<Tile27>(s, ax, a, lanes, other, along);
+    else launch_tile1<Tile16>(s, ax, a, lanes, other, along);
     return;
   }
   dim3 g((lanes + 127) / 128, other, (along + len - 1) / len);
@@ -865,25 +1118,41 @@ bool tune_axis(cudaStream_t s, int ax, const AxisArgs& a, int lanes, int other, 
   return ok && active;
 }
 
-// The default tile: 8 x 27 where the line splits into 27-voxel tiles with at
-// most 2 % of the last tile unused, else 16 x 16 (whole WENO5 stage on GB300,
-// M voxel-steps/s, 16 x 16 / 8 x 27: 512^3 516 / 532 (1.2 % unused),
-// 192^3 501 / 485 (12.5 % unused)).
+// The default tile at EMU 1: 8 x 27 where the line splits into 27-voxel tiles
+// with at most 2 % of the last tile unused, else 16 x 16.
 int tile_form_for(int along) {
   const int tiles = (along + Tile27::P - 1) / Tile27::P;
   return (int64_t)tiles * Tile27::P * 50 <= (int64_t)along * 51 ? 4 : 3;
 }
 
+// Below this many blocks for one axis the three axes share a launch (same
+// work, two launches fewer and one partly filled last round instead of three).
+constexpr int64_t kMergeBlocks = (int64_t)152 * kTileBlocks * 16;
+
 template <int EMU>
 void axes_at(cudaStream_t s, const Box& b, const double* phi, const double invs[3], double* const dp[3],
              double* const dm[3], const Ctl* ctl) {
   const int mode = axis_variant();
+  if (EMU == 2 && (mode == -1 || mode >= 3)) {
+    const int cap = mode == 3 ? 16 : (mode == 4 ? 27 : tile_cap_for(b));
+    cudaEvent_t e0 = ctl ? prof_open(s) : nullptr;
+    if (!e0 && b.fbx() * (int64_t)b.fby() * b.fbz() < kMergeBlocks * kTileL * kTileP) {
+      launch_tiles(s, b, phi, invs, dp, dm, ctl, 0, 3, cap);
+      return;
+    }
+    for (int ax = 0; ax < 3; ax++) {  // one launch per axis, timed one by one where asked for
+      if (ax && ctl) e0 = prof_open(s);
+      launch_tiles(s, b, phi, invs, dp, dm, ctl, ax, ax + 1, cap);
+      prof_close(s, e0, kProfAxisX + ax);
+    }
+    return;
+  }
   for (int ax = 0; ax < 3; ax++) {
     const int along = ax == 0 ? b.fbx() : (ax == 1 ? b.fby() : b.fbz());
     const int lanes = ax == 0 ? b.fby() : b.fbx();
     const int other = ax == 2 ? b.fby() : b.fbz();
-    // by default a tile form (tile_form_for), the fastest at every size
-    // measured on GB300 (64^3 .. 512^3, see k_weno_tile); of the two window forms, which are
+    // by default a tile form, the fastest at every size measured on GB300
+    // (64^3 .. 512^3); of the two window forms, which are
     // kept selectable, the shared-memory one is the faster from ~12 M fill
     // voxels on (register / shared-memory form, M voxel-steps/s: 128^3
     // 420 / 383, 192^3 411 / 385, 256^3 458 / 473, 512^3 469 / 488)
