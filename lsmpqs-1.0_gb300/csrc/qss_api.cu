@@ -52,14 +52,6 @@ SchemeSel scheme_of(const Options* o) {
 
 void sync(DevVolume& v) { QSS_CK(cudaStreamSynchronize(v.stream)); }
 
-void check_device_flags(DevVolume& v) {
-  QSS_CK(cudaMemcpyAsync(v.h_ctl, v.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, v.stream));
-  sync(v);
-  if (v.h_ctl->err)
-    throw Error(QSSGPU_ERR_DEVICE_CHECK, "a device-side iteration cap was reached (flags " +
-                                             std::to_string(v.h_ctl->err) + ")");
-}
-
 ImposeArgs impose_args(DevVolume& v, const Options* o) {
   return ImposeArgs{v.mask, v.mask_w, v.mask_nw, o->overlap, o->check_connectivity ? 1 : 0};
 }
@@ -138,21 +130,35 @@ void dev_trap(DevVolume& v, const Grid* g, const Options* o) {
   v.zero_on_return[H_SCRATCH1] = true;
 }
 
-double dev_volume(DevVolume& v, const double* f, const Grid* g, double eps) {
+// The reductions of an outer iteration are queued together and read back with
+// one synchronisation: volumes into dscal[0..1], the max norm's key and the
+// control block's error flags.
+void queue_volume(DevVolume& v, const double* f, const Grid* g, double eps, int slot) {
   PhaseTimer pt(v, PH_REDUCE);
-  launch_volume(v.stream, v.box, f, g->dx[0], g->dx[1], g->dx[2], eps, v.contrib, v.dscal);
-  QSS_CK(cudaMemcpyAsync(v.h_scal, v.dscal, sizeof(double), cudaMemcpyDeviceToHost, v.stream));
-  sync(v);
-  return v.h_scal[0];
+  launch_volume(v.stream, v.box, f, g->dx[0], g->dx[1], g->dx[2], eps, v.contrib, v.dscal + slot);
+  QSS_CK(cudaMemcpyAsync(v.h_scal + slot, v.dscal + slot, sizeof(double), cudaMemcpyDeviceToHost, v.stream));
 }
 
-double dev_maxnorm(DevVolume& v, const Options* o) {
+void queue_maxnorm(DevVolume& v, const Options* o) {
   PhaseTimer pt(v, PH_REDUCE);
   launch_maxnormdiff(v.stream, v.box, v.phi, v.phi_prev, o->err_check_zone, v.red + 2);
+  QSS_CK(cudaMemcpyAsync(v.h_scal + 2, v.red + 2, sizeof(unsigned long long), cudaMemcpyDeviceToHost, v.stream));
+}
+
+double fetched_maxnorm(const DevVolume& v) {
   unsigned long long key;
-  QSS_CK(cudaMemcpyAsync(&key, v.red + 2, sizeof key, cudaMemcpyDeviceToHost, v.stream));
+  memcpy(&key, v.h_scal + 2, sizeof key);
+  return maxnorm_of_key(key);
+}
+
+// waits for everything queued and checks the device-side error flags
+void sync_and_check(DevVolume& v) {
+  PhaseTimer pt(v, PH_REDUCE);
+  QSS_CK(cudaMemcpyAsync(v.h_ctl, v.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, v.stream));
   sync(v);
-  return key_to_double(key);
+  if (v.h_ctl->err)
+    throw Error(QSSGPU_ERR_DEVICE_CHECK, "a device-side iteration cap was reached (flags " +
+                                             std::to_string(v.h_ctl->err) + ")");
 }
 
 // ---------------------------------------------------------------------------
@@ -278,8 +284,14 @@ double dev_const_curv(DevVolume& v, bool var, Options* o, QSS_DataArrays* p, Gri
   const double vol_very_small = g->dx[0] * g->dx[1] * g->dx[2];
   const double eps = o->eps_coefficient * g->dx[0];
   const double max_satn = o->vol_frac_max;
-  const double vol_pore = dev_volume(v, v.mask, g, eps);
-  vol_phi = dev_volume(v, v.phi, g, eps);
+  queue_volume(v, v.mask, g, eps, 0);
+  queue_volume(v, v.phi, g, eps, 1);
+  {
+    PhaseTimer pt(v, PH_REDUCE);
+    sync(v);
+  }
+  const double vol_pore = v.h_scal[0];
+  vol_phi = v.h_scal[1];
   double satn = vol_phi / vol_pore, satn_old;
   while ((t < o->tmax) && (max_abs_err > o->eps_stop)) {
     v.outer_iters++;
@@ -321,10 +333,12 @@ double dev_const_curv(DevVolume& v, bool var, Options* o, QSS_DataArrays* p, Gri
     dev_reinit(v, &v.phi, 1, g, o);
     if (fp_out) fprintf(fp_out, "Reinitialized\n");
     v.dirty[H_PHI] = true;
-    max_abs_err = dev_maxnorm(v, o);
+    queue_maxnorm(v, o);
+    queue_volume(v, v.phi, g, eps, 1);
+    sync_and_check(v);
+    max_abs_err = fetched_maxnorm(v);
     satn_old = satn;
-    vol_phi = dev_volume(v, v.phi, g, eps);
-    check_device_flags(v);
+    vol_phi = v.h_scal[1];
     satn = vol_phi / vol_pore;
     if ((satn > max_satn) || (vol_phi <= vol_very_small)) return -1;
     if (o->checkpoint) {

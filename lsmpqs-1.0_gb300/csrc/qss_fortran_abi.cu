@@ -412,7 +412,7 @@ void qss3dmaxnormdifflocal_(double* max_norm_diff, const double* field1, GBN(a),
   unsigned long long k;
   d2h(&k, key, sizeof k);
   finish();
-  *max_norm_diff = key_to_double(k);
+  *max_norm_diff = maxnorm_of_key(k);
   ABI_END
 }
 

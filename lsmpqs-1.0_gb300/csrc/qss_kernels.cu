@@ -839,38 +839,20 @@ __global__ void k_maxnormdiff(Box b, const double* __restrict__ f1, const double
   const int i = b.ilo + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = b.jlo + blockIdx.y * blockDim.y + threadIdx.y;
   const int k = b.klo + blockIdx.z * blockDim.z + threadIdx.z;
-  double m = -1.0;
+  // magnitudes compared as integers (-1: none; NaN differences count as none):
+  // a native comparison occupies the FP64 pipe like an addition
+  long long m = -1;
   if (i <= b.ihi && j <= b.jhi && k <= b.khi) {
     const int64_t c = b.idx(i, j, k);
     const double a = f1[c];
-    if (fabs(a) < zone) m = fabs(a - f2[c]);
-  }
-  for (int o = 16; o > 0; o >>= 1) m = dmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
-  if (lane == 0 && m > -1.0) atomicMax(key, double_to_key(m));
-}
-
-// contribution of each fill-box voxel, stored in loop order (i fastest)
-__global__ void k_vol_contrib(Box b, const double* __restrict__ phi, double dV, double eps, double* contrib) {
-  const int64_t n = (int64_t)b.fbx() * b.fby() * b.fbz();
-  const double pi = 3.14159265358979323846;
-  const double one_over_pi = 0.31830988618379;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-    const int i = b.ilo + (int)(q % b.fbx());
-    const int64_t r = q / b.fbx();
-    const int j = b.jlo + (int)(r % b.fby());
-    const int k = b.klo + (int)(r / b.fby());
-    const double p = phi[b.idx(i, j, k)];
-    const double rr = p / eps;
-    double v = 0.0;
-    if (p < -eps) {
-      v = dV;
-    } else if (p < eps) {
-      const double one_minus_H = 0.5 * (1 - rr - one_over_pi * portable_sin(pi * rr));
-      v = one_minus_H * dV;
+    if (qss_emu::gt(zone, a) && qss_emu::gt(a, -zone)) {  // |a| < zone
+      m = (long long)qss_emu::bits(qss_emu::abs(a - f2[c]));
+      if (m > 0x7ff0000000000000ll) m = -1;
     }
-    contrib[q] = v;
   }
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
+  const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
+  if (lane == 0 && m >= 0) atomicMax(key, double_to_key(__longlong_as_double(m)));
 }
 
 // ---------------------------------------------------------------------------
@@ -1263,17 +1245,8 @@ void launch_impose_slab(cudaStream_t s, const Box& b, double* out, const double*
 
 void launch_maxnormdiff(cudaStream_t s, const Box& b, const double* f1, const double* f2, double zone,
                         unsigned long long* key) {
-  unsigned long long init = double_to_key(-1.0);
-  cudaMemcpyAsync(key, &init, sizeof init, cudaMemcpyHostToDevice, s);
+  cudaMemsetAsync(key, 0, sizeof *key, s);
   k_maxnormdiff<<<fb_grid(b, kBlk3), kBlk3, 0, s>>>(b, f1, f2, zone, key);
-}
-
-void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, double dy, double dz, double eps,
-                   double* scratch, double* out) {
-  const int64_t n = (int64_t)b.fbx() * b.fby() * b.fbz();
-  const double dV = dx * dy * dz;
-  k_vol_contrib<<<grid1(n), kBlk1, 0, s>>>(b, phi, dV, eps, scratch);
-  launch_loop_sum(s, scratch, n, scratch + n, out);
 }
 
 void launch_sphere(cudaStream_t s, const Box& b, double* phi, const double* x_lo_gb, const double* dxv, double cx,

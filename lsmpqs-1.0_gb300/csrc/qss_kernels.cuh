@@ -185,6 +185,9 @@ __host__ __device__ inline double key_to_double(unsigned long long k) {
   memcpy(&v, &u, 8);
   return v;
 }
+// *key: double_to_key of the largest |f1 - f2| where |f1| < zone, 0 where there is
+// none (maxnorm_of_key)
+inline double maxnorm_of_key(unsigned long long k) { return k ? key_to_double(k) : -1.0; }
 void launch_maxnormdiff(cudaStream_t s, const Box& b, const double* f1, const double* f2,
                         double zone, unsigned long long* key);
 // sequential (loop-order) smoothed volume of {phi < 0}; contrib is fill-box sized scratch

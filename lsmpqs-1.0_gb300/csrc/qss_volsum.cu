@@ -18,19 +18,24 @@
 // parallel and exactly (int64), valid when no element is a tie or not a
 // finite non-negative number and s / u + R stays below 2^53 - 1.
 //
-//   1. k_vol_chunk_sum: per chunk of 4096 contributions, its double sum (any
-//      order) -- only to estimate where the running sum stands;
-//   2. k_vol_scan: exclusive scan of those sums -> an estimate of s at the
+//   1. k_vol_contrib (volumes; the contributions are computed here) or
+//      k_vol_chunk_sum (a given sequence): per chunk of 4096 contributions,
+//      their sum -- only to estimate where the running sum stands;
+//   2. k_vol_scan (more than 4096 chunks only; else each block of 3 sums its
+//      predecessors): exclusive scan of those sums -> an estimate of s at the
 //      start of each chunk, good to far better than a factor of 2;
 //   3. k_vol_chunk_r: per chunk, R and a "not applicable" flag for the
 //      estimated binade and its two neighbours;
-//   4. k_vol_walk: one warp walks the chunks in order with the exact running
-//      sum: a chunk whose flag is clear for the binade s is actually in, and
-//      that does not reach the top of it, advances s by u * R in one integer
-//      addition; any other chunk (the first ones, binade crossings, ties,
-//      special values) is added element by element with native FP64
-//      additions in loop order.
-// Every result equals the sequential loop's bit for bit.
+//   4. k_vol_walk: one block walks the chunks in order with the exact running
+//      sum, 256 chunks at a time: a scan of their R finds the first chunk that
+//      does not apply (another binade, the top of the binade reached, a tie,
+//      special values); the sum advances to it in one integer addition, and
+//      that chunk goes the same way by groups of 16 elements, only the group
+//      that does not apply being added element by element.
+// Every result equals the sequential loop's bit for bit.  With one warp that
+// walked chunk by chunk and added a whole chunk element by element, a volume
+// took 0.42 ms at 24^3, 3.5 ms at 192^3 and 8.6 ms at 320^3 on GB300.
+#include "qss_emu.cuh"
 #include "qss_state.h"
 
 namespace qss {
@@ -39,7 +44,9 @@ namespace {
 
 constexpr int kVolChunk = 4096;
 constexpr int kVolThreads = 256;
-constexpr int kWalkBatch = 512;  // chunk descriptors staged in shared memory per round
+constexpr int kVolPer = kVolChunk / kVolThreads;  // elements per thread in the walk
+constexpr int kScanChunks = 4096;                 // from here on the estimates are scanned by a kernel
+constexpr int kSmallChunks = 4;                   // up to here the walk goes by elements alone
 
 __device__ __forceinline__ uint64_t dbits(double x) { return (uint64_t)__double_as_longlong(x); }
 __device__ __forceinline__ double dfrom(uint64_t b) { return __longlong_as_double((long long)b); }
@@ -99,25 +106,66 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_sum(const double* __r
   if (threadIdx.x == 0) csum[blockIdx.x] = red[0];
 }
 
+// contribution of each fill-box voxel in loop order (i fastest), and the
+// chunk's sum; one voxel in the smoothing band costs a division and a sine, any
+// other an integer comparison
+__global__ void __launch_bounds__(1024) k_vol_contrib(Box b, const double* __restrict__ phi, double dV, double eps,
+                                                      double* contrib, double* csum) {
+  __shared__ float red[32];
+  const double pi = 3.14159265358979323846;
+  const double one_over_pi = 0.31830988618379;
+  const uint32_t n = (uint32_t)b.fbx() * b.fby() * b.fbz();  // below 2^31
+  const uint32_t base = blockIdx.x * (uint32_t)kVolChunk;
+  float sum = 0.0f;
+  for (uint32_t t = threadIdx.x; t < kVolChunk; t += 1024) {
+    const uint32_t q = base + t;
+    if (q >= n) break;
+    const uint32_t r = q / (uint32_t)b.fbx();
+    const int i = b.ilo + (int)(q - r * (uint32_t)b.fbx());
+    const int k = b.klo + (int)(r / (uint32_t)b.fby());
+    const int j = b.jlo + (int)(r - (uint32_t)(k - b.klo) * (uint32_t)b.fby());
+    const double p = phi[b.idx(i, j, k)];
+    double v = 0.0;
+    if (qss_emu::gt(-eps, p)) {  // p < -eps
+      v = dV;
+    } else if (qss_emu::gt(eps, p)) {  // p < eps
+      const double rr = p / eps;
+      const double one_minus_H = 0.5 * (1 - rr - one_over_pi * portable_sin(pi * rr));
+      v = one_minus_H * dV;
+    }
+    contrib[q] = v;
+    // v as a float by its bits (a conversion is an FP64 instruction); values
+    // outside the float range do not matter for the estimate
+    const uint32_t h = qss_emu::hi32(v);
+    if (h - 0x38100000u < 0x0fe00000u) sum += __uint_as_float((h - 0x38000000u) << 3);
+  }
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    sum = red[threadIdx.x];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if (threadIdx.x == 0) csum[blockIdx.x] = (double)sum;
+  }
+}
+
 // exclusive scan of nc chunk sums in one block of 1024 threads
 __global__ void __launch_bounds__(1024) k_vol_scan(const double* __restrict__ csum, int64_t nc, double* est) {
-  __shared__ double part[1024];
+  __shared__ double part[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t per = (nc + 1023) / 1024;
   const int64_t lo = threadIdx.x * per, hi = lo + per < nc ? lo + per : nc;
   double s = 0;
   for (int64_t j = lo; j < hi; j++) s += csum[j];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double run = 0;
-    for (int t = 0; t < 1024; t++) {
-      const double x = part[t];
-      part[t] = run;
-      run += x;
-    }
+  double incl = s;
+  for (int o = 1; o < 32; o <<= 1) {
+    const double x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
   }
+  if (lane == 31) part[warp] = incl;
   __syncthreads();
-  double run = part[threadIdx.x];
+  double run = incl - s;
+  for (int w = 0; w < warp; w++) run += part[w];
   for (int64_t j = lo; j < hi; j++) {
     est[j] = run;
     run += csum[j];
@@ -126,12 +174,25 @@ __global__ void __launch_bounds__(1024) k_vol_scan(const double* __restrict__ cs
 
 // R[3j+q], F[3j+q] for E = exp(est[j]) - 1 + q
 __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __restrict__ c, int64_t n,
-                                                             const double* __restrict__ est, int64_t* R,
-                                                             int64_t* F) {
+                                                             const double* __restrict__ csum, bool scanned, double* est,
+                                                             int64_t* R, int64_t* F) {
   __shared__ unsigned long long rs[3][kVolThreads];
   __shared__ int fs[3][kVolThreads];
+  __shared__ double s_est[kVolThreads / 32];
   const int64_t j = blockIdx.x;
-  const int E0 = exp_of(est[j]);
+  double e = 0;
+  if (scanned) {
+    e = est[j];
+  } else {
+    for (int64_t q = threadIdx.x; q < j; q += kVolThreads) e += csum[q];
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if ((threadIdx.x & 31) == 0) s_est[threadIdx.x >> 5] = e;
+    __syncthreads();
+    e = 0;
+    for (int w = 0; w < kVolThreads / 32; w++) e += s_est[w];
+    if (threadIdx.x == 0) est[j] = e;
+  }
+  const int E0 = exp_of(e);
   const int64_t base = j * kVolChunk;
   unsigned long long r[3] = {0, 0, 0};
   bool bad[3] = {E0 < -1000, E0 < -1000, E0 < -1000};
@@ -168,63 +229,99 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __res
   }
 }
 
-// one warp: the exact running sum over the chunks in loop order
-__global__ void __launch_bounds__(32) k_vol_walk(const double* __restrict__ c, int64_t n, int64_t nc,
-                                                 const double* __restrict__ est, const int64_t* __restrict__ R,
-                                                 const int64_t* __restrict__ F, double* out) {
-  __shared__ double s_est[kWalkBatch];
-  __shared__ long long s_r[3 * kWalkBatch];
-  __shared__ int s_f[3 * kWalkBatch];
-  __shared__ int s_fast;
-  __shared__ double s_sum;
-  const int lane = threadIdx.x;
-  if (lane == 0) s_sum = 0.0;
-  for (int64_t j0 = 0; j0 < nc; j0 += kWalkBatch) {
-    const int cnt = (int)((nc - j0) < kWalkBatch ? (nc - j0) : kWalkBatch);
-    __syncwarp();
-    for (int t = lane; t < cnt; t += 32) s_est[t] = est[j0 + t];
-    for (int t = lane; t < 3 * cnt; t += 32) {
-      s_r[t] = R[3 * j0 + t];
-      s_f[t] = (int)F[3 * j0 + t];
-    }
-    __syncwarp();
-    for (int t = 0; t < cnt; t++) {
-      if (lane == 0) {
-        s_fast = 0;
-        const double s = s_sum;
-        const int E = exp_of(s), E0 = exp_of(s_est[t]);
-        const int k = E - (E0 - 1);
-        if (E > -1000 && E0 > -1000 && k >= 0 && k <= 2 && !s_f[3 * t + k]) {
-          const uint64_t M = (dbits(s) & ((1ull << 52) - 1)) | (1ull << 52);
-          const uint64_t Rj = (uint64_t)s_r[3 * t + k];
-          if (M + Rj < (1ull << 53) - 1) {
-            s_sum = dfrom(((uint64_t)(E + 1023) << 52) | (M + Rj - (1ull << 52)));
-            s_fast = 1;
-          }
-        }
-      }
-      __syncwarp();
-      if (!s_fast) {
-        // element by element, in loop order, skipping exact zeros
-        double v = s_sum;
-        const int64_t base = (j0 + t) * kVolChunk;
-        const int64_t end = base + kVolChunk < n ? base + kVolChunk : n;
-        for (int64_t b = base; b < end; b += 32) {
-          const int64_t q = b + lane;
-          const double x = (q < end) ? c[q] : 0.0;
-          unsigned nz = __ballot_sync(0xffffffffu, x != 0.0);
-          while (nz) {
-            const int l = __ffs(nz) - 1;
-            nz &= nz - 1;
-            v = v + __shfl_sync(0xffffffffu, x, l);
-          }
-        }
-        if (lane == 0) s_sum = v;
-      }
-      __syncwarp();
-    }
+// Inclusive scan of r over the block.  Then, with M the running sum in units of
+// its binade: the first thread that does not apply (bad, or M + its scan
+// reaches the top of the binade), kVolThreads if none, and the scan up to it.
+struct WalkScan {
+  unsigned long long warp_sum[kVolThreads / 32], before;
+  int warp_first[kVolThreads / 32];
+};
+__device__ __forceinline__ int walk_scan(WalkScan& w, unsigned long long r, bool bad, uint64_t M,
+                                         unsigned long long& before) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long incl = r;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
   }
-  if (lane == 0) *out = s_sum;
+  if (lane == 31) w.warp_sum[warp] = incl;
+  __syncthreads();
+  for (int q = 0; q < warp; q++) incl += w.warp_sum[q];
+  const unsigned stop = __ballot_sync(0xffffffffu, bad || M + incl >= (1ull << 53) - 1);
+  if (lane == 0) w.warp_first[warp] = stop ? 32 * warp + __ffs(stop) - 1 : kVolThreads;
+  __syncthreads();
+  int first = kVolThreads;
+  for (int q = 0; q < kVolThreads / 32; q++) first = min(first, w.warp_first[q]);
+  if ((int)threadIdx.x == (first < kVolThreads ? first : kVolThreads - 1)) w.before = first < kVolThreads ? incl - r : incl;
+  __syncthreads();
+  before = w.before;
+  return first;
+}
+
+// the running sum s, in a valid binade, advanced by R units of it
+__device__ __forceinline__ double advance(double s, unsigned long long R) {
+  return R ? dfrom(dbits(s) + R) : s;  // below the binade's top: the significand does not carry
+}
+
+// one block: the exact running sum over the chunks in loop order
+__global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restrict__ c, int64_t n, int64_t nc,
+                                                          const double* __restrict__ est, const int64_t* __restrict__ R,
+                                                          const int64_t* __restrict__ F, bool have_r, double* out) {
+  __shared__ WalkScan w;
+  __shared__ double s_sum;
+  const int t = threadIdx.x;
+  constexpr uint64_t hidden = 1ull << 52;
+  double s = 0.0;  // the same in every thread
+  for (int64_t j = 0; j < nc;) {
+    unsigned long long before;
+    if (have_r) {
+      const int E = exp_of(s);
+      bool ok = true;  // chunks past the end stop nothing
+      unsigned long long r = 0;
+      if (j + t < nc) {
+        const int64_t q = j + t;
+        const int E0 = exp_of(est[q]), k = E - (E0 - 1);
+        ok = E > -1000 && E0 > -1000 && k >= 0 && k <= 2;
+        if (ok) ok = F[3 * q + k] == 0;
+        if (ok) r = (unsigned long long)R[3 * q + k];
+      }
+      const int first = walk_scan(w, r, !ok, E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0, before);
+      s = advance(s, before);
+      j += first;
+      if (first == kVolThreads || j >= nc) continue;
+    }
+    // chunk j, kVolPer consecutive elements per thread
+    double x[kVolPer];
+#pragma unroll
+    for (int q = 0; q < kVolPer; q++) {
+      const int64_t e = j * kVolChunk + (int64_t)t * kVolPer + q;
+      x[q] = e < n ? c[e] : 0.0;
+    }
+    for (int start = 0; start < kVolThreads;) {
+      const int E = exp_of(s);
+      bool bad = false;
+      unsigned long long r = 0;
+      if (t >= start) {
+#pragma unroll
+        for (int q = 0; q < kVolPer; q++) r += rne_units(x[q], E, bad);
+      }
+      const int first = walk_scan(w, r, bad, E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0, before);
+      s = advance(s, before);
+      if (first == kVolThreads) break;
+      if (t == first) {  // element by element, in loop order, skipping exact zeros
+        double v = s;
+#pragma unroll
+        for (int q = 0; q < kVolPer; q++)
+          if (x[q] != 0.0) v = v + x[q];
+        s_sum = v;
+      }
+      __syncthreads();
+      s = s_sum;
+      start = first + 1;
+    }
+    j++;
+  }
+  if (t == 0) *out = s;
 }
 
 }  // namespace
@@ -234,20 +331,42 @@ int64_t loop_sum_scratch_doubles(int64_t n) {
   return 8 * nc + 64;
 }
 
-void launch_loop_sum(cudaStream_t s, const double* c, int64_t n, double* scratch, double* out) {
-  if (n <= 0) {
-    QSS_CK(cudaMemsetAsync(out, 0, sizeof(double), s));
-    return;
-  }
+namespace {
+
+// steps 2 to 4; the chunk sums are in scratch[0, nc) already
+void sum_chunks(cudaStream_t s, const double* c, int64_t n, double* scratch, double* out) {
   const int64_t nc = (n + kVolChunk - 1) / kVolChunk;
   double* csum = scratch;
   double* est = csum + nc;
   int64_t* R = reinterpret_cast<int64_t*>(est + nc);
   int64_t* F = R + 3 * nc;
-  k_vol_chunk_sum<<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum);
-  k_vol_scan<<<1, 1024, 0, s>>>(csum, nc, est);
-  k_vol_chunk_r<<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, est, R, F);
-  k_vol_walk<<<1, 32, 0, s>>>(c, n, nc, est, R, F, out);
+  const bool have_r = nc > kSmallChunks, scanned = nc > kScanChunks;
+  if (scanned) k_vol_scan<<<1, 1024, 0, s>>>(csum, nc, est);
+  if (have_r) k_vol_chunk_r<<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, scanned, est, R, F);
+  k_vol_walk<<<1, kVolThreads, 0, s>>>(c, n, nc, est, R, F, have_r, out);
+}
+
+}  // namespace
+
+void launch_loop_sum(cudaStream_t s, const double* c, int64_t n, double* scratch, double* out) {
+  if (n <= 0) {
+    QSS_CK(cudaMemsetAsync(out, 0, sizeof(double), s));
+    return;
+  }
+  k_vol_chunk_sum<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), kVolThreads, 0, s>>>(c, n, scratch);
+  sum_chunks(s, c, n, scratch, out);
+}
+
+void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, double dy, double dz, double eps,
+                   double* scratch, double* out) {
+  const int64_t n = (int64_t)b.fbx() * b.fby() * b.fbz();
+  if (n <= 0) {
+    QSS_CK(cudaMemsetAsync(out, 0, sizeof(double), s));
+    return;
+  }
+  const double dV = dx * dy * dz;
+  k_vol_contrib<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), 1024, 0, s>>>(b, phi, dV, eps, scratch, scratch + n);
+  sum_chunks(s, scratch, n, scratch + n, out);
 }
 
 }  // namespace qss
