@@ -41,6 +41,7 @@
 
 #include "qss_emu.cuh"
 #include "qss_kernels.cuh"
+#include "qss_stage.cuh"
 
 namespace qss {
 
@@ -801,12 +802,6 @@ __device__ __forceinline__ double godunov5(double vel, const double pp[3], const
   return vel * qss_emu::sqrt(ngps);
 }
 
-// |v| >= 1e-5 (false for NaN)
-__device__ __forceinline__ bool speed_valid(double v) {
-  const uint64_t a = qss_emu::bits(v) & qss_emu::kAbs;
-  return a >= qss_emu::bits(1.e-5) && a <= 0x7ff0000000000000ull;
-}
-
 // central curvature term (3d.f:2337-2379), same operations as curvature()
 // with the exact doublings, the threshold test and the division moved to the
 // integer pipes at EMU >= 1
@@ -934,6 +929,52 @@ __global__ void __launch_bounds__(128, 10) k_weno_combine(CombineArgs a) {
   }
   a.out[idx] = out;
   if (FINAL) a.phi_new[idx] = impose3_e<EMU>(out, idx, a.im);
+}
+
+// The combine kernel at EMU 2 (qss_stage.cuh), same patches and curvature skip.
+// Bound: FP64 pipe (~36 additions where the curvature is taken) and ~1400
+// integer instructions.  512^3 on GB300: 14.29 -> 8.75 ms a launch, 192^3 0.775 ->
+// 0.488 (64 registers, 8 blocks per SM; 10 blocks 8.66 / 0.484 with spills, 64^3
+// 8 % slower; 6 blocks 9.66 / 0.535).
+template <int STAGE, bool FINAL>
+__global__ void __launch_bounds__(128, 8) k_weno_combine2(CombineArgs a) {
+  if (STAGE != 0 && !a.ctl->active) return;
+  const Box& b = a.b;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = b.ilo + blockIdx.x * 32 + 8 * warp + (lane & 7);
+  const int j = b.jlo + blockIdx.y * 4 + (lane >> 3);
+  const int k = b.klo + blockIdx.z;
+  if (i > b.ihi || j > b.jhi || k > b.khi) return;
+  const int64_t idx = b.idx(i, j, k);
+  double pp[3], pm[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    pp[d] = a.dp[d][idx];
+    pm[d] = a.dm[d][idx];
+  }
+  const Inv one{1.0, 1.0, 1.0};
+  const double vel = a.c.vel_n[idx];
+  double rhs;
+  if (speed_valid(vel)) {
+    rhs = godunov_fast<WENO5, false>(vel, pp, pm, one);
+  } else {
+    const int src = a.c.nsrc[idx];
+    rhs = 0.0;
+    if (src >= 0)
+      rhs = godunov_native<WENO5>(a.c.vel_n[src], a.dp[0][src], a.dp[1][src], a.dp[2][src], a.dm[0][src], a.dm[1][src],
+                                  a.dm[2][src], 1.0, 1.0, 1.0);
+  }
+  // b * kappa is +-0 where b is +0, and (normal term + (+-0)) equals (normal
+  // term + 0.0) unless it is -0: there the curvature (finite: its denominator is
+  // at least 1e-5) changes nothing and is skipped
+  const double bco = a.c.b[idx];
+  if (qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign)
+    rhs = rhs + qss_emu::mul(bco, curvature_fast(a.phi_in, b, idx, a.fac));
+  rhs = add_advection<false>(rhs, a.c.vx[idx], a.c.vy[idx], a.c.vz[idx], pp, pm, one);
+  const double out =
+      rk_combine<STAGE>(rhs, STAGE ? a.ctl->dt : 0.0, STAGE ? __ldg(a.phi_in + idx) : 0.0, a.u_cur, idx);
+  a.out[idx] = out;
+  if (FINAL) a.phi_new[idx] = impose3_i(out, idx, a.im);
 }
 
 constexpr int64_t kRingVoxels = 12LL << 20;
@@ -1186,6 +1227,15 @@ void axes_at(cudaStream_t s, const Box& b, const double* phi, const double invs[
   }
 }
 
+void combine_fast(cudaStream_t s, int stage, bool fin, dim3 g, dim3 blk, const CombineArgs& a) {
+  switch (stage) {
+    case 0: k_weno_combine2<0, false><<<g, blk, 0, s>>>(a); break;
+    case 1: if (fin) k_weno_combine2<1, true><<<g, blk, 0, s>>>(a); else k_weno_combine2<1, false><<<g, blk, 0, s>>>(a); break;
+    case 2: if (fin) k_weno_combine2<2, true><<<g, blk, 0, s>>>(a); else k_weno_combine2<2, false><<<g, blk, 0, s>>>(a); break;
+    default: if (fin) k_weno_combine2<3, true><<<g, blk, 0, s>>>(a); else k_weno_combine2<3, false><<<g, blk, 0, s>>>(a); break;
+  }
+}
+
 template <int EMU>
 void combine_at(cudaStream_t s, int stage, bool final_stage, dim3 g, dim3 blk, const CombineArgs& a) {
   switch (stage) {
@@ -1231,7 +1281,10 @@ void launch_weno_combine(cudaStream_t s, int stage, bool final_stage, const Box&
   switch (emu_level()) {
     case 0: combine_at<0>(s, stage, final_stage, g, blk, a); break;
     case 1: combine_at<1>(s, stage, final_stage, g, blk, a); break;
-    default: combine_at<2>(s, stage, final_stage, g, blk, a); break;
+    default:
+      if (stage_factor(a.fac.x) && stage_factor(a.fac.y) && stage_factor(a.fac.z)) combine_fast(s, stage, final_stage, g, blk, a);
+      else combine_at<1>(s, stage, final_stage, g, blk, a);
+      break;
   }
   prof_close(s, e0, kProfCombine);
 }
