@@ -7,12 +7,14 @@
 // That label is a property of the component, not of the visiting order, so a
 // concurrent union-find that keeps the same rule (link the smaller root under
 // the larger, by compare-and-swap on the root) produces identical labels:
-//   1. per 8x8x8 tile, in shared memory: every foreground voxel unites with
-//      its preceding neighbours inside the tile; parent[v] = the global index
-//      of v's tile-local root (0 for background);
-//   2. voxels on a tile face unite, in global memory, with their preceding
-//      neighbours in other tiles (every adjacent pair is a preceding pair
-//      from one side);
+//   1. per tile of 32 x 8 x 8 voxels, in shared memory: the nodes are the runs of
+//      foreground voxels in the tile's 64 rows (one 32-bit mask each), named by
+//      their last voxel; one thread per row and preceding row unites the runs
+//      that touch; parent[v] = the global index of v's tile-local root (0 for
+//      background);
+//   2. across tiles, in global memory: a warp per row segment unites its runs
+//      with those of preceding rows in other tiles, each touching pair once,
+//      and its end voxels with the neighbouring segments;
 //   3. labels[v] = root(v), 0 for background.
 // Every write to parent[] increases it (hooking a root under a larger root,
 // or compressing a node to a larger ancestor), so parent[x] > x holds for
@@ -74,15 +76,24 @@ __device__ __forceinline__ void unite(int* parent, int a, int b, int* err) {
   }
 }
 
-// Tiles of 8 x 8 x 8 voxels: inside a tile the union-find runs in shared
-// memory (same rule: the smaller root is hung under the larger, so the local
-// root is the tile component's largest index, and the local order of a tile
-// is the global linear order restricted to it); then every voxel's global
-// parent is the global index of its local root (depth 1), and only the
-// adjacencies that cross a tile face are united in global memory.
-constexpr int kTile = 8;
-constexpr int kTileN = kTile * kTile * kTile;
-constexpr int kTileThreads = 256;
+// Tile of 32 x 8 x 8 voxels.  Rows r = lj + 8 lk, local index 32 r + li: the
+// local order is the global linear order restricted to the tile, so hanging the
+// smaller root under the larger makes a local root the component's last voxel.
+constexpr int kTileY = 8, kTileZ = 8, kRows = kTileY * kTileZ;
+constexpr int kTileN = 32 * kRows;
+constexpr int kTileThreads = 4 * kRows;  // one per row and preceding row
+
+// the four rows (dj, dk) that precede a row
+__device__ __forceinline__ void back_row(int m, int& dj, int& dk) {
+  dj = m == 3 ? 1 : (m == 2 ? 0 : -1);
+  dk = m == 0 ? 0 : -1;
+}
+
+// last position of the run of ones in `mask` that holds position p
+__device__ __forceinline__ int run_end(unsigned mask, int p) {
+  const unsigned z = ~mask & (0xffffffffu << p);  // zeros from p on
+  return z ? __ffs(z) - 2 : 31;
+}
 
 __device__ __forceinline__ int lfind(int* lp, int x, int* err) {
   int r = x;
@@ -126,143 +137,111 @@ __device__ __forceinline__ void lunite(int* lp, int a, int b, int* err) {
   }
 }
 
-// offsets of the 13 neighbours that precede a voxel in linear order
-__device__ __forceinline__ void back_offset(int m, int& di, int& dj, int& dk) {
-  if (m < 9) {
-    dk = -1;
-    dj = m / 3 - 1;
-    di = m % 3 - 1;
-  } else if (m < 12) {
-    dk = 0;
-    dj = -1;
-    di = m - 10;
-  } else {
-    dk = 0;
-    dj = 0;
-    di = -1;
-  }
-}
-
 // tile-local labelling; writes parent[] for every voxel of the tile
 // (background 0, foreground the global index of its local root)
 __global__ void __launch_bounds__(kTileThreads) k_uf_tile(Box b, const unsigned char* __restrict__ bin, int* parent,
                                                           Ctl* ctl) {
   __shared__ int lp[kTileN];
-  __shared__ unsigned char lb[kTileN];
-  const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, z0 = blockIdx.z * kTile;
+  __shared__ unsigned mask[kRows];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * kTileY, z0 = blockIdx.z * kTileZ;
   int err = 0;
-  for (int l = threadIdx.x; l < kTileN; l += kTileThreads) {
-    const int li = l % kTile, lj = (l / kTile) % kTile, lk = l / (kTile * kTile);
-    const int i = x0 + li, j = y0 + lj, k = z0 + lk;
+  for (int r = warp; r < kRows; r += kTileThreads / 32) {
+    const int i = x0 + lane, j = y0 + r % kTileY, k = z0 + r / kTileY;
     const bool in = i < b.nx && j < b.ny && k < b.nz;
-    const unsigned char v = in ? bin[b.idx(i, j, k)] : 0;
-    lb[l] = v;
-    lp[l] = l;
+    const unsigned m = __ballot_sync(0xffffffffu, in && bin[b.idx(i, j, k)]);
+    if (lane == 0) mask[r] = m;
+    lp[32 * r + lane] = 32 * r + lane;
   }
   __syncthreads();
-  for (int l = threadIdx.x; l < kTileN; l += kTileThreads) {
-    if (!lb[l]) continue;
-    const int li = l % kTile, lj = (l / kTile) % kTile, lk = l / (kTile * kTile);
-#pragma unroll
-    for (int m = 0; m < 13; m++) {
-      int di, dj, dk;
-      back_offset(m, di, dj, dk);
-      const int a = li + di, c = lj + dj, d = lk + dk;
-      if (a < 0 || c < 0 || d < 0 || a >= kTile || c >= kTile) continue;
-      const int l2 = a + kTile * (c + kTile * d);
-      if (lb[l2]) lunite(lp, l, l2, &err);
+  {
+    const int r = threadIdx.x % kRows;
+    int dj, dk;
+    back_row(threadIdx.x / kRows, dj, dk);
+    const int lj = r % kTileY + dj, lk = r / kTileY + dk;
+    if (lj >= 0 && lj < kTileY && lk >= 0) {
+      const int r2 = lj + kTileY * lk;
+      const unsigned B = mask[r2];
+      for (unsigned A = mask[r]; A;) {
+        const int p = __ffs(A) - 1, e = run_end(A, p);
+        const unsigned from_p = 0xffffffffu << p, to_e = 0xffffffffu >> (31 - e);
+        A &= ~to_e;
+        // the runs of B within one position of [p, e]
+        for (unsigned W = B & (from_p | (from_p >> 1)) & (to_e | (to_e << 1)); W;) {
+          const int e2 = run_end(B, __ffs(W) - 1);
+          lunite(lp, 32 * r + e, 32 * r2 + e2, &err);
+          W &= ~(0xffffffffu >> (31 - e2));
+        }
+      }
     }
   }
   __syncthreads();
-  for (int l = threadIdx.x; l < kTileN; l += kTileThreads) {
-    const int li = l % kTile, lj = (l / kTile) % kTile, lk = l / (kTile * kTile);
-    const int i = x0 + li, j = y0 + lj, k = z0 + lk;
+  for (int r = warp; r < kRows; r += kTileThreads / 32) {
+    const int i = x0 + lane, j = y0 + r % kTileY, k = z0 + r / kTileY;
     if (i >= b.nx || j >= b.ny || k >= b.nz) continue;
     int g = 0;
-    if (lb[l]) {
-      const int r = lfind(lp, l, &err);
-      const int ri = r % kTile, rj = (r / kTile) % kTile, rk = r / (kTile * kTile);
-      g = (int)b.idx(x0 + ri, y0 + rj, z0 + rk);
+    if (mask[r] >> lane & 1u) {
+      const int root = lfind(lp, 32 * r + run_end(mask[r], lane), &err);
+      const int rr = root / 32;
+      g = (int)b.idx(x0 + root % 32, y0 + rr % kTileY, z0 + rr / kTileY);
     }
     parent[b.idx(i, j, k)] = g;
   }
   if (err && ctl) atomicOr(&ctl->err, err);
 }
 
-// unions across tile faces: each voxel on a face of its tile with its
-// preceding neighbours in other tiles.  Neighbouring voxels mostly join the
-// same two tile components, so the lanes of a warp first agree on distinct
-// (parent, parent) pairs and only one lane per pair unites them (the parents
-// are in the same sets as the voxels).
-// Preceding offsets have di, dj in {-1, 0, 1} and dk in {-1, 0}, so only the
-// voxels of the tile's bottom plane (lk = 0) and of the ring li or lj in
-// {0, kTile-1} of every other plane have one outside the tile: 64 + 7 x 28 =
-// 260 of the 512.  face_voxel(f) enumerates them.
-constexpr int kFaceN = kTile * kTile + (kTile - 1) * 4 * (kTile - 1);
-
-__device__ __forceinline__ void face_voxel(int f, int& li, int& lj, int& lk) {
-  if (f < kTile * kTile) {
-    lk = 0;
-    li = f % kTile;
-    lj = f / kTile;
-    return;
+// The unions across tiles.  Given that voxels next to each other in a row are
+// united (in a tile by the runs, across tiles by lane 0 here), a row's voxel x and
+// the row before's voxels x-1, x, x+1 need one union where B[x] is set and the row
+// has no voxel x-1 (which would touch B[x] itself), and where B[x] is not set one
+// with B[x-1] under the same condition and one with B[x+1]: every pair of
+// touching runs once.  Lanes of a warp that join the same two tile components
+// agree on one of them (the parents are in the same sets as the voxels).
+__device__ __forceinline__ void unite_lanes(int* parent, bool pair, int64_t q, int64_t q2, int* err) {
+  if (!__any_sync(0xffffffffu, pair)) return;
+  const unsigned lane = threadIdx.x & 31u;
+  int ra = -1, rb = -1;
+  if (pair) {
+    ra = __ldcg(parent + q);
+    rb = __ldcg(parent + q2);
+    pair = ra != rb;
   }
-  const int g = f - kTile * kTile, ring = 4 * (kTile - 1);
-  lk = 1 + g / ring;
-  const int r = g % ring;
-  if (r < kTile) {
-    lj = 0;
-    li = r;
-  } else if (r < 2 * kTile) {
-    lj = kTile - 1;
-    li = r - kTile;
-  } else if (r < 3 * kTile - 2) {
-    li = 0;
-    lj = 1 + (r - 2 * kTile);
-  } else {
-    li = kTile - 1;
-    lj = 1 + (r - (3 * kTile - 2));
-  }
+  const unsigned lo = (unsigned)(ra < rb ? ra : rb), hi = (unsigned)(ra < rb ? rb : ra);
+  const unsigned long long key = pair ? (((unsigned long long)lo << 32) | hi) : (0xffffffff00000000ull | lane);
+  const unsigned peers = __match_any_sync(0xffffffffu, key);
+  if (pair && (unsigned)(__ffs(peers) - 1) == lane) unite(parent, ra, rb, err);
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_uf_cross(Box b, const unsigned char* __restrict__ bin, int* parent,
-                                                           Ctl* ctl) {
-  const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, z0 = blockIdx.z * kTile;
-  const unsigned lane = threadIdx.x & 31u;
+__global__ void __launch_bounds__(256) k_uf_cross(Box b, const unsigned char* __restrict__ bin, int* parent, Ctl* ctl) {
+  const int lane = threadIdx.x & 31;
+  const int x = blockIdx.x * 32 + lane, j = blockIdx.y * 8 + (threadIdx.x >> 5), k = blockIdx.z;
+  if (j >= b.ny) return;  // warp-uniform
+  const int64_t row = b.idx(0, j, k), q = row + x;
   int err = 0;
-  // the tile's face voxels, one per thread (warp-uniform loop: a warp runs a
-  // round while its first voxel exists)
-  for (int base = threadIdx.x - (int)lane; base < kFaceN; base += kTileThreads) {
-    const int l = base + (int)lane;
-    int li = 0, lj = 0, lk = 0;
-    if (l < kFaceN) face_voxel(l, li, lj, lk);
-    const int i = x0 + li, j = y0 + lj, k = z0 + lk;
-    const bool in = l < kFaceN && i < b.nx && j < b.ny && k < b.nz;
-    const int64_t q = in ? b.idx(i, j, k) : 0;
-    const bool fg = in && bin[q];
-#pragma unroll 1
-    for (int m = 0; m < 13; m++) {
-      int di, dj, dk;
-      back_offset(m, di, dj, dk);
-      int ra = -1, rb = -1;
-      if (fg) {
-        const int a = li + di, c = lj + dj, d = lk + dk;
-        const bool other_tile = !(a >= 0 && c >= 0 && d >= 0 && a < kTile && c < kTile);
-        const int i2 = i + di, j2 = j + dj, k2 = k + dk;
-        if (other_tile && i2 >= 0 && j2 >= 0 && k2 >= 0 && i2 < b.nx && j2 < b.ny) {
-          const int64_t q2 = b.idx(i2, j2, k2);
-          if (bin[q2]) {
-            ra = __ldcg(parent + q);
-            rb = __ldcg(parent + q2);
-          }
-        }
+  const bool fg = x < b.nx && bin[q];
+  const unsigned A = __ballot_sync(0xffffffffu, fg);
+  if (A) {
+    const bool left_a = lane == 0 && x > 0 && bin[q - 1];
+    const unsigned has_left = __ballot_sync(0xffffffffu, left_a) & 1u;  // A[x-1] of lane 0
+    const bool prev = lane ? (A >> (lane - 1)) & 1u : has_left;
+    unite_lanes(parent, fg && left_a, q, q - 1, &err);
+    for (int m = 0; m < 4; m++) {
+      int dj, dk;
+      back_row(m, dj, dk);
+      const int j2 = j + dj, k2 = k + dk;
+      if (j2 < 0 || j2 >= b.ny || k2 < 0) continue;  // warp-uniform
+      const bool same = j2 / kTileY == j / kTileY && k2 / kTileZ == k / kTileZ;
+      const int64_t q2 = b.idx(0, j2, k2) + x;
+      // within a tile only the end lanes look across; elsewhere every lane
+      const bool look = fg && (!same || lane == 0 || lane == 31);
+      const bool c1 = look && bin[q2];
+      bool c0 = look && x > 0 && bin[q2 - 1], c2 = look && x + 1 < b.nx && bin[q2 + 1];
+      if (same) {
+        c0 = c0 && lane == 0;
+        c2 = c2 && lane == 31;
       }
-      const bool pair = ra >= 0 && ra != rb;
-      const unsigned lo = (unsigned)(ra < rb ? ra : rb), hi = (unsigned)(ra < rb ? rb : ra);
-      const unsigned long long key =
-          pair ? (((unsigned long long)lo << 32) | hi) : (0xffffffff00000000ull | lane);
-      const unsigned peers = __match_any_sync(0xffffffffu, key);
-      if (pair && (unsigned)(__ffs(peers) - 1) == lane) unite(parent, ra, rb, &err);
+      unite_lanes(parent, look && !prev && ((c1 && !same) || (!c1 && c0)), q, c1 ? q2 : q2 - 1, &err);
+      unite_lanes(parent, look && !c1 && c2, q, q2 + 1, &err);
     }
   }
   if (err && ctl) atomicOr(&ctl->err, err);
@@ -375,9 +354,10 @@ unsigned grid_for(int64_t n) {
 
 void launch_label(cudaStream_t s, const Box& b, const unsigned char* bin, int* labels, Ctl* ctl) {
   const int64_t n = b.npts();
-  const dim3 tiles((b.nx + kTile - 1) / kTile, (b.ny + kTile - 1) / kTile, (b.nz + kTile - 1) / kTile);
+  const unsigned seg = (unsigned)((b.nx + 31) / 32);
+  const dim3 tiles(seg, (b.ny + kTileY - 1) / kTileY, (b.nz + kTileZ - 1) / kTileZ);
   k_uf_tile<<<tiles, kTileThreads, 0, s>>>(b, bin, labels, ctl);
-  k_uf_cross<<<tiles, kTileThreads, 0, s>>>(b, bin, labels, ctl);
+  k_uf_cross<<<dim3(seg, (b.ny + 7) / 8, b.nz), 256, 0, s>>>(b, bin, labels, ctl);
   k_uf_final<<<grid_for(n), 256, 0, s>>>(n, bin, labels, ctl);
 }
 
