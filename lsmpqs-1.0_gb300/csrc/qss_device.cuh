@@ -277,9 +277,12 @@ __device__ __forceinline__ double curvature(const double* __restrict__ phi, cons
 // values: the value stored at a ghost point equals the one the sequential
 // face sweeps would leave there.
 __device__ __forceinline__ double extrap(double f, double g, int dist) {
-  double s = copysign(1.0, f);
-  double slope = s * fabs(f - g);
-  return f + slope * (double)dist;
+  // slope = sign(f) |f - g|, the sign carried over in the high word
+  const double d = f - g;
+  const double slope = __hiloint2double((__double2hiint(d) & 0x7fffffff) | (__double2hiint(f) & 0x80000000),
+                                        __double2loint(d));
+  if (dist == 1) return f + slope;
+  return f + slope * (dist == 2 ? 2.0 : (dist == 3 ? 3.0 : (double)dist));
 }
 
 // value after the x faces at (i, j, k) with j, k inside the fill box

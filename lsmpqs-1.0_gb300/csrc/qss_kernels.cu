@@ -31,31 +31,98 @@ inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t
 // ---------------------------------------------------------------------------
 // inner step: dt
 
-template <int SCHEME, bool VAR>
-__global__ void k_dt(Box b, const double* __restrict__ phi, Coef c, int nslabs, double dx, double dy,
-                     double dz, Ctl* ctl) {
-  __shared__ double sh[32];
-  if (!ctl->active) return;
-  const Inv inv{1.0 / dx, 1.0 / dy, 1.0 / dz};
-  const int t = threadIdx.x;
-  double h = -1.0;
-  if (t < nslabs) {
-    int ns = b.khi - b.klo + 1;
-    int k = b.klo + (int)(((int64_t)ns * (t + 1)) / nslabs) - 1;
-    if (k > b.khi) k = b.khi;
-    int i = b.ihi, j = b.jhi;
-    double pp[3], pm[3];
-    upwind<SCHEME>(phi, b, i, j, k, inv, pp, pm);
-    double vel = VAR ? c.vel_n[b.idx(i, j, k)] : c.a_const;
-    h = cfl_h(vel, pp, pm, dx, dy, dz, inv);
+// weno5_side() with its products and divisions on the integer pipes, which here
+// are the lower latency
+__device__ __forceinline__ double weno5_side_e(double v1, double v2, double v3, double v4, double v5) {
+  using namespace qss_emu;
+  auto sq = [](double x) { return mul(x, x); };
+  const double m = dmax(dmax(dmax(dmax(sq(v1), sq(v2)), sq(v3)), sq(v4)), sq(v5));
+  const double eps = mul(1e-6, m) + 1.0e-35;
+  const double p1 = mul(1.0 / 3.0, v1) - mul(7.0 / 6.0, v2) + mul(11.0 / 6.0, v3);
+  const double p2 = -mul(1.0 / 6.0, v2) + mul(5.0 / 6.0, v3) + mul(1.0 / 3.0, v4);
+  const double p3 = mul(1.0 / 3.0, v3) + mul(5.0 / 6.0, v4) - mul(1.0 / 6.0, v5);
+  const double k1312 = 13.0 / 12.0;
+  const double S1 = mul(k1312, sq(v1 - scale2(v2, 1) + v3)) + scale2(sq(v1 - scale2(v2, 2) + mul(3.0, v3)), -2);
+  const double S2 = mul(k1312, sq(v2 - scale2(v3, 1) + v4)) + scale2(sq(v2 - v4), -2);
+  const double S3 = mul(k1312, sq(v3 - scale2(v4, 1) + v5)) + scale2(sq(mul(3.0, v3) - scale2(v4, 2) + v5), -2);
+  double a1 = div(0.1, sq(S1 + eps)), a2 = div(0.6, sq(S2 + eps)), a3 = div(0.3, sq(S3 + eps));
+  const double r = div(1.0, a1 + a2 + a3);
+  a1 = mul(a1, r);
+  a2 = mul(a2, r);
+  a3 = mul(a3, r);
+  return mul(a1, p1) + mul(a2, p2) + mul(a3, p3);
+}
+
+// one of the six one-sided derivatives of upwind(): axis 0..2, plus or minus
+template <int SCHEME>
+__device__ __forceinline__ double upwind_one(const double* __restrict__ phi, const Box& b, int i, int j, int k,
+                                             const Inv& inv, int axis, bool plus) {
+  const int64_t c = b.idx(i, j, k), st = axis == 0 ? 1 : (axis == 1 ? b.sy() : b.sz());
+  const double iv = axis == 0 ? inv.x : (axis == 1 ? inv.y : inv.z);
+  double p, m;
+  if (SCHEME == ENO2) {
+    double s[5];
+#pragma unroll
+    for (int o = -2; o <= 2; o++) s[o + 2] = __ldg(phi + c + o * st);
+    eno2_pm(s, iv, p, m);
+  } else if (SCHEME == ENO3) {
+    double s[7];
+#pragma unroll
+    for (int o = -3; o <= 3; o++) s[o + 3] = __ldg(phi + c + o * st);
+    if (axis == 0) s[6] = __ldg(phi + b.idx(i + 3, j, j));  // 3d.f:677
+    eno3_pm(s, iv, inv.x, p, m);
+  } else {
+    // v1..v5: faces i+3 .. i-1 (plus), i-2 .. i+2 (minus)
+    const int64_t d = plus ? -st : st;
+    const double* q = phi + c + (plus ? 3 * st : -2 * st);  // upper point of face v1
+    double v[5];
+#pragma unroll
+    for (int o = 0; o < 5; o++) v[o] = qss_emu::mul(__ldg(q + o * d) - __ldg(q + o * d - st), iv);
+    return weno5_side_e(v[0], v[1], v[2], v[3], v[4]);
   }
-  // max over slabs (the reference's critical section), -1 if none
-  for (int o = 16; o > 0; o >>= 1) h = dmax(h, __shfl_down_sync(0xffffffffu, h, o));
-  if ((t & 31) == 0) sh[t >> 5] = h;
+  return plus ? p : m;
+}
+
+// cfl_h() from the larger one-sided magnitudes
+__device__ __forceinline__ double cfl_h_e(double vel, double pxc, double pyc, double pzc, double dx, double dy,
+                                          double dz, const Inv& inv) {
+  using namespace qss_emu;
+  const double mdx = dmax(dmax(dx, dy), dz);
+  const double ngp = qss_emu::sqrt(mul(pxc, pxc) + mul(pyc, pyc) + mul(pzc, pzc) + mul(mdx, mdx));
+  return mul(div(qss_emu::abs(vel), ngp), mul(pxc, inv.x) + mul(pyc, inv.y) + mul(pzc, inv.z));
+}
+
+// One group of 8 lanes per slab, one lane per one-sided derivative: the step's
+// time is this kernel's latency (one thread computing all six with native
+// divisions took 28 us for WENO5, 8 us for ENO2).
+constexpr int kDtThreads = 256;
+
+template <int SCHEME, bool VAR>
+__global__ void __launch_bounds__(kDtThreads) k_dt(Box b, const double* __restrict__ phi, Coef c, int nslabs, double dx,
+                                                   double dy, double dz, Inv inv, Ctl* ctl) {
+  __shared__ double hs[1024];  // nslabs <= 1024
+  if (!ctl->active) return;
+  const int l = threadIdx.x & 7;
+  for (int t0 = 0; t0 < nslabs; t0 += blockDim.x >> 3) {
+    const int t = t0 + (threadIdx.x >> 3);
+    const int ts = t < nslabs ? t : nslabs - 1;
+    const int ns = b.khi - b.klo + 1;
+    int k = b.klo + (int)(((int64_t)ns * (ts + 1)) / nslabs) - 1;
+    if (k > b.khi) k = b.khi;
+    const int i = b.ihi, j = b.jhi;
+    const double d = l < 6 ? upwind_one<SCHEME>(phi, b, i, j, k, inv, l >> 1, (l & 1) == 0) : 0.0;
+    const double a = qss_emu::abs(d);
+    const double o = __shfl_xor_sync(0xffffffffu, a, 1);
+    const double mx = (l & 1) == 0 ? dmax(a, o) : dmax(o, a);  // dmax(|plus|, |minus|)
+    const double py = __shfl_down_sync(0xffffffffu, mx, 2, 8), pz = __shfl_down_sync(0xffffffffu, mx, 4, 8);
+    if (l == 0 && t < nslabs)
+      hs[t] = cfl_h_e(VAR ? c.vel_n[b.idx(i, j, k)] : c.a_const, mx, py, pz, dx, dy, dz, inv);
+  }
   __syncthreads();
-  if (t == 0) {
-    double m = -1.0;
-    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); w++) m = dmax(m, sh[w]);
+  if (threadIdx.x == 0) {
+    // max over slabs (the reference's critical section), -1 if none
+    double cur = -1.0;
+    for (int t = 0; t < nslabs; t++) cur = qss_emu::gt(hs[t], cur) ? hs[t] : cur;
     // loop condition of constCurvModel3d.c:127, evaluated before the step
     bool go = ctl->dt_sub < ctl->tplot;
     if (ctl->max_steps > 0 && ctl->steps >= ctl->max_steps) go = false;
@@ -63,9 +130,7 @@ __global__ void k_dt(Box b, const double* __restrict__ phi, Coef c, int nslabs, 
       ctl->active = 0;
       return;
     }
-    double cur = -1.0;
-    if (m > cur) cur = m;
-    double dt = 0.5 / (cur + ctl->b_max_over_dx + ctl->max_U_over_dx);
+    double dt = qss_emu::div(0.5, cur + ctl->b_max_over_dx + ctl->max_U_over_dx);
     ctl->cur_max_H = cur;
     ctl->dt = dt;
     ctl->dt_sub = ctl->dt_sub + dt;
@@ -274,46 +339,77 @@ __global__ void k_cfl_at(Box b, const double* __restrict__ phi, Coef c, int i, i
 // ---------------------------------------------------------------------------
 // ghost layers
 
-__global__ void k_ghost(Box b, double* a, double* phi_new, ImposeArgs im, const Ctl* ctl) {
+// bc_xyz() of qss_device.cuh for a warp's points at once: each axis has the nearest
+// fill-box index f, the one behind it g and the distance d (0 inside).  The axes
+// some lane of the warp lies outside of are found by votes, all loads they need
+// are issued together, then the extrapolations follow x, y, z.  (Point by point
+// with branches the loads came one after the other: 8 us at 24^3.)  32-bit
+// indices: the ghost box is below 2^31 points.
+struct GhostAxis {
+  int f, g, d;
+};
+__device__ __forceinline__ GhostAxis ghost_axis(int i, int lo, int hi) {
+  if (i < lo) return GhostAxis{lo, lo + 1, lo - i};
+  if (i > hi) return GhostAxis{hi, hi - 1, i - hi};
+  return GhostAxis{i, i, 0};
+}
+__device__ __forceinline__ double extrap_if(double f, double g, int d) { return d ? extrap(f, g, d) : f; }
+
+__global__ void __launch_bounds__(256) k_ghost(Box b, double* a, double* phi_new, ImposeArgs im, const Ctl* ctl) {
   if (ctl && !ctl->active) return;
-  const int64_t nxy = (int64_t)b.nx * b.ny;
-  const int nzg = b.klo + (b.nz - 1 - b.khi);    // z-ghost planes
-  const int nyg = b.jlo + (b.ny - 1 - b.jhi);    // y-ghost rows per plane
-  const int nxg = b.ilo + (b.nx - 1 - b.ihi);    // x-ghost points per row
-  const int64_t nz_cells = (int64_t)nzg * nxy;
-  const int64_t ny_cells = (int64_t)b.fbz() * nyg * b.nx;
-  const int64_t nx_cells = (int64_t)b.fbz() * b.fby() * nxg;
-  const int64_t total = nz_cells + ny_cells + nx_cells;
-  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-       q += (int64_t)gridDim.x * blockDim.x) {
+  const uint32_t nx = b.nx, nxy = (uint32_t)b.nx * b.ny;
+  const uint32_t nzg = b.klo + (b.nz - 1 - b.khi);  // z-ghost planes
+  const uint32_t nyg = b.jlo + (b.ny - 1 - b.jhi);  // y-ghost rows per plane
+  const uint32_t nxg = b.ilo + (b.nx - 1 - b.ihi);  // x-ghost points per row
+  const uint32_t nz_cells = nzg * nxy;
+  const uint32_t ny_cells = b.fbz() * nyg * nx;
+  const uint32_t total = nz_cells + ny_cells + (uint32_t)b.fbz() * b.fby() * nxg;
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t q0 = blockIdx.x * blockDim.x + threadIdx.x - lane; q0 < total; q0 += gridDim.x * blockDim.x) {
+    // lanes past the end repeat the last point and store nothing
+    const uint32_t q = q0 + lane < total ? q0 + lane : total - 1;
     int i, j, k;
     if (q < nz_cells) {
-      int p = (int)(q / nxy);
-      int64_t r = q - (int64_t)p * nxy;
-      k = (p < b.klo) ? p : b.khi + 1 + (p - b.klo);
-      j = (int)(r / b.nx);
-      i = (int)(r - (int64_t)j * b.nx);
+      const uint32_t row = q / nx, p = row / (uint32_t)b.ny;
+      i = (int)(q - row * nx);
+      j = (int)(row - p * b.ny);
+      k = (int)p < b.klo ? (int)p : b.khi + 1 + ((int)p - b.klo);
     } else if (q < nz_cells + ny_cells) {
-      int64_t r = q - nz_cells;
-      int64_t per = (int64_t)nyg * b.nx;
-      k = b.klo + (int)(r / per);
-      r -= (int64_t)(k - b.klo) * per;
-      int p = (int)(r / b.nx);
-      i = (int)(r - (int64_t)p * b.nx);
-      j = (p < b.jlo) ? p : b.jhi + 1 + (p - b.jlo);
+      const uint32_t r = q - nz_cells, row = r / nx, pl = row / nyg;
+      const int p = (int)(row - pl * nyg);
+      i = (int)(r - row * nx);
+      k = b.klo + (int)pl;
+      j = p < b.jlo ? p : b.jhi + 1 + (p - b.jlo);
     } else {
-      int64_t r = q - nz_cells - ny_cells;
-      int64_t per = (int64_t)b.fby() * nxg;
-      k = b.klo + (int)(r / per);
-      r -= (int64_t)(k - b.klo) * per;
-      j = b.jlo + (int)(r / nxg);
-      int p = (int)(r - (int64_t)(j - b.jlo) * nxg);
-      i = (p < b.ilo) ? p : b.ihi + 1 + (p - b.ilo);
+      const uint32_t r = q - nz_cells - ny_cells, row = r / nxg, pl = row / (uint32_t)b.fby();
+      const int p = (int)(r - row * nxg);
+      k = b.klo + (int)pl;
+      j = b.jlo + (int)(row - pl * b.fby());
+      i = p < b.ilo ? p : b.ihi + 1 + (p - b.ilo);
     }
-    const double v = bc_xyz(a, b, i, j, k);
-    const int64_t idx = b.idx(i, j, k);
-    a[idx] = v;
-    if (phi_new && k >= b.klo - 3 && k <= b.khi + 3) phi_new[idx] = impose3(v, idx, im);
+    const GhostAxis x = ghost_axis(i, b.ilo, b.ihi), y = ghost_axis(j, b.jlo, b.jhi), z = ghost_axis(k, b.klo, b.khi);
+    const bool ox = __any_sync(0xffffffffu, x.d), oy = __any_sync(0xffffffffu, y.d), oz = __any_sync(0xffffffffu, z.d);
+    double v[2][2][2];  // z, y, x: f, g
+#pragma unroll
+    for (int m = 0; m < 8; m++) {
+      const bool gx = m & 1, gy = m & 2, gz = m & 4;
+      if ((!gx || ox) && (!gy || oy) && (!gz || oz))
+        v[gz][gy][gx] = a[b.idx(gx ? x.g : x.f, gy ? y.g : y.f, gz ? z.g : z.f)];
+    }
+#pragma unroll
+    for (int gz = 0; gz < 2; gz++) {
+      if (gz && !oz) break;
+#pragma unroll
+      for (int gy = 0; gy < 2; gy++)
+        if ((!gy || oy) && ox) v[gz][gy][0] = extrap_if(v[gz][gy][0], v[gz][gy][1], x.d);
+      if (oy) v[gz][0][0] = extrap_if(v[gz][0][0], v[gz][1][0], y.d);
+    }
+    const double r = oz ? extrap_if(v[0][0][0], v[1][0][0], z.d) : v[0][0][0];
+    if (q0 + lane < total) {
+      const int64_t idx = b.idx(i, j, k);
+      a[idx] = r;
+      if (phi_new && k >= b.klo - 3 && k <= b.khi + 3) phi_new[idx] = impose3_i(r, idx, im);
+    }
   }
 }
 
@@ -1125,9 +1221,8 @@ static unsigned grid1(int64_t n) {
 
 void launch_dt(cudaStream_t s, int scheme, bool var, const Box& b, const double* phi, const Coef& c, int nslabs,
                double dx, double dy, double dz, Ctl* ctl) {
-  int threads = ((nslabs + 31) / 32) * 32;
-  if (threads < 32) threads = 32;
-#define QSS_DT(S, V) k_dt<S, V><<<1, threads, 0, s>>>(b, phi, c, nslabs, dx, dy, dz, ctl)
+  const Inv inv{1.0 / dx, 1.0 / dy, 1.0 / dz};
+#define QSS_DT(S, V) k_dt<S, V><<<1, nslabs <= 4 ? 32 : kDtThreads, 0, s>>>(b, phi, c, nslabs, dx, dy, dz, inv, ctl)
   if (scheme == ENO2) { if (var) QSS_DT(ENO2, true); else QSS_DT(ENO2, false); }
   else if (scheme == ENO3) { if (var) QSS_DT(ENO3, true); else QSS_DT(ENO3, false); }
   else { if (var) QSS_DT(WENO5, true); else QSS_DT(WENO5, false); }

@@ -106,57 +106,95 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_sum(const double* __r
   if (threadIdx.x == 0) csum[blockIdx.x] = red[0];
 }
 
-// contribution of each fill-box voxel in loop order (i fastest), and the
-// chunk's sum; one voxel in the smoothing band costs a division and a sine, any
-// other an integer comparison
-__global__ void __launch_bounds__(1024) k_vol_contrib(Box b, const double* __restrict__ phi, double dV, double eps,
-                                                      double* contrib, double* csum) {
-  __shared__ float red[32];
+// contribution of each fill-box voxel in loop order (i fastest), and the sum of
+// each quarter chunk.  A voxel outside the smoothing band costs an
+// integer comparison; those inside (about 15 % of the voxels, but a lane or more
+// of most warps) are first gathered, then evaluated by full warps: their division
+// and sine are ~45 FP64 instructions and the kernel's bound.  Blocks of 1024
+// voxels, so that small boxes use more SMs (24^3 49 us with whole chunks).
+constexpr int kContribVoxels = 1024, kContribThreads = 256;
+
+__global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const double* __restrict__ phi, double dV,
+                                                                 double eps, double* contrib, float* csum) {
+  __shared__ double band_p[kContribVoxels];
+  __shared__ uint32_t band_q[kContribVoxels];
+  __shared__ int band_n;
+  __shared__ float red[kContribThreads / 32];
   const double pi = 3.14159265358979323846;
   const double one_over_pi = 0.31830988618379;
   const uint32_t n = (uint32_t)b.fbx() * b.fby() * b.fbz();  // below 2^31
-  const uint32_t base = blockIdx.x * (uint32_t)kVolChunk;
-  float sum = 0.0f;
-  for (uint32_t t = threadIdx.x; t < kVolChunk; t += 1024) {
-    const uint32_t q = base + t;
-    if (q >= n) break;
-    const uint32_t r = q / (uint32_t)b.fbx();
-    const int i = b.ilo + (int)(q - r * (uint32_t)b.fbx());
-    const int k = b.klo + (int)(r / (uint32_t)b.fby());
-    const int j = b.jlo + (int)(r - (uint32_t)(k - b.klo) * (uint32_t)b.fby());
-    const double p = phi[b.idx(i, j, k)];
-    double v = 0.0;
-    if (qss_emu::gt(-eps, p)) {  // p < -eps
-      v = dV;
-    } else if (qss_emu::gt(eps, p)) {  // p < eps
-      const double rr = p / eps;
-      const double one_minus_H = 0.5 * (1 - rr - one_over_pi * portable_sin(pi * rr));
-      v = one_minus_H * dV;
-    }
-    contrib[q] = v;
-    // v as a float by its bits (a conversion is an FP64 instruction); values
-    // outside the float range do not matter for the estimate
+  const uint32_t base = blockIdx.x * (uint32_t)kContribVoxels;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) band_n = 0;
+  __syncthreads();
+  // a value as a float by its bits (a conversion is an FP64 instruction); values
+  // outside the float range do not matter for the estimate
+  auto approx = [](double v) {
     const uint32_t h = qss_emu::hi32(v);
-    if (h - 0x38100000u < 0x0fe00000u) sum += __uint_as_float((h - 0x38000000u) << 3);
+    return h - 0x38100000u < 0x0fe00000u ? __uint_as_float((h - 0x38000000u) << 3) : 0.0f;
+  };
+  float sum = 0.0f;
+#pragma unroll
+  for (int t = 0; t < kContribVoxels; t += kContribThreads) {
+    const uint32_t q = base + t + threadIdx.x;
+    bool band = false;
+    double p = 0.0;
+    if (q < n) {
+      const uint32_t r = q / (uint32_t)b.fbx();
+      const int i = b.ilo + (int)(q - r * (uint32_t)b.fbx());
+      const int k = b.klo + (int)(r / (uint32_t)b.fby());
+      const int j = b.jlo + (int)(r - (uint32_t)(k - b.klo) * (uint32_t)b.fby());
+      p = phi[b.idx(i, j, k)];
+      const bool inside = qss_emu::gt(-eps, p);  // p < -eps
+      band = !inside && qss_emu::gt(eps, p);     // p < eps
+      if (!band) contrib[q] = inside ? dV : 0.0;
+      if (inside) sum += approx(dV);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, band);
+    int at = 0;
+    if (lane == 0 && m) at = atomicAdd(&band_n, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
+    if (band) {
+      band_p[at] = p;
+      band_q[at] = q;
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < band_n; t += kContribThreads) {
+    const double rr = band_p[t] / eps;
+    const double one_minus_H = 0.5 * (1 - rr - one_over_pi * portable_sin(pi * rr));
+    const double v = one_minus_H * dV;
+    contrib[band_q[t]] = v;
+    sum += approx(v);
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  if (lane == 0) red[threadIdx.x >> 5] = sum;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    sum = red[threadIdx.x];
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-    if (threadIdx.x == 0) csum[blockIdx.x] = (double)sum;
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kContribThreads / 32; w++) sum += red[w];
+    csum[blockIdx.x] = sum;
   }
 }
 
+// the estimate of chunk j's sum from PER partial sums (past np: none)
+template <typename T, int PER>
+__device__ __forceinline__ double chunk_estimate(const T* __restrict__ csum, int64_t np, int64_t j) {
+  double s = 0;
+#pragma unroll
+  for (int q = 0; q < PER; q++)
+    if (PER * j + q < np) s += (double)csum[PER * j + q];
+  return s;
+}
+
 // exclusive scan of nc chunk sums in one block of 1024 threads
-__global__ void __launch_bounds__(1024) k_vol_scan(const double* __restrict__ csum, int64_t nc, double* est) {
+template <typename T, int PER>
+__global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, int64_t np, int64_t nc, double* est) {
   __shared__ double part[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t per = (nc + 1023) / 1024;
   const int64_t lo = threadIdx.x * per, hi = lo + per < nc ? lo + per : nc;
   double s = 0;
-  for (int64_t j = lo; j < hi; j++) s += csum[j];
+  for (int64_t j = lo; j < hi; j++) s += chunk_estimate<T, PER>(csum, np, j);
   double incl = s;
   for (int o = 1; o < 32; o <<= 1) {
     const double x = __shfl_up_sync(0xffffffffu, incl, o);
@@ -168,14 +206,15 @@ __global__ void __launch_bounds__(1024) k_vol_scan(const double* __restrict__ cs
   for (int w = 0; w < warp; w++) run += part[w];
   for (int64_t j = lo; j < hi; j++) {
     est[j] = run;
-    run += csum[j];
+    run += chunk_estimate<T, PER>(csum, np, j);
   }
 }
 
 // R[3j+q], F[3j+q] for E = exp(est[j]) - 1 + q
+template <typename T, int PER>
 __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __restrict__ c, int64_t n,
-                                                             const double* __restrict__ csum, bool scanned, double* est,
-                                                             int64_t* R, int64_t* F) {
+                                                             const T* __restrict__ csum, int64_t np, bool scanned,
+                                                             double* est, int64_t* R, int* F) {
   __shared__ unsigned long long rs[3][kVolThreads];
   __shared__ int fs[3][kVolThreads];
   __shared__ double s_est[kVolThreads / 32];
@@ -184,7 +223,7 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __res
   if (scanned) {
     e = est[j];
   } else {
-    for (int64_t q = threadIdx.x; q < j; q += kVolThreads) e += csum[q];
+    for (int64_t q = threadIdx.x; q < PER * j; q += kVolThreads) e += (double)csum[q];
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
     if ((threadIdx.x & 31) == 0) s_est[threadIdx.x >> 5] = e;
     __syncthreads();
@@ -266,9 +305,10 @@ __device__ __forceinline__ double advance(double s, unsigned long long R) {
 // one block: the exact running sum over the chunks in loop order
 __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restrict__ c, int64_t n, int64_t nc,
                                                           const double* __restrict__ est, const int64_t* __restrict__ R,
-                                                          const int64_t* __restrict__ F, bool have_r, double* out) {
+                                                          const int* __restrict__ F, bool have_r, double* out) {
   __shared__ WalkScan w;
   __shared__ double s_sum;
+  __shared__ double x[kVolChunk];
   const int t = threadIdx.x;
   constexpr uint64_t hidden = 1ull << 52;
   double s = 0.0;  // the same in every thread
@@ -290,34 +330,42 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restri
       j += first;
       if (first == kVolThreads || j >= nc) continue;
     }
-    // chunk j, kVolPer consecutive elements per thread
-    double x[kVolPer];
+    // chunk j: windows of kVolThreads * per consecutive elements, per of them to a
+    // thread.  The sum takes about as many elements again to leave a binade as it
+    // took to enter it, so per grows with the elements behind.
+    __syncthreads();  // the previous chunk's elements are no longer read
+    const int64_t base = j * kVolChunk;
 #pragma unroll
     for (int q = 0; q < kVolPer; q++) {
-      const int64_t e = j * kVolChunk + (int64_t)t * kVolPer + q;
-      x[q] = e < n ? c[e] : 0.0;
+      const int64_t e = base + q * kVolThreads + t;
+      x[q * kVolThreads + t] = e < n ? c[e] : 0.0;
     }
-    for (int start = 0; start < kVolThreads;) {
+    __syncthreads();
+    for (int start = 0; start < kVolChunk;) {
       const int E = exp_of(s);
+      const int64_t behind = (base + start) / (2 * kVolThreads);
+      const int per = behind < 1 ? 1 : (behind < kVolPer ? (int)behind : kVolPer);
       bool bad = false;
       unsigned long long r = 0;
-      if (t >= start) {
-#pragma unroll
-        for (int q = 0; q < kVolPer; q++) r += rne_units(x[q], E, bad);
-      }
+      const int lo = start + t * per, hi = lo + per < kVolChunk ? lo + per : kVolChunk;
+      for (int q = lo; q < hi; q++) r += rne_units(x[q], E, bad);
       const int first = walk_scan(w, r, bad, E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0, before);
       s = advance(s, before);
-      if (first == kVolThreads) break;
+      if (first == kVolThreads) {
+        start += kVolThreads * per;
+        continue;
+      }
       if (t == first) {  // element by element, in loop order, skipping exact zeros
         double v = s;
-#pragma unroll
-        for (int q = 0; q < kVolPer; q++)
-          if (x[q] != 0.0) v = v + x[q];
+        for (int q = lo; q < hi; q++) {
+          const double y = x[q];
+          if ((dbits(y) << 1) != 0) v = v + y;
+        }
         s_sum = v;
       }
       __syncthreads();
       s = s_sum;
-      start = first + 1;
+      start += (first + 1) * per;
     }
     j++;
   }
@@ -333,16 +381,19 @@ int64_t loop_sum_scratch_doubles(int64_t n) {
 
 namespace {
 
-// steps 2 to 4; the chunk sums are in scratch[0, nc) already
-void sum_chunks(cudaStream_t s, const double* c, int64_t n, double* scratch, double* out) {
+// steps 2 to 4; np partial sums, PER a chunk, are at the start of scratch
+// (2 nc doubles), then the estimates (nc), R (3 nc) and F (3 nc ints)
+template <typename T, int PER>
+void sum_chunks(cudaStream_t s, const double* c, int64_t n, int64_t np, double* scratch, double* out) {
+  static_assert(PER * sizeof(T) <= 2 * sizeof(double), "partial sums outgrow their part of the scratch");
   const int64_t nc = (n + kVolChunk - 1) / kVolChunk;
-  double* csum = scratch;
-  double* est = csum + nc;
+  const T* csum = reinterpret_cast<const T*>(scratch);
+  double* est = scratch + 2 * nc;
   int64_t* R = reinterpret_cast<int64_t*>(est + nc);
-  int64_t* F = R + 3 * nc;
+  int* F = reinterpret_cast<int*>(R + 3 * nc);
   const bool have_r = nc > kSmallChunks, scanned = nc > kScanChunks;
-  if (scanned) k_vol_scan<<<1, 1024, 0, s>>>(csum, nc, est);
-  if (have_r) k_vol_chunk_r<<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, scanned, est, R, F);
+  if (scanned) k_vol_scan<T, PER><<<1, 1024, 0, s>>>(csum, np, nc, est);
+  if (have_r) k_vol_chunk_r<T, PER><<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, np, scanned, est, R, F);
   k_vol_walk<<<1, kVolThreads, 0, s>>>(c, n, nc, est, R, F, have_r, out);
 }
 
@@ -354,7 +405,7 @@ void launch_loop_sum(cudaStream_t s, const double* c, int64_t n, double* scratch
     return;
   }
   k_vol_chunk_sum<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), kVolThreads, 0, s>>>(c, n, scratch);
-  sum_chunks(s, c, n, scratch, out);
+  sum_chunks<double, 1>(s, c, n, (n + kVolChunk - 1) / kVolChunk, scratch, out);
 }
 
 void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, double dy, double dz, double eps,
@@ -365,8 +416,9 @@ void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, d
     return;
   }
   const double dV = dx * dy * dz;
-  k_vol_contrib<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), 1024, 0, s>>>(b, phi, dV, eps, scratch, scratch + n);
-  sum_chunks(s, scratch, n, scratch + n, out);
+  const unsigned np = (unsigned)((n + kContribVoxels - 1) / kContribVoxels);
+  k_vol_contrib<<<np, kContribThreads, 0, s>>>(b, phi, dV, eps, scratch, reinterpret_cast<float*>(scratch + n));
+  sum_chunks<float, kVolChunk / kContribVoxels>(s, scratch, n, np, scratch + n, out);
 }
 
 }  // namespace qss

@@ -1027,18 +1027,19 @@ int even_len(int along, int cap) {
   return (along + tiles - 1) / tiles;
 }
 
-// The longest tiles (the smallest halo) that leave about four rounds of blocks
-// for the GPU, down to 8 positions.  Whole stage, M voxel-steps/s, 8-line tiles
-// of up to 8 / 16 / 24 / 27 positions: 24^3 70 / 66 / 63 / 63, 48^3 337 / 340 /
-// 347 / 347, 96^3 703 / 743 / 761 / 760, 128^3 773 / 827 / 837 / 851.
+// The longest tiles (the smallest halo) that leave about three rounds of blocks
+// for the GPU, down to 16 positions (one round of sides for 128 threads; shorter
+// ones leave threads idle).  Whole stage, M voxel-steps/s, 8-line tiles of up to
+// 8 / 16 / 24 / 27 positions: 24^3 70 / 66 / 63 / 63, 48^3 337 / 340 / 347 / 347,
+// 96^3 703 / 743 / 761 / 760, 128^3 773 / 827 / 837 / 851.
 int tile_cap_for(const Box& b) {
   int cap = kTileP;
-  while (cap > 8) {
+  while (cap > 16) {
     int64_t blocks = 0;
     for (int ax = 0; ax < 3; ax++)
       blocks += (int64_t)((line_lanes(b, ax) + kTileL - 1) / kTileL) * line_rows(b, ax) *
                 ((line_len(b, ax) + cap - 1) / cap);
-    if (blocks >= (int64_t)152 * kTileBlocks * 4) break;
+    if (blocks >= (int64_t)152 * kTileBlocks * 3) break;
     cap /= 2;
   }
   return cap;
