@@ -228,10 +228,15 @@ __global__ void __launch_bounds__(128) k_adj_carry(AdjPointArgs a) {
 //   d value / d T_k = -2 w_k (p_k - value) / T_k,   T_k = S_k + eps,
 //   d value / d p_k = w_k,  d eps / d u_j = 2e-6 u_j at the maximum square
 // (the later operand of the reference's MAX chain on ties, per side).
-// Each thread owns one of nseg equal segments of a line's points and
-// recomputes the windows on either side of it whose faces it needs, so every
-// point's adjoint is written once, in a fixed order: lam(p) += inv (F(p) -
-// F(p+1)), F the face adjoints.
+// A block holds a tile of 4 lines x up to 58 points and goes through it in
+// phases, each value once in shared memory: faces v, centre differences a, the
+// windows (their five face adjoints and the adjoints of the three indicators'
+// first terms), the centre terms' adjoints, the faces' sums in a fixed order, and
+// lam(p) += inv (F(p) - F(p+1)).  A tile recomputes the windows of 3 points on
+// either side; tiles of 58 points make 64 windows of them, full warps.
+// Bound: FP64 pipe (~145 instructions a window, 77 cycles each).  With a thread
+// walking a segment of a line instead (32 points and more, so that a 72^3 box had
+// 324 warps for 608 schedulers) a pass took 0.30 ms at 72^3.
 struct AdjAxisArgs {
   Box b;
   const double* phi;
@@ -239,41 +244,46 @@ struct AdjAxisArgs {
   const double* bm;
   double* lam;
   double inv;
-  int nseg;
+  int len;  // points per tile
 };
+constexpr int kAdjL = 4, kAdjP = 58, kAdjThreads = 128;
+constexpr int kAdjW = kAdjP + 6;   // windows p0-2 .. p0+P+3
+constexpr int kAdjF = kAdjP + 10;  // faces p0-4 .. p0+P+5
+constexpr int kAdjC = kAdjP + 8;   // centres p0-3 .. p0+P+4
+constexpr size_t kAdjBytes = sizeof(double) * kAdjL * (kAdjF + kAdjC + 8 * kAdjW);
+static_assert(kAdjBytes <= 48 * 1024, "dynamic shared memory without the opt-in attribute");
 
 template <int AX>
-__global__ void __launch_bounds__(128) k_adj_axis(AdjAxisArgs a) {
+__global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
+  constexpr int L = kAdjL;
+  extern __shared__ double adj_smem[];
+  double* const sv = adj_smem;             // faces; later the face adjoints F
+  double* const sa = sv + L * kAdjF;       // centre differences; later their terms' adjoints
+  double* const sd = sa + L * kAdjC;       // [8][window]: d0 .. d4, bS1 .. bS3
+  constexpr int W = L * kAdjW;
   const Box& b = a.b;
-  int p, q, lo, hi;
+  const int line = threadIdx.x % L;
+  int p, q, lo, hi, plast_line;
   if (AX == 0) {
-    p = b.jlo + blockIdx.x * blockDim.x + threadIdx.x;  // j
-    q = b.klo + blockIdx.y;                              // k
-    if (p > b.jhi) return;
+    p = b.jlo + blockIdx.x * L + line;  // j
+    q = b.klo + blockIdx.y;             // k
+    plast_line = b.jhi;
     lo = b.ilo;
     hi = b.ihi;
   } else {
-    p = b.ilo + blockIdx.x * blockDim.x + threadIdx.x;  // i
+    p = b.ilo + blockIdx.x * L + line;  // i
     q = (AX == 1 ? b.klo : b.jlo) + blockIdx.y;
-    if (p > b.ihi) return;
+    plast_line = b.ihi;
     lo = (AX == 1) ? b.jlo : b.klo;
     hi = (AX == 1) ? b.jhi : b.khi;
   }
-  const int len = hi - lo + 7;  // points lo-3 .. hi+3
-  const int p0 = lo - 3 + (int)(((int64_t)blockIdx.z * len) / a.nseg);
-  const int pend = lo - 3 + (int)(((int64_t)(blockIdx.z + 1) * len) / a.nseg) - 1;
-  if (pend < p0) return;
-  int64_t base, stride;
-  if (AX == 0) {
-    base = b.idx(0, p, q);
-    stride = 1;
-  } else if (AX == 1) {
-    base = b.idx(p, 0, q);
-    stride = b.nx;
-  } else {
-    base = b.idx(p, q, 0);
-    stride = (int64_t)b.nx * b.ny;
-  }
+  const bool line_ok = p <= plast_line;
+  if (!line_ok) p = plast_line;  // loads stay in the box; nothing is stored
+  const int p0 = lo - 3 + (int)blockIdx.z * a.len;  // points lo-3 .. hi+3 in all
+  int tp = hi + 3 - p0 + 1;
+  if (tp > a.len) tp = a.len;
+  const int64_t base = AX == 0 ? b.idx(0, p, q) : (AX == 1 ? b.idx(p, 0, q) : b.idx(p, q, 0));
+  const int64_t stride = AX == 0 ? 1 : (AX == 1 ? (int64_t)b.nx : (int64_t)b.nx * b.ny);
   const double* __restrict__ phi = a.phi;
   const double inv = a.inv;
   const int last = (AX == 0 ? b.nx : (AX == 1 ? b.ny : b.nz)) - 1;
@@ -286,55 +296,51 @@ __global__ void __launch_bounds__(128) k_adj_axis(AdjAxisArgs a) {
     return (m >= lo && m <= hi) ? __ldg(arr + base + (int64_t)m * stride) : 0.0;
   };
   using qss_emu::bits;
-  // window c = p0 - 2 first: faces c-2 .. c+1 now, face c+2 in the loop
-  const int c0 = p0 - 2;
-  double f_m3 = ld(c0 - 3), f_m2 = ld(c0 - 2), f_m1 = ld(c0 - 1), f_0 = ld(c0), f_p1 = ld(c0 + 1);
-  double u0 = (f_m2 - f_m3) * inv, u1 = (f_m1 - f_m2) * inv, u2 = (f_0 - f_m1) * inv, u3 = (f_p1 - f_0) * inv;
-  double s0 = u0 * u0, s1 = u1 * u1, s2 = u2 * u2, s3 = u3 * u3;
-  double plast = f_p1;
-  double F0 = 0, F1 = 0, F2 = 0, F3 = 0, F4 = 0;  // adjoints of faces c-2 .. c+2
-  double prevF = 0;                                // completed adjoint of face c-3
-  // the second difference a(m) = v(m-1) - 2 v(m) + v(m+1) of centre m and its
-  // term 13/12 a^2 enter S1 of window m+1, S2 of window m and S3 of window
-  // m-1: kept for centres c-1, c (c+1 computed per window), their adjoints
-  // summed over the three windows
-  double am_ = (u0 - 2.0 * u1) + u2, a0_ = (u1 - 2.0 * u2) + u3;
-  double Am_ = k1312 * (am_ * am_), A0_ = k1312 * (a0_ * a0_);
-  double BAm = 0, BA0 = 0, BAp = 0;  // adjoints of the terms of centres c-1, c, c+1
-#pragma unroll 1
-  for (int c = c0; c <= pend + 3; c++) {
-    const double pn = ld(c + 2);
-    const double u4 = (pn - plast) * inv;
-    plast = pn;
-    const double s4 = u4 * u4;
-    const double ap_ = (u2 - 2.0 * u3) + u4;
-    const double Ap_ = k1312 * (ap_ * ap_);
+  for (int it = threadIdx.x; it < (tp + 10) * L; it += kAdjThreads) {
+    const int m = p0 - 4 + it / L;
+    sv[it] = (ld(m) - ld(m - 1)) * inv;
+  }
+  __syncthreads();
+  // a(m) = v(m-1) - 2 v(m) + v(m+1); its term 13/12 a^2 enters S1 of window m+1,
+  // S2 of window m and S3 of window m-1
+  for (int it = threadIdx.x; it < (tp + 8) * L; it += kAdjThreads) {
+    const double* const v = sv + it;
+    sa[it] = (v[0] - 2.0 * v[L]) + v[2 * L];
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < (tp + 6) * L; it += kAdjThreads) {
+    const int c = p0 - 2 + it / L;
+    double d0 = 0, d1 = 0, d2 = 0, d3 = 0, d4 = 0, bS1 = 0, bS2 = 0, bS3 = 0;
     const double gm = ldbar(a.bm, c), gp = ldbar(a.bp, c - 1);
     if (gm != 0.0 || gp != 0.0) {
-      // eps and the position of the largest square for each reading direction
-      const long long b0 = (long long)bits(s0), b1 = (long long)bits(s1), b2 = (long long)bits(s2),
-                      b3 = (long long)bits(s3), b4 = (long long)bits(s4);
-      long long mx = b0;
+      const double* const v = sv + it;
+      const double u0 = v[0], u1 = v[L], u2 = v[2 * L], u3 = v[3 * L], u4 = v[4 * L];
+      const double* const aa = sa + it;
+      // eps and the position of the largest square (of the largest magnitude) for
+      // each reading direction
+      const uint64_t b0 = bits(u0) << 1, b1 = bits(u1) << 1, b2 = bits(u2) << 1, b3 = bits(u3) << 1,
+                     b4 = bits(u4) << 1;
+      uint64_t mx = b0;
       int im = 0;  // minus: u0 .. u4, later wins ties
       if (b1 >= mx) { mx = b1; im = 1; }
       if (b2 >= mx) { mx = b2; im = 2; }
       if (b3 >= mx) { mx = b3; im = 3; }
       if (b4 >= mx) { mx = b4; im = 4; }
-      long long mp = b4;
-      int ip = 4;  // plus: u4 .. u0, later wins ties
-      if (b3 >= mp) { mp = b3; ip = 3; }
-      if (b2 >= mp) { mp = b2; ip = 2; }
-      if (b1 >= mp) { mp = b1; ip = 1; }
-      if (b0 >= mp) { mp = b0; ip = 0; }
-      const double eps = 1e-6 * qss_emu::from_bits((unsigned long long)mx) + 1.0e-35;
+      int ip = 0;  // plus: u4 .. u0, later wins ties
+      if (b0 == mx) ip = 0;
+      else if (b1 == mx) ip = 1;
+      else if (b2 == mx) ip = 2;
+      else if (b3 == mx) ip = 3;
+      else ip = 4;
+      const double um = im == 0 ? u0 : im == 1 ? u1 : im == 2 ? u2 : im == 3 ? u3 : u4;
+      const double eps = 1e-6 * (um * um) + 1.0e-35;
       const double b1t = (u0 - 4.0 * u1) + 3.0 * u2, e2 = u1 - u3, b3t = (3.0 * u2 - 4.0 * u3) + u4;
-      const double S1 = Am_ + 0.25 * (b1t * b1t);
-      const double S2 = A0_ + 0.25 * (e2 * e2);
-      const double S3 = Ap_ + 0.25 * (b3t * b3t);
+      const double S1 = k1312 * (aa[0] * aa[0]) + 0.25 * (b1t * b1t);
+      const double S2 = k1312 * (aa[L] * aa[L]) + 0.25 * (e2 * e2);
+      const double S3 = k1312 * (aa[2 * L] * aa[2 * L]) + 0.25 * (b3t * b3t);
       const double r1 = qss_emu::div(1.0, S1 + eps), r2 = qss_emu::div(1.0, S2 + eps),
                    r3 = qss_emu::div(1.0, S3 + eps);
-      // products of the weights on the integer pipes (the FP64 pipe bounds
-      // this kernel, its integer pipes are ~90 % idle)
+      // products of the weights on the integer pipes (the FP64 pipe bounds this kernel)
       using qss_emu::mul;
       const double q1 = mul(r1, r1), q2 = mul(r2, r2), q3 = mul(r3, r3);
       const double am2 = mul(0.6, q2);
@@ -358,24 +364,22 @@ __global__ void __launch_bounds__(128) k_adj_axis(AdjAxisArgs a) {
       // x_k = 2 r_k; the minus sign of d value / d T_k is folded into the differences
       const double m1 = P1 * (vm - pm1) * x1, m2 = P2 * (vm - pm2) * x2, m3 = P3 * (vm - pm3) * x3;
       const double n1 = Q1 * (vp - pq1) * x1, n2 = Q2 * (vp - pq2) * x2, n3 = Q3 * (vp - pq3) * x3;
-      const double bS1 = m1 + n1, bS2 = m2 + n2, bS3 = m3 + n3;
+      bS1 = m1 + n1;
+      bS2 = m2 + n2;
+      bS3 = m3 + n3;
       const double bem = m1 + m2 + m3, bep = n1 + n2 + n3;
-      BAm += bS1;
-      BA0 += bS2;
-      BAp += bS3;
       const double bb1 = bS1 * qss_emu::scale2(b1t, -1);
       const double be2 = bS2 * qss_emu::scale2(e2, -1);
       const double bb3 = bS3 * qss_emu::scale2(b3t, -1);
-      double d0 = bb1 + kC13 * P1 - kC16 * Q1;
-      double d1 = -4.0 * bb1 + be2 - kC76 * P1 - kC16 * P2 + kC56 * Q1 + kC13 * Q2;
-      double d2 = 3.0 * bb1 + 3.0 * bb3 + kC116 * P1 + kC56 * P2 + kC13 * P3 + kC13 * Q1 + kC56 * Q2 +
+      d0 = bb1 + kC13 * P1 - kC16 * Q1;
+      d1 = -4.0 * bb1 + be2 - kC76 * P1 - kC16 * P2 + kC56 * Q1 + kC13 * Q2;
+      d2 = 3.0 * bb1 + 3.0 * bb3 + kC116 * P1 + kC56 * P2 + kC13 * P3 + kC13 * Q1 + kC56 * Q2 +
                   kC116 * Q3;
-      double d3 = -be2 - 4.0 * bb3 + kC13 * P2 + kC56 * P3 - kC16 * Q2 - kC76 * Q3;
-      double d4 = bb3 - kC16 * P3 + kC13 * Q3;
+      d3 = -be2 - 4.0 * bb3 + kC13 * P2 + kC56 * P3 - kC16 * Q2 - kC76 * Q3;
+      d4 = bb3 - kC16 * P3 + kC13 * Q3;
       // eps = 1e-6 max(u^2) + 1e-35, per reading direction
       {
         // both directions usually pick the same face: one sum, then selects
-        const double um = im == 0 ? u0 : im == 1 ? u1 : im == 2 ? u2 : im == 3 ? u3 : u4;
         const double up = ip == 0 ? u0 : ip == 1 ? u1 : ip == 2 ? u2 : ip == 3 ? u3 : u4;
         const double cm = 2e-6 * um * bem, cp = 2e-6 * up * bep;
         const double cs = (im == ip) ? cm + cp : cm;
@@ -386,49 +390,37 @@ __global__ void __launch_bounds__(128) k_adj_axis(AdjAxisArgs a) {
         d3 += ex(3);
         d4 += ex(4);
       }
-      F0 += d0;
-      F1 += d1;
-      F2 += d2;
-      F3 += d3;
-      F4 += d4;
     }
-    // centre c-1 is complete: its term 13/12 a^2 back to faces c-2, c-1, c
-    {
-      const double ba = BAm * (k136 * am_);
-      F0 += ba;
-      F1 -= 2.0 * ba;
-      F2 += ba;
-    }
-    // face c-2 is complete: the point between faces c-3 and c-2 is done
-    const int m = c - 2;
-    if (m > p0) {
-      const int pt = m - 1;
-      double* l = a.lam + base + (int64_t)pt * stride;
-      *l += inv * (prevF - F0);
-    }
-    prevF = F0;
-    // slide the window by one face
-    u0 = u1;
-    u1 = u2;
-    u2 = u3;
-    u3 = u4;
-    s0 = s1;
-    s1 = s2;
-    s2 = s3;
-    s3 = s4;
-    F0 = F1;
-    F1 = F2;
-    F2 = F3;
-    F3 = F4;
-    F4 = 0;
-    am_ = a0_;
-    a0_ = ap_;
-    Am_ = A0_;
-    A0_ = Ap_;
-    BAm = BA0;
-    BA0 = BAp;
-    BAp = 0;
+    sd[it] = d0;
+    sd[W + it] = d1;
+    sd[2 * W + it] = d2;
+    sd[3 * W + it] = d3;
+    sd[4 * W + it] = d4;
+    sd[5 * W + it] = bS1;
+    sd[6 * W + it] = bS2;
+    sd[7 * W + it] = bS3;
   }
+  __syncthreads();
+  // adjoint of a(m) for the centres p0-1 .. p0+tp+1 the tile's faces touch (window
+  // index w = m - p0 + 2): its term sits in S1 of window w+1, S2 of w, S3 of w-1
+  for (int it = threadIdx.x; it < (tp + 3) * L; it += kAdjThreads) {
+    const int w = it + L;  // the window of centre m = p0 - 1 + it / L
+    const double ba = (sd[5 * W + w + L] + sd[6 * W + w]) + sd[7 * W + w - L];
+    sa[it + 2 * L] = ba * (k136 * sa[it + 2 * L]);  // centre m is entry m - p0 + 3
+  }
+  __syncthreads();
+  // face f = p0 .. p0+tp: slot k of window f + 2 - k, and the three centres on it
+  for (int it = threadIdx.x; it < (tp + 1) * L; it += kAdjThreads) {
+    const double* const d = sd + it + 4 * L;  // window f + 2
+    const double* const c = sa + it + 2 * L;  // centre f - 1
+    double F = ((d[0] + d[W - L]) + (d[2 * W - 2 * L] + d[3 * W - 3 * L])) + d[4 * W - 4 * L];
+    F += (c[0] + c[2 * L]) - 2.0 * c[L];
+    sv[it] = F;  // the faces' v is no longer read
+  }
+  __syncthreads();
+  if (!line_ok) return;
+  for (int it = threadIdx.x; it < tp * L; it += kAdjThreads)
+    a.lam[base + (int64_t)(p0 + it / L) * stride] += inv * (sv[it] - sv[it + L]);
 }
 
 // lam_out[p] += coef * lam_in[p] (fill box) + the curvature partials of the
@@ -467,11 +459,27 @@ __global__ void k_adj_curv(Box b, const double* __restrict__ cc, int64_t npts, c
 // layers' adjoints go to the two boundary points they were built from, and
 // are cleared.  axis 2: all (i, j); axis 1: all i, k in the fill box;
 // axis 0: j, k in the fill box (the forward's sweep domains).
-__device__ __forceinline__ void extrap_bwd(double f, double g, int dist, double gb, double& fb, double& gbb) {
-  const double s = copysign(1.0, f);
-  const double dsd = (f - g) > 0 ? 1.0 : ((f - g) < 0 ? -1.0 : 0.0);
-  fb += gb * (1.0 + s * dsd * dist);
-  gbb += gb * (-s * dsd * dist);
+// With t = sign(f) sign(f - g) in {-1, 0, 1}, a layer at distance d adds lam (1 +
+// t d) to f and -lam t d to g: two sums per side, all layers' loads first.
+__device__ __forceinline__ void extrap_bwd(double* lam, int64_t p0, int64_t st, int layers, double f, double g,
+                                           double& fb, double& gb) {
+  double s = 0, sd = 0;
+  for (int m0 = 0; m0 < layers; m0 += 3) {
+    double x[3];
+#pragma unroll
+    for (int m = 0; m < 3; m++) x[m] = m0 + m < layers ? lam[p0 + (m0 + m) * st] : 0.0;
+#pragma unroll
+    for (int m = 0; m < 3; m++) {
+      s += x[m];
+      sd += x[m] * (double)(m0 + m + 1);
+      if (m0 + m < layers) lam[p0 + (m0 + m) * st] = 0.0;
+    }
+  }
+  const double d = f - g;
+  const bool neg = (int64_t)(qss_emu::bits(f) ^ qss_emu::bits(d)) < 0;
+  const double t = (qss_emu::bits(d) << 1) == 0 ? 0.0 : (neg ? -sd : sd);
+  fb = s + t;
+  gb = -t;
 }
 
 __global__ void k_adj_bc(Box b, int axis, const double* __restrict__ val, double* lam) {
@@ -510,19 +518,11 @@ __global__ void k_adj_bc(Box b, int axis, const double* __restrict__ val, double
     hi = b.ihi;
     len = b.nx;
   }
-  double blo = 0, blo1 = 0, bhi = 0, bhi1 = 0;
+  double blo, blo1, bhi, bhi1;
   const double flo = val[base + lo * st], flo1 = val[base + (lo + 1) * st];
   const double fhi = val[base + hi * st], fhi1 = val[base + (hi - 1) * st];
-  for (int m = 0; m < lo; m++) {
-    const int64_t p = base + m * st;
-    extrap_bwd(flo, flo1, lo - m, lam[p], blo, blo1);
-    lam[p] = 0.0;
-  }
-  for (int m = hi + 1; m < len; m++) {
-    const int64_t p = base + m * st;
-    extrap_bwd(fhi, fhi1, m - hi, lam[p], bhi, bhi1);
-    lam[p] = 0.0;
-  }
+  extrap_bwd(lam, base + (lo - 1) * st, -st, lo, flo, flo1, blo, blo1);
+  extrap_bwd(lam, base + (hi + 1) * st, st, len - 1 - hi, fhi, fhi1, bhi, bhi1);
   lam[base + lo * st] += blo;
   lam[base + (lo + 1) * st] += blo1;
   lam[base + hi * st] += bhi;
@@ -868,23 +868,20 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
     ar.npts = n;
     const dim3 blk(32, 4, 1);
     const dim3 grd((b.fbx() + 31) / 32, (b.fby() + 3) / 4, b.fbz());
-    // line kernels: lanes along i for the y and z passes, along j for x; each
-    // line cut into equal segments of at least 32 points (the windows a
-    // segment recomputes at its ends cost 5 per segment), enough of them for
-    // about two waves of 20 warps per SM
-    auto nseg_of = [&](int ax) {
-      const int len = (ax == 0 ? b.fbx() : ax == 1 ? b.fby() : b.fbz()) + 6;
-      const int64_t lines = (ax == 0) ? (int64_t)b.fby() * b.fbz()
-                                      : (ax == 1 ? (int64_t)b.fbx() * b.fbz() : (int64_t)b.fbx() * b.fby());
-      const int64_t want = 2LL * 152 * 20 * 32;
-      int64_t ns = (want + lines - 1) / lines;
-      if (ns > len / 32) ns = len / 32;
-      return (int)(ns < 1 ? 1 : ns);
-    };
-    const int ns0 = nseg_of(0), ns1 = nseg_of(1), ns2 = nseg_of(2);
-    const dim3 ag0((unsigned)((b.fby() + 127) / 128), (unsigned)b.fbz(), (unsigned)ns0);
-    const dim3 ag1((unsigned)((b.fbx() + 127) / 128), (unsigned)b.fbz(), (unsigned)ns1);
-    const dim3 ag2((unsigned)((b.fbx() + 127) / 128), (unsigned)b.fby(), (unsigned)ns2);
+    // the axis passes' tiles: a line's points split evenly; shorter tiles on small
+    // boxes, so that four blocks per SM have about two rounds of them
+    AdjAxisArgs axs[3];
+    dim3 agrid[3];
+    for (int d = 0; d < 3; d++) {
+      const int len = (d == 0 ? b.fbx() : d == 1 ? b.fby() : b.fbz()) + 6;
+      const unsigned lx = (unsigned)(((d == 0 ? b.fby() : b.fbx()) + kAdjL - 1) / kAdjL);
+      const unsigned ly = (unsigned)(d == 2 ? b.fby() : b.fbz());
+      int cap = kAdjP;
+      while (cap > 16 && (int64_t)lx * ly * ((len + cap - 1) / cap) < 152 * 4 * 2) cap /= 2;
+      const int tiles = (len + cap - 1) / cap;
+      axs[d] = AdjAxisArgs{b, nullptr, ar.bp[d], ar.bm[d], nullptr, 1.0 / g->dx[d], (len + tiles - 1) / tiles};
+      agrid[d] = dim3(lx, ly, (unsigned)((len + axs[d].len - 1) / axs[d].len));
+    }
     auto bc_bwd = [&](const double* val, double* l) {
       const int n2 = b.nx * b.ny, n1 = b.nx * b.fbz(), n0 = b.fby() * b.fbz();
       k_adj_bc<<<(n2 + 255) / 256, 256, 0, a.s>>>(b, 2, val, l);
@@ -912,22 +909,13 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
       ar.coef_l = coef_l;
       k_adj_point<<<grd, blk, 0, a.s>>>(ar);
       k_adj_carry<<<grd, blk, 0, a.s>>>(ar);
-      AdjAxisArgs ax{b, in, nullptr, nullptr, lam_out, 0.0, 1};
-      ax.bp = ar.bp[0];
-      ax.bm = ar.bm[0];
-      ax.inv = 1.0 / g->dx[0];
-      ax.nseg = ns0;
-      k_adj_axis<0><<<ag0, 128, 0, a.s>>>(ax);
-      ax.bp = ar.bp[1];
-      ax.bm = ar.bm[1];
-      ax.inv = 1.0 / g->dx[1];
-      ax.nseg = ns1;
-      k_adj_axis<1><<<ag1, 128, 0, a.s>>>(ax);
-      ax.bp = ar.bp[2];
-      ax.bm = ar.bm[2];
-      ax.inv = 1.0 / g->dx[2];
-      ax.nseg = ns2;
-      k_adj_axis<2><<<ag2, 128, 0, a.s>>>(ax);
+      for (auto& x : axs) {
+        x.phi = in;
+        x.lam = lam_out;
+      }
+      k_adj_axis<0><<<agrid[0], kAdjThreads, kAdjBytes, a.s>>>(axs[0]);
+      k_adj_axis<1><<<agrid[1], kAdjThreads, kAdjBytes, a.s>>>(axs[1]);
+      k_adj_axis<2><<<agrid[2], kAdjThreads, kAdjBytes, a.s>>>(axs[2]);
       k_adj_curv<<<g1(n), 256, 0, a.s>>>(b, cc, n, lam_in, coef_id, lam_out);
     };
     // recomputation of segment k's states from its checkpoint, on stream st
