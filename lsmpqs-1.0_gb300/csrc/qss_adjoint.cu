@@ -607,16 +607,27 @@ unsigned g1(int64_t n) {
   return (unsigned)(b < 1 ? 1 : b);
 }
 
+// the call's stream and, on it, its device arrays; an exception may leave work of
+// either stream in flight, which is waited for before they go
 struct DBufs {
-  std::vector<double*> ptrs;
-  double* get(int64_t n) {
-    double* p = nullptr;
-    QSS_CK(cudaMalloc(&p, (size_t)(n > 0 ? n : 1) * sizeof(double)));
-    ptrs.push_back(p);
-    return p;
+  cudaStream_t s = nullptr;
+  std::vector<std::pair<void*, size_t>> ptrs;
+  bool done = false;  // every stream has been waited for
+  DBufs() { QSS_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
+  DBufs(const DBufs&) = delete;
+  DBufs& operator=(const DBufs&) = delete;
+  template <class T = double>
+  T* get(int64_t n) {
+    const size_t bytes = (size_t)(n > 0 ? n : 1) * sizeof(T);
+    ptrs.reserve(ptrs.size() + 1);
+    void* p = scratch_alloc(bytes, s);
+    ptrs.emplace_back(p, bytes);
+    return (T*)p;
   }
   ~DBufs() {
-    for (double* p : ptrs) cudaFree(p);
+    if (!done) cudaDeviceSynchronize();
+    for (const auto& p : ptrs) scratch_free(p.first, p.second, s);
+    cudaStreamDestroy(s);
   }
 };
 
@@ -719,8 +730,8 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
     a.b = b;
     a.n = n;
     for (int d = 0; d < 3; d++) a.dx[d] = g->dx[d];
-    QSS_CK(cudaStreamCreateWithFlags(&a.s, cudaStreamNonBlocking));
     DBufs buf;
+    a.s = buf.s;
     double* mask = buf.get(n);
     double* mxyz[3] = {buf.get(n), buf.get(n), buf.get(n)};
     double* th = buf.get(n);
@@ -732,17 +743,13 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
       a.dp[d] = buf.get(n);
       a.dm[d] = buf.get(n);
     }
-    int* nsrc = nullptr;
-    QSS_CK(cudaMalloc(&nsrc, (size_t)n * sizeof(int)));
+    int* nsrc = buf.get<int>(n);
     const int64_t rows = (int64_t)b.fby() * b.fbz();
-    int *rowlast = nullptr, *carry = nullptr;
-    unsigned long long* cnt = nullptr;
-    unsigned long long* red = nullptr;
-    QSS_CK(cudaMalloc(&rowlast, (size_t)rows * sizeof(int)));
-    QSS_CK(cudaMalloc(&carry, (size_t)rows * sizeof(int)));
-    QSS_CK(cudaMalloc(&cnt, sizeof(unsigned long long)));
-    QSS_CK(cudaMalloc(&red, 4 * sizeof(unsigned long long)));
-    QSS_CK(cudaMalloc(&a.ctl, sizeof(Ctl)));
+    int* rowlast = buf.get<int>(rows);
+    int* carry = buf.get<int>(rows);
+    unsigned long long* cnt = buf.get<unsigned long long>(1);
+    unsigned long long* red = buf.get<unsigned long long>(4);
+    a.ctl = buf.get<Ctl>(1);
     QSS_CK(cudaMemcpyAsync(mask, p->mask, bytes, cudaMemcpyHostToDevice, a.s));
     QSS_CK(cudaMemcpyAsync(th, theta, bytes, cudaMemcpyHostToDevice, a.s));
     QSS_CK(cudaMemcpyAsync(tgt, target, bytes, cudaMemcpyHostToDevice, a.s));
@@ -781,6 +788,7 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
       for (int k = 0; k < nseg - 1; k++) cp[k] = buf.get(n);
       size_t free_b = 0, total_b = 0;
       QSS_CK(cudaMemGetInfo(&free_b, &total_b));
+      free_b += scratch_idle_bytes();
       const double per_set = (double)ckpt * (4 + 18) * bytes;
       const double rest = (double)(15 + 8) * bytes;
       const bool derivs = per_set + rest < 0.6 * (double)free_b;
@@ -823,13 +831,7 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
     QSS_CK(cudaGetLastError());
     if (!want_grad) {
       QSS_CK(cudaStreamSynchronize(a.s));
-      cudaFree(nsrc);
-      cudaFree(rowlast);
-      cudaFree(carry);
-      cudaFree(cnt);
-      cudaFree(red);
-      cudaFree(a.ctl);
-      cudaStreamDestroy(a.s);
+      buf.done = true;
       return 0;
     }
     // backward
@@ -998,13 +1000,7 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
     Ctl hc;
     QSS_CK(cudaMemcpy(&hc, a.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
     host_err = hc.err;
-    cudaFree(nsrc);
-    cudaFree(rowlast);
-    cudaFree(carry);
-    cudaFree(cnt);
-    cudaFree(red);
-    cudaFree(a.ctl);
-    cudaStreamDestroy(a.s);
+    buf.done = true;
     if (host_err) throw Error(QSSGPU_ERR_DEVICE_CHECK, "device check failed in the adjoint run");
     return 0;
   } catch (const std::exception& e) {

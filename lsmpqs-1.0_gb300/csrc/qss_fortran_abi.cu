@@ -33,10 +33,8 @@ cudaStream_t abi_stream() {
 struct DBuf {
   void* p = nullptr;
   size_t bytes = 0;
-  explicit DBuf(size_t b) : bytes(b) { QSS_CK(cudaMalloc(&p, b ? b : 8)); }
-  ~DBuf() {
-    if (p) cudaFree(p);
-  }
+  explicit DBuf(size_t b) : p(scratch_alloc(b, abi_stream())), bytes(b) {}
+  ~DBuf() { scratch_free(p, bytes, abi_stream()); }
   DBuf(const DBuf&) = delete;
   DBuf& operator=(const DBuf&) = delete;
   double* d() { return (double*)p; }
@@ -102,7 +100,6 @@ void rhs_entry(int scheme, bool var, const double* phi, const double* vel_n, con
   h2d(dphi, phi, bytes);
   h2d(drhs, lse_rhs, bytes);
   Coef c{};
-  std::vector<DBuf*> keep;
   DBuf dv(var ? bytes : 8), db(var ? bytes : 8), dvx(var ? bytes : 8), dvy(var ? bytes : 8),
       dvz(var ? bytes : 8), dns(var ? (size_t)bx.npts() * sizeof(int) : 8),
       drow(var ? (size_t)bx.fby() * bx.fbz() * sizeof(int) : 8),
@@ -133,7 +130,6 @@ void rhs_entry(int scheme, bool var, const double* phi, const double* vel_n, con
     double* const dm[3] = {d3.d(), d4.d(), d5.d()};
     launch_weno_axes(s, bx, dphi.d(), dx, dy, dz, dp, dm, nullptr);
     launch_weno_combine(s, 0, false, bx, dx, dy, dz, dphi.d(), nullptr, drhs.d(), nullptr, dp, dm, c, im, nullptr);
-    QSS_CK(cudaStreamSynchronize(s));
   } else {
     launch_stage(s, scheme, var, 0, false, bx, dx, dy, dz, dphi.d(), nullptr, drhs.d(), nullptr, c, im, nullptr);
   }

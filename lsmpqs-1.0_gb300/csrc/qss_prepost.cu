@@ -107,16 +107,19 @@ unsigned g1(int64_t n) {
 }
 
 struct Buf {
-  std::vector<void*> ptrs;
+  cudaStream_t s;
+  std::vector<std::pair<void*, size_t>> ptrs;
+  explicit Buf(cudaStream_t stream) : s(stream) {}
   template <class T>
   T* get(int64_t n) {
-    void* p = nullptr;
-    QSS_CK(cudaMalloc(&p, (size_t)(n > 0 ? n : 1) * sizeof(T)));
-    ptrs.push_back(p);
+    const size_t bytes = (size_t)(n > 0 ? n : 1) * sizeof(T);
+    ptrs.reserve(ptrs.size() + 1);
+    void* p = scratch_alloc(bytes, s);
+    ptrs.emplace_back(p, bytes);
     return (T*)p;
   }
   ~Buf() {
-    for (void* p : ptrs) cudaFree(p);
+    for (const auto& p : ptrs) scratch_free(p.first, p.second, s);
   }
 };
 
@@ -179,7 +182,7 @@ void qss_reinitialize_mask(QSS_DataArrays* p, Grid* g, Options* o) {
     const int64_t n = b.npts();
     const size_t bytes = (size_t)n * sizeof(double);
     Stream st;
-    Buf buf;
+    Buf buf(st.s);
     double *mask = buf.get<double>(n), *s1 = buf.get<double>(n), *s2 = buf.get<double>(n),
            *rhs = buf.get<double>(n), *next = buf.get<double>(n);
     h2d(st.s, mask, p->mask, bytes);
@@ -210,7 +213,7 @@ int qssgpu_create_mask_ubc(const unsigned char* ubc, QSS_DataArrays* p, Grid* g,
     const int64_t n = b.npts(), nfb = (int64_t)b.fbx() * b.fby() * b.fbz();
     const size_t bytes = (size_t)n * sizeof(double);
     Stream st;
-    Buf buf;
+    Buf buf(st.s);
     unsigned char* img = buf.get<unsigned char>(nfb);
     double *mask = buf.get<double>(n), *s1 = buf.get<double>(n), *s2 = buf.get<double>(n),
            *rhs = buf.get<double>(n), *next = buf.get<double>(n);
@@ -255,7 +258,7 @@ int qssgpu_create_init_from_mask(QSS_DataArrays* p, Grid* g, Options* o) {
       cz = 0.5 * (g->x_lo[2] + g->x_hi[2]);
     }
     Stream st;
-    Buf buf;
+    Buf buf(st.s);
     double *mask = buf.get<double>(n), *phi = buf.get<double>(n);
     h2d(st.s, mask, p->mask, bytes);
     launch_sphere(st.s, b, phi, g->x_lo_ghostbox, g->dx, cx, cy, cz, radius, -1);  // createSphere(.., -1, g)
@@ -279,7 +282,7 @@ int qssgpu_diff_steps(const double* step_a, const double* step_b, Grid* g, doubl
     const int64_t n = b.npts();
     const size_t bytes = (size_t)n * sizeof(double);
     Stream st;
-    Buf buf;
+    Buf buf(st.s);
     double *a = buf.get<double>(n), *bb = buf.get<double>(n), *phi = buf.get<double>(n);
     unsigned char* bin = buf.get<unsigned char>(n);
     int* labels = buf.get<int>(n);
@@ -329,7 +332,7 @@ int qssgpu_phase_uchar(const double* phi, const double* mask, Grid* g, char phas
     const int64_t n = b.npts(), nfb = (int64_t)b.fbx() * b.fby() * b.fbz();
     const size_t bytes = (size_t)n * sizeof(double);
     Stream st;
-    Buf buf;
+    Buf buf(st.s);
     double* dphi = need_phi ? buf.get<double>(n) : nullptr;
     double* dmask = need_mask ? buf.get<double>(n) : nullptr;
     unsigned char* dfull = bin_full ? buf.get<unsigned char>(n) : nullptr;

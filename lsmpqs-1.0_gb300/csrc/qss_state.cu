@@ -197,9 +197,97 @@ int emu_level() {
   return m < 0 ? 0 : (m > 2 ? 2 : m);
 }
 
+// ---------------------------------------------------------------------------
+// scratch pool, one per device (see qss_state.h)
+
+namespace {
+constexpr size_t kPoolBlock = 1ull << 30;  // larger blocks bypass the pool
+constexpr size_t kPoolKeep = 4ull << 30;
+constexpr int kPoolDevices = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kPoolDevices] = {};
+
+// the current device's pool; with create false, null where there is none yet
+cudaMemPool_t scratch_pool(bool create) {
+  int dev = 0;
+  QSS_CK(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kPoolDevices) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool[dev] && create) {
+    int ok = 0;
+    QSS_CK(cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev));
+    if (!ok) return nullptr;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    QSS_CK(cudaMemPoolCreate(&pool, &props));
+    uint64_t keep = kPoolKeep;
+    const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      QSS_CK(e);
+    }
+    g_pool[dev] = pool;
+  }
+  return g_pool[dev];
+}
+
+// cudaMalloc, once more after the pool has given its unused memory back
+cudaError_t malloc_trimming(void** ptr, size_t bytes) {
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    scratch_trim();
+    e = cudaMalloc(ptr, bytes);
+  }
+  return e;
+}
+}  // namespace
+
+void* scratch_alloc(size_t bytes, cudaStream_t s) {
+  void* ptr = nullptr;
+  if (bytes == 0) bytes = 8;
+  cudaMemPool_t pool = bytes <= kPoolBlock ? scratch_pool(true) : nullptr;
+  if (pool) QSS_CK(cudaMallocFromPoolAsync(&ptr, bytes, pool, s));
+  else QSS_CK(malloc_trimming(&ptr, bytes));
+  return ptr;
+}
+
+void scratch_free(void* ptr, size_t bytes, cudaStream_t s) {
+  if (!ptr) return;
+  cudaMemPool_t pool = nullptr;
+  if (bytes <= kPoolBlock) {
+    try {
+      pool = scratch_pool(false);
+    } catch (const Error&) {
+    }
+  }
+  if (pool) cudaFreeAsync(ptr, s);
+  else cudaFree(ptr);
+}
+
+void scratch_trim() {
+  try {
+    cudaMemPool_t pool = scratch_pool(false);
+    if (pool) cudaMemPoolTrimTo(pool, 0);
+  } catch (const Error&) {
+  }
+}
+
+size_t scratch_idle_bytes() {
+  cudaMemPool_t pool = scratch_pool(false);
+  if (!pool) return 0;
+  uint64_t reserved = 0, used = 0;
+  QSS_CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+  QSS_CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return (size_t)(reserved > used ? reserved - used : 0);
+}
+
 template <class T>
 static void dalloc(T*& ptr, int64_t count) {
-  if (!ptr) QSS_CK(cudaMalloc((void**)&ptr, (size_t)count * sizeof(T)));
+  if (!ptr) QSS_CK(malloc_trimming((void**)&ptr, (size_t)count * sizeof(T)));
 }
 
 static void destroy_volume(DevVolume* v) {
@@ -296,6 +384,7 @@ static void alloc_volume(DevVolume* v) {
 }
 
 void release_volume(const QSS_DataArrays* p) {
+  scratch_trim();
   std::lock_guard<std::mutex> lk(g_mu);
   auto it = g_table.find(p);
   if (it == g_table.end()) return;
@@ -457,13 +546,13 @@ void download_dirty(DevVolume& v, QSS_DataArrays* p) {
         // ghost values must survive, so only fill-box rows travel
         const Box& b = v.box;
         const size_t pitch = (size_t)b.nx * sizeof(double);
-        const cudaStream_t st = lane();
-        for (int k = b.klo; k <= b.khi; k++) {
-          const size_t off = (size_t)b.idx(b.ilo, b.jlo, k) * sizeof(double);
-          QSS_CK(cudaMemcpy2DAsync((char*)h + off, pitch, (const char*)d + off, pitch,
-                                   (size_t)b.fbx() * sizeof(double), (size_t)b.fby(), cudaMemcpyDeviceToHost,
-                                   st));
-        }
+        cudaMemcpy3DParms c{};
+        c.srcPtr = make_cudaPitchedPtr(d, pitch, pitch, (size_t)b.ny);
+        c.dstPtr = make_cudaPitchedPtr(h, pitch, pitch, (size_t)b.ny);
+        c.srcPos = c.dstPos = make_cudaPos((size_t)b.ilo * sizeof(double), (size_t)b.jlo, (size_t)b.klo);
+        c.extent = make_cudaExtent((size_t)b.fbx() * sizeof(double), (size_t)b.fby(), (size_t)b.fbz());
+        c.kind = cudaMemcpyDeviceToHost;
+        QSS_CK(cudaMemcpy3DAsync(&c, lane()));
       } else {
         QSS_CK(cudaMemcpyAsync(h, d, (size_t)v.n * elem_size(w), cudaMemcpyDeviceToHost, lane()));
       }
