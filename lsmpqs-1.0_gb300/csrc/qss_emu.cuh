@@ -66,6 +66,13 @@ constexpr uint64_t kHidden = 1ull << 52;
 constexpr uint64_t kSign = 1ull << 63;
 constexpr uint64_t kAbs = ~kSign;
 
+// Twice the magnitude bits, for comparisons of magnitudes: the sign is shifted
+// out because the compiler takes (bits of a double) & kAbs for fabs and issues
+// it on the FP64 pipe (77 cycles; two such tests were a fifth of the
+// reinitialisation sweep).
+QSS_EMU_HD uint64_t mag2(uint64_t b) { return b << 1; }
+constexpr uint64_t kInf2 = 0x7ff0000000000000ull << 1;
+
 QSS_EMU_HD uint64_t bits(double x) {
 #ifdef __CUDA_ARCH__
   return (uint64_t)__double_as_longlong(x);
@@ -213,12 +220,12 @@ QSS_EMU_HD uint32_t recip30(uint32_t mh, uint32_t ml, bool& ok) {
   return S0 * 64u - (uint32_t)c;
 }
 
-// quotient of the normal numbers (xh:xl) / (yh:yl) where it is normal
-QSS_EMU_HD double div_win(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl, bool& ok) {
+// quotient of the normal numbers (xh:xl) / (yh:yl) where it is normal; S1 is
+// recip30 of y's significand, which a loop over one divisor computes once
+QSS_EMU_HD double div_recip(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl, uint32_t S1) {
   const uint32_t mxh = mant_hi(xh), myh = mant_hi(yh);
   const uint64_t mx = pack64(mxh, xl), my = pack64(myh, yl);
   const uint32_t s = mx < my ? 1u : 0u;
-  const uint32_t S1 = recip30(myh, yl, ok);
   const uint32_t nh = fsr(xl, mxh, 22u - s);
   const uint32_t q1 = (mulhi32(nh, S1) - 2u) >> 2;
   const uint64_t R1c = pack64(fsl(xl, mxh, 26u + s), xl << (26u + s)) + (1ull << 23) - (uint64_t)q1 * my;  // R1 + 2^23
@@ -228,6 +235,9 @@ QSS_EMU_HD double div_win(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl, bo
   // (exponent - 1) << 52 plus the 53-bit significand; the signs add up mod 2
   const uint32_t e = (xh - mxh) - (yh - myh) + ((1022u - s) << 20);
   return from_bits(pack64((uint32_t)(Q >> 32) + e, (uint32_t)Q));
+}
+QSS_EMU_HD double div_win(uint32_t xh, uint32_t xl, uint32_t yh, uint32_t yl, bool& ok) {
+  return div_recip(xh, xl, yh, yl, recip30(mant_hi(yh), yl, ok));
 }
 
 QSS_EMU_HD double div(double x, double y) {
@@ -300,7 +310,7 @@ QSS_EMU_HD double sqrt(double x) {
     bool ok = true;
     const double r = sqrt_win(xh, lo32(x), ok);
     if (ok) return r;
-  } else if ((bits(x) & kAbs) == 0) {
+  } else if (mag2(bits(x)) == 0) {
     return x;  // sqrt(+-0) = +-0
   }
   return QSS_EMU_FALLBACK(3, ::sqrt(x));
@@ -341,7 +351,7 @@ QSS_EMU_HD double mul(double x, double y) {
   if (in_window(xh, yh)) return mul_win(xh, lo32(x), yh, lo32(y));
   const uint64_t bx = bits(x), by = bits(y);
   const uint32_t ex = (xh >> 20) & 0x7ffu, ey = (yh >> 20) & 0x7ffu;
-  if ((((bx & kAbs) == 0) && ey != 0x7ffu) || (((by & kAbs) == 0) && ex != 0x7ffu))
+  if ((mag2(bx) == 0 && ey != 0x7ffu) || (mag2(by) == 0 && ex != 0x7ffu))
     return from_bits((bx ^ by) & kSign);  // zero times a finite number
   return QSS_EMU_FALLBACK(1, native_mul(x, y));
 }
@@ -437,7 +447,7 @@ QSS_EMU_HD double scale2(double x, int k) {
   const int e = (int)((b >> 52) & 0x7ffu);
   if (e >= 1 && e <= 2046 && e + k >= 1 && e + k <= 2046)
     return from_bits(b + ((uint64_t)(int64_t)k << 52));
-  if ((b & kAbs) == 0) return x;
+  if (mag2(b) == 0) return x;
 #ifdef __CUDA_ARCH__
   return x * __longlong_as_double((long long)((uint64_t)(1023 + k) << 52));
 #else
@@ -474,7 +484,7 @@ QSS_EMU_HD double abs(double x) {
 // ---------------------------------------------------------------------------
 // comparisons with IEEE semantics (false for NaN operands, -0 == +0)
 
-QSS_EMU_HD bool isnan_bits(uint64_t b) { return (b & kAbs) > 0x7ff0000000000000ull; }
+QSS_EMU_HD bool isnan_bits(uint64_t b) { return mag2(b) > kInf2; }
 
 // x > 0
 QSS_EMU_HD bool gt0(double x) {
@@ -496,9 +506,10 @@ QSS_EMU_HD bool lt0(double x) {
 QSS_EMU_HD bool gt(double x, double y) {
   const uint64_t a = bits(x), b = bits(y);
   if (isnan_bits(a) || isnan_bits(b)) return false;
-  if (((a | b) & kAbs) == 0) return false;  // both zero
-  const int64_t ka = (int64_t)a >= 0 ? (int64_t)a : -(int64_t)(a & kAbs);
-  const int64_t kb = (int64_t)b >= 0 ? (int64_t)b : -(int64_t)(b & kAbs);
+  if (mag2(a | b) == 0) return false;  // both zero
+  // negative numbers order as their magnitudes' complements
+  const int64_t ka = (int64_t)a ^ (((int64_t)a >> 63) & (int64_t)kAbs);
+  const int64_t kb = (int64_t)b ^ (((int64_t)b >> 63) & (int64_t)kAbs);
   return ka > kb;
 }
 

@@ -560,7 +560,7 @@ __global__ void k_distance0(Box b, const double* __restrict__ phi0, double* dist
   // opposite signs, zero counted as negative; the tests on the integer pipes
   // (a native comparison occupies the FP64 pipe like an addition)
   bool near = false;
-  const bool pos = qss_emu::gt0(cc), nonpos = qss_emu::lt0(cc) || (qss_emu::bits(cc) & qss_emu::kAbs) == 0;
+  const bool pos = qss_emu::gt0(cc), nonpos = qss_emu::lt0(cc) || qss_emu::mag2(qss_emu::bits(cc)) == 0;
 #pragma unroll
   for (int q = 0; q < 6; q++) {
     const bool np = qss_emu::gt0(n[q]);
@@ -638,13 +638,13 @@ __device__ __forceinline__ double reinit_rhs_e(const double* __restrict__ phi, c
                                                const double* __restrict__ distance0, const Box& b, int64_t c,
                                                const Inv& inv, double max_dx, uint64_t far_bits) {
   using namespace qss_emu;
-  const uint64_t tol_bits = bits(1.e-5);
+  const uint64_t tol2 = mag2(bits(1.e-5));
   const int64_t sy = b.sy(), sz = b.sz();
   auto scale = [](double d, double f) -> double { return EMU >= 2 ? qss_emu::mul(d, f) : d * f; };
   const double cc = __ldg(phi + c);
   const double p0 = phi0[c];
-  const uint64_t ap0 = bits(p0) & kAbs;
-  const bool sgn_nz = ap0 > tol_bits && ap0 <= 0x7ff0000000000000ull;  // fabs(p0) > 1e-5
+  const uint64_t ap0 = mag2(bits(p0));
+  const bool sgn_nz = ap0 > tol2 && ap0 <= kInf2;  // fabs(p0) > 1e-5
   const bool sgn_neg = (int64_t)bits(p0) < 0;
   const double sgn = sgn_nz ? (sgn_neg ? -1.0 : 1.0) : 0.0;
   const double d0 = distance0[c];
@@ -667,8 +667,8 @@ __device__ __forceinline__ double reinit_rhs_e(const double* __restrict__ phi, c
       }
       gs[d] = max_nonneg(a_, b_);
     }
-    const uint64_t acc = bits(cc) & kAbs;
-    if (acc > tol_bits && acc <= 0x7ff0000000000000ull) {  // fabs(cc) > 1e-5
+    const uint64_t acc = mag2(bits(cc));
+    if (acc > tol2 && acc <= kInf2) {  // fabs(cc) > 1e-5
       const double ngps = scale(gs[0], gs[0]) + scale(gs[1], gs[1]) + scale(gs[2], gs[2]);
       const double s = qss_emu::sqrt(ngps);
       if (!sgn_nz) return sgn - sgn * s;
@@ -688,10 +688,10 @@ __device__ __forceinline__ double reinit_rhs_e(const double* __restrict__ phi, c
 __device__ __forceinline__ double reinit_rhs_diffs(double cc, double p0, double d0, const double gp[3],
                                                    const double gm[3], double max_dx, uint64_t far_bits) {
   using namespace qss_emu;
-  const uint64_t tol_bits = bits(1.e-5);
+  const uint64_t tol2 = mag2(bits(1.e-5));
   auto scale = [](double d, double f) -> double { return qss_emu::mul(d, f); };
-  const uint64_t ap0 = bits(p0) & kAbs;
-  const bool sgn_nz = ap0 > tol_bits && ap0 <= 0x7ff0000000000000ull;  // fabs(p0) > 1e-5
+  const uint64_t ap0 = mag2(bits(p0));
+  const bool sgn_nz = ap0 > tol2 && ap0 <= kInf2;  // fabs(p0) > 1e-5
   const bool sgn_neg = (int64_t)bits(p0) < 0;
   const double sgn = sgn_nz ? (sgn_neg ? -1.0 : 1.0) : 0.0;
   if (bits(d0) == far_bits) {
@@ -709,8 +709,8 @@ __device__ __forceinline__ double reinit_rhs_diffs(double cc, double p0, double 
       }
       gs[d] = max_nonneg(a_, b_);
     }
-    const uint64_t acc = bits(cc) & kAbs;
-    if (acc > tol_bits && acc <= 0x7ff0000000000000ull) {  // fabs(cc) > 1e-5
+    const uint64_t acc = mag2(bits(cc));
+    if (acc > tol2 && acc <= kInf2) {  // fabs(cc) > 1e-5
       const double ngps = scale(gs[0], gs[0]) + scale(gs[1], gs[1]) + scale(gs[2], gs[2]);
       const double s = qss_emu::sqrt(ngps);
       if (!sgn_nz) return sgn - sgn * s;
@@ -741,9 +741,17 @@ __device__ __forceinline__ double reinit_rhs_diffs(double cc, double p0, double 
 // test per operation.  The floor of 2^-255 in place of a zero changes no bit:
 // the root it could reach is below 2^-100, and sgn - root, and phi + dt r,
 // round to the same number.  Differences of 2^100 or more (infinities and
-// NaNs among them) take the general path, reinit_rhs_diffs.  FP64
-// instructions per voxel: 3.4 differences, 2 sums, sgn - root, phi + dt r;
-// that is the kernel's bound.
+// NaNs among them) take the general path, reinit_rhs_diffs.  A voxel next to
+// the interface differs in two operands only, d0 - |phi| / max_dx in place of
+// sgn - root, so it shares the subtraction and the update; the reciprocal of
+// max_dx is computed once per thread.  (Sent through the general path, the ~10 %
+// of a sphere pack's voxels that lie there cost most warps a second set of FP64
+// instructions: 200^3, 311 us a sweep against 185.)
+//
+// FP64 instructions per voxel: 3 differences and the edges', 2 sums,
+// sgn - root, phi + dt r; they take 616 cycles of the ~720 the sweep takes per
+// warp and plane, and with one or both sums moved to the integer pipes it is
+// 1 and 5 % slower.
 //
 // GHOST: the layer next to the fill box is not read but extrapolated from the
 // two voxels inside it (extrap with distance 1, as k_ghost would leave it), so
@@ -793,6 +801,9 @@ __global__ void __launch_bounds__(128, 10) k_reinit_walk(Box b, ReinitSweep a) {
   const int k1 = k0 + a.walk - 1 < b.khi ? k0 + a.walk - 1 : b.khi;
   const int64_t sy = b.sy(), sz = b.sz();
   const Inv inv = a.inv;
+  const uint32_t dxh = hi32(a.max_dx), dxl = lo32(a.max_dx);
+  bool seed_ok = true;
+  const uint32_t dx_recip = recip30(mant_hi(dxh), dxl, seed_ok);
   int64_t c = b.idx(i, j, k0);
   // the lane's share of the low edges: a neighbour's offset from c, and whether
   // that neighbour lies in the ghost layer
@@ -838,20 +849,26 @@ __global__ void __launch_bounds__(128, 10) k_reinit_walk(Box b, ReinitSweep a) {
       const int64_t wx = ux > vx ? ux : vx, wy = uy > vy ? uy : vy, wz = uz > vz ? uz : vz;
       const int hx = max((int)(wx >> 32), 0x30000000), hy = max((int)(wy >> 32), 0x30000000),
                 hz = max((int)(wz >> 32), 0x30000000);
-      const uint64_t acc = bits(cc) & kAbs, ap0 = bits(p0) & kAbs;
-      constexpr uint64_t inf = 0x7ff0000000000000ull;
-      const uint64_t tol = 0x3ee4f8b588e368f1ull;  // 1e-5
+      const uint64_t acc2 = mag2(bits(cc)), ap02 = mag2(bits(p0)), tol2 = mag2(0x3ee4f8b588e368f1ull);  // 1e-5
+      const uint32_t ach = hi32(cc) & 0x7fffffffu;
+      const bool far = bits(d0) == a.far_bits;
+      const bool plain = far ? max(max(hx, hy), hz) < 0x46300000 && acc2 > tol2 && acc2 <= kInf2
+                             : ach - 0x3af00000u < 0x0b400000u && (hi32(d0) & 0x7fffffffu) < 0x46300000u;
       double r;
-      if (bits(d0) == a.far_bits && max(max(hx, hy), hz) < 0x46300000 && acc > tol && acc <= inf && ap0 > tol &&
-          ap0 <= inf) {
-        const double gx = mul_win((uint32_t)hx, (uint32_t)wx, hi32(inv.x), lo32(inv.x));
-        const double gy = mul_win((uint32_t)hy, (uint32_t)wy, hi32(inv.y), lo32(inv.y));
-        const double gz = mul_win((uint32_t)hz, (uint32_t)wz, hi32(inv.z), lo32(inv.z));
-        const double n2 = sq_win(hi32(gx), lo32(gx)) + sq_win(hi32(gy), lo32(gy)) + sq_win(hi32(gz), lo32(gz));
-        const double root = sqrt_win(hi32(n2), lo32(n2));
+      if (plain && ap02 > tol2 && ap02 <= kInf2) {
         const uint32_t neg0 = hi32(p0) & 0x80000000u;  // sgn = +-1
-        const double sgn = __hiloint2double((int)(0x3ff00000u | neg0), 0);
-        r = sgn + __hiloint2double((int)(hi32(root) ^ neg0 ^ 0x80000000u), (int)lo32(root));
+        double from = d0, mag;
+        if (far) {
+          const double gx = mul_win((uint32_t)hx, (uint32_t)wx, hi32(inv.x), lo32(inv.x));
+          const double gy = mul_win((uint32_t)hy, (uint32_t)wy, hi32(inv.y), lo32(inv.y));
+          const double gz = mul_win((uint32_t)hz, (uint32_t)wz, hi32(inv.z), lo32(inv.z));
+          const double n2 = sq_win(hi32(gx), lo32(gx)) + sq_win(hi32(gy), lo32(gy)) + sq_win(hi32(gz), lo32(gz));
+          mag = sqrt_win(hi32(n2), lo32(n2));
+          from = __hiloint2double((int)(0x3ff00000u | neg0), 0);
+        } else {
+          mag = div_recip(ach, lo32(cc), dxh, dxl, dx_recip);
+        }
+        r = from + __hiloint2double((int)(hi32(mag) ^ neg0 ^ 0x80000000u), (int)lo32(mag));
         if (!a.rhs_only) {
           // dt r with |r| raised to 2^-255 (r = 0: phi + tiny rounds to phi)
           const uint32_t ar = hi32(r) & 0x7fffffffu;

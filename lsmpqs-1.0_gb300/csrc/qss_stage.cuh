@@ -29,8 +29,8 @@ __device__ __forceinline__ double sqw(double x) { return qss_emu::sq_win(qss_emu
 
 // |v| >= 1e-5 (false for NaN)
 __device__ __forceinline__ bool speed_valid(double v) {
-  const uint64_t a = qss_emu::bits(v) & qss_emu::kAbs;
-  return a >= qss_emu::bits(1.e-5) && a <= 0x7ff0000000000000ull;
+  const uint64_t a = qss_emu::mag2(qss_emu::bits(v));
+  return a >= 0x7dc9f16b11c6d1e2ull && a <= qss_emu::kInf2;
 }
 
 // host: factors the fast paths accept
