@@ -935,53 +935,183 @@ __device__ __forceinline__ MaskGeom mask_geom(double m, double mx, double my, do
   return g;
 }
 
-__global__ void k_setvarnorm(Box b, const double* __restrict__ mask, const double* __restrict__ mx,
-                             const double* __restrict__ my, const double* __restrict__ mz, double* vel_n,
-                             double a0, const double* theta_field, double theta, double dx) {
-  const int i = b.ilo + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = b.jlo + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = b.klo + blockIdx.z * blockDim.z + threadIdx.z;
-  if (i > b.ihi || j > b.jhi || k > b.khi) return;
-  const int64_t c = b.idx(i, j, k);
+// The coefficients from the mask and its gradient: CURV the curvature
+// coefficient and the advection velocity with their CFL maxima, otherwise the
+// normal velocity.  The smoothed step of the mask is 0 or 1 for most voxels,
+// and what is left of the expressions there needs no FP64 instruction in the
+// pore space (a0; the curvature coefficient and signed zeros) and four in the
+// solid.  The voxels inside the smoothing band, whose sines and divisions are
+// ~70 FP64 instructions, and those with operands out of range (SetVar::plain,
+// coef_plain) are gathered per block of 1024 voxels and evaluated by full warps.
+// The maxima go over integer keys: a native comparison occupies the FP64 pipe
+// like an addition.  With everything evaluated natively everywhere the two
+// kernels took 2.4 ms each at 192^3.
+struct SetVar {
+  const double *mask, *mx, *my, *mz, *theta_field;
+  double *vel_n, *vb, *vx, *vy, *vz;
+  double coef;  // a0, or the constant curvature coefficient
+  double theta, dx;
+  bool plain;
+  unsigned long long* red;
+  double eps, inv, coef0;  // 1.5 dx, 1 / dx, 0 coef
+};
+constexpr int kSetVoxels = 1024, kSetThreads = 256;
+
+struct SetVarOut {
+  double a, x, y, z;  // normal velocity; or curvature coefficient and velocity
+};
+
+template <bool CURV>
+__device__ __noinline__ SetVarOut setvar_native(double m, double gx, double gy, double gz, double theta, double coef,
+                                                double dx) {
   const double C2 = 1;
-  MaskGeom g = mask_geom(mask[c], mx[c], my[c], mz[c], dx);
-  const double ca = theta_field ? theta_field[c] : theta;
-  vel_n[c] = g.h1 * a0 - g.s * g.h2 * C2 * portable_cos(ca) * g.absgrad;
+  const MaskGeom g = mask_geom(m, gx, gy, gz, dx);
+  if (CURV) return {g.h1 * coef, g.s * C2 * gx * g.h2, g.s * C2 * gy * g.h2, g.s * C2 * gz * g.h2};
+  return {g.h1 * coef - g.s * g.h2 * C2 * portable_cos(theta) * g.absgrad, 0.0, 0.0, 0.0};
 }
 
-__global__ void k_setvarcurvadv(Box b, const double* __restrict__ mask, const double* __restrict__ mx,
-                                const double* __restrict__ my, const double* __restrict__ mz, double* vb,
-                                double* vx, double* vy, double* vz, double const_b, double dx,
-                                unsigned long long* red) {
-  const int i = b.ilo + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = b.jlo + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = b.klo + blockIdx.z * blockDim.z + threadIdx.z;
-  double bm = -1.0, um = -1.0;
-  if (i <= b.ihi && j <= b.jhi && k <= b.khi) {
-    const int64_t c = b.idx(i, j, k);
-    const double C1 = const_b, C2 = 1;
-    const double inv_dx = 1.0 / dx, inv_dy = 1.0 / dx, inv_dz = 1.0 / dx;
-    const double gx = mx[c], gy = my[c], gz = mz[c];
-    MaskGeom g = mask_geom(mask[c], gx, gy, gz, dx);
-    const double bv = g.h1 * C1;
-    vb[c] = bv;
-    bm = bv;
-    const double ux = g.s * C2 * gx * g.h2;
-    const double uy = g.s * C2 * gy * g.h2;
-    const double uz = g.s * C2 * gz * g.h2;
-    vx[c] = ux;
-    vy[c] = uy;
-    vz[c] = uz;
-    um = fabs(ux) * inv_dx + fabs(uy) * inv_dy + fabs(uz) * inv_dz;
+// the mask in [2^-127, 2^129) and the gradient below 2^129
+__device__ __forceinline__ bool coef_plain(double m, double gx, double gy, double gz, uint32_t& top) {
+  using namespace qss_emu;
+  top = max(max(hi32(gx) & 0x7fffffffu, hi32(gy) & 0x7fffffffu), hi32(gz) & 0x7fffffffu);
+  return win8(m) < kWin8 && top < 0x48000000u;
+}
+
+// s and |gradient| of mask_geom, where the largest component is 2^-127 or more
+// (the floor of 2^-255 under the others changes no sum)
+__device__ __forceinline__ void sign_geom(double m, double gx, double gy, double gz, double dx, double& s, double& ag) {
+  using namespace qss_emu;
+  auto sq = [](double v) { return sq_win(max(hi32(v) & 0x7fffffffu, 0x30000000u), lo32(v)); };
+  const double a2 = sq(gx) + sq(gy) + sq(gz);
+  ag = sqrt_win(hi32(a2), lo32(a2));
+  const double x2 = sqw(m) + mulw(mulw(mulw(ag, dx), ag), dx);
+  const double x = sqrt_win(hi32(x2), lo32(x2));
+  bool ok = true;
+  s = div_win(hi32(m), lo32(m), hi32(x), lo32(x), ok);
+}
+
+template <bool CURV>
+__global__ void __launch_bounds__(kSetThreads) k_setvar(Box b, SetVar a) {
+  using namespace qss_emu;
+  __shared__ uint16_t band[kSetVoxels];
+  __shared__ int band_n;
+  __shared__ double cos_theta;
+  const uint32_t fbx = (uint32_t)b.fbx(), fby = (uint32_t)b.fby();
+  const int64_t base = (int64_t)blockIdx.x * kSetVoxels, n = (int64_t)fbx * fby * b.fbz();
+  const int64_t row0 = base / fbx;
+  const uint32_t i0 = (uint32_t)(base - row0 * fbx), k0 = (uint32_t)(row0 / fby),
+                 j0 = (uint32_t)(row0 - (int64_t)k0 * fby);
+  auto at = [&](uint32_t t) {  // index of the block's voxel t
+    const uint32_t x = i0 + t, r = x / fbx, y = j0 + r, q = y / fby;
+    return b.idx(b.ilo + (int)(x - r * fbx), b.jlo + (int)(y - q * fby), b.klo + (int)(k0 + q));
+  };
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) band_n = 0;
+  if (!CURV && !a.theta_field && threadIdx.x < 32) {
+    const double ct = portable_cos(a.theta);
+    if (threadIdx.x == 0) cos_theta = ct;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    bm = dmax(bm, __shfl_down_sync(0xffffffffu, bm, o));
-    um = dmax(um, __shfl_down_sync(0xffffffffu, um, o));
+  __syncthreads();
+  const double eps = a.eps, inv = a.inv;
+  unsigned long long bm = 0, um = 0;  // keys, 0: none; NaNs count as none
+  auto keep = [&](const SetVarOut& r) {
+    const double u = qss_emu::abs(r.x) * inv + qss_emu::abs(r.y) * inv + qss_emu::abs(r.z) * inv;
+    const unsigned long long kb = isnan_bits(bits(r.a)) ? 0 : double_to_key(r.a);
+    const unsigned long long ku = isnan_bits(bits(u)) ? 0 : double_to_key(u);
+    bm = kb > bm ? kb : bm;
+    um = ku > um ? ku : um;
+  };
+  auto put = [&](int64_t c, const SetVarOut& r) {
+    if (CURV) {
+      a.vb[c] = r.a;
+      a.vx[c] = r.x;
+      a.vy[c] = r.y;
+      a.vz[c] = r.z;
+    } else {
+      a.vel_n[c] = r.a;
+    }
+  };
+  for (int t0 = 0; t0 < kSetVoxels; t0 += kSetThreads) {
+    const uint32_t t = t0 + threadIdx.x;
+    bool rest = false;
+    if (base + t < n) {
+      const int64_t c = at(t);
+      const double m = a.mask[c], gx = a.mx[c], gy = a.my[c], gz = a.mz[c];
+      uint32_t top;
+      rest = !(a.plain && coef_plain(m, gx, gy, gz, top));
+      const bool pore = gt(neg(eps), m), solid = gt(m, eps);
+      rest = rest || !(pore || (solid && top >= 0x38000000u));
+      if (!CURV && a.theta_field) rest = rest || (hi32(a.theta_field[c]) & 0x7fffffffu) >= 0x41300000u;  // 2^20
+      if (!rest) {
+        SetVarOut r{};
+        if (pore) {
+          r.a = a.coef;
+          if (CURV) {  // s is negative
+            r.x = __hiloint2double((int)(~hi32(gx) & 0x80000000u), 0);
+            r.y = __hiloint2double((int)(~hi32(gy) & 0x80000000u), 0);
+            r.z = __hiloint2double((int)(~hi32(gz) & 0x80000000u), 0);
+            const unsigned long long kb = double_to_key(r.a), ku = double_to_key(0.0);
+            bm = kb > bm ? kb : bm;
+            um = ku > um ? ku : um;
+          }
+          put(c, r);
+        } else {
+          double s, ag;
+          sign_geom(m, gx, gy, gz, a.dx, s, ag);
+          if (CURV) {
+            r.a = a.coef0;
+            r.x = mul(s, gx);
+            r.y = mul(s, gy);
+            r.z = mul(s, gz);
+            keep(r);
+            put(c, r);
+          } else {
+            const double v = mul(mul(s, a.theta_field ? portable_cos(a.theta_field[c]) : cos_theta), ag);
+            r.a = neg(v);  // 0 a0 - v
+            rest = mag2(bits(v)) == 0;
+            if (!rest) put(c, r);
+          }
+        }
+      }
+    }
+    const unsigned vote = __ballot_sync(0xffffffffu, rest);
+    int slot = 0;
+    if (lane == 0 && vote) slot = atomicAdd(&band_n, __popc(vote));
+    slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(vote & ((1u << lane) - 1u));
+    if (rest) band[slot] = (uint16_t)t;
   }
-  const int lane = (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z)) & 31;
-  if (lane == 0) {
-    atomicMax(&red[0], double_to_key(bm));
-    atomicMax(&red[1], double_to_key(um));
+  __syncthreads();
+  for (int e = threadIdx.x; e < band_n; e += kSetThreads) {
+    const int64_t c = at(band[e]);
+    const double m = a.mask[c], gx = a.mx[c], gy = a.my[c], gz = a.mz[c];
+    uint32_t top;
+    SetVarOut r{};
+    if (a.plain && coef_plain(m, gx, gy, gz, top) && top >= 0x38000000u && gt(m, neg(eps)) && gt(eps, m) &&
+        !(!CURV && a.theta_field)) {
+      // both smoothed steps from one quotient and one sine, which are odd in m
+      double s, ag;
+      sign_geom(m, gx, gy, gz, a.dx, s, ag);
+      const double pi = 3.14159265358979323846, one_over_pi = 0.31830988618379;
+      const double q = div(m, 2 * eps), w = (0.5 * one_over_pi) * portable_sin(div(mul(pi, m), eps));
+      const double h1 = 0.5 - q - w, h2 = 0.5 + q + w;
+      if (CURV) r = {h1 * a.coef, mul(mul(s, gx), h2), mul(mul(s, gy), h2), mul(mul(s, gz), h2)};
+      else r.a = h1 * a.coef - mul(mul(mul(s, h2), cos_theta), ag);
+    } else {
+      r = setvar_native<CURV>(m, gx, gy, gz, CURV ? 0.0 : (a.theta_field ? a.theta_field[c] : a.theta), a.coef, a.dx);
+    }
+    if (CURV) keep(r);
+    put(c, r);
+  }
+  if (CURV) {
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long x = __shfl_down_sync(0xffffffffu, bm, o), y = __shfl_down_sync(0xffffffffu, um, o);
+      bm = x > bm ? x : bm;
+      um = y > um ? y : um;
+    }
+    if (lane == 0) {
+      atomicMax(&a.red[0], bm);
+      atomicMax(&a.red[1], um);
+    }
   }
 }
 
@@ -1444,10 +1574,16 @@ void launch_central_grad(cudaStream_t s, const Box& b, const double* f, double* 
   k_central_grad<<<fb_grid(b, kBlk3), kBlk3, 0, s>>>(b, f, fx, fy, fz, Fac{0.5 / dx, 0.5 / dy, 0.5 / dz});
 }
 
+static unsigned setvar_blocks(const Box& b) {
+  return (unsigned)(((int64_t)b.fbx() * b.fby() * b.fbz() + kSetVoxels - 1) / kSetVoxels);
+}
+
 void launch_setvarnorm(cudaStream_t s, const Box& b, const double* mask, const double* mx, const double* my,
                        const double* mz, double* vel_n, double a0, const double* theta_field, double theta,
                        double dx) {
-  k_setvarnorm<<<fb_grid(b, kBlk3), kBlk3, 0, s>>>(b, mask, mx, my, mz, vel_n, a0, theta_field, theta, dx);
+  SetVar a{mask, mx, my, mz, theta_field, vel_n, nullptr, nullptr, nullptr, nullptr, a0, theta, dx, false, nullptr, 1.5 * dx, 1.0 / dx, 0.0};
+  a.plain = stage_factor(dx) && a0 != 0.0 && isfinite(a0) && (theta_field || fabs(theta) < 0x1p20);
+  k_setvar<false><<<setvar_blocks(b), kSetThreads, 0, s>>>(b, a);
 }
 
 void launch_setvarcurvadv(cudaStream_t s, const Box& b, const double* mask, const double* mx, const double* my,
@@ -1455,7 +1591,9 @@ void launch_setvarcurvadv(cudaStream_t s, const Box& b, const double* mask, cons
                           double dx, unsigned long long* red) {
   unsigned long long init[2] = {double_to_key(-1.0), double_to_key(-1.0)};
   cudaMemcpyAsync(red, init, sizeof init, cudaMemcpyHostToDevice, s);
-  k_setvarcurvadv<<<fb_grid(b, kBlk3), kBlk3, 0, s>>>(b, mask, mx, my, mz, vb, vx, vy, vz, const_b, dx, red);
+  SetVar a{mask, mx, my, mz, nullptr, nullptr, vb, vx, vy, vz, const_b, 0.0, dx, false, red, 1.5 * dx, 1.0 / dx, 0.0 * const_b};
+  a.plain = stage_factor(dx) && isfinite(const_b);
+  k_setvar<true><<<setvar_blocks(b), kSetThreads, 0, s>>>(b, a);
 }
 
 void launch_trapvel(cudaStream_t s, const Box& b, const double* test, double* vel_n, double* vb, double* vx,
