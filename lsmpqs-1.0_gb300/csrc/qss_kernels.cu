@@ -162,6 +162,7 @@ struct StageArgs {
   Coef c;
   ImposeArgs im;
   const Ctl* ctl;
+  int walk;  // planes per block (k_eno2)
 };
 
 template <int SCHEME, bool VAR, int STAGE, bool FINAL>
@@ -233,25 +234,18 @@ __global__ void __launch_bounds__(128) k_stage(StageArgs a) {
 // ---------------------------------------------------------------------------
 // ENO2 / ENO3 stage at EMU 2: the one-sided differences with native additions and
 // integer comparisons, the rest as in qss_stage.cuh.  Blocks of four 8 x 4
-// patches (see k_weno_combine).  Bound: FP64 pipe (66 additions a voxel for ENO2).
-// A stage of constant coefficients on GB300, ENO2: 128^3 0.69 -> 0.32 ms, 64^3 0.085
-// -> 0.054 ms against k_stage (80 registers, 6 blocks per SM; 8 blocks the same).
+// patches (see k_weno_combine).  Bound: FP64 pipe.  ENO2 with every voxel by itself
+// takes 63 FP64 instructions a voxel, with the differences shared (k_eno2) 48; a step of
+// constant coefficients on GB300 0.54 -> 0.48 ms at 128^3, 0.116 -> 0.109 ms at 64^3
+// (two stages, ghost layers and the CFL step).  Walks of k_eno2 as long as
+// kEno2Target blocks per SM allow: at 128^3 6 per SM 0.60 ms, 12 0.52, 18 to 40
+// 0.48, 60 0.49; 7 or 8 resident blocks the same as 6.
+constexpr int kEno2Blocks = 6, kEno2Target = 32, kEno2Walk = 16;
 
 // |x| < |y| (false where y is NaN)
 __device__ __forceinline__ bool abs_lt(double x, double y) {
   const uint64_t a = qss_emu::bits(x) << 1, b = qss_emu::bits(y) << 1;
   return a < b && b <= 0xffe0000000000000ull;
-}
-
-// eno2_pm without the scaling by inv
-__device__ __forceinline__ void eno2_raw(const double s[5], double& plus, double& minus) {
-  using qss_emu::scale2;
-  const double D1 = s[2] - s[1], D1p = s[3] - s[2];
-  const double D2 = s[3] + s[1] - scale2(s[2], 1);
-  const double D2p = s[4] + s[2] - scale2(s[3], 1);
-  const double D2m = s[0] + s[2] - scale2(s[1], 1);
-  plus = D1p - scale2(abs_lt(D2, D2p) ? D2 : D2p, -1);
-  minus = D1 + scale2(abs_lt(D2m, D2) ? D2m : D2, -1);
 }
 
 // eno3_pm without the scaling
@@ -275,23 +269,17 @@ __device__ __forceinline__ void eno3_raw(const double s[7], double& plus, double
   minus = (D1 + scale2(m ? D2m : D2, -1)) + (m ? tm : neg(tm));
 }
 
-// unscaled one-sided differences of the three axes at (i, j, k)
-template <int SCHEME>
-__device__ __forceinline__ void eno_raw(const double* __restrict__ phi, const Box& b, int i, int j, int64_t c,
-                                        double pp[3], double pm[3]) {
-  constexpr int R = SCHEME == ENO2 ? 2 : 3;
+// unscaled ENO3 one-sided differences of the three axes at (i, j, k)
+__device__ __forceinline__ void eno3_axes(const double* __restrict__ phi, const Box& b, int i, int j, int64_t c,
+                                          double pp[3], double pm[3]) {
   const int64_t st[3] = {1, b.sy(), b.sz()};
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    double s[2 * R + 1];
+    double s[7];
 #pragma unroll
-    for (int o = -R; o <= R; o++) s[o + R] = __ldg(phi + c + o * st[d]);
-    if (SCHEME == ENO2) {
-      eno2_raw(s, pp[d], pm[d]);
-    } else {
-      if (d == 0) s[2 * R] = __ldg(phi + b.idx(i + 3, j, j));  // 3d.f:677
-      eno3_raw(s, pp[d], pm[d]);
-    }
+    for (int o = -3; o <= 3; o++) s[o + 3] = __ldg(phi + c + o * st[d]);
+    if (d == 0) s[6] = __ldg(phi + b.idx(i + 3, j, j));  // 3d.f:677
+    eno3_raw(s, pp[d], pm[d]);
   }
 }
 
@@ -304,8 +292,31 @@ __device__ __noinline__ double carried_norm(const double* __restrict__ phi, cons
   return godunov_norm<SCHEME>(vel_n[src], qp, qm);
 }
 
-template <int SCHEME, bool VAR, int STAGE, bool FINAL>
-__global__ void __launch_bounds__(128, 6) k_eno(StageArgs a) {
+// the rest of a stage at one voxel from its unscaled one-sided differences
+template <int SCHEME, bool VAR, int STAGE, bool FINAL, bool INT>
+__device__ __forceinline__ void eno_finish(const StageArgs& a, int64_t idx, const double pp[3], const double pm[3]) {
+  const Box& b = a.b;
+  const double* __restrict__ phi = a.phi_in;
+  const double vel = VAR ? a.c.vel_n[idx] : a.c.a_const;
+  double rhs = 0.0;
+  if (speed_valid(vel)) {
+    rhs = godunov_fast<SCHEME, true, INT>(vel, pp, pm, a.inv);
+  } else if (VAR) {
+    // a voxel at rest keeps the term of the closest preceding voxel of its slab
+    const int src = a.c.nsrc[idx];
+    if (src >= 0) rhs = carried_norm<SCHEME>(phi, b, src, a.inv, a.c.vel_n);
+  }
+  const double bco = VAR ? a.c.b[idx] : a.c.b_const;
+  if (!VAR || qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign)  // as in k_weno_combine2
+    rhs = rhs + qss_emu::mul(bco, curvature_fast<INT>(phi, b, idx, a.fac));
+  if (VAR) rhs = add_advection<true>(rhs, a.c.vx[idx], a.c.vy[idx], a.c.vz[idx], pp, pm, a.inv);
+  const double out = rk_combine<STAGE>(rhs, STAGE ? a.ctl->dt : 0.0, STAGE ? __ldg(phi + idx) : 0.0, a.u_cur, idx);
+  a.out[idx] = out;
+  if (FINAL) a.phi_new[idx] = impose3_i(out, idx, a.im);
+}
+
+template <bool VAR, int STAGE, bool FINAL>
+__global__ void __launch_bounds__(128, 6) k_eno3(StageArgs a) {
   if (STAGE != 0 && !a.ctl->active) return;
   const Box& b = a.b;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -314,25 +325,90 @@ __global__ void __launch_bounds__(128, 6) k_eno(StageArgs a) {
   const int k = b.klo + blockIdx.z;
   if (i > b.ihi || j > b.jhi) return;
   const int64_t idx = b.idx(i, j, k);
-  const double* __restrict__ phi = a.phi_in;
   double pp[3], pm[3];
-  eno_raw<SCHEME>(phi, b, i, j, idx, pp, pm);
-  const double vel = VAR ? a.c.vel_n[idx] : a.c.a_const;
-  double rhs = 0.0;
-  if (speed_valid(vel)) {
-    rhs = godunov_fast<SCHEME, true>(vel, pp, pm, a.inv);
-  } else if (VAR) {
-    // a voxel at rest keeps the term of the closest preceding voxel of its slab
-    const int src = a.c.nsrc[idx];
-    if (src >= 0) rhs = carried_norm<SCHEME>(phi, b, src, a.inv, a.c.vel_n);
+  eno3_axes(a.phi_in, b, i, j, idx, pp, pm);
+  eno_finish<ENO3, VAR, STAGE, FINAL, false>(a, idx, pp, pm);
+}
+
+// ENO2 with each difference computed once.  On an axis, with d1(v) = phi(v + 1) -
+// phi(v), d2(v) = phi(v + 1) + phi(v - 1) - 2 phi(v) and m(v) the smaller of d2(v)
+// and d2(v + 1) in magnitude, the plus difference of v is d1(v) - m(v) / 2 and the
+// minus difference d1(v - 1) + m(v - 1) / 2: three FP64 instructions for d1 and d2
+// and two for the sums, against ten for a voxel by itself.  A warp owns an 8 x 4
+// patch (x neighbours one lane apart, y neighbours eight) and walks `walk` planes
+// along k with the z terms carried; d2 outside the patch's four edges, and d1 below
+// the two low ones, is one more evaluation by 24 of the lanes.  The sums of squares
+// go over the integer pipes, which have the time.
+template <bool VAR, int STAGE, bool FINAL>
+__global__ void __launch_bounds__(128, kEno2Blocks) k_eno2(StageArgs a) {
+  using qss_emu::scale2;
+  if (STAGE != 0 && !a.ctl->active) return;
+  const Box& b = a.b;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int li = lane & 7, lj = lane >> 3;
+  const int i0 = b.ilo + blockIdx.x * 32 + 8 * warp, j0 = b.jlo + blockIdx.y * 4;
+  if (i0 > b.ihi) return;  // the whole warp
+  // lanes past the fill box work on its last row / column and store nothing
+  const int lx = min(7, b.ihi - i0), ly = min(3, b.jhi - j0);
+  const bool ok = li <= lx && lj <= ly;
+  const int k0 = b.klo + blockIdx.z * a.walk, k1 = min(k0 + a.walk - 1, b.khi);
+  const int64_t sy = b.sy(), sz = b.sz();
+  const double* __restrict__ phi = a.phi_in;
+  int64_t c = b.idx(i0 + min(li, lx), j0 + min(lj, ly), k0);
+  // the lane's voxel outside the patch: below (0 - 7) and above (8 - 15) in y, below
+  // (16 - 19) and above (20 - 23) in x; its own for the rest
+  const bool ey = lane < 16;
+  const int er = min(lane & 3, ly);
+  const int64_t e0 = ey ? b.idx(i0 + min(li, lx), lane < 8 ? j0 - 1 : j0 + ly + 1, k0)
+                        : (lane < 24 ? b.idx(lane < 20 ? i0 - 1 : i0 + lx + 1, j0 + er, k0) : c);
+  const int64_t eo = e0 - c, es = ey ? sy : 1;
+  auto d2_of = [](double lo, double mid, double hi) { return __fma_rn(-2.0, mid, hi + lo); };
+  auto pick = [](double x, double y) { return abs_lt(x, y) ? x : y; };
+  auto from = [](double v, int src) { return __shfl_sync(0xffffffffu, v, src); };
+  double cc = __ldg(phi + c), zp = __ldg(phi + c + sz), d2z, d1zl, mzl;
+  {
+    const double zm = __ldg(phi + c - sz);
+    d1zl = cc - zm;
+    d2z = d2_of(zm, cc, zp);
+    mzl = pick(d2_of(__ldg(phi + c - 2 * sz), zm, cc), d2z);
   }
-  const double bco = VAR ? a.c.b[idx] : a.c.b_const;
-  if (!VAR || qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign)  // as in k_weno_combine2
-    rhs = rhs + qss_emu::mul(bco, curvature_fast(phi, b, idx, a.fac));
-  if (VAR) rhs = add_advection<true>(rhs, a.c.vx[idx], a.c.vy[idx], a.c.vz[idx], pp, pm, a.inv);
-  const double out = rk_combine<STAGE>(rhs, STAGE ? a.ctl->dt : 0.0, STAGE ? __ldg(phi + idx) : 0.0, a.u_cur, idx);
-  a.out[idx] = out;
-  if (FINAL) a.phi_new[idx] = impose3_i(out, idx, a.im);
+  for (int k = k0; k <= k1; k++) {
+    const double xp = __ldg(phi + c + 1), xm = __ldg(phi + c - 1), yp = __ldg(phi + c + sy), ym = __ldg(phi + c - sy);
+    const double em = __ldg(phi + c + eo - es), ec = __ldg(phi + c + eo), ep = __ldg(phi + c + eo + es);
+    const double zpp = __ldg(phi + c + 2 * sz);
+    const double d1e = ep - ec, d2e = d2_of(em, ec, ep);
+    const double d1x = xp - cc, d1y = yp - cc, d1z = zp - cc;
+    const double d2x = d2_of(xm, cc, xp), d2y = d2_of(ym, cc, yp), d2zp = d2_of(cc, zp, zpp);
+    double up = __shfl_down_sync(0xffffffffu, d2x, 1), edge = from(d2e, 20 + lj);
+    const double mx = pick(d2x, li >= lx ? edge : up);
+    up = __shfl_down_sync(0xffffffffu, d2y, 8);
+    edge = from(d2e, 8 + li);
+    const double my = pick(d2y, lj >= ly ? edge : up);
+    const double mz = pick(d2z, d2zp);
+    double mxl = __shfl_up_sync(0xffffffffu, mx, 1), d1xl = __shfl_up_sync(0xffffffffu, d1x, 1);
+    edge = from(d2e, 16 + lj);
+    double d1 = from(d1e, 16 + lj);
+    if (li == 0) {
+      mxl = pick(edge, d2x);
+      d1xl = d1;
+    }
+    double myl = __shfl_up_sync(0xffffffffu, my, 8), d1yl = __shfl_up_sync(0xffffffffu, d1y, 8);
+    edge = from(d2e, li);
+    d1 = from(d1e, li);
+    if (lj == 0) {
+      myl = pick(edge, d2y);
+      d1yl = d1;
+    }
+    const double pp[3] = {d1x - scale2(mx, -1), d1y - scale2(my, -1), d1z - scale2(mz, -1)};
+    const double pm[3] = {d1xl + scale2(mxl, -1), d1yl + scale2(myl, -1), d1zl + scale2(mzl, -1)};
+    if (ok) eno_finish<ENO2, VAR, STAGE, FINAL, true>(a, c, pp, pm);
+    d1zl = d1z;
+    mzl = mz;
+    d2z = d2zp;
+    cc = zp;
+    zp = zpp;
+    c += sz;
+  }
 }
 
 template <int SCHEME, bool VAR>
@@ -793,6 +869,7 @@ __global__ void __launch_bounds__(128, 10) k_reinit_walk(Box b, ReinitSweep a) {
   const int field = blockIdx.z / a.chunks, chunk = blockIdx.z - field * a.chunks;
   const double* __restrict__ data = a.data[field];
   const int i0 = b.ilo + blockIdx.x * 32 + 8 * warp, j0 = b.jlo + blockIdx.y * 4;
+  if (i0 > b.ihi) return;  // the whole warp
   const bool ok = i0 + li <= b.ihi && j0 + lj <= b.jhi;
   // lanes past the fill box work on its last row/column (in the box), store nothing
   const int i = i0 + li <= b.ihi ? i0 + li : b.ihi;
@@ -809,7 +886,7 @@ __global__ void __launch_bounds__(128, 10) k_reinit_walk(Box b, ReinitSweep a) {
   // that neighbour lies in the ghost layer
   const bool edge_y = lj == 0, edge_x = li == 0 && lj != 0, corner_x = lane == 9;
   const bool edge = edge_y || edge_x || corner_x;
-  const int64_t ec = corner_x ? b.idx(i0 <= b.ihi ? i0 : b.ihi, j0, k0) - 1 - c : (edge_y ? -sy : -1);
+  const int64_t ec = corner_x ? b.idx(i0, j0, k0) - 1 - c : (edge_y ? -sy : -1);
   const bool edge_ghost = GHOST && ((edge_y && j0 == b.jlo) || ((edge_x || corner_x) && i0 == b.ilo));
   const bool xlast = GHOST && i == b.ihi, ylast = GHOST && j == b.jhi;
   double cc = __ldg(data + c);
@@ -1392,14 +1469,17 @@ static void stage_dispatch(cudaStream_t s, int stage, bool fin, dim3 g, dim3 blk
   }
 }
 
-template <int S, bool V>
-static void eno_dispatch(cudaStream_t s, int stage, bool fin, dim3 g, const StageArgs& a) {
+template <bool V>
+static void eno_dispatch(cudaStream_t s, int scheme, int stage, bool fin, dim3 g, const StageArgs& a) {
+#define QSS_ENO(S, F) \
+  { if (scheme == ENO2) k_eno2<V, S, F><<<g, 128, 0, s>>>(a); else k_eno3<V, S, F><<<g, 128, 0, s>>>(a); }
   switch (stage) {
-    case 0: k_eno<S, V, 0, false><<<g, 128, 0, s>>>(a); break;
-    case 1: if (fin) k_eno<S, V, 1, true><<<g, 128, 0, s>>>(a); else k_eno<S, V, 1, false><<<g, 128, 0, s>>>(a); break;
-    case 2: if (fin) k_eno<S, V, 2, true><<<g, 128, 0, s>>>(a); else k_eno<S, V, 2, false><<<g, 128, 0, s>>>(a); break;
-    default: if (fin) k_eno<S, V, 3, true><<<g, 128, 0, s>>>(a); else k_eno<S, V, 3, false><<<g, 128, 0, s>>>(a); break;
+    case 0: QSS_ENO(0, false) break;
+    case 1: if (fin) QSS_ENO(1, true) else QSS_ENO(1, false) break;
+    case 2: if (fin) QSS_ENO(2, true) else QSS_ENO(2, false) break;
+    default: if (fin) QSS_ENO(3, true) else QSS_ENO(3, false) break;
   }
+#undef QSS_ENO
 }
 
 void launch_stage(cudaStream_t s, int scheme, bool var, int stage, bool final_stage, const Box& b, double dx,
@@ -1421,9 +1501,13 @@ void launch_stage(cudaStream_t s, int scheme, bool var, int stage, bool final_st
   // ENO3 scales its y and z minus differences by 1/dx, the plus ones by 1/dy, 1/dz
   const bool fast = emu_level() >= 2 && scheme != WENO5 && stage_factor(a.fac.x) && stage_factor(a.fac.y) &&
                     stage_factor(a.fac.z) && (scheme == ENO2 || (dx == dy && dx == dz));
-  const dim3 ge((b.fbx() + 31) / 32, (b.fby() + 3) / 4, b.fbz());
-  if (fast && scheme == ENO2) { if (var) eno_dispatch<ENO2, true>(s, stage, final_stage, ge, a); else eno_dispatch<ENO2, false>(s, stage, final_stage, ge, a); }
-  else if (fast) { if (var) eno_dispatch<ENO3, true>(s, stage, final_stage, ge, a); else eno_dispatch<ENO3, false>(s, stage, final_stage, ge, a); }
+  dim3 ge((b.fbx() + 31) / 32, (b.fby() + 3) / 4, b.fbz());
+  if (fast && scheme == ENO2) {
+    const int64_t walk = (int64_t)ge.x * ge.y * b.fbz() / (152 * kEno2Target);
+    a.walk = (int)(walk < 1 ? 1 : (walk > kEno2Walk ? kEno2Walk : walk));
+    ge.z = (b.fbz() + a.walk - 1) / a.walk;
+  }
+  if (fast) { if (var) eno_dispatch<true>(s, scheme, stage, final_stage, ge, a); else eno_dispatch<false>(s, scheme, stage, final_stage, ge, a); }
   else if (scheme == ENO2) { if (var) stage_dispatch<ENO2, true>(s, stage, final_stage, g, kBlk3, a); else stage_dispatch<ENO2, false>(s, stage, final_stage, g, kBlk3, a); }
   else if (scheme == ENO3) { if (var) stage_dispatch<ENO3, true>(s, stage, final_stage, g, kBlk3, a); else stage_dispatch<ENO3, false>(s, stage, final_stage, g, kBlk3, a); }
   else { if (var) stage_dispatch<WENO5, true>(s, stage, final_stage, g, kBlk3, a); else stage_dispatch<WENO5, false>(s, stage, final_stage, g, kBlk3, a); }

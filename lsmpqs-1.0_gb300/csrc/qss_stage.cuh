@@ -42,7 +42,14 @@ static __device__ __noinline__ double curvature_native(const double* __restrict_
   return curvature(phi, b, c, f);
 }
 
+// a + b + c of squares; INT: on the integer pipes
+template <bool INT>
+__device__ __forceinline__ double sum_sq(double a, double b, double c) {
+  return INT ? qss_emu::add_pos(qss_emu::add_pos(a, b), c) : a + b + c;
+}
+
 // curvature() (3d.f:2337-2379), the same operations
+template <bool INT = false>
 __device__ __forceinline__ double curvature_fast(const double* __restrict__ phi, const Box& b, int64_t c,
                                                  const Fac& f) {
   const int64_t sy = b.sy(), sz = b.sz();
@@ -61,7 +68,7 @@ __device__ __forceinline__ double curvature_fast(const double* __restrict__ phi,
   const uint32_t w = win8(dx) | win8(dy) | win8(dz) | win8(dxx) | win8(dyy) | win8(dzz) | win8(dxy) | win8(dxz) | win8(dyz);
   if (w >= kWin8) return curvature_native(phi, b, c, f);
   const double x = mulw(dx, f.x), y = mulw(dy, f.y), z = mulw(dz, f.z);
-  const double g2 = sqw(x) + sqw(y) + sqw(z);
+  const double g2 = sum_sq<INT>(sqw(x), sqw(y), sqw(z));
   if (qss_emu::bits(g2) < 0x3ee4f8b588e368f1ull) return 0.0;  // 1e-5
   const double xx = mulw(mulw(dxx, f.x), f.x);
   const double yy = mulw(mulw(dyy, f.y), f.y);
@@ -88,7 +95,7 @@ __device__ __noinline__ double godunov_native(double vel, double px, double py, 
 // The larger of the two candidates of an axis is picked before it is scaled and
 // squared (rounding is monotone), as a signed integer maximum raised to 2^-255:
 // beside a largest candidate of 2^-127 or more the floor changes no sum.
-template <int SCHEME, bool SCALE>
+template <int SCHEME, bool SCALE, bool INT = false>
 __device__ __forceinline__ double godunov_fast(double vel, const double pp[3], const double pm[3], const Inv& inv) {
   using namespace qss_emu;
   const uint64_t sm = gt0(vel) ? 0 : kSign, sp = sm ^ kSign;  // vel > 0: max(pm, -pp, 0), else max(-pm, pp, 0)
@@ -111,7 +118,7 @@ __device__ __forceinline__ double godunov_fast(double vel, const double pp[3], c
       if (SCALE) g = mulw(g, iv[d]);
       s[d] = sqw(g);
     }
-    const double n2 = s[0] + s[1] + s[2];
+    const double n2 = sum_sq<INT>(s[0], s[1], s[2]);
     const double r = mulw(vel, sqrt_win(hi32(n2), lo32(n2)));
     return SCHEME == WENO5 ? r : neg(r);
   }
