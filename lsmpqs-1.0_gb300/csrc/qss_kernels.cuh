@@ -197,9 +197,10 @@ void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, d
                    double eps, double* scratch, double* out);
 // the sequentially rounded sum c[0] + c[1] + ... + c[n-1] (qss_volsum.cu);
 // scratch holds loop_sum_scratch_doubles(n) doubles
-int64_t loop_sum_scratch_doubles(int64_t n);
+constexpr int kVolChunk = 1024;  // consecutive elements to a chunk of the sum
+constexpr int64_t loop_sum_scratch_doubles(int64_t n) { return 8 * ((n + kVolChunk - 1) / kVolChunk) + 64; }
 void launch_loop_sum(cudaStream_t s, const double* c, int64_t n, double* scratch, double* out);
-inline int64_t volume_scratch_doubles(int64_t nfb) { return nfb + loop_sum_scratch_doubles(nfb); }
+constexpr int64_t volume_scratch_doubles(int64_t nfb) { return nfb + loop_sum_scratch_doubles(nfb); }
 
 // ---- geometry ------------------------------------------------------------
 void launch_sphere(cudaStream_t s, const Box& b, double* phi, const double* x_lo_gb, const double* dxv,

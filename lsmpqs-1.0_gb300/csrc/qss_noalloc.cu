@@ -23,10 +23,10 @@
 using namespace qss;
 
 // Largest fill box accepted: 2^21 voxels (128^3) -> 16 MiB of scratch per GPU
-// (one contribution per voxel, plus 8 doubles per chunk of 4096 for the
+// (one contribution per voxel, plus 8 doubles per chunk of 1024 for the
 // parallel loop-order sum and 64 of padding).
 #define QSSGPU_NOALLOC_MAX_FB_VOXELS (1 << 21)
-#define QSSGPU_NOALLOC_SCRATCH_DOUBLES (QSSGPU_NOALLOC_MAX_FB_VOXELS + 8 * (QSSGPU_NOALLOC_MAX_FB_VOXELS / 4096) + 64)
+#define QSSGPU_NOALLOC_SCRATCH_DOUBLES (qss::volume_scratch_doubles(QSSGPU_NOALLOC_MAX_FB_VOXELS))
 
 static __device__ __align__(256) double g_noalloc_contrib[QSSGPU_NOALLOC_SCRATCH_DOUBLES];
 
@@ -93,8 +93,6 @@ int qssgpu_volume_noalloc(const double* d_phi, const int gb[6], const int ib[6],
                                       "); use qss3dvolumeregionphilessthanzero_ for larger boxes");
     // Every scratch entry the sum reads is written first by the contribution
     // and chunk kernels, so nothing has to be cleared between calls.
-    static_assert(QSSGPU_NOALLOC_SCRATCH_DOUBLES >= QSSGPU_NOALLOC_MAX_FB_VOXELS + 8 * ((QSSGPU_NOALLOC_MAX_FB_VOXELS + 4095) / 4096) + 64,
-                  "scratch below volume_scratch_doubles of the largest box");
     if (volume_scratch_doubles(nfb) > QSSGPU_NOALLOC_SCRATCH_DOUBLES)
       throw Error(QSSGPU_ERR_ARG, "qssgpu_volume_noalloc: scratch too small");
     launch_volume(s, b, d_phi, dx, dy, dz, epsilon, scratch, d_volume);

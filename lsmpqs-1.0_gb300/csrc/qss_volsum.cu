@@ -11,42 +11,49 @@
 // never decreases.  While s stays inside one binade [2^E, 2^(E+1)), every
 // representable value there is a multiple of u = 2^(E-52), and
 //     RN(s + c) = s + u * rne(c / u)
-// where rne rounds to the nearest integer -- unless c / u is exactly halfway
-// between two integers (then the tie goes to the even significand, which
-// depends on s).  So for a chunk of contributions and a known binade, the
-// chunk's effect on s is one integer R = sum of rne(c / u), computable in
-// parallel and exactly (int64), valid when no element is a tie or not a
-// finite non-negative number and s / u + R stays below 2^53 - 1.
+// where rne rounds to the nearest integer.  If c / u is exactly halfway between
+// two integers, the tie goes to the even significand, so what c adds depends on
+// the parity of s / u.  A run of contributions in a known binade is therefore two
+// integers (struct Units): what it adds to an even and to an odd significand,
+// computable in parallel and exactly.  It applies when no element is negative or
+// not finite and s / u plus that stays below 2^53 - 1.
 //
 //   1. k_vol_contrib (volumes; the contributions are computed here) or
-//      k_vol_chunk_sum (a given sequence): per chunk of 4096 contributions,
+//      k_vol_chunk_sum (a given sequence): per chunk of 1024 contributions,
 //      their sum -- only to estimate where the running sum stands;
-//   2. k_vol_scan (more than 4096 chunks only; else each block of 3 sums its
+//   2. k_vol_scan (more than 2048 chunks only; else each block of 3 sums its
 //      predecessors): exclusive scan of those sums -> an estimate of s at the
 //      start of each chunk, good to far better than a factor of 2;
-//   3. k_vol_chunk_r: per chunk, R and a "not applicable" flag for the
-//      estimated binade and its two neighbours;
+//   3. k_vol_chunk_r: per chunk, its Units and a "not applicable" flag for the
+//      estimated binade and its two neighbours, or that all of it is zero;
 //   4. k_vol_walk: one block walks the chunks in order with the exact running
-//      sum, 256 chunks at a time: a scan of their R finds the first chunk that
-//      does not apply (another binade, the top of the binade reached, a tie,
-//      special values); the sum advances to it in one integer addition, and
-//      that chunk goes the same way by groups of 16 elements, only the group
-//      that does not apply being added element by element.
-// Every result equals the sequential loop's bit for bit.  With one warp that
-// walked chunk by chunk and added a whole chunk element by element, a volume
-// took 0.42 ms at 24^3, 3.5 ms at 192^3 and 8.6 ms at 320^3 on GB300.
+//      sum, 256 chunks at a time: a scan of their Units finds the first chunk that
+//      does not apply (another binade, the top of the binade reached, special
+//      values); the sum advances to it in one integer addition, and that chunk
+//      goes the same way by groups of up to 4 elements, only the group that does
+//      not apply being added element by element.
+// Every result equals the sequential loop's bit for bit.
+//
+// The walk is bound by latency: 1 to 2 us for each binade the sum crosses, in opening
+// its chunk and scanning windows of it.  Chunks of 4096 elements, whose ties and
+// leading zero chunks did not apply and whose windows were four times as long, took
+// 49 us at 24^3, 117 us at 64^3 and 224 us at 128^3 on GB300; these chunks of 1024
+// take 46, 63 and 109 us.  (One warp walking chunk by chunk, adding a whole chunk
+// element by element: 0.42 ms at 24^3, 3.5 ms at 192^3.)  Windows of one warp for the
+// first elements, without barriers, were slower; so was the rounding with branches.
 #include "qss_emu.cuh"
+#include "qss_kernels.cuh"
 #include "qss_state.h"
 
 namespace qss {
 
 namespace {
 
-constexpr int kVolChunk = 4096;
 constexpr int kVolThreads = 256;
 constexpr int kVolPer = kVolChunk / kVolThreads;  // elements per thread in the walk
-constexpr int kScanChunks = 4096;                 // from here on the estimates are scanned by a kernel
-constexpr int kSmallChunks = 4;                   // up to here the walk goes by elements alone
+constexpr int kScanChunks = 2048;                 // from here on the estimates are scanned by a kernel
+constexpr int kSmallChunks = 2;                   // up to here the walk goes by elements alone
+constexpr int kWalkChunks = 8;                    // chunks to a thread of the walk, at most
 
 __device__ __forceinline__ uint64_t dbits(double x) { return (uint64_t)__double_as_longlong(x); }
 __device__ __forceinline__ double dfrom(uint64_t b) { return __longlong_as_double((long long)b); }
@@ -59,34 +66,52 @@ __device__ __forceinline__ int exp_of(double x) {
   return e - 1023;
 }
 
-// rne(c / u) for u = 2^(E - 52) (below 2^52 + 1, so 4096 of them fit in
-// 64 bits); bad = a tie, a negative or non-finite c, or c >= 2^E
-__device__ __forceinline__ uint64_t rne_units(double c, int E, bool& bad) {
+// c / u rounded to an integer, for u = 2^(E - 52); on a tie, rounded down.  bad: a
+// negative or non-finite c, or c >= 2^E.  Without branches, so that a thread's
+// elements overlap.
+__device__ __forceinline__ uint64_t rne_units(double c, int E, bool& bad, bool& tie) {
   const uint64_t b = dbits(c);
-  if ((b << 1) == 0) return 0;  // +-0 leaves s unchanged
-  const int ec = (int)((b >> 52) & 0x7ff);
-  if ((b >> 63) || ec == 0x7ff) {
-    bad = true;
-    return 0;
-  }
-  uint64_t m = b & ((1ull << 52) - 1);
-  int ce;  // c = m 2^ce
-  if (ec == 0) {
-    ce = -1074;
-  } else {
-    m |= 1ull << 52;
-    ce = ec - 1075;
-  }
-  const int sh = (E - 52) - ce;  // c / u = m / 2^sh
-  if (sh <= 0) {  // c >= 2^E: s leaves the binade within this chunk
-    bad = true;
-    return 0;
-  }
-  if (sh >= 64) return 0;  // m < 2^53 <= 2^(sh-11): far below half a unit
-  const uint64_t q = m >> sh, rem = m & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-  if (rem == half) bad = true;
-  return q + (rem > half ? 1u : 0u);
+  const uint32_t hi = (uint32_t)(b >> 32), ec = (hi >> 20) & 0x7ffu;
+  // c = m 2^(max(ec, 1) - 1075), c / u = m / 2^sh
+  const uint64_t m = (b & ((1ull << 52) - 1)) | (ec ? 1ull << 52 : 0ull);
+  const int sh = E + 1023 - (ec ? (int)ec : 1);
+  // sh <= 0: c >= 2^E, s leaves the binade.  +-0 leaves s unchanged.
+  bad = bad || (((hi >> 31) || ec == 0x7ffu || sh <= 0) && (b << 1) != 0);
+  const int d = min(max(sh, 1), 55) - 1;  // from 54 on below half a unit
+  const uint64_t h = m >> d;              // c / u in halves, rounded down
+  tie = (h & 1) && (h << d) == m;
+  return (h + (tie ? 0 : 1)) >> 1;
 }
+
+// What a run of contributions adds to the significand of s: r units where it is
+// even before the run, r + d where it is odd.  A tie goes to the even sum; two
+// significands one apart end 0, 1 or 2 apart, and stay so once they are of one
+// parity, so d is -1, 0 or 1.
+struct Units {
+  unsigned long long r;
+  int d;
+};
+__device__ __forceinline__ void add_units(Units& a, uint64_t q, bool tie) {
+  if (tie) {
+    const unsigned long long even = a.r + q, odd = even + (unsigned long long)(long long)a.d + 1;
+    a.d = (int)(odd + (odd & 1) - 1 - even - (even & 1));
+    a.r = even + (even & 1);
+  } else {
+    a.r += q;
+  }
+}
+// a, then b
+__device__ __forceinline__ Units join(const Units& a, const Units& b) {
+  const bool odd = a.r & 1;
+  return {a.r + b.r + (unsigned long long)(long long)(odd ? b.d : 0), a.d != 0 ? a.d : (odd ? -b.d : b.d)};
+}
+// the significand m after the run
+__device__ __forceinline__ unsigned long long after(unsigned long long m, const Units& a) {
+  return m + a.r + (unsigned long long)(long long)((m & 1) ? a.d : 0);
+}
+// kVolPer consecutive elements to a thread, without bank conflicts
+constexpr int kVolStage = kVolChunk + kVolChunk / kVolPer;
+__device__ __forceinline__ int stage_at(int e) { return e + e / kVolPer; }
 
 __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_sum(const double* __restrict__ c, int64_t n,
                                                                double* csum) {
@@ -210,96 +235,165 @@ __global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, i
   }
 }
 
-// R[3j+q], F[3j+q] for E = exp(est[j]) - 1 + q
+// R[3j+q], F[3j+q] for E = exp(est[j]) - 1 + q.  F: kZeroChunk, all contributions
+// zero (nothing changes whatever the sum); kBadChunk, not applicable; else d + 1
+constexpr int kBadChunk = 4, kZeroChunk = 5;
 template <typename T, int PER>
 __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __restrict__ c, int64_t n,
                                                              const T* __restrict__ csum, int64_t np, bool scanned,
                                                              double* est, int64_t* R, int* F) {
-  __shared__ unsigned long long rs[3][kVolThreads];
-  __shared__ int fs[3][kVolThreads];
+  __shared__ double x[kVolStage];
+  __shared__ Units part[3][kVolThreads / 32];
   __shared__ double s_est[kVolThreads / 32];
-  const int64_t j = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t j = blockIdx.x, base = j * kVolChunk;
+  bool some = false;
+#pragma unroll
+  for (int q = 0; q < kVolPer; q++) {
+    const int e = q * kVolThreads + threadIdx.x;
+    const double v = base + e < n ? c[base + e] : 0.0;
+    x[stage_at(e)] = v;
+    some = some || (dbits(v) << 1) != 0;
+  }
   double e = 0;
   if (scanned) {
     e = est[j];
   } else {
     for (int64_t q = threadIdx.x; q < PER * j; q += kVolThreads) e += (double)csum[q];
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    if ((threadIdx.x & 31) == 0) s_est[threadIdx.x >> 5] = e;
-    __syncthreads();
+    if (lane == 0) s_est[warp] = e;
+  }
+  if (!__syncthreads_or(some)) {
+    if (threadIdx.x < 3) F[3 * j + threadIdx.x] = kZeroChunk;
+    if (threadIdx.x == 0 && !scanned) est[j] = 0.0;  // not used
+    return;
+  }
+  if (!scanned) {
     e = 0;
     for (int w = 0; w < kVolThreads / 32; w++) e += s_est[w];
     if (threadIdx.x == 0) est[j] = e;
   }
   const int E0 = exp_of(e);
-  const int64_t base = j * kVolChunk;
-  unsigned long long r[3] = {0, 0, 0};
+  Units u[3] = {};
   bool bad[3] = {E0 < -1000, E0 < -1000, E0 < -1000};
   if (E0 >= -1000) {
-    for (int t = threadIdx.x; t < kVolChunk; t += kVolThreads) {
-      const int64_t q = base + t;
-      if (q >= n) break;
-      const double x = c[q];
-#pragma unroll
-      for (int k = 0; k < 3; k++) r[k] += rne_units(x, E0 - 1 + k, bad[k]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    rs[k][threadIdx.x] = r[k];
-    fs[k][threadIdx.x] = bad[k] ? 1 : 0;
-  }
-  __syncthreads();
-  for (int w = kVolThreads / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
+    for (int q = 0; q < kVolPer; q++) {
+      const double v = x[stage_at(threadIdx.x * kVolPer + q)];
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        rs[k][threadIdx.x] += rs[k][threadIdx.x + w];
-        fs[k][threadIdx.x] |= fs[k][threadIdx.x + w];
+        bool tie;
+        const uint64_t r = rne_units(v, E0 - 1 + k, bad[k], tie);
+        add_units(u[k], r, tie);
       }
     }
-    __syncthreads();
   }
+  int any = 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    if (bad[k] || u[k].r >= (1ull << 53)) {  // the second also keeps the sums below 2^63
+      any |= 1 << k;
+      u[k] = Units{0, 0};
+    }
+    for (int o = 1; o < 32; o <<= 1) {
+      const Units v{__shfl_down_sync(0xffffffffu, u[k].r, o), __shfl_down_sync(0xffffffffu, u[k].d, o)};
+      if ((lane & (2 * o - 1)) == 0) u[k] = join(u[k], v);
+    }
+    if (lane == 0) part[k][warp] = u[k];
+  }
+  __shared__ int s_any;
+  if (threadIdx.x == 0) s_any = 0;
+  __syncthreads();
+  if (any) atomicOr(&s_any, any);
+  __syncthreads();
   if (threadIdx.x < 3) {
     const int k = threadIdx.x;
+    Units t = part[k][0];
+    for (int w = 1; w < kVolThreads / 32; w++) t = join(t, part[k][w]);
     // a chunk sum that does not fit the significand range is not applicable
-    R[3 * j + k] = (int64_t)rs[k][0];
-    F[3 * j + k] = (fs[k][0] || rs[k][0] >= (1ull << 53)) ? 1 : 0;
+    R[3 * j + k] = (int64_t)t.r;
+    F[3 * j + k] = ((s_any >> k) & 1) || t.r >= (1ull << 53) ? kBadChunk : t.d + 1;
   }
 }
 
-// Inclusive scan of r over the block.  Then, with M the running sum in units of
-// its binade: the first thread that does not apply (bad, or M + its scan
-// reaches the top of the binade), kVolThreads if none, and the scan up to it.
+// The significand m through the block's runs u in thread order: the first thread
+// that does not apply (bad, or the top of the binade reached), kVolThreads if none,
+// and in `before` the significand ahead of it.
 struct WalkScan {
-  unsigned long long warp_sum[kVolThreads / 32], before;
-  int warp_first[kVolThreads / 32];
+  Units warp_sum[kVolThreads / 32];
+  unsigned long long before[kVolThreads / 32];
+  int first[kVolThreads / 32];
 };
-__device__ __forceinline__ int walk_scan(WalkScan& w, unsigned long long r, bool bad, uint64_t M,
-                                         unsigned long long& before) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long incl = r;
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long x = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += x;
+__device__ __forceinline__ Units warp_join(Units u, int lane) {
+  if (__any_sync(0xffffffffu, u.d != 0)) {
+    for (int o = 1; o < 32; o <<= 1) {
+      const Units v{__shfl_up_sync(0xffffffffu, u.r, o), __shfl_up_sync(0xffffffffu, u.d, o)};
+      if (lane >= o) u = join(v, u);
+    }
+  } else {
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, u.r, o);
+      if (lane >= o) u.r += v;
+    }
   }
-  if (lane == 31) w.warp_sum[warp] = incl;
+  return u;
+}
+constexpr unsigned long long kBinadeTop = (1ull << 53) - 1;
+__device__ __forceinline__ int walk_scan(WalkScan& w, Units u, bool bad, unsigned long long m,
+                                         unsigned long long& before) {
+  constexpr int kWarps = kVolThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  u = warp_join(u, lane);
+  if (lane == 31) w.warp_sum[warp] = u;
   __syncthreads();
-  for (int q = 0; q < warp; q++) incl += w.warp_sum[q];
-  const unsigned stop = __ballot_sync(0xffffffffu, bad || M + incl >= (1ull << 53) - 1);
-  if (lane == 0) w.warp_first[warp] = stop ? 32 * warp + __ffs(stop) - 1 : kVolThreads;
+#pragma unroll
+  for (int q = 0; q < kWarps - 1; q++) {
+    const Units v = w.warp_sum[q];
+    if (q < warp) m = after(m, v);
+  }
+  const unsigned long long end = after(m, u), prev = __shfl_up_sync(0xffffffffu, end, 1);
+  const unsigned stop = __ballot_sync(0xffffffffu, bad || end >= kBinadeTop);
+  const int at = stop ? __ffs(stop) - 1 : 31;
+  if (lane == at) {
+    w.first[warp] = stop ? 32 * warp + at : kVolThreads;
+    w.before[warp] = !stop ? end : (lane ? prev : m);
+  }
   __syncthreads();
   int first = kVolThreads;
-  for (int q = 0; q < kVolThreads / 32; q++) first = min(first, w.warp_first[q]);
-  if ((int)threadIdx.x == (first < kVolThreads ? first : kVolThreads - 1)) w.before = first < kVolThreads ? incl - r : incl;
-  __syncthreads();
-  before = w.before;
+  before = w.before[kWarps - 1];
+#pragma unroll
+  for (int q = kWarps - 1; q >= 0; q--) {
+    if (w.first[q] < kVolThreads) {
+      first = w.first[q];
+      before = w.before[q];
+    }
+  }
   return first;
 }
 
-// the running sum s, in a valid binade, advanced by R units of it
-__device__ __forceinline__ double advance(double s, unsigned long long R) {
-  return R ? dfrom(dbits(s) + R) : s;  // below the binade's top: the significand does not carry
+// the running sum s, with significand m and in a valid binade, once the significand is `to`
+__device__ __forceinline__ double advance(double s, unsigned long long m, unsigned long long to) {
+  return dfrom(dbits(s) + (to - m));  // below the binade's top: the significand does not carry
+}
+
+__device__ __forceinline__ double add_nonzero(double s, double y) { return (dbits(y) << 1) != 0 ? s + y : s; }
+
+// the elements [lo, hi) of a staged chunk in the binade E
+__device__ __forceinline__ Units window_units(const double* x, int lo, int hi, int E, bool& bad) {
+  Units u{0, 0};
+  bad = false;
+#pragma unroll
+  for (int q = 0; q < kVolPer; q++) {
+    if (lo + q < hi) {
+      bool tie;
+      const uint64_t r = rne_units(x[stage_at(lo + q)], E, bad, tie);
+      add_units(u, r, tie);
+    }
+  }
+  if (bad || u.r >= (1ull << 53)) {  // past the binade; also keeps sums over the block below 2^63
+    bad = true;
+    u = Units{0, 0};
+  }
+  return u;
 }
 
 // one block: the exact running sum over the chunks in loop order
@@ -308,62 +402,91 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restri
                                                           const int* __restrict__ F, bool have_r, double* out) {
   __shared__ WalkScan w;
   __shared__ double s_sum;
-  __shared__ double x[kVolChunk];
+  __shared__ int s_start;
+  __shared__ unsigned long long s_at;
+  __shared__ double x[kVolStage];
   const int t = threadIdx.x;
   constexpr uint64_t hidden = 1ull << 52;
-  double s = 0.0;  // the same in every thread
+  double s = 0.0;    // the same in every thread
+  int64_t born = 0;  // where s left zero, to a few elements
+  auto significand = [&](int E) { return E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0ull; };
   for (int64_t j = 0; j < nc;) {
     unsigned long long before;
     if (have_r) {
-      const int E = exp_of(s);
-      bool ok = true;  // chunks past the end stop nothing
-      unsigned long long r = 0;
-      if (j + t < nc) {
-        const int64_t q = j + t;
-        const int E0 = exp_of(est[q]), k = E - (E0 - 1);
-        ok = E > -1000 && E0 > -1000 && k >= 0 && k <= 2;
-        if (ok) ok = F[3 * q + k] == 0;
-        if (ok) r = (unsigned long long)R[3 * q + k];
+      // the sum takes about as many chunks again to leave a binade as it took to enter it
+      const int E = exp_of(s), cpt = j < 256 ? 1 : (j < 256 * kWalkChunks ? (int)(j / 256) : kWalkChunks);
+      auto chunk_units = [&](int64_t q, bool& ok) {  // chunks past the end stop nothing
+        if (q >= nc) return Units{0, 0};
+        const double e = est[q];
+        const int f[3] = {F[3 * q], F[3 * q + 1], F[3 * q + 2]};
+        const int64_t r[3] = {R[3 * q], R[3 * q + 1], R[3 * q + 2]};
+        if (f[0] == kZeroChunk) return Units{0, 0};
+        const int E0 = exp_of(e), k = E - (E0 - 1), fk = k == 0 ? f[0] : (k == 1 ? f[1] : f[2]);
+        if (E <= -1000 || E0 <= -1000 || k < 0 || k > 2 || fk == kBadChunk) {
+          ok = false;
+          return Units{0, 0};
+        }
+        return Units{(unsigned long long)(k == 0 ? r[0] : (k == 1 ? r[1] : r[2])), fk - 1};
+      };
+      bool ok = true;
+      Units u{0, 0};
+      for (int i = 0; i < cpt; i++) u = join(u, chunk_units(j + (int64_t)t * cpt + i, ok));
+      const unsigned long long m = significand(E);
+      const int first = walk_scan(w, u, !ok, m, before);
+      if (first < kVolThreads && cpt > 1) {  // which of the thread's chunks
+        if (t == first) {
+          int i = 0;
+          unsigned long long at = before;
+          for (; i < cpt; i++) {
+            bool fits = true;
+            const unsigned long long end = after(at, chunk_units(j + (int64_t)t * cpt + i, fits));
+            if (!fits || end >= kBinadeTop) break;
+            at = end;
+          }
+          s_at = at;
+          s_start = i;
+        }
+        __syncthreads();
+        before = s_at;
+        j += s_start;
       }
-      const int first = walk_scan(w, r, !ok, E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0, before);
-      s = advance(s, before);
-      j += first;
+      s = advance(s, m, before);
+      j += (int64_t)first * cpt;
       if (first == kVolThreads || j >= nc) continue;
     }
-    // chunk j: windows of kVolThreads * per consecutive elements, per of them to a
-    // thread.  The sum takes about as many elements again to leave a binade as it
-    // took to enter it, so per grows with the elements behind.
+    // chunk j, by windows of consecutive elements, per of them to a thread.  The sum
+    // takes about as many elements again to leave a binade as it took to enter it,
+    // so per grows with the elements since it left zero.
     __syncthreads();  // the previous chunk's elements are no longer read
     const int64_t base = j * kVolChunk;
 #pragma unroll
     for (int q = 0; q < kVolPer; q++) {
       const int64_t e = base + q * kVolThreads + t;
-      x[q * kVolThreads + t] = e < n ? c[e] : 0.0;
+      x[stage_at(q * kVolThreads + t)] = e < n ? c[e] : 0.0;
     }
     __syncthreads();
-    for (int start = 0; start < kVolChunk;) {
+    int start = 0;
+    while (start < kVolChunk) {
       const int E = exp_of(s);
-      const int64_t behind = (base + start) / (2 * kVolThreads);
-      const int per = behind < 1 ? 1 : (behind < kVolPer ? (int)behind : kVolPer);
-      bool bad = false;
-      unsigned long long r = 0;
+      const int64_t since = base + start - born;
+      const int per = since < 512 ? 1 : (since < 512 * kVolPer ? (int)(since / 512) : kVolPer);
       const int lo = start + t * per, hi = lo + per < kVolChunk ? lo + per : kVolChunk;
-      for (int q = lo; q < hi; q++) r += rne_units(x[q], E, bad);
-      const int first = walk_scan(w, r, bad, E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0, before);
-      s = advance(s, before);
+      bool bad;
+      const Units u = window_units(x, lo, hi, E, bad);
+      const unsigned long long m = significand(E);
+      const int first = walk_scan(w, u, bad, m, before);
+      s = advance(s, m, before);
       if (first == kVolThreads) {
         start += kVolThreads * per;
         continue;
       }
       if (t == first) {  // element by element, in loop order, skipping exact zeros
         double v = s;
-        for (int q = lo; q < hi; q++) {
-          const double y = x[q];
-          if ((dbits(y) << 1) != 0) v = v + y;
-        }
+        for (int q = lo; q < hi; q++) v = add_nonzero(v, x[stage_at(q)]);
         s_sum = v;
       }
       __syncthreads();
+      if ((dbits(s) << 1) == 0) born = base + start + first * per;
       s = s_sum;
       start += (first + 1) * per;
     }
@@ -373,11 +496,6 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restri
 }
 
 }  // namespace
-
-int64_t loop_sum_scratch_doubles(int64_t n) {
-  const int64_t nc = (n + kVolChunk - 1) / kVolChunk;
-  return 8 * nc + 64;
-}
 
 namespace {
 
