@@ -73,9 +73,14 @@ constexpr uint64_t kAbs = ~kSign;
 QSS_EMU_HD uint64_t mag2(uint64_t b) { return b << 1; }
 constexpr uint64_t kInf2 = 0x7ff0000000000000ull << 1;
 
+// Opaque to the compiler on the device: it takes tests of the bits for what they
+// say about the number ((bits << 1) == 0 for x == 0, bits & kAbs for fabs) and issues
+// them on the FP64 pipe, where one costs as much as a whole integer-pipe product.
 QSS_EMU_HD uint64_t bits(double x) {
 #ifdef __CUDA_ARCH__
-  return (uint64_t)__double_as_longlong(x);
+  uint64_t u;
+  asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+  return u;
 #else
   uint64_t u;
   memcpy(&u, &x, 8);
