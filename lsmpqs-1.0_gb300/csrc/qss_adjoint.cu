@@ -44,8 +44,23 @@ namespace qss {
 
 namespace {
 
-constexpr double kC13 = 1.0 / 3.0, kC76 = 7.0 / 6.0, kC116 = 11.0 / 6.0, kC16 = 1.0 / 6.0, kC56 = 5.0 / 6.0;
 constexpr double k1312 = 13.0 / 12.0, k136 = 13.0 / 6.0;
+
+__device__ __noinline__ double mul_rare(double x, double y) { return x * y; }
+
+// x * y on the integer pipes where zeros are common (adjoints of parts at rest, exactly
+// linear parts): qss_emu::mul sends them down the branch of its FP64 instruction, which
+// then takes the pipe for the whole warp
+__device__ __forceinline__ double mulz(double x, double y) {
+  using namespace qss_emu;
+  const uint32_t xh = hi32(x), yh = hi32(y);
+  const uint32_t wx = win(xh), wy = win(yh);
+  const bool zx = mag2(bits(x)) == 0, zy = mag2(bits(y)) == 0;
+  double r = mul_win(xh, lo32(x), yh, lo32(y));
+  r = zx || zy ? __hiloint2double((int)((xh ^ yh) & 0x80000000u), 0) : r;
+  if ((!zx && wx >= 0x40000000u) || (!zy && wy >= 0x40000000u)) r = mul_rare(x, y);
+  return r;
+}
 
 // Godunov term of WENO5 (3d.f:2251-2276) and its partials: dtn/d(pp, pm), dtn/dvel
 __device__ __forceinline__ double godunov_bwd(double vel, const double pp[3], const double pm[3], double ppb[3],
@@ -230,13 +245,17 @@ __global__ void __launch_bounds__(128) k_adj_carry(AdjPointArgs a) {
 // (the later operand of the reference's MAX chain on ties, per side).
 // A block holds a tile of 4 lines x up to 58 points and goes through it in
 // phases, each value once in shared memory: faces v, centre differences a, the
-// windows (their five face adjoints and the adjoints of the three indicators'
-// first terms), the centre terms' adjoints, the faces' sums in a fixed order, and
-// lam(p) += inv (F(p) - F(p+1)).  A tile recomputes the windows of 3 points on
+// windows (their adjoints of five faces and three centre differences, times six),
+// the centres' sums, the faces' sums in a fixed order, and lam(p) += inv / 6 (F(p)
+// - F(p+1)).  Only distances between the candidates count, so the candidates are
+// taken relative to a midpoint, where they are multiples of the centre differences.  A tile recomputes the windows of 3 points on
 // either side; tiles of 58 points make 64 windows of them, full warps.
-// Bound: FP64 pipe (~145 instructions a window, 77 cycles each).  With a thread
-// walking a segment of a line instead (32 points and more, so that a 72^3 box had
-// 324 warps for 608 schedulers) a pass took 0.30 ms at 72^3.
+// Bound: FP64 pipe, about 80 % of its time busy with 57 instructions a window and 15 a
+// point (145 a window with the candidates as stencils of their own, products and
+// comparisons on the FP64 pipe: 72^3, 150 us a pass against 92).  Full tiles and a
+// remainder rather than equal ones: their windows are whole rounds of the block.
+// With a thread walking a segment of a line instead (32 points and more, so that a 72^3 box
+// had 324 warps for 608 schedulers) a pass took 0.30 ms.
 struct AdjAxisArgs {
   Box b;
   const double* phi;
@@ -254,7 +273,7 @@ constexpr size_t kAdjBytes = sizeof(double) * kAdjL * (kAdjF + kAdjC + 8 * kAdjW
 static_assert(kAdjBytes <= 48 * 1024, "dynamic shared memory without the opt-in attribute");
 
 template <int AX>
-__global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
+__global__ void __launch_bounds__(kAdjThreads, 5) k_adj_axis(AdjAxisArgs a) {
   constexpr int L = kAdjL;
   extern __shared__ double adj_smem[];
   double* const sv = adj_smem;             // faces; later the face adjoints F
@@ -285,7 +304,7 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
   const int64_t base = AX == 0 ? b.idx(0, p, q) : (AX == 1 ? b.idx(p, 0, q) : b.idx(p, q, 0));
   const int64_t stride = AX == 0 ? 1 : (AX == 1 ? (int64_t)b.nx : (int64_t)b.nx * b.ny);
   const double* __restrict__ phi = a.phi;
-  const double inv = a.inv;
+  const double inv = a.inv, inv6 = a.inv * (1.0 / 6.0);
   const int last = (AX == 0 ? b.nx : (AX == 1 ? b.ny : b.nz)) - 1;
   // loads outside the line only feed windows without adjoints
   auto ld = [&](int m) -> double {
@@ -308,11 +327,30 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
     sa[it] = (v[0] - 2.0 * v[L]) + v[2 * L];
   }
   __syncthreads();
+  // windows with an adjoint: c = lo .. hi + 1; the others add nothing
+  const int w0 = (p0 - 2 < lo ? lo - (p0 - 2) : 0) * L, w1 = (p0 + tp + 3 > hi + 1 ? hi + 1 - (p0 - 2) + 1 : tp + 6) * L;
   for (int it = threadIdx.x; it < (tp + 6) * L; it += kAdjThreads) {
+    if (it >= w0 && it < w1) continue;
+#pragma unroll
+    for (int o = 0; o < 8; o++) sd[o * W + it] = 0.0;
+  }
+  for (int it = w0 + threadIdx.x; it < w1; it += kAdjThreads) {
     const int c = p0 - 2 + it / L;
-    double d0 = 0, d1 = 0, d2 = 0, d3 = 0, d4 = 0, bS1 = 0, bS2 = 0, bS3 = 0;
-    const double gm = ldbar(a.bm, c), gp = ldbar(a.bp, c - 1);
-    if (gm != 0.0 || gp != 0.0) {
+    double d0 = 0, d1 = 0, d2 = 0, d3 = 0, d4 = 0, A1 = 0, A2 = 0, A3 = 0;
+    double gm = ldbar(a.bm, c), gp = ldbar(a.bp, c - 1);
+    if (((bits(gm) | bits(gp)) << 1) != 0) {
+      // Adjoints fall off by orders of magnitude per voxel ahead of the front.  Below
+      // 2^-160 the window, linear in them, is evaluated on a multiple: their products
+      // would leave the range of the integer ones, and one lane's FP64 instruction costs
+      // its warp as much as 32.
+      using qss_emu::hi32;
+      using qss_emu::scale2;
+      const uint32_t top = max(hi32(gm) & 0x7fffffffu, hi32(gp) & 0x7fffffffu);
+      const int up2 = top >= 0x35f00000u ? 0 : (top >= 0x23300000u ? 300 : 700);
+      if (up2) {
+        gm = scale2(gm, up2);
+        gp = scale2(gp, up2);
+      }
       const double* const v = sv + it;
       const double u0 = v[0], u1 = v[L], u2 = v[2 * L], u3 = v[3 * L], u4 = v[4 * L];
       const double* const aa = sa + it;
@@ -333,62 +371,65 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
       else if (b3 == mx) ip = 3;
       else ip = 4;
       const double um = im == 0 ? u0 : im == 1 ? u1 : im == 2 ? u2 : im == 3 ? u3 : u4;
-      const double eps = 1e-6 * (um * um) + 1.0e-35;
-      const double b1t = (u0 - 4.0 * u1) + 3.0 * u2, e2 = u1 - u3, b3t = (3.0 * u2 - 4.0 * u3) + u4;
-      const double S1 = k1312 * (aa[0] * aa[0]) + 0.25 * (b1t * b1t);
-      const double S2 = k1312 * (aa[L] * aa[L]) + 0.25 * (e2 * e2);
-      const double S3 = k1312 * (aa[2 * L] * aa[2 * L]) + 0.25 * (b3t * b3t);
-      const double r1 = qss_emu::div(1.0, S1 + eps), r2 = qss_emu::div(1.0, S2 + eps),
-                   r3 = qss_emu::div(1.0, S3 + eps);
-      // products of the weights on the integer pipes (the FP64 pipe bounds this kernel)
-      using qss_emu::mul;
-      const double q1 = mul(r1, r1), q2 = mul(r2, r2), q3 = mul(r3, r3);
-      const double am2 = mul(0.6, q2);
-      const double am1 = mul(0.1, q1), am3 = mul(0.3, q3);  // minus: 0.1, 0.6, 0.3
-      const double ap1 = mul(0.3, q1), ap3 = mul(0.1, q3);  // plus (on S1, S2, S3): 0.3, 0.6, 0.1
+      auto sq = [](double x) { return mulz(x, x); };
+      const double eps = fma(1e-6, sq(um), 1.0e-35);
+      const double a1 = aa[0], a2 = aa[L], a3 = aa[2 * L];
+      const double s1 = u2 - u1, s2 = u3 - u2, e2 = s1 + s2;
+      const double b1t = fma(2.0, s1, a1), b3t = fma(-2.0, s2, a3);  // u0 - 4 u1 + 3 u2, 3 u2 - 4 u3 + u4
+      const double r1 = qss_emu::div(1.0, fma(k1312, sq(a1), fma(0.25, sq(b1t), eps))),
+                   r2 = qss_emu::div(1.0, fma(k1312, sq(a2), fma(0.25, sq(e2), eps))),
+                   r3 = qss_emu::div(1.0, fma(k1312, sq(a3), fma(0.25, sq(b3t), eps)));
+      const double q1 = mulz(r1, r1), q2 = mulz(r2, r2), q3 = mulz(r3, r3);
+      const double am2 = mulz(0.6, q2);
+      const double am1 = mulz(0.1, q1), am3 = mulz(0.3, q3);  // minus: 0.1, 0.6, 0.3
+      const double ap1 = mulz(0.3, q1), ap3 = mulz(0.1, q3);  // plus (on S1, S2, S3): 0.3, 0.6, 0.1
       const double iam = qss_emu::div(1.0, am1 + am2 + am3), iap = qss_emu::div(1.0, ap1 + am2 + ap3);
-      const double wm1 = mul(am1, iam), wm2 = mul(am2, iam), wm3 = mul(am3, iam);
-      const double wp1 = mul(ap1, iap), wp2 = mul(am2, iap), wp3 = mul(ap3, iap);
-      // candidate stencils: minus reads u0..u4, plus reads u4..u0
-      const double pm1 = kC13 * u0 - kC76 * u1 + kC116 * u2;
-      const double pm2 = -kC16 * u1 + kC56 * u2 + kC13 * u3;
-      const double pm3 = kC13 * u2 + kC56 * u3 - kC16 * u4;
-      const double pq1 = -kC16 * u0 + kC56 * u1 + kC13 * u2;  // plus stencil on S1 (its third)
-      const double pq2 = kC13 * u1 + kC56 * u2 - kC16 * u3;   // on S2
-      const double pq3 = kC116 * u2 - kC76 * u3 + kC13 * u4;  // on S3 (its first)
-      const double vm = wm1 * pm1 + wm2 * pm2 + wm3 * pm3;
-      const double vp = wp1 * pq1 + wp2 * pq2 + wp3 * pq3;
-      const double P1 = mul(gm, wm1), P2 = mul(gm, wm2), P3 = mul(gm, wm3);
-      const double Q1 = mul(gp, wp1), Q2 = mul(gp, wp2), Q3 = mul(gp, wp3);
-      const double x1 = qss_emu::scale2(r1, 1), x2 = qss_emu::scale2(r2, 1), x3 = qss_emu::scale2(r3, 1);
-      // x_k = 2 r_k; the minus sign of d value / d T_k is folded into the differences
-      const double m1 = P1 * (vm - pm1) * x1, m2 = P2 * (vm - pm2) * x2, m3 = P3 * (vm - pm3) * x3;
-      const double n1 = Q1 * (vp - pq1) * x1, n2 = Q2 * (vp - pq2) * x2, n3 = Q3 * (vp - pq3) * x3;
-      bS1 = m1 + n1;
-      bS2 = m2 + n2;
-      bS3 = m3 + n3;
-      const double bem = m1 + m2 + m3, bep = n1 + n2 + n3;
-      const double bb1 = bS1 * qss_emu::scale2(b1t, -1);
-      const double be2 = bS2 * qss_emu::scale2(e2, -1);
-      const double bb3 = bS3 * qss_emu::scale2(b3t, -1);
-      d0 = bb1 + kC13 * P1 - kC16 * Q1;
-      d1 = -4.0 * bb1 + be2 - kC76 * P1 - kC16 * P2 + kC56 * Q1 + kC13 * Q2;
-      d2 = 3.0 * bb1 + 3.0 * bb3 + kC116 * P1 + kC56 * P2 + kC13 * P3 + kC13 * Q1 + kC56 * Q2 +
-                  kC116 * Q3;
-      d3 = -be2 - 4.0 * bb3 + kC13 * P2 + kC56 * P3 - kC16 * Q2 - kC76 * Q3;
-      d4 = bb3 - kC16 * P3 + kC13 * Q3;
-      // eps = 1e-6 max(u^2) + 1e-35, per reading direction
-      {
-        // both directions usually pick the same face: one sum, then selects
-        const double up = ip == 0 ? u0 : ip == 1 ? u1 : ip == 2 ? u2 : ip == 3 ? u3 : u4;
-        const double cm = 2e-6 * um * bem, cp = 2e-6 * up * bep;
-        const double cs = (im == ip) ? cm + cp : cm;
-        auto ex = [&](int j) { return j == im ? cs : (j == ip && im != ip ? cp : 0.0); };
-        d0 += ex(0);
-        d1 += ex(1);
-        d2 += ex(2);
-        d3 += ex(3);
-        d4 += ex(4);
+      // the weights first: in flat parts the sums are 1e70 and their inverses out of range beside gm
+      const double wm1 = mulz(am1, iam), wm2 = mulz(am2, iam), wm3 = mulz(am3, iam);
+      const double wp1 = mulz(ap1, iap), wp2 = mulz(am2, iap), wp3 = mulz(ap3, iap);
+      // candidates, six times their distance from (u2 + u3) / 2 (minus) and
+      // (u1 + u2) / 2 (plus): c1, -a2, -a3 and -a1, -a2, c3
+      const double a23 = -3.0 * a2, c1 = fma(2.0, a1, a23), c3 = fma(2.0, a3, a23);
+      const double vm = fma(-wm3, a3, fma(-wm2, a2, mulz(wm1, c1)));
+      const double vp = fma(-wp1, a1, fma(-wp2, a2, mulz(wp3, c3)));
+      // three times the adjoints of the indicators, without their sign: P_k (value - p_k) r_k for
+      // each direction and both
+      const double P1 = mulz(gm, wm1), P2 = mulz(gm, wm2), P3 = mulz(gm, wm3);
+      const double Q1 = mulz(gp, wp1), Q2 = mulz(gp, wp2), Q3 = mulz(gp, wp3);
+      const double m1 = mulz(r1, mulz(P1, vm - c1)), m2 = mulz(r2, mulz(P2, vm + a2)), m3 = mulz(r3, mulz(P3, vm + a3));
+      const double n1 = mulz(r1, mulz(Q1, vp + a1)), n2 = mulz(r2, mulz(Q2, vp + a2)), n3 = mulz(r3, mulz(Q3, vp - c3));
+      const double bS1 = m1 + n1, bS2 = m2 + n2, bS3 = m3 + n3;
+      // six times everything from here on: adjoints of the centres a1, a2, a3 ...
+      A1 = fma(bS1, fma(2.0 * k136, a1, b1t), fma(2.0, P1, -Q1));
+      A2 = fma(2.0 * k136, mulz(bS2, a2), fma(-3.0, P1 + Q3, -(P2 + Q2)));
+      A3 = fma(bS3, fma(2.0 * k136, a3, b3t), fma(2.0, Q3, -P3));
+      // ... of the differences s1, s2 ...
+      const double be = mulz(bS2, e2);
+      const double g1 = fma(-3.0, gp, fma(2.0, mulz(bS1, b1t), be)), g2 = fma(3.0, gm, fma(-2.0, mulz(bS3, b3t), be));
+      // ... and of the faces
+      d1 = -g1;
+      d2 = fma(6.0, gm + gp, g1 - g2);
+      d3 = g2;
+      // eps = 1e-6 max(u^2) + 1e-35, per reading direction; two faces of exactly the same
+      // magnitude, where the directions differ, are common enough not to branch on
+      const double up = ip == 0 ? u0 : ip == 1 ? u1 : ip == 2 ? u2 : ip == 3 ? u3 : u4;
+      const double cm = mulz(mulz(4e-6, um), (m1 + m2) + m3), cp = mulz(mulz(4e-6, up), (n1 + n2) + n3);
+      const double cs = im == ip ? cm + cp : cm;
+      auto ex = [&](int j) { return j == im ? cs : (j == ip ? cp : 0.0); };
+      d0 = ex(0);
+      d1 += ex(1);
+      d2 += ex(2);
+      d3 += ex(3);
+      d4 = ex(4);
+      if (up2) {
+        d0 = scale2(d0, -up2);
+        d1 = scale2(d1, -up2);
+        d2 = scale2(d2, -up2);
+        d3 = scale2(d3, -up2);
+        d4 = scale2(d4, -up2);
+        A1 = scale2(A1, -up2);
+        A2 = scale2(A2, -up2);
+        A3 = scale2(A3, -up2);
       }
     }
     sd[it] = d0;
@@ -396,17 +437,16 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
     sd[2 * W + it] = d2;
     sd[3 * W + it] = d3;
     sd[4 * W + it] = d4;
-    sd[5 * W + it] = bS1;
-    sd[6 * W + it] = bS2;
-    sd[7 * W + it] = bS3;
+    sd[5 * W + it] = A1;
+    sd[6 * W + it] = A2;
+    sd[7 * W + it] = A3;
   }
   __syncthreads();
   // adjoint of a(m) for the centres p0-1 .. p0+tp+1 the tile's faces touch (window
-  // index w = m - p0 + 2): its term sits in S1 of window w+1, S2 of w, S3 of w-1
+  // index w = m - p0 + 2): it is a1 of window w+1, a2 of w, a3 of w-1
   for (int it = threadIdx.x; it < (tp + 3) * L; it += kAdjThreads) {
     const int w = it + L;  // the window of centre m = p0 - 1 + it / L
-    const double ba = (sd[5 * W + w + L] + sd[6 * W + w]) + sd[7 * W + w - L];
-    sa[it + 2 * L] = ba * (k136 * sa[it + 2 * L]);  // centre m is entry m - p0 + 3
+    sa[it + 2 * L] = (sd[5 * W + w + L] + sd[6 * W + w]) + sd[7 * W + w - L];  // centre m is entry m - p0 + 3
   }
   __syncthreads();
   // face f = p0 .. p0+tp: slot k of window f + 2 - k, and the three centres on it
@@ -414,13 +454,13 @@ __global__ void __launch_bounds__(kAdjThreads, 4) k_adj_axis(AdjAxisArgs a) {
     const double* const d = sd + it + 4 * L;  // window f + 2
     const double* const c = sa + it + 2 * L;  // centre f - 1
     double F = ((d[0] + d[W - L]) + (d[2 * W - 2 * L] + d[3 * W - 3 * L])) + d[4 * W - 4 * L];
-    F += (c[0] + c[2 * L]) - 2.0 * c[L];
+    F += fma(-2.0, c[L], c[0] + c[2 * L]);
     sv[it] = F;  // the faces' v is no longer read
   }
   __syncthreads();
   if (!line_ok) return;
   for (int it = threadIdx.x; it < tp * L; it += kAdjThreads)
-    a.lam[base + (int64_t)(p0 + it / L) * stride] += inv * (sv[it] - sv[it + L]);
+    a.lam[base + (int64_t)(p0 + it / L) * stride] += inv6 * (sv[it] - sv[it + L]);
 }
 
 // lam_out[p] += coef * lam_in[p] (fill box) + the curvature partials of the
@@ -870,8 +910,8 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
     ar.npts = n;
     const dim3 blk(32, 4, 1);
     const dim3 grd((b.fbx() + 31) / 32, (b.fby() + 3) / 4, b.fbz());
-    // the axis passes' tiles: a line's points split evenly; shorter tiles on small
-    // boxes, so that four blocks per SM have about two rounds of them
+    // the axis passes' tiles: full ones and a remainder; shorter tiles on small boxes, so
+    // that four blocks per SM have about two rounds of them
     AdjAxisArgs axs[3];
     dim3 agrid[3];
     for (int d = 0; d < 3; d++) {
@@ -880,8 +920,7 @@ int adjoint_run(Options* o, QSS_DataArrays* p, Grid* g, const double* theta, con
       const unsigned ly = (unsigned)(d == 2 ? b.fby() : b.fbz());
       int cap = kAdjP;
       while (cap > 16 && (int64_t)lx * ly * ((len + cap - 1) / cap) < 152 * 4 * 2) cap /= 2;
-      const int tiles = (len + cap - 1) / cap;
-      axs[d] = AdjAxisArgs{b, nullptr, ar.bp[d], ar.bm[d], nullptr, 1.0 / g->dx[d], (len + tiles - 1) / tiles};
+      axs[d] = AdjAxisArgs{b, nullptr, ar.bp[d], ar.bm[d], nullptr, 1.0 / g->dx[d], len < cap ? len : cap};
       agrid[d] = dim3(lx, ly, (unsigned)((len + axs[d].len - 1) / axs[d].len));
     }
     auto bc_bwd = [&](const double* val, double* l) {
