@@ -63,7 +63,7 @@ __device__ __forceinline__ double mulz(double x, double y) {
 }
 
 // Godunov term of WENO5 (3d.f:2251-2276) and its partials: dtn/d(pp, pm), dtn/dvel
-__device__ __forceinline__ double godunov_bwd(double vel, const double pp[3], const double pm[3], double ppb[3],
+__device__ __forceinline__ void godunov_bwd(double vel, const double pp[3], const double pm[3], double ppb[3],
                                               double pmb[3], double& velb) {
   double a[3], c[3];
   bool use_a[3];
@@ -78,20 +78,27 @@ __device__ __forceinline__ double godunov_bwd(double vel, const double pp[3], co
       a[d] = qss_emu::lt0(pm[d]) ? pm[d] : 0.0;
       c[d] = qss_emu::gt0(pp[d]) ? pp[d] : 0.0;
     }
-    const double aa = a[d] * a[d], cc = c[d] * c[d];
+    const double aa = mulz(a[d], a[d]), cc = mulz(c[d], c[d]);
     use_a[d] = (long long)qss_emu::bits(aa) > (long long)qss_emu::bits(cc);
     ngps += use_a[d] ? aa : cc;
   }
   const double norm = qss_emu::sqrt(ngps);
   velb = norm;
-  const double nb = qss_emu::gt0(norm) ? qss_emu::div(vel, 2.0 * norm) : 0.0;
+  // vel / (2 norm), the other 2 of the square's derivative folded in
+  const double nb = qss_emu::gt0(norm) ? qss_emu::div(vel, norm) : 0.0;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    if (use_a[d]) pmb[d] = nb * 2.0 * a[d];
-    else ppb[d] = nb * 2.0 * c[d];
+    if (use_a[d]) pmb[d] = mulz(nb, a[d]);
+    else ppb[d] = mulz(nb, c[d]);
   }
-  return vel * norm;
 }
+
+// |v| >= 1e-5
+__device__ __forceinline__ bool moving(double v) {
+  const uint64_t a = qss_emu::mag2(qss_emu::bits(v));
+  return a >= 0x7dc9f16b11c6d1e2ull && a <= qss_emu::kInf2;
+}
+__device__ __forceinline__ bool nonzero(double v) { return qss_emu::mag2(qss_emu::bits(v)) != 0; }
 
 struct AdjPointArgs {
   Box b;
@@ -123,7 +130,7 @@ struct AdjPointArgs {
 // A block of 32 x 4 threads covers 32 (i) x 4 (j) voxels; each warp an 8 x 4
 // patch of them, so that warps inside the grains (b = 0) skip the curvature
 // partials together.
-__global__ void __launch_bounds__(128) k_adj_point(AdjPointArgs a) {
+__global__ void __launch_bounds__(128, 7) k_adj_point(AdjPointArgs a) {
   const Box& b = a.b;
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int i = b.ilo + blockIdx.x * 32 + 8 * warp + (lane & 7);
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(128) k_adj_point(AdjPointArgs a) {
   const int k = b.klo + blockIdx.z;
   if (i > b.ihi || j > b.jhi || k > b.khi) return;
   const int64_t q = b.idx(i, j, k);
-  const double w = a.coef_l * a.lam_in[q];
+  const double w = mulz(a.coef_l, a.lam_in[q]);
   const int64_t st[3] = {1, (int64_t)b.nx, (int64_t)b.nx * b.ny};
   const double* __restrict__ phi = a.phi;
   double pp[3], pm[3];
@@ -142,57 +149,62 @@ __global__ void __launch_bounds__(128) k_adj_point(AdjPointArgs a) {
   }
   const double vel = a.vel_n[q];
   double ppb[3] = {0, 0, 0}, pmb[3] = {0, 0, 0};
-  if (fabs(vel) >= 1.e-5) {
+  if (moving(vel)) {
     double velb;
     godunov_bwd(vel, pp, pm, ppb, pmb, velb);
-    a.adj_vel[q] += w * velb;
+    a.adj_vel[q] += mulz(w, velb);
   }
   const double vxyz[3] = {a.vx[q], a.vy[q], a.vz[q]};
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    if (qss_emu::ge0(vxyz[d])) pmb[d] += -vxyz[d];
-    else ppb[d] += -vxyz[d];
-    a.bp[d][q] = w * ppb[d];
-    a.bm[d][q] = w * pmb[d];
+    const bool up = qss_emu::ge0(vxyz[d]);
+    if (nonzero(vxyz[d])) (up ? pmb[d] : ppb[d]) -= vxyz[d];
+    a.bp[d][q] = mulz(w, ppb[d]);
+    a.bm[d][q] = mulz(w, pmb[d]);
   }
   double out[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  {
+  // nothing flows through b kappa where b is zero (grain interiors)
+  const double bco = a.bcoef[q];
+  if (nonzero(w) && nonzero(bco)) {
     const double fx = a.fac[0], fy = a.fac[1], fz = a.fac[2];
     // first differences as the forward computes them (the threshold test on
     // their squares must take the forward's branch)
-    const double phx = (phi[q + st[0]] - phi[q - st[0]]) * fx;
-    const double phy = (phi[q + st[1]] - phi[q - st[1]]) * fy;
-    const double phz = (phi[q + st[2]] - phi[q - st[2]]) * fz;
-    const double grad = __dadd_rn(__dadd_rn(__dmul_rn(phx, phx), __dmul_rn(phy, phy)), __dmul_rn(phz, phz));
-    // nothing flows through b kappa where b is zero (grain interiors)
-    if (w != 0.0 && a.bcoef[q] != 0.0 && qss_emu::bits(grad) >= qss_emu::bits(1.e-5)) {  // grad >= 1e-5
+    const double phx = mulz(phi[q + st[0]] - phi[q - st[0]], fx);
+    const double phy = mulz(phi[q + st[1]] - phi[q - st[1]], fy);
+    const double phz = mulz(phi[q + st[2]] - phi[q - st[2]], fz);
+    const double sx = mulz(phx, phx), sy = mulz(phy, phy), sz = mulz(phz, phz);
+    const double grad = __dadd_rn(__dadd_rn(sx, sy), sz);
+    if (qss_emu::bits(grad) >= 0x3ee4f8b588e368f1ull) {  // grad >= 1e-5
       const double cc = phi[q];
-      const double pxx = (phi[q + 2 * st[0]] + phi[q - 2 * st[0]] - 2 * cc) * a.f2[0];
-      const double pyy = (phi[q + 2 * st[1]] + phi[q - 2 * st[1]] - 2 * cc) * a.f2[1];
-      const double pzz = (phi[q + 2 * st[2]] + phi[q - 2 * st[2]] - 2 * cc) * a.f2[2];
-      const double pxy = (phi[q + st[0] + st[1]] + phi[q - st[0] - st[1]] - phi[q - st[0] + st[1]] -
-                          phi[q + st[0] - st[1]]) * a.f2[3];
-      const double pxz = (phi[q + st[0] + st[2]] + phi[q - st[0] - st[2]] - phi[q - st[0] + st[2]] -
-                          phi[q + st[0] - st[2]]) * a.f2[4];
-      const double pyz = (phi[q + st[1] + st[2]] + phi[q - st[1] - st[2]] - phi[q - st[1] + st[2]] -
-                          phi[q + st[1] - st[2]]) * a.f2[5];
-      const double sx = phx * phx, sy = phy * phy, sz = phz * phz;
+      const double pxx = mulz(fma(-2.0, cc, phi[q + 2 * st[0]] + phi[q - 2 * st[0]]), a.f2[0]);
+      const double pyy = mulz(fma(-2.0, cc, phi[q + 2 * st[1]] + phi[q - 2 * st[1]]), a.f2[1]);
+      const double pzz = mulz(fma(-2.0, cc, phi[q + 2 * st[2]] + phi[q - 2 * st[2]]), a.f2[2]);
+      const double pxy = mulz(phi[q + st[0] + st[1]] + phi[q - st[0] - st[1]] - phi[q - st[0] + st[1]] -
+                              phi[q + st[0] - st[1]], a.f2[3]);
+      const double pxz = mulz(phi[q + st[0] + st[2]] + phi[q - st[0] - st[2]] - phi[q - st[0] + st[2]] -
+                              phi[q + st[0] - st[2]], a.f2[4]);
+      const double pyz = mulz(phi[q + st[1] + st[2]] + phi[q - st[1] - st[2]] - phi[q - st[1] + st[2]] -
+                              phi[q + st[1] - st[2]], a.f2[5]);
+      const double yz = sy + sz, xz = sx + sz, xy = sx + sy;
+      const double hxy = mulz(phx, phy), hxz = mulz(phx, phz), hyz = mulz(phy, phz);
       // kappa numerator (3d.f:2337-2379), regrouped
-      const double curv = pxx * (sy + sz) + pyy * (sx + sz) + pzz * (sx + sy) -
-                          2 * (pxy * phx * phy + pxz * phx * phz + pyz * phy * phz);
+      const double curv = fma(pxx, yz, fma(pyy, xz, mulz(pzz, xy))) -
+                          2 * fma(pxy, hxy, fma(pxz, hxz, mulz(pyz, hyz)));
       const double ig = qss_emu::div(1.0, grad);
-      const double cb = w * a.bcoef[q] * ig;  // d RHS / d numerator
-      const double gb = -cb * curv * ig;      // d RHS / d grad
-      out[0] = 2 * (phx * (cb * (pyy + pzz) + gb) - cb * (pxy * phy + pxz * phz)) * fx;
-      out[1] = 2 * (phy * (cb * (pxx + pzz) + gb) - cb * (pxy * phx + pyz * phz)) * fy;
-      out[2] = 2 * (phz * (cb * (pxx + pyy) + gb) - cb * (pxz * phx + pyz * phy)) * fz;
-      out[3] = cb * (sy + sz) * a.f2[0];
-      out[4] = cb * (sx + sz) * a.f2[1];
-      out[5] = cb * (sx + sy) * a.f2[2];
-      const double m2cb = -2 * cb;
-      out[6] = m2cb * phx * phy * a.f2[3];
-      out[7] = m2cb * phx * phz * a.f2[4];
-      out[8] = m2cb * phy * phz * a.f2[5];
+      const double cb = mulz(mulz(w, bco), ig);         // d RHS / d numerator
+      const double gb = -mulz(mulz(cb, curv), ig);      // d RHS / d grad
+      const double c2 = cb + cb;
+      const double cx = mulz(c2, phx), cy = mulz(c2, phy), cz = mulz(c2, phz), g2 = gb + gb;
+      // 2 (ph (cb (the two second differences across) + gb) - cb (mixed terms)) f
+      out[0] = mulz(fma(cx, pyy + pzz, fma(g2, phx, -fma(pxy, cy, mulz(pxz, cz)))), fx);
+      out[1] = mulz(fma(cy, pxx + pzz, fma(g2, phy, -fma(pxy, cx, mulz(pyz, cz)))), fy);
+      out[2] = mulz(fma(cz, pxx + pyy, fma(g2, phz, -fma(pxz, cx, mulz(pyz, cy)))), fz);
+      out[3] = mulz(mulz(cb, yz), a.f2[0]);
+      out[4] = mulz(mulz(cb, xz), a.f2[1]);
+      out[5] = mulz(mulz(cb, xy), a.f2[2]);
+      out[6] = -mulz(mulz(cx, phy), a.f2[3]);
+      out[7] = -mulz(mulz(cx, phz), a.f2[4]);
+      out[8] = -mulz(mulz(cy, phz), a.f2[5]);
     }
   }
 #pragma unroll
@@ -210,7 +222,7 @@ __global__ void __launch_bounds__(128) k_adj_carry(AdjPointArgs a) {
   const int k = b.klo + blockIdx.z * blockDim.z + threadIdx.z;
   if (i > b.ihi || j > b.jhi || k > b.khi) return;
   const int64_t q = b.idx(i, j, k);
-  if (fabs(a.vel_n[q]) >= 1.e-5) return;
+  if (moving(a.vel_n[q])) return;
   const double w = a.coef_l * a.lam_in[q];
   const int src = a.nsrc[q];
   if (w == 0.0 || src < 0) return;
