@@ -217,33 +217,21 @@ KERNEL_NAME = {0: "k_stage<WENO5,var> (fused RHS + TVD-RK stage)",
 WINDOW_NAME = {1: "k_weno_axis<0> (WENO5 x-pass, sliding window)",
                2: "k_weno_axis<1> (WENO5 y-pass, sliding window)",
                3: "k_weno_axis<2> (WENO5 z-pass, sliding window)"}
-# FP64-pipe instructions (DADD + DMUL) per fill-box voxel of one tile-form axis
-# pass by tile geometry, from ncu (smsp__sass_thread_inst_executed_op_{dadd,dmul}_pred_on.sum
-# of one launch over its voxels; 16 x 16 at 192^3: 50.94 + 5.07, 8 x 27 at
-# 216^3: 49.33 + 4.66); the rest of the 98 algorithmic operations (divisions,
-# squares, scalings, maxima, scaled copies, the weights' products) run on the
-# integer pipes.  FP64_PIPE_BUSY_TILE: sm__inst_executed_pipe_fp64 (pct of
-# peak, active) of the same launches (a build before the out-of-line division
-# and product, which leave the FP64 instruction counts unchanged).
-FP64_INSTR_PER_VOXEL_TILE = {"16 x 16": 56.0, "8 x 27": 54.0}
-FP64_PIPE_BUSY_TILE = {"16 x 16": ("192^3", 72.8), "8 x 27": ("216^3", 76.0)}
-
-
-def tile_geometry(line: int) -> str:
-    """The library's default tile for a line of `line` voxels: 8 x 27 where the
-    last 27-voxel tile is at most 2 % idle, else 16 x 16."""
-    tiles = -(-line // 27)
-    return "8 x 27" if tiles * 27 * 50 <= line * 51 else "16 x 16"
+# FP64-pipe instructions per fill-box voxel of one tile-form axis pass, by the longest
+# tile along the line, from ncu (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}
+# _pred_on.sum of the three passes over their voxels); the rest of the 98 algorithmic
+# operations run on the integer pipes.  FP64_PIPE_BUSY_TILE: the pipe's cycles, 77 an
+# instruction, over the active ones of the same launches.
+FP64_INSTR_PER_VOXEL_TILE = {"4 x 64": 38.4}
+FP64_PIPE_BUSY_TILE = {"4 x 64": ("256^3", 93.0)}
 N_KINDS = 5
 # DRAM bytes per fill-box voxel of one launch of each stage kernel, measured at
 # 512^3 with ncu (dram__bytes_read.sum + dram__bytes_write.sum, one pass):
 # x pass 7.74 GB, y pass 3.40 GB, z pass 3.37 GB, combine 14.22 GB for 134.2 M
 # voxels; the fused kernel was not captured
 TRAFFIC_BYTES_PER_VOXEL = {1: 57.7, 2: 25.3, 3: 25.1, 4: 105.9}
-# the same for the 16 x 16 tile form of the axis passes and the combine kernel,
-# measured at 256^3 with ncu (one kernel and at most three launches per
-# capture): x pass 474.2 MB, y 363.9 MB, z 362.2 MB, combine 2470.3 MB for
-# 16.78 M voxels
+# the same for the tile form of the axis passes and the combine kernel, measured at
+# 256^3 with ncu (one kernel and at most three launches per capture)
 TRAFFIC_BYTES_PER_VOXEL_TILE = {1: 28.3, 2: 21.7, 3: 21.6, 4: 147.2}
 # algorithmic HBM bytes per voxel-step (each array touched once per stage):
 # stage 1 phi + 5 coefficients -> phi1, stage 2 phi1 + phi + 5 coeff -> phi2,
@@ -280,7 +268,7 @@ def gpu_arm(args, dist: Dist):
     top = int(out[4])
     top_ms = out[1]
     window = args.axis_variant in (0, 1, 2)
-    geom = {None: tile_geometry(n), 3: "16 x 16", 4: "8 x 27"}.get(args.axis_variant)
+    geom = {3: "4 x 16", 4: "4 x 27"}.get(args.axis_variant, "4 x 64")
 
     def kname(k):
         return (WINDOW_NAME if window and k in WINDOW_NAME else KERNEL_NAME)[k].format(geom)
@@ -344,20 +332,20 @@ def gpu_arm(args, dist: Dist):
     tile = top in (1, 2, 3) and not window
     if tile or (top == 4 and not window):
         traffic_table = dict(TRAFFIC_BYTES_PER_VOXEL_TILE)
-        traffic_unit = "bytes per launch (ncu at 256^3 with 16 x 16 tiles, scaled per voxel to this size)"
+        traffic_unit = "bytes per launch (ncu at 256^3, scaled per voxel to this size)"
     else:
         traffic_table = TRAFFIC_BYTES_PER_VOXEL
         traffic_unit = "bytes per launch (ncu at 512^3, scaled per voxel to this size)"
     fp64_pipe = None
-    if tile and top_ms > 0:
+    if tile and top_ms > 0 and geom in FP64_INSTR_PER_VOXEL_TILE:
         per_voxel = FP64_INSTR_PER_VOXEL_TILE[geom]
         instr = per_voxel * nvox / (top_ms / 1e3) / 1e12
         fp64_pipe = {"instructions_per_voxel": per_voxel, "tile": geom, "achieved": round(instr, 4),
                      "peak": fp64_peak, "unit": "T instructions/s", "frac": round(instr / fp64_peak, 4),
                      "ncu_busy_pct": FP64_PIPE_BUSY_TILE[geom][1], "ncu_case": FP64_PIPE_BUSY_TILE[geom][0],
-                     "note": "FP64-pipe instructions (DADD + DMUL, ncu count per voxel) over the launch time, "
-                             "against the non-FMA issue rate; ncu_busy_pct is sm__inst_executed_pipe_fp64 "
-                             "(pct of peak) of the same kernel in the ncu_case capture"}
+                     "note": "FP64-pipe instructions (ncu count per voxel) over the launch time, "
+                             "against the non-FMA issue rate; ncu_busy_pct is the pipe's cycles over the active "
+                             "ones of the same kernel in the ncu_case capture"}
     # HBM: the step's algorithmic bytes over the time of all its stage kernels
     stage_total_ms = out[3] / args.steps
     achieved_gbs = BYTES_PER_VOXEL_STEP * nvox / (stage_total_ms / 1e3) / 1e9 if stage_total_ms > 0 else 0.0
@@ -784,7 +772,7 @@ def main():
                     help="skip the adjoint run that keeps the whole trajectory in HBM (no recomputation)")
     ap.add_argument("--axis-variant", type=int, default=None,
                     help="WENO5 axis passes: 0 registers, 1 shared memory, 2 launch shapes tuned by timing, "
-                         "3 tiles with one voxel per thread (default: tiles)")
+                         "3 / 4 tiles of up to 16 / 27 voxels along the line (default: tiles of up to 64)")
     ap.add_argument("--traffic", type=float, default=None,
                     help="DRAM bytes per launch of the roofline kernel (overrides the measured table)")
     args = ap.parse_args()

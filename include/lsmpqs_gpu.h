@@ -225,9 +225,10 @@ int qssgpu_set_weno_split(int mode);
    products and sums; -1 restores the default.  Results are identical at
    every level.  Returns the previous level. */
 int qssgpu_set_emu_level(int level);
-/* form of the WENO5 axis passes at levels >= 1: -1 (default) and 3 tiles
-   of 16 lines x 16 voxels, one voxel per thread, every face and centre of a
-   tile computed once into shared memory; 4 tiles of 8 lines x 27 voxels; 0
+/* form of the WENO5 axis passes at levels >= 1: tiles, every face and centre
+   of a tile computed once into shared memory, -1 (default) of 4 lines x up to
+   64 voxels, shorter on small boxes; 3 / 4 of 4 lines x up to 16 / 27 voxels
+   (16 x 16 and 8 x 27 at level 1, whose default is one of the two); 0
    sliding window in registers; 1 the window's scaled copies in shared
    memory and the smoothness squares on the integer pipes; 2 tuned: the
    first pass over each line shape times every distinct (form, segment
@@ -323,7 +324,8 @@ int qssgpu_forward_theta(Options *o, QSS_DataArrays *p, Grid *g, const double *t
    elsewhere; the volume integrals use the same code.  0 on success. */
 int qssgpu_loop_sum(const double *values, long long n, double *out);
 int qssgpu_get_slabs(const Grid *g);
-/* frees the device copy kept for p (destroyQSSDataArrays calls it) */
+/* frees the device copy kept for p (destroyQSSDataArrays calls it), and the unused
+   scratch memory the library holds on the current GPU */
 void qssgpu_release(QSS_DataArrays *p);
 /* page-locked, zeroed host memory for the arrays of a QSS_DataArrays (the
    copies to and from the device then skip the driver's staging); NULL on

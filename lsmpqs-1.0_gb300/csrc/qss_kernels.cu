@@ -26,8 +26,6 @@ inline dim3 fb_grid(const Box& b, dim3 blk) {
   return dim3((b.fbx() + blk.x - 1) / blk.x, (b.fby() + blk.y - 1) / blk.y, (b.fbz() + blk.z - 1) / blk.z);
 }
 
-inline unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
-
 // ---------------------------------------------------------------------------
 // inner step: dt
 

@@ -77,11 +77,10 @@ void launch_stage(cudaStream_t s, int scheme, bool var, int stage, bool final_st
 
 // emulation level of the split WENO5 kernels (defined in qss_state.cu)
 int emu_level();
-// form of the WENO5 axis passes at integer-pipe levels >= 1: 0 the sliding
-// window in registers, 1 the faces' scaled copies in shared memory with the
-// smoothness squares on the integer pipes (faster from ~12 M fill voxels),
-// -1 (default) chosen by the launch's size ($QSSGPU_AXIS_VARIANT,
-// qssgpu_set_axis_variant); both give identical results
+// form of the WENO5 axis passes at integer-pipe levels >= 1: -1 (default) tiles, 3 / 4
+// tiles of up to 16 / 27 voxels along the line, 0 the sliding window in registers, 1
+// the faces' scaled copies in shared memory, 2 tuned by timing ($QSSGPU_AXIS_VARIANT,
+// qssgpu_set_axis_variant); all give identical results
 int axis_variant();
 
 // WENO5 variable-coefficient stage as three axis passes (one-sided
