@@ -306,7 +306,7 @@ __device__ __forceinline__ void eno_finish(const StageArgs& a, int64_t idx, cons
   }
   const double bco = VAR ? a.c.b[idx] : a.c.b_const;
   if (!VAR || qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign)  // as in k_weno_combine2
-    rhs = rhs + qss_emu::mul(bco, curvature_fast<INT>(phi, b, idx, a.fac));
+    rhs = rhs + qss_emu::mul(bco, curvature_fast<INT, SCHEME == ENO2>(phi, b, idx, a.fac));
   if (VAR) rhs = add_advection<true>(rhs, a.c.vx[idx], a.c.vy[idx], a.c.vz[idx], pp, pm, a.inv);
   const double out = rk_combine<STAGE>(rhs, STAGE ? a.ctl->dt : 0.0, STAGE ? __ldg(phi + idx) : 0.0, a.u_cur, idx);
   a.out[idx] = out;

@@ -21,6 +21,7 @@ namespace qss {
 // one OR
 __device__ __forceinline__ uint32_t win8(double x) { return qss_emu::hi32(x) * 2u - 0x70000000u; }
 constexpr uint32_t kWin8 = 0x20000000u;
+__device__ __forceinline__ bool is_zero(double x) { return ((qss_emu::hi32(x) * 2u) | qss_emu::lo32(x)) == 0; }
 
 __device__ __forceinline__ double mulw(double x, double y, int k = 0) {
   return qss_emu::mul_win(qss_emu::hi32(x), qss_emu::lo32(x), qss_emu::hi32(y), qss_emu::lo32(y), k);
@@ -48,8 +49,13 @@ __device__ __forceinline__ double sum_sq(double a, double b, double c) {
   return INT ? qss_emu::add_pos(qss_emu::add_pos(a, b), c) : a + b + c;
 }
 
-// curvature() (3d.f:2337-2379), the same operations
-template <bool INT = false>
+// curvature() (3d.f:2337-2379), the same operations.  ZERO: exact zeros among the
+// differences (planes, symmetric parts) stay in the straight line, where a product
+// with one holds nothing of use and its term is replaced by a signed zero; otherwise
+// they take the native form.  ENO2 on GB300: drainage 64^3, where plane parts are
+// common, stages 9.13 -> 8.13 ms.  The WENO5 combine kernel goes without: 24^3 6 % and
+// 110^3 1 % faster with it, 192^3 and 320^3 1 % slower (registers).
+template <bool INT = false, bool ZERO = false>
 __device__ __forceinline__ double curvature_fast(const double* __restrict__ phi, const Box& b, int64_t c,
                                                  const Fac& f) {
   const int64_t sy = b.sy(), sz = b.sz();
@@ -65,22 +71,34 @@ __device__ __forceinline__ double curvature_fast(const double* __restrict__ phi,
   const double dxy = __ldg(q + 1 + sy) + __ldg(q - 1 - sy) - __ldg(q - 1 + sy) - __ldg(q + 1 - sy);
   const double dxz = __ldg(q + 1 + sz) + __ldg(q - 1 - sz) - __ldg(q - 1 + sz) - __ldg(q + 1 - sz);
   const double dyz = __ldg(q + sy + sz) + __ldg(q - sy - sz) - __ldg(q - sy + sz) - __ldg(q + sy - sz);
-  const uint32_t w = win8(dx) | win8(dy) | win8(dz) | win8(dxx) | win8(dyy) | win8(dzz) | win8(dxy) | win8(dxz) | win8(dyz);
+  auto zero = [](double d) { return ZERO && is_zero(d); };
+  const bool zx = zero(dx), zy = zero(dy), zz = zero(dz);
+  const bool zxx = zero(dxx), zyy = zero(dyy), zzz = zero(dzz);
+  const bool zxy = zero(dxy), zxz = zero(dxz), zyz = zero(dyz);
+  auto out = [](bool z, double d) { return z ? 0u : win8(d); };
+  const uint32_t w = out(zx, dx) | out(zy, dy) | out(zz, dz) | out(zxx, dxx) | out(zyy, dyy) | out(zzz, dzz) |
+                     out(zxy, dxy) | out(zxz, dxz) | out(zyz, dyz);
   if (w >= kWin8) return curvature_native(phi, b, c, f);
+  auto term = [](bool zero, uint32_t sign, double v) {
+    return zero ? __hiloint2double((int)(sign & 0x80000000u), 0) : v;
+  };
+  const uint32_t hx = qss_emu::hi32(dx), hy = qss_emu::hi32(dy), hz = qss_emu::hi32(dz);
+  const uint32_t hxx = qss_emu::hi32(dxx), hyy = qss_emu::hi32(dyy), hzz = qss_emu::hi32(dzz);
   const double x = mulw(dx, f.x), y = mulw(dy, f.y), z = mulw(dz, f.z);
-  const double g2 = sum_sq<INT>(sqw(x), sqw(y), sqw(z));
+  const double g2 = sum_sq<INT>(term(zx, 0, sqw(x)), term(zy, 0, sqw(y)), term(zz, 0, sqw(z)));
   if (qss_emu::bits(g2) < 0x3ee4f8b588e368f1ull) return 0.0;  // 1e-5
   const double xx = mulw(mulw(dxx, f.x), f.x);
   const double yy = mulw(mulw(dyy, f.y), f.y);
-  double curv = mulw(mulw(xx, y), y) + mulw(mulw(yy, x), x);
-  curv = curv - mulw(mulw(mulw(mulw(dxy, f.x), f.y, 1), x), y);
-  curv = curv + mulw(mulw(xx, z), z);
-  const double zz = mulw(mulw(dzz, f.z), f.z);
-  curv = curv + mulw(mulw(zz, x), x);
-  curv = curv - mulw(mulw(mulw(mulw(dxz, f.x), f.z, 1), x), z);
-  curv = curv + mulw(mulw(yy, z), z);
-  curv = curv + mulw(mulw(zz, y), y);
-  curv = curv - mulw(mulw(mulw(mulw(dyz, f.y), f.z, 1), y), z);
+  double curv = term(zxx || zy, hxx, mulw(mulw(xx, y), y)) + term(zyy || zx, hyy, mulw(mulw(yy, x), x));
+  curv = curv - term(zxy || zx || zy, qss_emu::hi32(dxy) ^ hx ^ hy, mulw(mulw(mulw(mulw(dxy, f.x), f.y, 1), x), y));
+  curv = curv + term(zxx || zz, hxx, mulw(mulw(xx, z), z));
+  const double zzv = mulw(mulw(dzz, f.z), f.z);
+  curv = curv + term(zzz || zx, hzz, mulw(mulw(zzv, x), x));
+  curv = curv - term(zxz || zx || zz, qss_emu::hi32(dxz) ^ hx ^ hz, mulw(mulw(mulw(mulw(dxz, f.x), f.z, 1), x), z));
+  curv = curv + term(zyy || zz, hyy, mulw(mulw(yy, z), z));
+  curv = curv + term(zzz || zy, hzz, mulw(mulw(zzv, y), y));
+  curv = curv - term(zyz || zy || zz, qss_emu::hi32(dyz) ^ hy ^ hz, mulw(mulw(mulw(mulw(dyz, f.y), f.z, 1), y), z));
+  if (ZERO && is_zero(curv)) return curv;  // over a positive g2
   return qss_emu::div(curv, g2);
 }
 
