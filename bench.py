@@ -212,7 +212,7 @@ KERNEL_NAME = {0: "k_stage<WENO5,var> (fused RHS + TVD-RK stage)",
                1: "k_weno_tile<0> (WENO5 x-pass, {} tiles, shared sub-expressions)",
                2: "k_weno_tile<1> (WENO5 y-pass, {} tiles, shared sub-expressions)",
                3: "k_weno_tile<2> (WENO5 z-pass, {} tiles, shared sub-expressions)",
-               4: "k_weno_combine (Godunov + advection + curvature + TVD-RK)"}
+               4: "k_weno_combine2 (Godunov + advection + curvature + TVD-RK)"}
 # the window forms (--axis-variant 0/1/2) run k_weno_axis<axis> instead
 WINDOW_NAME = {1: "k_weno_axis<0> (WENO5 x-pass, sliding window)",
                2: "k_weno_axis<1> (WENO5 y-pass, sliding window)",
@@ -222,8 +222,8 @@ WINDOW_NAME = {1: "k_weno_axis<0> (WENO5 x-pass, sliding window)",
 # _pred_on.sum of the three passes over their voxels); the rest of the 98 algorithmic
 # operations run on the integer pipes.  FP64_PIPE_BUSY_TILE: the pipe's cycles, 77 an
 # instruction, over the active ones of the same launches.
-FP64_INSTR_PER_VOXEL_TILE = {"4 x 64": 38.4}
-FP64_PIPE_BUSY_TILE = {"4 x 64": ("256^3", 93.0)}
+FP64_INSTR_PER_VOXEL_TILE = {"4 x 64": 37.8}
+FP64_PIPE_BUSY_TILE = {"4 x 64": ("256^3", 94.0)}
 N_KINDS = 5
 # DRAM bytes per fill-box voxel of one launch of each stage kernel, measured at
 # 512^3 with ncu (dram__bytes_read.sum + dram__bytes_write.sum, one pass):
@@ -232,7 +232,7 @@ N_KINDS = 5
 TRAFFIC_BYTES_PER_VOXEL = {1: 57.7, 2: 25.3, 3: 25.1, 4: 105.9}
 # the same for the tile form of the axis passes and the combine kernel, measured at
 # 256^3 with ncu (one kernel and at most three launches per capture)
-TRAFFIC_BYTES_PER_VOXEL_TILE = {1: 28.3, 2: 21.7, 3: 21.6, 4: 147.2}
+TRAFFIC_BYTES_PER_VOXEL_TILE = {1: 25.2, 2: 22.3, 3: 22.2, 4: 122.9}
 # algorithmic HBM bytes per voxel-step (each array touched once per stage):
 # stage 1 phi + 5 coefficients -> phi1, stage 2 phi1 + phi + 5 coeff -> phi2,
 # stage 3 phi2 + phi + 5 coeff + 3 masks -> phi1, phi
@@ -358,7 +358,7 @@ def gpu_arm(args, dist: Dist):
                 "launch_ms": round(top_ms, 4), "kernels": kinds,
                 "peak_source": peak_src, "dfma_peak_tflops": dfma_tflops,
                 "note": "achieved = the kernel's algorithmic FP64 operations per launch over its mean launch time "
-                        "(CUDA events); about a third of them (divisions, squares, power-of-two scalings, maxima, "
+                        "(CUDA events); most of them (divisions, products, squares, power-of-two scalings, maxima, "
                         "scaled copies) run bit-exactly on the integer pipes, so frac against the FP64 pipe's "
                         "non-FMA ceiling can exceed 1; fp64_pipe is the pipe's own utilisation",
                 "fp64_pipe": fp64_pipe,
