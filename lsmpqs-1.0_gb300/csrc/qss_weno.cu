@@ -10,16 +10,16 @@
 // on identical operands wherever it appears, so computing it once per line
 // and reusing it reproduces the reference's values bit for bit while cutting
 // the FP64 instructions per voxel -- the resource that bounds this kernel on
-// GB300 (one FP64 warp instruction per ~64 cycles per scheduler).
+// GB300 (one FP64 warp instruction per 77 cycles per scheduler).
 //
 // A stage runs as three axis passes and one combine kernel:
-//   k_weno_tile<AX> (the default): a block computes every face and centre of
+//   k_weno_tile (the default): a block computes every face and centre of
 //     a tile of lines once into shared memory, then one thread per voxel the
 //     two reconstructions, and writes the plus and minus one-sided
 //     derivatives of that axis (2 doubles per voxel);
 //   k_weno_axis<AX> (selectable): each thread walks a segment of voxels along
 //     axis AX with a sliding window of faces / centres, same outputs;
-//   k_weno_combine: Godunov normal term (with the carried term of voxels whose
+//   k_weno_combine2 (level 2), k_weno_combine: Godunov normal term (with the carried term of voxels whose
 //     speed is below 1e-5), upwind advection, central curvature, TVD-RK
 //     combination and, on the last stage, the three mask impositions.
 // The extra traffic (48 B written + 48 B read per voxel and stage) costs about
@@ -933,8 +933,8 @@ __global__ void __launch_bounds__(128, 10) k_weno_combine(CombineArgs a) {
 
 // The combine kernel at EMU 2 (qss_stage.cuh), same patches and curvature skip.
 // Bound: FP64 pipe (~36 additions where the curvature is taken) and ~1400
-// integer instructions.  512^3 on GB300: 14.29 -> 8.75 ms a launch, 192^3 0.775 ->
-// 0.488 (64 registers, 8 blocks per SM; 10 blocks 8.66 / 0.484 with spills, 64^3
+// integer instructions.  512^3 on GB300: 14.29 -> 8.75 ms a launch (8.35 since its tests of
+// bits left the FP64 pipe), 192^3 0.775 -> 0.488 (64 registers, 8 blocks per SM; 10 blocks 8.66 / 0.484 with spills, 64^3
 // 8 % slower; 6 blocks 9.66 / 0.535).
 template <int STAGE, bool FINAL>
 __global__ void __launch_bounds__(128, 8) k_weno_combine2(CombineArgs a) {
