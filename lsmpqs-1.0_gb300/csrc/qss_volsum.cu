@@ -409,7 +409,9 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restri
   constexpr uint64_t hidden = 1ull << 52;
   double s = 0.0;    // the same in every thread
   int64_t born = 0;  // where s left zero, to a few elements
-  auto significand = [&](int E) { return E > -1000 ? (dbits(s) & (hidden - 1)) | hidden : 0ull; };
+  // of every normal s, so that the top of its binade is seen; zero for any other s, whose
+  // windows apply to zeros only
+  auto significand = [&](int E) { return E >= -1022 ? (dbits(s) & (hidden - 1)) | hidden : 0ull; };
   for (int64_t j = 0; j < nc;) {
     unsigned long long before;
     if (have_r) {
