@@ -9,25 +9,9 @@
 // "3d.f" = src/spatial_derivatives/qss_spatial_derivatives3d.f of the reference.
 #pragma once
 #include <cstdint>
+#include "qss_box.cuh"
 
 namespace qss {
-
-// Index space of one volume: ghost box [0,nx)x[0,ny)x[0,nz), fill box
-// [ilo,ihi]x[jlo,jhi]x[klo,khi], column-major with i fastest.
-struct Box {
-  int nx, ny, nz;
-  int ilo, ihi, jlo, jhi, klo, khi;
-  __host__ __device__ int64_t sx() const { return 1; }
-  __host__ __device__ int64_t sy() const { return nx; }
-  __host__ __device__ int64_t sz() const { return (int64_t)nx * ny; }
-  __host__ __device__ int64_t idx(int i, int j, int k) const {
-    return (int64_t)i + (int64_t)nx * ((int64_t)j + (int64_t)ny * k);
-  }
-  __host__ __device__ int64_t npts() const { return (int64_t)nx * ny * nz; }
-  __host__ __device__ int fbx() const { return ihi - ilo + 1; }
-  __host__ __device__ int fby() const { return jhi - jlo + 1; }
-  __host__ __device__ int fbz() const { return khi - klo + 1; }
-};
 
 enum Scheme { ENO2 = 2, ENO3 = 3, WENO5 = 5 };
 

@@ -643,14 +643,7 @@ __global__ void __launch_bounds__(kNearThreads) k_distance0(Box b, const double*
   using namespace qss_emu;
   __shared__ uint16_t near_t[kNearVoxels];
   __shared__ int near_n;
-  const uint32_t fbx = (uint32_t)b.fbx(), fby = (uint32_t)b.fby();
-  const int64_t base = (int64_t)blockIdx.x * kNearVoxels, n = (int64_t)fbx * fby * b.fbz(), row0 = base / fbx;
-  const uint32_t i0 = (uint32_t)(base - row0 * fbx), k0 = (uint32_t)(row0 / fby),
-                 j0 = (uint32_t)(row0 - (int64_t)k0 * fby);
-  auto at = [&](uint32_t t) {  // index of the block's voxel t
-    const uint32_t x = i0 + t, r = x / fbx, y = j0 + r, q = y / fby;
-    return b.idx(b.ilo + (int)(x - r * fbx), b.jlo + (int)(y - q * fby), b.klo + (int)(k0 + q));
-  };
+  const FillBlock blk(b, blockIdx.x, kNearVoxels);
   const int64_t st[6] = {1, -1, b.sy(), -b.sy(), b.sz(), -b.sz()};
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) near_n = 0;
@@ -658,8 +651,8 @@ __global__ void __launch_bounds__(kNearThreads) k_distance0(Box b, const double*
   for (int t0 = 0; t0 < kNearVoxels; t0 += kNearThreads) {
     const uint32_t t = t0 + threadIdx.x;
     bool near = false;
-    if (base + t < n) {
-      const int64_t c = at(t);
+    if (blk.in(t)) {
+      const int64_t c = blk.at(b, t);
       const double cc = phi0[c];
       // opposite signs, zero counted as negative
       const bool pos = gt0(cc), nonpos = lt0(cc) || mag2(bits(cc)) == 0;
@@ -679,7 +672,7 @@ __global__ void __launch_bounds__(kNearThreads) k_distance0(Box b, const double*
   }
   __syncthreads();
   for (int e = threadIdx.x; e < near_n; e += kNearThreads) {
-    const int64_t c = at(near_t[e]);
+    const int64_t c = blk.at(b, near_t[e]);
     const double cc = phi0[c];
     double v[6];
     uint64_t top = mag2(bits(cc));
@@ -1118,15 +1111,7 @@ __global__ void __launch_bounds__(kSetThreads) k_setvar(Box b, SetVar a) {
   __shared__ uint16_t band[kSetVoxels];
   __shared__ int band_n;
   __shared__ double cos_theta;
-  const uint32_t fbx = (uint32_t)b.fbx(), fby = (uint32_t)b.fby();
-  const int64_t base = (int64_t)blockIdx.x * kSetVoxels, n = (int64_t)fbx * fby * b.fbz();
-  const int64_t row0 = base / fbx;
-  const uint32_t i0 = (uint32_t)(base - row0 * fbx), k0 = (uint32_t)(row0 / fby),
-                 j0 = (uint32_t)(row0 - (int64_t)k0 * fby);
-  auto at = [&](uint32_t t) {  // index of the block's voxel t
-    const uint32_t x = i0 + t, r = x / fbx, y = j0 + r, q = y / fby;
-    return b.idx(b.ilo + (int)(x - r * fbx), b.jlo + (int)(y - q * fby), b.klo + (int)(k0 + q));
-  };
+  const FillBlock blk(b, blockIdx.x, kSetVoxels);
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) band_n = 0;
   if (!CURV && !a.theta_field && threadIdx.x < 32) {
@@ -1156,8 +1141,8 @@ __global__ void __launch_bounds__(kSetThreads) k_setvar(Box b, SetVar a) {
   for (int t0 = 0; t0 < kSetVoxels; t0 += kSetThreads) {
     const uint32_t t = t0 + threadIdx.x;
     bool rest = false;
-    if (base + t < n) {
-      const int64_t c = at(t);
+    if (blk.in(t)) {
+      const int64_t c = blk.at(b, t);
       const double m = a.mask[c], gx = a.mx[c], gy = a.my[c], gz = a.mz[c];
       uint32_t top;
       rest = !(a.plain && coef_plain(m, gx, gy, gz, top));
@@ -1204,7 +1189,7 @@ __global__ void __launch_bounds__(kSetThreads) k_setvar(Box b, SetVar a) {
   }
   __syncthreads();
   for (int e = threadIdx.x; e < band_n; e += kSetThreads) {
-    const int64_t c = at(band[e]);
+    const int64_t c = blk.at(b, band[e]);
     const double m = a.mask[c], gx = a.mx[c], gy = a.my[c], gz = a.mz[c];
     uint32_t top;
     SetVarOut r{};

@@ -142,13 +142,13 @@ constexpr int kContribVoxels = 1024, kContribThreads = 256;
 __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const double* __restrict__ phi, double dV,
                                                                  double eps, double* contrib, float* csum) {
   __shared__ double band_p[kContribVoxels];
-  __shared__ uint32_t band_q[kContribVoxels];
+  __shared__ uint16_t band_t[kContribVoxels];
   __shared__ int band_n;
   __shared__ float red[kContribThreads / 32];
   const double pi = 3.14159265358979323846;
   const double one_over_pi = 0.31830988618379;
-  const uint32_t n = (uint32_t)b.fbx() * b.fby() * b.fbz();  // below 2^31
-  const uint32_t base = blockIdx.x * (uint32_t)kContribVoxels;
+  const FillBlock blk(b, blockIdx.x, kContribVoxels);
+  contrib += blk.base;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) band_n = 0;
   __syncthreads();
@@ -160,19 +160,15 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
   };
   float sum = 0.0f;
 #pragma unroll
-  for (int t = 0; t < kContribVoxels; t += kContribThreads) {
-    const uint32_t q = base + t + threadIdx.x;
+  for (int t0 = 0; t0 < kContribVoxels; t0 += kContribThreads) {
+    const uint32_t t = t0 + threadIdx.x;
     bool band = false;
     double p = 0.0;
-    if (q < n) {
-      const uint32_t r = q / (uint32_t)b.fbx();
-      const int i = b.ilo + (int)(q - r * (uint32_t)b.fbx());
-      const int k = b.klo + (int)(r / (uint32_t)b.fby());
-      const int j = b.jlo + (int)(r - (uint32_t)(k - b.klo) * (uint32_t)b.fby());
-      p = phi[b.idx(i, j, k)];
+    if (blk.in(t)) {
+      p = phi[blk.at(b, t)];
       const bool inside = qss_emu::gt(-eps, p);  // p < -eps
       band = !inside && qss_emu::gt(eps, p);     // p < eps
-      if (!band) contrib[q] = inside ? dV : 0.0;
+      if (!band) contrib[t] = inside ? dV : 0.0;
       if (inside) sum += approx(dV);
     }
     const unsigned m = __ballot_sync(0xffffffffu, band);
@@ -181,15 +177,15 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << lane) - 1u));
     if (band) {
       band_p[at] = p;
-      band_q[at] = q;
+      band_t[at] = (uint16_t)t;
     }
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < band_n; t += kContribThreads) {
-    const double rr = band_p[t] / eps;
+  for (int e = threadIdx.x; e < band_n; e += kContribThreads) {
+    const double rr = band_p[e] / eps;
     const double one_minus_H = 0.5 * (1 - rr - one_over_pi * portable_sin(pi * rr));
     const double v = one_minus_H * dV;
-    contrib[band_q[t]] = v;
+    contrib[band_t[e]] = v;
     sum += approx(v);
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
