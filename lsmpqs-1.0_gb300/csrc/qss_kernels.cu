@@ -305,7 +305,8 @@ __device__ __forceinline__ void eno_finish(const StageArgs& a, int64_t idx, cons
     if (src >= 0) rhs = carried_norm<SCHEME>(phi, b, src, a.inv, a.c.vel_n);
   }
   const double bco = VAR ? a.c.b[idx] : a.c.b_const;
-  if (!VAR || qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign)  // as in k_weno_combine2
+  // b * kappa is +-0 where b is +0 and kappa finite, and changes no term but -0
+  if (!VAR || qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign || !curvature_finite(phi, b, idx))
     rhs = rhs + qss_emu::mul(bco, curvature_fast<INT, SCHEME == ENO2>(phi, b, idx, a.fac));
   if (VAR) rhs = add_advection<true>(rhs, a.c.vx[idx], a.c.vy[idx], a.c.vz[idx], pp, pm, a.inv);
   const double out = rk_combine<STAGE>(rhs, STAGE ? a.ctl->dt : 0.0, STAGE ? __ldg(phi + idx) : 0.0, a.u_cur, idx);

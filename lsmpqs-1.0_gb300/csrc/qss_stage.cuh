@@ -102,6 +102,31 @@ __device__ __forceinline__ double curvature_fast(const double* __restrict__ phi,
   return qss_emu::div(curv, g2);
 }
 
+// whether curvature() is certainly finite: every point it reads below 2^200 in magnitude
+// (grid factors of at most 2^50: numerator below 2^810, over at least 1e-5).  25 loads of
+// high words in place of the curvature's FP64 instructions: the ENO2 stages with variable
+// coefficients take 6.24 ms of a 128^3 step against 6.00 without the look, GB300.
+__device__ __forceinline__ bool curvature_finite(const double* __restrict__ phi, const Box& b, int64_t c) {
+  const int64_t st[3] = {1, b.sy(), b.sz()};
+  const double* __restrict__ q = phi + c;
+  uint32_t top = 0;
+  auto see = [&](int64_t o) { top = max(top, __ldg(reinterpret_cast<const uint32_t*>(q + o) + 1) * 2u); };
+  see(0);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const int64_t s = st[d], t = st[(d + 1) % 3];
+    see(s);
+    see(-s);
+    see(2 * s);
+    see(-2 * s);
+    see(s + t);
+    see(s - t);
+    see(t - s);
+    see(-s - t);
+  }
+  return top < 0x98e00000u;  // 2 x the high word of 2^200
+}
+
 template <int SCHEME>
 __device__ __noinline__ double godunov_native(double vel, double px, double py, double pz, double mx, double my,
                                               double mz, double ix, double iy, double iz) {
