@@ -361,7 +361,13 @@ __global__ void __launch_bounds__(128, kEno2Blocks) k_eno2(StageArgs a) {
   const int64_t e0 = ey ? b.idx(i0 + min(li, lx), lane < 8 ? j0 - 1 : j0 + ly + 1, k0)
                         : (lane < 24 ? b.idx(lane < 20 ? i0 - 1 : i0 + lx + 1, j0 + er, k0) : c);
   const int64_t eo = e0 - c, es = ey ? sy : 1;
-  auto d2_of = [](double lo, double mid, double hi) { return __fma_rn(-2.0, mid, hi + lo); };
+  // an FMA does not overflow in 2 mid: where that is infinite (2^1023 and more), mid is made so
+  auto d2_of = [](double lo, double mid, double hi) {
+    const uint32_t h = qss_emu::hi32(mid);
+    const bool over = (h & 0x7ff00000u) == 0x7fe00000u;
+    const double m = __hiloint2double((int)(over ? (h & 0x80000000u) | 0x7ff00000u : h), (int)(over ? 0u : qss_emu::lo32(mid)));
+    return __fma_rn(-2.0, m, hi + lo);
+  };
   auto pick = [](double x, double y) { return abs_lt(x, y) ? x : y; };
   auto from = [](double v, int src) { return __shfl_sync(0xffffffffu, v, src); };
   double cc = __ldg(phi + c), zp = __ldg(phi + c + sz), d2z, d1zl, mzl;
