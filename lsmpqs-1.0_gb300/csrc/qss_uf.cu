@@ -214,13 +214,14 @@ __device__ __forceinline__ void unite_lanes(int* parent, bool pair, int64_t q, i
 
 __global__ void __launch_bounds__(256) k_uf_cross(Box b, const unsigned char* __restrict__ bin, int* parent, Ctl* ctl) {
   const int lane = threadIdx.x & 31;
-  const int x = blockIdx.x * 32 + lane, j = blockIdx.y * 8 + (threadIdx.x >> 5), k = blockIdx.z;
+  const int x = blockIdx.x * 32 + lane, j = blockIdx.y * 8 + (threadIdx.x >> 5);
   if (j >= b.ny) return;  // warp-uniform
-  const int64_t row = b.idx(0, j, k), q = row + x;
   int err = 0;
-  const bool fg = x < b.nx && bin[q];
-  const unsigned A = __ballot_sync(0xffffffffu, fg);
-  if (A) {
+  for (int k = blockIdx.z; k < b.nz; k += gridDim.z) {
+    const int64_t q = b.idx(0, j, k) + x;
+    const bool fg = x < b.nx && bin[q];
+    const unsigned A = __ballot_sync(0xffffffffu, fg);
+    if (!A) continue;
     const bool left_a = lane == 0 && x > 0 && bin[q - 1];
     const unsigned has_left = __ballot_sync(0xffffffffu, left_a) & 1u;  // A[x-1] of lane 0
     const bool prev = lane ? (A >> (lane - 1)) & 1u : has_left;
@@ -357,7 +358,8 @@ void launch_label(cudaStream_t s, const Box& b, const unsigned char* bin, int* l
   const unsigned seg = (unsigned)((b.nx + 31) / 32);
   const dim3 tiles(seg, (b.ny + kTileY - 1) / kTileY, (b.nz + kTileZ - 1) / kTileZ);
   k_uf_tile<<<tiles, kTileThreads, 0, s>>>(b, bin, labels, ctl);
-  k_uf_cross<<<dim3(seg, (b.ny + 7) / 8, b.nz), 256, 0, s>>>(b, bin, labels, ctl);
+  // a plane to a block; a block of a grid at its limit goes on to further planes
+  k_uf_cross<<<dim3(seg, (b.ny + 7) / 8, b.nz < 65535 ? b.nz : 65535), 256, 0, s>>>(b, bin, labels, ctl);
   k_uf_final<<<grid_for(n), 256, 0, s>>>(n, bin, labels, ctl);
 }
 
