@@ -38,7 +38,7 @@ int qssgpu_fp64_peak(double* out) {
     QSS_CK(cudaGetDevice(&dev));
     QSS_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     double* d = nullptr;
-    QSS_CK(cudaMalloc(&d, sizeof(double)));
+    device_malloc((void**)&d, sizeof(double));
     const int iters = 4096, threads = 256, blocks = sms * 8;
     cudaEvent_t e0, e1;
     QSS_CK(cudaEventCreate(&e0));

@@ -161,9 +161,9 @@ int qssgpu_emu_selftest(long long n, unsigned long long seed, long long* counts,
     unsigned long long* dc = nullptr;
     int* dflag = nullptr;
     double* dfirst = nullptr;
-    QSS_CK(cudaMalloc(&dc, 9 * sizeof(unsigned long long)));
-    QSS_CK(cudaMalloc(&dflag, sizeof(int)));
-    QSS_CK(cudaMalloc(&dfirst, 3 * sizeof(double)));
+    device_malloc((void**)&dc, 9 * sizeof(unsigned long long));
+    device_malloc((void**)&dflag, sizeof(int));
+    device_malloc((void**)&dfirst, 3 * sizeof(double));
     QSS_CK(cudaMemset(dc, 0, 9 * sizeof(unsigned long long)));
     QSS_CK(cudaMemset(dflag, 0, sizeof(int)));
     QSS_CK(cudaMemset(dfirst, 0, 3 * sizeof(double)));
@@ -197,7 +197,7 @@ int qssgpu_op_rates(double* out) {
     QSS_CK(cudaGetDevice(&dev));
     QSS_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     double* d = nullptr;
-    QSS_CK(cudaMalloc(&d, sizeof(double)));
+    device_malloc((void**)&d, sizeof(double));
     const int threads = 256, blocks = sms * 4, iters = 512;
     const double ops = (double)blocks * threads * iters * 8;
     const float t[7] = {time_rate<0, false>(d, blocks, threads, iters), time_rate<0, true>(d, blocks, threads, iters),

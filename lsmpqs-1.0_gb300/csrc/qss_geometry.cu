@@ -24,12 +24,14 @@ Box full_box(const Grid* g) {
   return b;
 }
 
+// call scratch on the legacy default stream, where these calls launch and copy
 struct Dev {
-  void* p = nullptr;
-  explicit Dev(size_t bytes) { QSS_CK(cudaMalloc(&p, bytes ? bytes : 8)); }
-  ~Dev() {
-    if (p) cudaFree(p);
-  }
+  void* p;
+  size_t bytes;
+  explicit Dev(size_t n) : p(scratch_alloc(n, nullptr)), bytes(n) {}
+  ~Dev() { scratch_free(p, bytes, nullptr); }
+  Dev(const Dev&) = delete;
+  Dev& operator=(const Dev&) = delete;
   template <class T>
   T* as() {
     return (T*)p;

@@ -234,24 +234,29 @@ cudaMemPool_t scratch_pool(bool create) {
   return g_pool[dev];
 }
 
-// cudaMalloc, once more after the pool has given its unused memory back
-cudaError_t malloc_trimming(void** ptr, size_t bytes) {
-  cudaError_t e = cudaMalloc(ptr, bytes);
+// an allocation, once more after the pool has given its unused memory back
+template <class F>
+void alloc_trimming(F allocate) {
+  cudaError_t e = allocate();
   if (e == cudaErrorMemoryAllocation) {
     (void)cudaGetLastError();
     scratch_trim();
-    e = cudaMalloc(ptr, bytes);
+    e = allocate();
   }
-  return e;
+  QSS_CK(e);
 }
 }  // namespace
+
+void device_malloc(void** ptr, size_t bytes) {
+  alloc_trimming([&] { return cudaMalloc(ptr, bytes); });
+}
 
 void* scratch_alloc(size_t bytes, cudaStream_t s) {
   void* ptr = nullptr;
   if (bytes == 0) bytes = 8;
   cudaMemPool_t pool = bytes <= kPoolBlock ? scratch_pool(true) : nullptr;
-  if (pool) QSS_CK(cudaMallocFromPoolAsync(&ptr, bytes, pool, s));
-  else QSS_CK(malloc_trimming(&ptr, bytes));
+  if (pool) alloc_trimming([&] { return cudaMallocFromPoolAsync(&ptr, bytes, pool, s); });
+  else device_malloc(&ptr, bytes);
   return ptr;
 }
 
@@ -271,7 +276,12 @@ void scratch_free(void* ptr, size_t bytes, cudaStream_t s) {
 void scratch_trim() {
   try {
     cudaMemPool_t pool = scratch_pool(false);
-    if (pool) cudaMemPoolTrimTo(pool, 0);
+    uint64_t reserved = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess || !reserved)
+      return;
+    // a free on a stream counts as in use until the host has seen that it is done
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(pool, 0);
   } catch (const Error&) {
   }
 }
@@ -287,7 +297,7 @@ size_t scratch_idle_bytes() {
 
 template <class T>
 static void dalloc(T*& ptr, int64_t count) {
-  if (!ptr) QSS_CK(malloc_trimming((void**)&ptr, (size_t)count * sizeof(T)));
+  if (!ptr) device_malloc((void**)&ptr, (size_t)count * sizeof(T));
 }
 
 static void destroy_volume(DevVolume* v) {

@@ -133,13 +133,14 @@ struct DevVolume {
 // a memory pool of the library's own (CUDA's stream-ordered allocator: reuse is
 // ordered between streams and threads by the runtime), which keeps up to 4 GiB
 // across calls; larger blocks are cudaMalloc / cudaFree.  The pool gives its unused
-// memory back in qssgpu_release / destroyQSSDataArrays and when an allocation of
-// the library fails.
+// memory back, after waiting for the device, in qssgpu_release / destroyQSSDataArrays
+// and when an allocation of the library, all of which come through here, fails.
 // A call with 15 arrays spent more time in cudaMalloc and cudaFree (which waits
 // for the device) than in its kernels: getrhs3d5th_ at 130 x 96 x 75, 2.08 ms.
 void* scratch_alloc(size_t bytes, cudaStream_t s);
 void scratch_free(void* ptr, size_t bytes, cudaStream_t s);  // work queued on s may still use ptr
 void scratch_trim();
+void device_malloc(void** ptr, size_t bytes);  // cudaMalloc
 size_t scratch_idle_bytes();  // held by the pool, in use by no call
 
 DevVolume& volume_for(const QSS_DataArrays* p, const Grid* g);

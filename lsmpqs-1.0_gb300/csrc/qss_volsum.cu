@@ -541,6 +541,30 @@ void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, d
 
 using namespace qss;
 
+namespace {
+
+// a call's stream and its device arrays
+struct SumCall {
+  cudaStream_t s = nullptr;
+  void* p[3] = {};
+  size_t bytes[3] = {};
+  int count = 0;
+  SumCall() { QSS_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking)); }
+  ~SumCall() {
+    for (int k = 0; k < count; k++) scratch_free(p[k], bytes[k], s);
+    cudaStreamDestroy(s);
+  }
+  SumCall(const SumCall&) = delete;
+  SumCall& operator=(const SumCall&) = delete;
+  double* get(int64_t n) {
+    bytes[count] = (size_t)n * sizeof(double);
+    p[count] = scratch_alloc(bytes[count], s);
+    return (double*)p[count++];
+  }
+};
+
+}  // namespace
+
 // ---------------------------------------------------------------------------
 extern "C" {
 
@@ -549,22 +573,15 @@ int qssgpu_loop_sum(const double* values, long long n, double* out) {
   try {
     ensure_device();
     if (n < 0 || (n > 0 && !values) || !out) throw Error(QSSGPU_ERR_ARG, "qssgpu_loop_sum: bad argument");
-    cudaStream_t s = nullptr;
-    QSS_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    double *dv = nullptr, *scratch = nullptr, *dout = nullptr;
+    SumCall call;
+    const cudaStream_t s = call.s;
     const int64_t nn = n > 0 ? n : 1;
-    QSS_CK(cudaMalloc(&dv, nn * sizeof(double)));
-    QSS_CK(cudaMalloc(&scratch, loop_sum_scratch_doubles(nn) * sizeof(double)));
-    QSS_CK(cudaMalloc(&dout, sizeof(double)));
+    double *dv = call.get(nn), *scratch = call.get(loop_sum_scratch_doubles(nn)), *dout = call.get(1);
     if (n > 0) QSS_CK(cudaMemcpyAsync(dv, values, n * sizeof(double), cudaMemcpyHostToDevice, s));
     launch_loop_sum(s, dv, n, scratch, dout);
     QSS_CK(cudaGetLastError());
     QSS_CK(cudaMemcpyAsync(out, dout, sizeof(double), cudaMemcpyDeviceToHost, s));
     QSS_CK(cudaStreamSynchronize(s));
-    cudaFree(dv);
-    cudaFree(scratch);
-    cudaFree(dout);
-    cudaStreamDestroy(s);
     return 0;
   } catch (const std::exception& e) {
     return report_exception(e);
