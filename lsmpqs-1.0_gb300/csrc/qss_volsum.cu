@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) band_n = 0;
   __syncthreads();
-  // a value as a float by its bits (a conversion is an FP64 instruction); values
-  // outside the float range do not matter for the estimate
+  // the estimate is in units of dV, which itself may lie outside the float range; a value
+  // as a float by its bits (a conversion is an FP64 instruction)
   auto approx = [](double v) {
     const uint32_t h = qss_emu::hi32(v);
     return h - 0x38100000u < 0x0fe00000u ? __uint_as_float((h - 0x38000000u) << 3) : 0.0f;
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
       const bool inside = qss_emu::gt(-eps, p);  // p < -eps
       band = !inside && qss_emu::gt(eps, p);     // p < eps
       if (!band) contrib[t] = inside ? dV : 0.0;
-      if (inside) sum += approx(dV);
+      if (inside) sum += 1.0f;
     }
     const unsigned m = __ballot_sync(0xffffffffu, band);
     int at = 0;
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
     const double one_minus_H = 0.5 * (1 - rr - one_over_pi * portable_sin(pi * rr));
     const double v = one_minus_H * dV;
     contrib[band_t[e]] = v;
-    sum += approx(v);
+    sum += approx(one_minus_H);
   }
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
   if (lane == 0) red[threadIdx.x >> 5] = sum;
@@ -213,9 +213,10 @@ __device__ __forceinline__ double chunk_estimate(const T* __restrict__ csum, int
   return s;
 }
 
-// exclusive scan of nc chunk sums in one block of 1024 threads
+// exclusive scan of nc chunk sums, in units of `unit`, in one block of 1024 threads
 template <typename T, int PER>
-__global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, int64_t np, int64_t nc, double* est) {
+__global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, int64_t np, int64_t nc, double unit,
+                                                   double* est) {
   __shared__ double part[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t per = (nc + 1023) / 1024;
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, i
   double run = incl - s;
   for (int w = 0; w < warp; w++) run += part[w];
   for (int64_t j = lo; j < hi; j++) {
-    est[j] = run;
+    est[j] = run * unit;
     run += chunk_estimate<T, PER>(csum, np, j);
   }
 }
@@ -242,8 +243,8 @@ __global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, i
 constexpr int kBadChunk = 4, kZeroChunk = 5;
 template <typename T, int PER>
 __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __restrict__ c, int64_t n,
-                                                             const T* __restrict__ csum, int64_t np, bool scanned,
-                                                             double* est, int64_t* R, int* F) {
+                                                             const T* __restrict__ csum, int64_t np, double unit,
+                                                             bool scanned, double* est, int64_t* R, int* F) {
   __shared__ double x[kVolStage];
   __shared__ Units part[3][kVolThreads / 32];
   __shared__ double s_est[kVolThreads / 32];
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __res
   if (!scanned) {
     e = 0;
     for (int w = 0; w < kVolThreads / 32; w++) e += s_est[w];
+    e *= unit;
     if (threadIdx.x == 0) est[j] = e;
   }
   const int E0 = exp_of(e);
@@ -510,10 +512,10 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restri
 
 namespace {
 
-// steps 2 to 4; np partial sums, PER a chunk, are at the start of scratch
+// steps 2 to 4; np partial sums in units of `unit`, PER a chunk, are at the start of scratch
 // (2 nc doubles), then the estimates (nc), R (3 nc) and F (3 nc ints)
 template <typename T, int PER>
-void sum_chunks(cudaStream_t s, const double* c, int64_t n, int64_t np, double* scratch, double* out) {
+void sum_chunks(cudaStream_t s, const double* c, int64_t n, int64_t np, double unit, double* scratch, double* out) {
   static_assert(PER * sizeof(T) <= 2 * sizeof(double), "partial sums outgrow their part of the scratch");
   const int64_t nc = (n + kVolChunk - 1) / kVolChunk;
   const T* csum = reinterpret_cast<const T*>(scratch);
@@ -521,8 +523,8 @@ void sum_chunks(cudaStream_t s, const double* c, int64_t n, int64_t np, double* 
   int64_t* R = reinterpret_cast<int64_t*>(est + nc);
   int* F = reinterpret_cast<int*>(R + 3 * nc);
   const bool have_r = nc > kSmallChunks, scanned = nc > kScanChunks;
-  if (scanned) k_vol_scan<T, PER><<<1, 1024, 0, s>>>(csum, np, nc, est);
-  if (have_r) k_vol_chunk_r<T, PER><<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, np, scanned, est, R, F);
+  if (scanned) k_vol_scan<T, PER><<<1, 1024, 0, s>>>(csum, np, nc, unit, est);
+  if (have_r) k_vol_chunk_r<T, PER><<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, np, unit, scanned, est, R, F);
   k_vol_walk<<<1, kVolThreads, 0, s>>>(c, n, nc, est, R, F, have_r, out);
 }
 
@@ -534,7 +536,7 @@ void launch_loop_sum(cudaStream_t s, const double* c, int64_t n, double* scratch
     return;
   }
   k_vol_chunk_sum<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), kVolThreads, 0, s>>>(c, n, scratch);
-  sum_chunks<double, 1>(s, c, n, (n + kVolChunk - 1) / kVolChunk, scratch, out);
+  sum_chunks<double, 1>(s, c, n, (n + kVolChunk - 1) / kVolChunk, 1.0, scratch, out);
 }
 
 void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, double dy, double dz, double eps,
@@ -547,7 +549,7 @@ void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, d
   const double dV = dx * dy * dz;
   const unsigned np = (unsigned)((n + kContribVoxels - 1) / kContribVoxels);
   k_vol_contrib<<<np, kContribThreads, 0, s>>>(b, phi, dV, eps, scratch, reinterpret_cast<float*>(scratch + n));
-  sum_chunks<float, kVolChunk / kContribVoxels>(s, scratch, n, np, scratch + n, out);
+  sum_chunks<float, kVolChunk / kContribVoxels>(s, scratch, n, np, dV, scratch + n, out);
 }
 
 }  // namespace qss
