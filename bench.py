@@ -209,21 +209,33 @@ FLOP_PER_VOXEL = {0: 3 * (16 + 2 * 75) + 10 + 5 + 72 + 2 + 5,
                   1: 9 + 35 + 2 + 2 * 26, 2: 9 + 35 + 2 + 2 * 26, 3: 9 + 35 + 2 + 2 * 26,
                   4: 10 + 5 + 72 + 2 + 5}
 KERNEL_NAME = {0: "k_stage<WENO5,var> (fused RHS + TVD-RK stage)",
-               1: "k_weno_tile<0> (WENO5 x-pass, {} tiles, shared sub-expressions)",
-               2: "k_weno_tile<1> (WENO5 y-pass, {} tiles, shared sub-expressions)",
-               3: "k_weno_tile<2> (WENO5 z-pass, {} tiles, shared sub-expressions)",
+               1: "k_weno_tile:x (WENO5 x-pass, {} tiles, shared sub-expressions)",
+               2: "k_weno_tile:y (WENO5 y-pass, {} tiles, shared sub-expressions)",
+               3: "k_weno_tile:z (WENO5 z-pass, {} tiles, shared sub-expressions)",
                4: "k_weno_combine2 (Godunov + advection + curvature + TVD-RK)"}
 # the window forms (--axis-variant 0/1/2) run k_weno_axis<axis> instead
 WINDOW_NAME = {1: "k_weno_axis<0> (WENO5 x-pass, sliding window)",
                2: "k_weno_axis<1> (WENO5 y-pass, sliding window)",
                3: "k_weno_axis<2> (WENO5 z-pass, sliding window)"}
-# FP64-pipe instructions per fill-box voxel of one tile-form axis pass, by the longest
-# tile along the line, from ncu (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}
+# FP64-pipe instructions per fill-box voxel of one tile-form axis pass, by its tile (the
+# shorter tiles of small boxes do more for their halo and were not measured), from ncu (smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}
 # _pred_on.sum of the three passes over their voxels); the rest of the 98 algorithmic
 # operations run on the integer pipes.  FP64_PIPE_BUSY_TILE: the pipe's cycles, 77 an
 # instruction, over the active ones of the same launches.
 FP64_INSTR_PER_VOXEL_TILE = {"4 x 64": 37.8}
 FP64_PIPE_BUSY_TILE = {"4 x 64": ("256^3", 94.0)}
+
+
+def tile_shape(n: int, variant: int | None) -> str:
+    """The library's tile for the lines of an n^3 box: the longest that leaves three rounds
+    of 7 blocks on 152 SMs, of 64 positions down to 16 (16 and 27 for variants 3 and 4),
+    the line split evenly."""
+    cap = {3: 16, 4: 27}.get(variant, 64)
+    while variant not in (3, 4) and cap > 16 and 3 * -(-n // 4) * n * -(-n // cap) < 152 * 7 * 3:
+        cap //= 2
+    return f"4 x {-(-n // -(-n // cap))}"
+
+
 N_KINDS = 5
 # DRAM bytes per fill-box voxel of one launch of each stage kernel, measured at
 # 512^3 with ncu (dram__bytes_read.sum + dram__bytes_write.sum, one pass):
@@ -268,7 +280,7 @@ def gpu_arm(args, dist: Dist):
     top = int(out[4])
     top_ms = out[1]
     window = args.axis_variant in (0, 1, 2)
-    geom = {3: "4 x 16", 4: "4 x 27"}.get(args.axis_variant, "4 x 64")
+    geom = tile_shape(n, args.axis_variant)
 
     def kname(k):
         return (WINDOW_NAME if window and k in WINDOW_NAME else KERNEL_NAME)[k].format(geom)

@@ -30,8 +30,8 @@
 //      sum, 256 chunks at a time: a scan of their Units finds the first chunk that
 //      does not apply (another binade, the top of the binade reached, special
 //      values); the sum advances to it in one integer addition, and that chunk
-//      goes the same way by groups of up to 4 elements, only the group that does
-//      not apply being added element by element.
+//      goes the same way by groups of up to 4 elements, the group that does not
+//      apply being added element by element (and more where none applies, kWalkClose).
 // Every result equals the sequential loop's bit for bit.
 //
 // The walk is bound by latency: 1 to 2 us for each binade the sum crosses, in opening
@@ -138,22 +138,22 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_sum(const double* __r
 }
 
 // contribution of each fill-box voxel in loop order (i fastest), and the sum of
-// each quarter chunk.  A voxel outside the smoothing band costs an
+// each chunk in units of dV.  A voxel outside the smoothing band costs an
 // integer comparison; those inside (about 15 % of the voxels, but a lane or more
 // of most warps) are first gathered, then evaluated by full warps: their division
-// and sine are ~45 FP64 instructions and the kernel's bound.  Blocks of 1024
-// voxels, so that small boxes use more SMs (24^3 49 us with whole chunks).
-constexpr int kContribVoxels = 1024, kContribThreads = 256;
+// and sine are ~45 FP64 instructions and the kernel's bound.  A block is a chunk:
+// 1024 voxels, so that small boxes use more SMs (24^3 49 us with 4096).
+constexpr int kContribThreads = 256;
 
 __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const double* __restrict__ phi, double dV,
                                                                  double eps, double* contrib, float* csum) {
-  __shared__ double band_p[kContribVoxels];
-  __shared__ uint16_t band_t[kContribVoxels];
+  __shared__ double band_p[kVolChunk];
+  __shared__ uint16_t band_t[kVolChunk];
   __shared__ int band_n;
   __shared__ float red[kContribThreads / 32];
   const double pi = 3.14159265358979323846;
   const double one_over_pi = 0.31830988618379;
-  const FillBlock blk(b, blockIdx.x, kContribVoxels);
+  const FillBlock blk(b, blockIdx.x, kVolChunk);
   contrib += blk.base;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) band_n = 0;
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
   };
   float sum = 0.0f;
 #pragma unroll
-  for (int t0 = 0; t0 < kContribVoxels; t0 += kContribThreads) {
+  for (int t0 = 0; t0 < kVolChunk; t0 += kContribThreads) {
     const uint32_t t = t0 + threadIdx.x;
     bool band = false;
     double p = 0.0;
@@ -203,26 +203,15 @@ __global__ void __launch_bounds__(kContribThreads) k_vol_contrib(Box b, const do
   }
 }
 
-// the estimate of chunk j's sum from PER partial sums (past np: none)
-template <typename T, int PER>
-__device__ __forceinline__ double chunk_estimate(const T* __restrict__ csum, int64_t np, int64_t j) {
-  double s = 0;
-#pragma unroll
-  for (int q = 0; q < PER; q++)
-    if (PER * j + q < np) s += (double)csum[PER * j + q];
-  return s;
-}
-
 // exclusive scan of nc chunk sums, in units of `unit`, in one block of 1024 threads
-template <typename T, int PER>
-__global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, int64_t np, int64_t nc, double unit,
-                                                   double* est) {
+template <typename T>
+__global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, int64_t nc, double unit, double* est) {
   __shared__ double part[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t per = (nc + 1023) / 1024;
   const int64_t lo = threadIdx.x * per, hi = lo + per < nc ? lo + per : nc;
   double s = 0;
-  for (int64_t j = lo; j < hi; j++) s += chunk_estimate<T, PER>(csum, np, j);
+  for (int64_t j = lo; j < hi; j++) s += (double)csum[j];
   double incl = s;
   for (int o = 1; o < 32; o <<= 1) {
     const double x = __shfl_up_sync(0xffffffffu, incl, o);
@@ -234,16 +223,16 @@ __global__ void __launch_bounds__(1024) k_vol_scan(const T* __restrict__ csum, i
   for (int w = 0; w < warp; w++) run += part[w];
   for (int64_t j = lo; j < hi; j++) {
     est[j] = run * unit;
-    run += chunk_estimate<T, PER>(csum, np, j);
+    run += (double)csum[j];
   }
 }
 
 // R[3j+q], F[3j+q] for E = exp(est[j]) - 1 + q.  F: kZeroChunk, all contributions
 // zero (nothing changes whatever the sum); kBadChunk, not applicable; else d + 1
 constexpr int kBadChunk = 4, kZeroChunk = 5;
-template <typename T, int PER>
+template <typename T>
 __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __restrict__ c, int64_t n,
-                                                             const T* __restrict__ csum, int64_t np, double unit,
+                                                             const T* __restrict__ csum, double unit,
                                                              bool scanned, double* est, int64_t* R, int* F) {
   __shared__ double x[kVolStage];
   __shared__ Units part[3][kVolThreads / 32];
@@ -262,7 +251,7 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_chunk_r(const double* __res
   if (scanned) {
     e = est[j];
   } else {
-    for (int64_t q = threadIdx.x; q < PER * j; q += kVolThreads) e += (double)csum[q];
+    for (int64_t q = threadIdx.x; q < j; q += kVolThreads) e += (double)csum[q];
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
     if (lane == 0) s_est[warp] = e;
   }
@@ -512,19 +501,18 @@ __global__ void __launch_bounds__(kVolThreads) k_vol_walk(const double* __restri
 
 namespace {
 
-// steps 2 to 4; np partial sums in units of `unit`, PER a chunk, are at the start of scratch
-// (2 nc doubles), then the estimates (nc), R (3 nc) and F (3 nc ints)
-template <typename T, int PER>
-void sum_chunks(cudaStream_t s, const double* c, int64_t n, int64_t np, double unit, double* scratch, double* out) {
-  static_assert(PER * sizeof(T) <= 2 * sizeof(double), "partial sums outgrow their part of the scratch");
+// steps 2 to 4; the chunks' sums in units of `unit` are at the start of scratch, from its
+// double 2 nc on the estimates (nc), R (3 nc) and F (3 nc ints)
+template <typename T>
+void sum_chunks(cudaStream_t s, const double* c, int64_t n, double unit, double* scratch, double* out) {
   const int64_t nc = (n + kVolChunk - 1) / kVolChunk;
   const T* csum = reinterpret_cast<const T*>(scratch);
   double* est = scratch + 2 * nc;
   int64_t* R = reinterpret_cast<int64_t*>(est + nc);
   int* F = reinterpret_cast<int*>(R + 3 * nc);
   const bool have_r = nc > kSmallChunks, scanned = nc > kScanChunks;
-  if (scanned) k_vol_scan<T, PER><<<1, 1024, 0, s>>>(csum, np, nc, unit, est);
-  if (have_r) k_vol_chunk_r<T, PER><<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, np, unit, scanned, est, R, F);
+  if (scanned) k_vol_scan<<<1, 1024, 0, s>>>(csum, nc, unit, est);
+  if (have_r) k_vol_chunk_r<<<(unsigned)nc, kVolThreads, 0, s>>>(c, n, csum, unit, scanned, est, R, F);
   k_vol_walk<<<1, kVolThreads, 0, s>>>(c, n, nc, est, R, F, have_r, out);
 }
 
@@ -536,7 +524,7 @@ void launch_loop_sum(cudaStream_t s, const double* c, int64_t n, double* scratch
     return;
   }
   k_vol_chunk_sum<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), kVolThreads, 0, s>>>(c, n, scratch);
-  sum_chunks<double, 1>(s, c, n, (n + kVolChunk - 1) / kVolChunk, 1.0, scratch, out);
+  sum_chunks<double>(s, c, n, 1.0, scratch, out);
 }
 
 void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, double dy, double dz, double eps,
@@ -547,9 +535,9 @@ void launch_volume(cudaStream_t s, const Box& b, const double* phi, double dx, d
     return;
   }
   const double dV = dx * dy * dz;
-  const unsigned np = (unsigned)((n + kContribVoxels - 1) / kContribVoxels);
-  k_vol_contrib<<<np, kContribThreads, 0, s>>>(b, phi, dV, eps, scratch, reinterpret_cast<float*>(scratch + n));
-  sum_chunks<float, kVolChunk / kContribVoxels>(s, scratch, n, np, dV, scratch + n, out);
+  k_vol_contrib<<<(unsigned)((n + kVolChunk - 1) / kVolChunk), kContribThreads, 0, s>>>(
+      b, phi, dV, eps, scratch, reinterpret_cast<float*>(scratch + n));
+  sum_chunks<float>(s, scratch, n, dV, scratch + n, out);
 }
 
 }  // namespace qss

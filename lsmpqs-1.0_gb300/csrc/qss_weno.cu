@@ -14,14 +14,15 @@
 //
 // A stage runs as three axis passes and one combine kernel:
 //   k_weno_tile (the default): a block computes every face and centre of
-//     a tile of lines once into shared memory, then one thread per voxel the
-//     two reconstructions, and writes the plus and minus one-sided
+//     a tile of lines once into shared memory, then one thread per voxel and
+//     side the reconstruction, and writes the plus and minus one-sided
 //     derivatives of that axis (2 doubles per voxel);
 //   k_weno_axis<AX> (selectable): each thread walks a segment of voxels along
 //     axis AX with a sliding window of faces / centres, same outputs;
-//   k_weno_combine2 (level 2), k_weno_combine: Godunov normal term (with the carried term of voxels whose
-//     speed is below 1e-5), upwind advection, central curvature, TVD-RK
-//     combination and, on the last stage, the three mask impositions.
+//   k_weno_combine2 (level 2; k_weno_combine at levels 0 and 1): Godunov normal
+//     term (with the carried term of voxels whose speed is below 1e-5), upwind
+//     advection, central curvature, TVD-RK combination and, on the last stage,
+//     the three mask impositions.
 // The extra traffic (48 B written + 48 B read per voxel and stage) costs about
 // 2 % of the stage time at 512^3; HBM is idle otherwise.
 //
@@ -55,12 +56,10 @@ constexpr int SEG = 16;  // voxels per thread along the pass axis
 //   0: native FP64 instructions only;
 //   1: divisions, square roots, power-of-two scalings and comparisons on the
 //      integer pipes;
-//   2: level 1 plus a share of the products: in the axis passes the five
-//      scaled copies of each face and the normalised weights, in the combine
-//      kernel the second derivatives and the curvature numerator.  The
-//      combine kernel runs ~10 warps per scheduler and overlaps these with
-//      its FP64 work; the axis passes hold ~120 registers per thread (4 warps
-//      per scheduler) and gain only a few percent from them.
+//   2: level 1 plus a share of the products: here, in the window forms of the
+//      axis passes, the five scaled copies of each face and the normalised
+//      weights; the default tile form and the combine kernel of level 2 have
+//      arithmetic of their own (k_weno_tile, qss_stage.cuh).
 template <int EMU>
 struct Ar {
   static __device__ __forceinline__ double div(double a, double b) {
@@ -189,7 +188,7 @@ struct AxisArgs {
   double* dminus;
   double inv;
   const Ctl* ctl;
-  int seg_len;  // voxels per thread (window forms, EMU >= 1) or positions per tile (tile form, EMU 2)
+  int seg_len;  // voxels per thread (window forms, EMU >= 1)
 };
 
 // One thread: SEG consecutive voxels along axis AX starting at s0, inside
@@ -776,7 +775,7 @@ struct CombineArgs {
 };
 
 // Godunov normal term of the WENO5 scheme, vel * |grad| (3d.f:2251-2276),
-// with the sign tests and maxima on the integer pipes at EMU >= 1
+// with the sign tests and maxima on the integer pipes at EMU 1
 template <int EMU>
 __device__ __forceinline__ double godunov5(double vel, const double pp[3], const double pm[3]) {
   if (EMU == 0) return godunov_norm<WENO5>(vel, pp, pm);
@@ -804,7 +803,7 @@ __device__ __forceinline__ double godunov5(double vel, const double pp[3], const
 
 // central curvature term (3d.f:2337-2379), same operations as curvature()
 // with the exact doublings, the threshold test and the division moved to the
-// integer pipes at EMU >= 1
+// integer pipes at EMU 1
 template <int EMU>
 __device__ __forceinline__ double curvature_e(const double* __restrict__ phi, const Box& b, int64_t c, const Fac& f) {
   if (EMU == 0) return curvature(phi, b, c, f);
@@ -815,25 +814,23 @@ __device__ __forceinline__ double curvature_e(const double* __restrict__ phi, co
   const double phi_x = (__ldg(phi + c + 1) - __ldg(phi + c - 1)) * f.x;
   const double phi_y = (__ldg(phi + c + sy) - __ldg(phi + c - sy)) * f.y;
   const double phi_z = (__ldg(phi + c + sz) - __ldg(phi + c - sz)) * f.z;
-  const double phi_xx = Q::mul2((__ldg(phi + c + 2) + __ldg(phi + c - 2) - cc2) * f.x, f.x);
-  const double phi_zz = Q::mul2((__ldg(phi + c + 2 * sz) + __ldg(phi + c - 2 * sz) - cc2) * f.z, f.z);
-  const double phi_yy = Q::mul2((__ldg(phi + c + 2 * sy) + __ldg(phi + c - 2 * sy) - cc2) * f.y, f.y);
-  const double phi_xy = Q::mul2((__ldg(phi + c + 1 + sy) + __ldg(phi + c - 1 - sy) - __ldg(phi + c - 1 + sy) -
-                                 __ldg(phi + c + 1 - sy)) * f.x, f.y);
-  const double phi_xz = Q::mul2((__ldg(phi + c + 1 + sz) + __ldg(phi + c - 1 - sz) - __ldg(phi + c - 1 + sz) -
-                                 __ldg(phi + c + 1 - sz)) * f.x, f.z);
-  const double phi_yz = Q::mul2((__ldg(phi + c + sy + sz) + __ldg(phi + c - sy - sz) - __ldg(phi + c - sy + sz) -
-                                 __ldg(phi + c + sy - sz)) * f.y, f.z);
-  const double grad_mag2 = Q::mul2(phi_x, phi_x) + Q::mul2(phi_y, phi_y) + Q::mul2(phi_z, phi_z);
+  const double phi_xx = (__ldg(phi + c + 2) + __ldg(phi + c - 2) - cc2) * f.x * f.x;
+  const double phi_zz = (__ldg(phi + c + 2 * sz) + __ldg(phi + c - 2 * sz) - cc2) * f.z * f.z;
+  const double phi_yy = (__ldg(phi + c + 2 * sy) + __ldg(phi + c - 2 * sy) - cc2) * f.y * f.y;
+  const double phi_xy = (__ldg(phi + c + 1 + sy) + __ldg(phi + c - 1 - sy) - __ldg(phi + c - 1 + sy) -
+                         __ldg(phi + c + 1 - sy)) * f.x * f.y;
+  const double phi_xz = (__ldg(phi + c + 1 + sz) + __ldg(phi + c - 1 - sz) - __ldg(phi + c - 1 + sz) -
+                         __ldg(phi + c + 1 - sz)) * f.x * f.z;
+  const double phi_yz = (__ldg(phi + c + sy + sz) + __ldg(phi + c - sy - sz) - __ldg(phi + c - sy + sz) -
+                         __ldg(phi + c + sy - sz)) * f.y * f.z;
+  const double grad_mag2 = phi_x * phi_x + phi_y * phi_y + phi_z * phi_z;
   // grad_mag2 < 1e-5: a sum of squares is +0, positive or NaN
   if (qss_emu::bits(grad_mag2) < qss_emu::bits(1.e-5)) return 0.0;
-  // at level 2 the products of the curvature numerator run on the integer
-  // pipes (the FP64 pipe is the combine kernel's bound; its integer pipes idle)
-  const double curv = phi_xx * phi_y * phi_y + Q::mul2(Q::mul2(phi_yy, phi_x), phi_x) -
-                      Q::mul2(Q::mul2(Q::s2(phi_xy, 1), phi_x), phi_y) + Q::mul2(Q::mul2(phi_xx, phi_z), phi_z) +
-                      Q::mul2(Q::mul2(phi_zz, phi_x), phi_x) - Q::mul2(Q::mul2(Q::s2(phi_xz, 1), phi_x), phi_z) +
-                      Q::mul2(Q::mul2(phi_yy, phi_z), phi_z) + Q::mul2(Q::mul2(phi_zz, phi_y), phi_y) -
-                      Q::mul2(Q::mul2(Q::s2(phi_yz, 1), phi_y), phi_z);
+  const double curv = phi_xx * phi_y * phi_y + phi_yy * phi_x * phi_x -
+                      Q::s2(phi_xy, 1) * phi_x * phi_y + phi_xx * phi_z * phi_z +
+                      phi_zz * phi_x * phi_x - Q::s2(phi_xz, 1) * phi_x * phi_z +
+                      phi_yy * phi_z * phi_z + phi_zz * phi_y * phi_y -
+                      Q::s2(phi_yz, 1) * phi_y * phi_z;
   return Q::div(curv, grad_mag2);
 }
 
@@ -855,8 +852,8 @@ __device__ __forceinline__ double impose3_e(double v, int64_t idx, const ImposeA
 // One block: 32 (i) x 4 (j) voxels of one k plane; each warp covers an 8 x 4
 // patch of them, so that the warps that lie wholly where the curvature
 // coefficient is zero (inside the grains) skip the curvature term together.
-// Compiled for 10 resident blocks per SM (48 registers; 64 without the bound):
-// 557 against 553 M voxel-steps/s for the whole stage at 512^3 on GB300.
+// Levels 0 and 1 (and level 2 where a grid factor is out of its range).  Compiled
+// for 10 resident blocks per SM (48 registers; 64 without the bound).
 template <int STAGE, bool FINAL, int EMU>
 __global__ void __launch_bounds__(128, 10) k_weno_combine(CombineArgs a) {
   if (STAGE != 0 && !a.ctl->active) return;
@@ -1028,10 +1025,12 @@ int even_len(int along, int cap) {
 }
 
 // The longest tiles (the smallest halo) that leave about three rounds of blocks
-// for the GPU, down to 16 positions (one round of sides for 128 threads; shorter
-// ones leave threads idle).  Whole stage, M voxel-steps/s, 8-line tiles of up to
-// 8 / 16 / 24 / 27 positions: 24^3 70 / 66 / 63 / 63, 48^3 337 / 340 / 347 / 347,
-// 96^3 703 / 743 / 761 / 760, 128^3 773 / 827 / 837 / 851.
+// for the GPU, down to 16 positions (one round of sides for 128 threads).  Inner loop
+// of a curvature step on GB300, ms, tiles of up to 16 / 32 / 64 positions (8 is slower
+// everywhere): 16 x 16 x 64 1.09 / 1.11 / 1.16, 12 x 12 x 200 1.25 / 1.25 / 1.31 (few
+// long lines: the rule), 36^3 1.54 / 1.54 / 1.48, 48^3 2.26 / 2.19 / 2.13, 64^3 3.53 /
+// 3.32 / 3.25 (2 to 4 % lost by the rule, which takes 12, 24 and 32 there), 96^3 9.84 /
+// 9.06 / 8.70, 192^3 72.6 / 66.1 / 62.5 (64: the rule).
 int tile_cap_for(const Box& b) {
   int cap = kTileP;
   while (cap > 16) {
@@ -1167,8 +1166,12 @@ int tile_form_for(int along) {
   return (int64_t)tiles * Tile27::P * 50 <= (int64_t)along * 51 ? 4 : 3;
 }
 
-// Below this many blocks for one axis the three axes share a launch (same
-// work, two launches fewer and one partly filled last round instead of three).
+// Below this many blocks of full tiles for one axis (4.36 M voxels) the three axes share
+// a launch: the same work, two launches fewer and one partly filled last round instead of
+// three, but blocks without work where the sides differ.  Inner loop of a curvature step
+// on GB300, ms, three launches / one: 24^3 1.21 / 0.96, 64^3 3.72 / 3.31, 128^3 21.7 / 21.2,
+// 192^3 62.5 / 62.0, 320^3 282.6 / 282.0, 400 x 100 x 100 41.1 / 41.1, 100 x 400 x 400
+// 143.9 / 147.5.
 constexpr int64_t kMergeBlocks = (int64_t)152 * kTileBlocks * 16;
 
 template <int EMU>
@@ -1193,8 +1196,7 @@ void axes_at(cudaStream_t s, const Box& b, const double* phi, const double invs[
     const int along = ax == 0 ? b.fbx() : (ax == 1 ? b.fby() : b.fbz());
     const int lanes = ax == 0 ? b.fby() : b.fbx();
     const int other = ax == 2 ? b.fby() : b.fbz();
-    // by default a tile form, the fastest at every size measured on GB300
-    // (64^3 .. 512^3); of the two window forms, which are
+    // by default a tile form; of the two window forms, which are
     // kept selectable, the shared-memory one is the faster from ~12 M fill
     // voxels on (register / shared-memory form, M voxel-steps/s: 128^3
     // 420 / 383, 192^3 411 / 385, 256^3 458 / 473, 512^3 469 / 488)
