@@ -24,12 +24,14 @@ Box full_box(const Grid* g) {
   return b;
 }
 
-// call scratch on the legacy default stream, where these calls launch and copy
+// Not from the scratch pool: these calls run on the legacy default stream, and blocks that
+// it gave back made later calls on other streams slower (a 24^3 right-hand side 167 -> 188 us).
 struct Dev {
-  void* p;
-  size_t bytes;
-  explicit Dev(size_t n) : p(scratch_alloc(n, nullptr)), bytes(n) {}
-  ~Dev() { scratch_free(p, bytes, nullptr); }
+  void* p = nullptr;
+  explicit Dev(size_t bytes) { device_malloc(&p, bytes ? bytes : 8); }
+  ~Dev() {
+    if (p) cudaFree(p);
+  }
   Dev(const Dev&) = delete;
   Dev& operator=(const Dev&) = delete;
   template <class T>
