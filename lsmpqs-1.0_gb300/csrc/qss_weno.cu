@@ -901,9 +901,10 @@ __global__ void __launch_bounds__(128, 10) k_weno_combine(CombineArgs a) {
     az = (vz >= 0) ? pm[2] : pp[2];
   }
   const double temp_vel = -(vx * ax + vy * ay + vz * az);
-  // b * kappa is +-0 where b is +0, and (temp_norm + (+-0)) equals
-  // (temp_norm + 0.0) unless temp_norm is -0: there the curvature (finite:
-  // its denominator is at least 1e-5) changes nothing and is skipped
+  // b * kappa is +-0 where b is +0 and kappa finite, and (temp_norm + (+-0)) equals
+  // (temp_norm + 0.0) unless temp_norm is -0: elsewhere the curvature is skipped.  A
+  // level set whose curvature is not finite there (infinities, NaNs, differences
+  // beyond 2^200) loses the NaN that 0 x kappa would give
   const double bco = a.c.b[idx];
   const double temp_curv = (qss_emu::bits(bco) == 0 && qss_emu::bits(temp_norm) != qss_emu::kSign)
                                ? 0.0
@@ -961,9 +962,9 @@ __global__ void __launch_bounds__(128, 8) k_weno_combine2(CombineArgs a) {
       rhs = godunov_native<WENO5>(a.c.vel_n[src], a.dp[0][src], a.dp[1][src], a.dp[2][src], a.dm[0][src], a.dm[1][src],
                                   a.dm[2][src], 1.0, 1.0, 1.0);
   }
-  // b * kappa is +-0 where b is +0, and (normal term + (+-0)) equals (normal
-  // term + 0.0) unless it is -0: there the curvature (finite: its denominator is
-  // at least 1e-5) changes nothing and is skipped
+  // b * kappa is +-0 where b is +0 and kappa finite, and (normal term + (+-0)) equals
+  // (normal term + 0.0) unless it is -0: elsewhere the curvature is skipped.  A level
+  // set whose curvature is not finite there loses the NaN that 0 x kappa would give
   const double bco = a.c.b[idx];
   if (qss_emu::bits(bco) != 0 || qss_emu::bits(rhs) == qss_emu::kSign)
     rhs = rhs + qss_emu::mul(bco, curvature_fast(a.phi_in, b, idx, a.fac));
